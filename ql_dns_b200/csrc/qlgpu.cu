@@ -171,9 +171,7 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
         if (prc != QLGPU_OK) return fail(nullptr, prc, msg);
     }
     Variant var;
-    const char* ps = std::getenv("QLGPU_PRIV_SMEM");
-    const bool use_tmem = !(ps && ps[0] == '1');
-    if (!pick_variant(p.NZ, p.model, p.integrator, use_tmem, &var))
+    if (!pick_variant(p.NZ, p.model, p.integrator, &var))
         return fail(nullptr, QLGPU_ERR_UNSUPPORTED,
                     "unsupported NZ: must be a power of two in [16, 256]");
     int ndev = 0;
@@ -203,71 +201,22 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     const DevParams& d = h->dp;
 
     ktables(p, h->kx_tab, h->ky_tab, h->kxi_tab, h->kyi_tab);
-    // Launch geometry: as many CTAs as fit, at most one mode per group
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) {
         h->err = "cudaGetDeviceProperties failed";
         return bail(QLGPU_ERR_CUDA);
     }
-    // CTA width: the number of warps (up to 16 or 8, as compiled) that maximises resident
-    // warps per SM, given shared memory, registers and (for the TMEM store) 512 TMEM columns per SM.
-    int best_w = 1, best_res = -1, best_per_sm = 1;
-    for (int w = var.max_warps; w >= 1; --w) {
-        const size_t sm_bytes = var.smem(w);
-        if (sm_bytes > (size_t)prop.sharedMemPerBlockOptin) continue;
-        if (ensure_smem_attr(var.kernel(), sm_bytes) !=
-            cudaSuccess)
-            continue;
-        const int tc = var.tmem(w);
-        if (tc > 512) continue;
-        int want = tc > 0 ? 512 / tc : 32;
-        const size_t per_cta = sm_bytes + 1024;
-        while (want > 1 && per_cta * want > (size_t)prop.sharedMemPerMultiprocessor) --want;
-        int pct = (int)((100.0 * per_cta * want) / (double)prop.sharedMemPerMultiprocessor + 0.999);
-        if (pct > 100) pct = 100;
-        cudaFuncSetAttribute(var.kernel(), cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-        int occ = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, var.kernel(), 32 * w, sm_bytes);
-        if (tc > 0 && occ > 512 / tc) occ = 512 / tc;
-        if (occ < 1) continue;
-        // warps that hold work at once: the CTAs the modes need (one mode per pair of
-        // groups), capped by what the GPU holds.  Narrower CTAs win ties: the same
-        // warps spread over more SMs.
-        const int modes_per_cta = w * (32 / var.T) / 2;
-        const long need = (h->nxy + modes_per_cta - 1) / modes_per_cta;
-        const long cap = (long)prop.multiProcessorCount * occ;
-        const int res = (int)((need < cap ? need : cap) * w);
-        if (best_res < 0 || res >= best_res * 0.98) {
-            best_res = res;
-            best_w = w;
-            best_per_sm = occ;
-        }
-    }
-    h->warps = best_w;
+    const StageGeom sg = stage_geometry(p.model, p.NZ, h->nxy, prop.multiProcessorCount, 64 * RED_GROUP);
+    h->warps = sg.warps;
     h->block = 32 * h->warps;
     h->smem = var.smem(h->warps);
-    if (ensure_smem_attr(var.kernel(), h->smem) != cudaSuccess) {
+    h->grid = sg.grid;
+    h->per_sm = 1;
+    if (h->smem > (size_t)prop.sharedMemPerBlockOptin || ensure_smem_attr(var.kernel(), h->smem) != cudaSuccess) {
         h->err = "shared memory request too large";
         return bail(QLGPU_ERR_CUDA);
     }
-    {
-        int want = var.tmem(h->warps) > 0 ? 512 / var.tmem(h->warps) : 32;
-        const size_t per_cta = h->smem + 1024;
-        while (want > 1 && per_cta * want > (size_t)prop.sharedMemPerMultiprocessor) --want;
-        int pct = (int)((100.0 * per_cta * want) / (double)prop.sharedMemPerMultiprocessor + 0.999);
-        if (pct > 100) pct = 100;
-        cudaFuncSetAttribute(var.kernel(), cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-    }
-    h->tmem_cols = var.tmem(h->warps);
-    int per_sm = best_per_sm;
-    h->per_sm = per_sm;
-    // one mode per pair of transform groups
-    const int modes_per_cta = h->warps * (32 / var.T) / 2;
-    int need = (h->nxy + modes_per_cta - 1) / modes_per_cta;
-    int cap = prop.multiProcessorCount * per_sm;
-    h->grid = need < cap ? need : cap;
-    if (h->grid > 64 * RED_GROUP) h->grid = 64 * RED_GROUP;
-    if (h->grid < 1) h->grid = 1;
+    cudaFuncSetAttribute(var.kernel(), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     const int ngroups = (h->grid + RED_GROUP - 1) / RED_GROUP;
 
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -293,7 +242,7 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     QLGPU_ALLOC(h->d_ky, h->nxy * sizeof(double));
     QLGPU_ALLOC(h->d_kxi, h->nxy * sizeof(int));
     QLGPU_ALLOC(h->d_kyi, h->nxy * sizeof(int));
-    QLGPU_ALLOC(h->d_tw, h->NZ * sizeof(cplx));
+    QLGPU_ALLOC(h->d_tw, 2 * h->NZ * sizeof(cplx));
     QLGPU_ALLOC(h->d_partials, (size_t)h->grid * var.PL * sizeof(double));
     QLGPU_ALLOC(h->d_gpartials, (size_t)ngroups * var.PL * sizeof(double));
     QLGPU_ALLOC(h->d_clk, sizeof(DevClock));
@@ -302,7 +251,7 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     QLGPU_ALLOC(h->d_mfr, (size_t)8 * h->NZ * sizeof(double));
     QLGPU_ALLOC(h->d_ekz, (size_t)6 * h->nz * sizeof(double));
     QLGPU_ALLOC(h->d_dbg, sizeof(int));
-    const std::vector<double> tw = twiddles(h->NZ, var.T);
+    const std::vector<double> tw = stage_twiddles(h->NZ);
     cudaMemcpyAsync(h->d_tw, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     h->il2_tab = ilap2_table(p, h->nz);
     h->ekz_tab = ekz_table(p, d);
@@ -486,7 +435,7 @@ static int step_forced(qlgpu_t* h, int nsteps, int diag_every, double* diag_out,
         h->dt_sum += dt;
         ++h->steps_taken;
         if (diag_every > 0 && (n + 1) % diag_every == 0 && nd < max_diag) {
-            h->var.diag(h->d_lin[h->cur], h->d_mf, h->d_kx0, h->d_ky, h->d_kxi, h->d_kyi, h->dp, t,
+            launch_diag(h->d_lin[h->cur], h->d_mf, h->d_kx0, h->d_ky, h->d_kyi, h->dp, t,
                         h->d_diag + 15 * (size_t)nd, h->stream);
             ++nd;
         }
@@ -623,7 +572,7 @@ int qlgpu_diagnostics(qlgpu_t* h, double* out15) {
     double t = 0;
     QLGPU_CK(cudaMemcpyAsync(&t, &h->d_clk->t, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     QLGPU_CK(cudaStreamSynchronize(h->stream));
-    h->var.diag(h->d_lin[h->cur], h->d_mf, h->d_kx0, h->d_ky, h->d_kxi, h->d_kyi, h->dp, t, h->d_out15, h->stream);
+    launch_diag(h->d_lin[h->cur], h->d_mf, h->d_kx0, h->d_ky, h->d_kyi, h->dp, t, h->d_out15, h->stream);
     int rc = check_launch(h);
     if (rc) return rc;
     QLGPU_CK(cudaMemcpyAsync(out15, h->d_out15, 15 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -693,8 +642,8 @@ int qlgpu_launch_info(const qlgpu_t* h, int* info8) {
     info8[1] = h->block;
     info8[2] = (int)h->smem;
     info8[3] = h->per_sm;
-    info8[4] = h->tmem_cols;
-    info8[5] = h->var.T;
+    info8[4] = 0;  // the stage kernel allocates no tensor memory
+    info8[5] = h->NZ / 8;
     info8[6] = h->nxy;
     info8[7] = h->warps;
     return QLGPU_OK;
@@ -774,7 +723,7 @@ struct NoallocLayout {
 NoallocLayout noalloc_layout(int NZ, int nxy, int nyh, int nz, int grid, int PL) {
     NoallocLayout L;
     size_t o = 0;
-    L.tw = o; o = align256(o + sizeof(cplx) * NZ);
+    L.tw = o; o = align256(o + sizeof(cplx) * 2 * NZ);
     L.ky = o; o = align256(o + sizeof(double) * nxy);
     L.kxi = o; o = align256(o + sizeof(int) * nxy);
     L.kyi = o; o = align256(o + sizeof(int) * nxy);
@@ -801,15 +750,14 @@ __global__ void noalloc_tables_kernel(unsigned char* base, NoallocLayout L, int 
     double* il2 = reinterpret_cast<double*>(base + L.il2);
     DevClock* clk = reinterpret_cast<DevClock*>(base + L.clk);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    const int P = NZ / T;
-    for (int i = tid; i < NZ; i += nth) {
-        const int n2 = i / T, t = i % T;
-        const int m = (n2 * t) % NZ;
+    for (int i = tid; i < 2 * NZ; i += nth) {
+        // [P][T] of the adjoint's layout, then [8][NZ/8]
+        const int Tl = i < NZ ? T : NZ / 8, j = i < NZ ? i : i - NZ;
+        const int m = ((j / Tl) * (j % Tl)) % NZ;
         double sn, cs;
         sincospi(2.0 * (double)m / (double)NZ, &sn, &cs);
         tw[i] = mk(cs, sn);
     }
-    (void)P;
     for (int i = tid; i < nxy; i += nth) {
         // mode index j + (Ny/2) i with the kx Nyquist column dropped
         const int col = i / nyh, j = i % nyh;
@@ -856,7 +804,7 @@ extern "C" int qlgpu_rhs_noalloc(const qlgpu_params* pp, double t, double dt_lin
         if (bits & 15) return fail(nullptr, QLGPU_ERR_ARG, "device pointers must be 16-byte aligned");
     }
     Variant var;
-    if (!pick_variant(p.NZ, p.model, QLGPU_INTEG_RK3CN_ELIN, true, &var))
+    if (!pick_variant(p.NZ, p.model, QLGPU_INTEG_RK3CN_ELIN, &var))
         return fail(nullptr, QLGPU_ERR_UNSUPPORTED, "unsupported NZ: must be a power of two in [16, 256]");
     const int nz = 1 + 2 * int(p.NZ / 3.0), nxy = (p.nx - 1) * (p.ny / 2), nyh = p.ny / 2;
     const int nmf = p.model == QLGPU_MODEL_MHD_BQLIN ? 2 : 4;
@@ -888,16 +836,12 @@ extern "C" int qlgpu_rhs_noalloc(const qlgpu_params* pp, double t, double dt_lin
         nd = c;
     }
     void* base = nd.ptr;
-    // Launch geometry: as in qlgpu_create, at most one CTA per SM and one mode per pair of groups.
-    int warps = 8;
-    while (warps > 1 && var.smem(warps) > (size_t)nd.smem_optin) warps >>= 1;
+    // Launch geometry: as in qlgpu_create.
+    const StageGeom sg = stage_geometry(p.model, p.NZ, nxy, nd.sms, QLGPU_NOALLOC_MAX_GRID);
+    const int warps = sg.warps, grid = sg.grid;
     const size_t smem = var.smem(warps);
     if (ensure_smem_attr(var.kernel(), smem) != cudaSuccess)
         return fail(nullptr, QLGPU_ERR_CUDA, "shared memory request too large");
-    const int modes_per_cta = warps * (32 / var.T) / 2;
-    int grid = (nxy + modes_per_cta - 1) / modes_per_cta;
-    if (grid > nd.sms) grid = nd.sms;
-    if (grid > QLGPU_NOALLOC_MAX_GRID) grid = QLGPU_NOALLOC_MAX_GRID;
     const NoallocLayout L = noalloc_layout(p.NZ, nxy, nyh, nz, grid, var.PL);
     if (L.end > QLGPU_NOALLOC_SCRATCH_BYTES)
         return fail(nullptr, QLGPU_ERR_ARG, "case exceeds the 4 MiB no-allocation scratch");

@@ -16,7 +16,7 @@
 // step loop, frees its TMEM and returns.  The host launches the kernel with the
 // cooperative attribute, so all CTAs are co-resident or the launch fails.
 #pragma once
-#include "qlgpu_kernel.cuh"
+#include "qlgpu_wide.cuh"
 
 namespace qlgpu {
 
@@ -65,18 +65,8 @@ __device__ __forceinline__ void cta_copy8(void* dst, const void* src, int n) {
 // keeps the compile time of the kernel linear in the number of classes.  The
 // shared-memory objects are declared here so that every access stays a
 // shared-space access.
-// Field staging in the persistent kernel: only for transforms of up to 8 points
-// per thread (NZ <= 64).  At NZ = 128 the staging buffers cost the warp per SM
-// that the 255-register CTA could still hold; the batch measured 8% faster
-// without them (the single-case kernel keeps them: 6% faster with).
-template <int NZ>
-struct BatchStaging {
-    static constexpr bool ON = Geom<NZ>::P <= 8;
-};
-
-template <int NZ, int MODEL, int INTEG, int MAXNZ>
-__device__ __noinline__ bool batch_item_stage(const BatchCase* cs, int s, int swap, int cta, int ncta, uint32_t tmem,
-                                              int n) {
+template <int NZ, int MODEL, int INTEG>
+__device__ __noinline__ bool batch_item_stage(const BatchCase* cs, int s, int swap, int cta, int ncta, int n) {
     static_assert(sizeof(StageArgs) % 8 == 0 && sizeof(DevParams) % 8 == 0, "8-byte copies");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StageShared ss;
@@ -87,7 +77,6 @@ __device__ __noinline__ bool batch_item_stage(const BatchCase* cs, int s, int sw
     cta_copy8(&sA, &cs->A[s], (int)sizeof(StageArgs));
     __syncthreads();
     if (threadIdx.x == 0) {
-        ss.tmem = tmem;
         if (swap) {
             const cplx* in = sA.lin_in;
             sA.lin_in = sA.lin_out;
@@ -104,34 +93,20 @@ __device__ __noinline__ bool batch_item_stage(const BatchCase* cs, int s, int sw
         }
     }
     __syncthreads();
-    return stage_body<NZ, MODEL, INTEG, true, BatchStaging<NZ>::ON>(sA, sP, cta, ncta, smem_raw, ss);
+    return stage_body<NZ, MODEL, INTEG>(sA, sP, cta, ncta, smem_raw, ss);
 }
 
-// MAXNZ: the largest NZ class the kernel steps.  With TMEM one CTA runs per
-// SM; classes up to NZ = 64 hold 8 points per thread, fit 128 registers and
-// run 16-warp CTAs, the NZ = 128 / 256 classes (16 points per thread) 8-warp CTAs.
-template <int MAXNZ>
-struct BatchOcc {
-    static constexpr int MAX_THREADS = MAXNZ <= 64 ? 512 : 256;
-};
-
-template <int MODEL, int INTEG, int MAXNZ>
-__global__ void __launch_bounds__(BatchOcc<MAXNZ>::MAX_THREADS, 1) batch_kernel(BatchLaunch L) {
-    __shared__ uint32_t s_tmem;
+template <int MODEL, int INTEG>
+__global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) batch_kernel(const __grid_constant__ BatchLaunch L) {
     __shared__ int s_ok;
     __shared__ BatchSlot s_items[BATCH_MAX_SLOTS];
     __shared__ int s_top[BATCH_MAX_SLOTS];
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const BatchCta* me = L.ctas + blockIdx.x;
     const int nitems = min(me->nslots, BATCH_MAX_SLOTS);
-    const int tcols = me->tcols;
     if (tid < nitems * 4) reinterpret_cast<int*>(s_items)[tid] = reinterpret_cast<const int*>(me->slot)[tid];
     if (blockIdx.x == 0 && tid == 0) L.ctl->t_start = gtimer();
-    if (tcols > 0 && warp == 0) tmem_alloc(&s_tmem, (uint32_t)tcols);
-    tmem_fence_before_sync();
     __syncthreads();
-    tmem_fence_after_sync();
-    const uint32_t tmem = tcols > 0 ? s_tmem : 0u;
     bool ok = true;
     unsigned k = 0;  // stages completed by every case in this launch
     for (int n = 0; n < L.nsteps && ok; ++n) {
@@ -142,17 +117,12 @@ __global__ void __launch_bounds__(BatchOcc<MAXNZ>::MAX_THREADS, 1) batch_kernel(
                 const BatchSlot it = s_items[i];
                 const BatchCase* cs = L.cases + QLGPU_CHECK_INDEX(it.c, L.ncases, &L.ctl->status);
                 bool top = false;
-                if (it.NZ == 16) {
-                    top = batch_item_stage<16, MODEL, INTEG, MAXNZ>(cs, s, swap, it.cta, it.ncta, tmem, n);
-                } else if (it.NZ == 32) {
-                    top = batch_item_stage<32, MODEL, INTEG, MAXNZ>(cs, s, swap, it.cta, it.ncta, tmem, n);
-                } else if (it.NZ == 64) {
-                    top = batch_item_stage<64, MODEL, INTEG, MAXNZ>(cs, s, swap, it.cta, it.ncta, tmem, n);
-                } else if constexpr (MAXNZ >= 128) {
-                    if (it.NZ == 128)
-                        top = batch_item_stage<128, MODEL, INTEG, MAXNZ>(cs, s, swap, it.cta, it.ncta, tmem, n);
-                    else if (it.NZ == 256)
-                        top = batch_item_stage<256, MODEL, INTEG, MAXNZ>(cs, s, swap, it.cta, it.ncta, tmem, n);
+                switch (it.NZ) {
+                    case 16: top = batch_item_stage<16, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
+                    case 32: top = batch_item_stage<32, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
+                    case 64: top = batch_item_stage<64, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
+                    case 128: top = batch_item_stage<128, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
+                    default: top = batch_item_stage<256, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
                 }
                 if (tid == 0) s_top[i] = top ? 1 : 0;
                 if (top) {
@@ -178,10 +148,6 @@ __global__ void __launch_bounds__(BatchOcc<MAXNZ>::MAX_THREADS, 1) batch_kernel(
             ok = s_ok != 0;
         }
     }
-    tmem_fence_before_sync();
-    __syncthreads();
-    tmem_fence_after_sync();
-    if (tcols > 0 && warp == 0) tmem_dealloc(s_tmem, (uint32_t)tcols);
 }
 
 }  // namespace qlgpu

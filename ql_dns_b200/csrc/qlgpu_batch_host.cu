@@ -3,8 +3,8 @@
 // descriptors of the persistent kernel, the CTA mapping and its autotuner, and
 // the CUDA-graph launch of the persistent kernel.
 //
-// Mapping model.  A CTA of w warps steps mpc = w*(32/T)/2 modes of a case at a
-// time (one mode per pair of transform groups).  Giving case c k CTAs costs it
+// Mapping model.  A CTA of w warps steps mpc = teams(w) * 256/NZ modes of a case at
+// a time (one block of modes per team of warps).  Giving case c k CTAs costs it
 // rounds(c, k) = ceil(nxy_c / (k*mpc)) passes of its stage pipeline per stage.
 // A CTA that owns several work items runs them one after the other, so its
 // stage time is modelled as the sum over its items of
@@ -268,10 +268,13 @@ size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 // one arena slot: the buffer and, in the debug build, its guard zone
 size_t gslot(size_t x) { return al256(x + QLGPU_GUARD_BYTES); }
 
-int modes_per_cta(int warps, int T) { return warps * (32 / T) / 2; }
+// modes a CTA of `warps` warps steps at once
+int modes_per_cta(const CaseHost& c, int warps) {
+    return stage_teams(c.p.model, warps) * block_modes(c.NZ);
+}
 
 int rounds_of(const CaseHost& c, int k, int warps) {
-    const int m = modes_per_cta(warps, c.T) * k;
+    const int m = modes_per_cta(c, warps) * k;
     return (c.nxy + m - 1) / m;
 }
 
@@ -284,18 +287,13 @@ void drop_graphs(qlgpu_batch_t* b) {
 // CTAs per SM and dynamic shared memory of a CTA width over the NZ classes present.
 bool width_limits(qlgpu_batch_t* b, int warps, int* per_sm, size_t* smem) {
     size_t sm = 0;
-    int tc = 0;
-    for (const CaseHost& c : b->cs) {
-        sm = std::max(sm, b->bk.smem(c.NZ, warps));
-        tc = std::max(tc, b->bk.tmem(c.NZ, warps));
-    }
-    if (sm > b->smem_optin || tc > 512) return false;
+    for (const CaseHost& c : b->cs) sm = std::max(sm, b->bk.smem(c.NZ, warps));
+    if (sm > b->smem_optin) return false;
     if (ensure_smem_attr(b->bk.kernel(), sm) != cudaSuccess)
         return false;
     cudaFuncSetAttribute(b->bk.kernel(), cudaFuncAttributePreferredSharedMemoryCarveout, 100);
     int occ = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, b->bk.kernel(), 32 * warps, sm) != cudaSuccess) return false;
-    if (tc > 0) occ = std::min(occ, 512 / tc);  // TMEM columns per SM: an allocation beyond them would wait
     if (occ < 1) return false;
     *per_sm = occ;
     *smem = sm;
@@ -324,7 +322,7 @@ bool plan(const qlgpu_batch_t* b, int warps, int G, const CostModel& cm, const i
                 while (kk < kmax && item_cost(c, kk) > M) {
                     // next CTA count that lowers the number of passes
                     const int r = rounds_of(h, kk, warps);
-                    const int m = modes_per_cta(warps, h.T);
+                    const int m = modes_per_cta(h, warps);
                     int nk = r > 1 ? (h.nxy + m * (r - 1) - 1) / (m * (r - 1)) : kk + 1;
                     if (nk <= kk) nk = kk + 1;
                     kk = std::min(nk, kmax);
@@ -443,16 +441,13 @@ int apply_mapping(qlgpu_batch_t* b, int warps, int per_sm, size_t smem, const st
         BatchCta& m = ctas[j];
         std::memset(&m, 0, sizeof(m));
         m.nslots = (int)bins[j].size();
-        int tc = 0;
         for (int i = 0; i < m.nslots; ++i) {
             const Item& it = bins[j][i];
             m.slot[i].c = it.c;
             m.slot[i].cta = it.i;
             m.slot[i].ncta = it.k;
             m.slot[i].NZ = b->cs[it.c].NZ;
-            tc = std::max(tc, b->bk.tmem(b->cs[it.c].NZ, warps));
         }
-        m.tcols = tc;
     }
     if (ensure_smem_attr(b->bk.kernel(), smem) != cudaSuccess)
         return bfail(b, QLGPU_ERR_CUDA, "batch kernel: shared memory request too large");
@@ -472,7 +467,7 @@ int plan_and_apply(qlgpu_batch_t* b, int warps, const int* fixed_k) {
     int per_sm = 0;
     size_t smem = 0;
     if (!width_limits(b, warps, &per_sm, &smem))
-        return bfail(b, QLGPU_ERR_UNSUPPORTED, "batch: CTA width does not fit (shared memory / TMEM)");
+        return bfail(b, QLGPU_ERR_UNSUPPORTED, "batch: CTA width does not fit (shared memory)");
     const int G = std::min(b->sms * per_sm, b->sms * 2);
     std::vector<int> k;
     std::vector<std::vector<Item>> bins;
@@ -872,9 +867,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         b->err = "cudaSetDevice failed";
         return bail(QLGPU_ERR_NODEVICE);
     }
-    int max_nz = 0;
-    for (int c = 0; c < ncases; ++c) max_nz = std::max(max_nz, cases[c].NZ);
-    if (!pick_batch_kernel(b->model, b->integ, max_nz > 64, &b->bk)) {
+    if (!pick_batch_kernel(b->model, b->integ, &b->bk)) {
         b->err = "no batch kernel for this model / integrator";
         return bail(QLGPU_ERR_UNSUPPORTED);
     }
@@ -912,11 +905,10 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         h.nz = h.dp.nz;
         h.NZ = h.p.NZ;
         h.nmf = h.dp.nmf;
-        h.T = group_threads(h.NZ);
         h.PL = (h.nmf == 2 ? 2 : 4) * h.NZ + 8;
-        h.max_cta = std::min(max_grid, (h.nxy + modes_per_cta(4, h.T) - 1) / modes_per_cta(4, h.T));
+        h.max_cta = std::min(max_grid, (h.nxy + modes_per_cta(h, 4) - 1) / modes_per_cta(h, 4));
         h.max_cta = std::min(h.max_cta, 64 * RED_GROUP);
-        if (!pick_variant(h.NZ, b->model, b->integ, true, &h.var)) {
+        if (!pick_variant(h.NZ, b->model, b->integ, &h.var)) {
             b->err = "unsupported NZ";
             return bail(QLGPU_ERR_UNSUPPORTED);
         }
@@ -926,7 +918,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         o += 3 * gslot(nmfe * sizeof(cplx));                       // mf, Fmf1, Fmf2
         o += 3 * gslot(h.nxy * sizeof(double));                    // kx0, ky, kx_init
         o += 2 * gslot(h.nxy * sizeof(int));                       // kxi, kyi
-        o += gslot(h.NZ * sizeof(cplx));                           // twiddles
+        o += gslot(2 * h.NZ * sizeof(cplx));                       // twiddles
         o += gslot((size_t)(h.p.ny / 2) * h.nz * sizeof(double));  // 1/lap2
         o += gslot((size_t)h.max_cta * h.PL * sizeof(double));     // partials
         o += gslot((size_t)((h.max_cta + RED_GROUP - 1) / RED_GROUP) * h.PL * sizeof(double));
@@ -962,7 +954,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         h.ky = reinterpret_cast<double*>(take(h.nxy * sizeof(double)));
         h.kxi = reinterpret_cast<int*>(take(h.nxy * sizeof(int)));
         h.kyi = reinterpret_cast<int*>(take(h.nxy * sizeof(int)));
-        h.tw = reinterpret_cast<cplx*>(take(h.NZ * sizeof(cplx)));
+        h.tw = reinterpret_cast<cplx*>(take(2 * h.NZ * sizeof(cplx)));
         h.il2 = reinterpret_cast<double*>(take((size_t)(h.p.ny / 2) * h.nz * sizeof(double)));
         h.partials = reinterpret_cast<double*>(take((size_t)h.max_cta * h.PL * sizeof(double)));
         h.gpartials = reinterpret_cast<double*>(
@@ -974,7 +966,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         std::vector<double> ky;
         std::vector<int> kxi, kyi;
         ktables(h.p, h.kx_tab, ky, kxi, kyi);
-        const std::vector<double> tw = twiddles(h.NZ, h.T);
+        const std::vector<double> tw = stage_twiddles(h.NZ);
         const std::vector<double> il2 = ilap2_table(h.p, h.nz);
         const std::vector<double> ekz = ekz_table(h.p, h.dp);
         cudaMemcpyAsync(h.kx0, h.kx_tab.data(), h.nxy * sizeof(double), cudaMemcpyHostToDevice, b->stream);
@@ -1199,7 +1191,7 @@ int qlgpu_batch_diagnostics(qlgpu_batch_t* b, int c, double* out15) {
     double t = 0;
     QB_CK(cudaMemcpyAsync(&t, &h.clk->t, sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     QB_CK(cudaStreamSynchronize(b->stream));
-    h.var.diag(h.lin[b->cur], h.mf, h.kx0, h.ky, h.kxi, h.kyi, h.dp, t, b->d_out15, b->stream);
+    launch_diag(h.lin[b->cur], h.mf, h.kx0, h.ky, h.kyi, h.dp, t, b->d_out15, b->stream);
     QB_CK(cudaGetLastError());
     QB_CK(cudaMemcpyAsync(out15, b->d_out15, 15 * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
     QB_CK(cudaStreamSynchronize(b->stream));

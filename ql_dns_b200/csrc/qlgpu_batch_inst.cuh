@@ -6,7 +6,7 @@
 
 namespace qlgpu {
 
-template <int MODEL, int INTEG, int MAXNZ>
+template <int MODEL, int INTEG>
 cudaError_t batch_launch(const BatchLaunch& L, int grid, int block, size_t smem, cudaStream_t st) {
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
@@ -19,42 +19,29 @@ cudaError_t batch_launch(const BatchLaunch& L, int grid, int block, size_t smem,
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, batch_kernel<MODEL, INTEG, MAXNZ>, L);
+    return cudaLaunchKernelEx(&cfg, batch_kernel<MODEL, INTEG>, L);
 }
-template <int MODEL, int INTEG, int MAXNZ>
+template <int MODEL, int INTEG>
 const void* batch_ptr() {
-    return reinterpret_cast<const void*>(&batch_kernel<MODEL, INTEG, MAXNZ>);
+    return reinterpret_cast<const void*>(&batch_kernel<MODEL, INTEG>);
 }
 template <int MODEL>
 size_t batch_smem(int NZ, int warps) {
     switch (NZ) {
-        case 16: return StageKind<16, MODEL, true, BatchStaging<16>::ON>::SM::bytes(warps);
-        case 32: return StageKind<32, MODEL, true, BatchStaging<32>::ON>::SM::bytes(warps);
-        case 64: return StageKind<64, MODEL, true, BatchStaging<64>::ON>::SM::bytes(warps);
-        case 128: return StageKind<128, MODEL, true, BatchStaging<128>::ON>::SM::bytes(warps);
-        case 256: return StageKind<256, MODEL, true, BatchStaging<256>::ON>::SM::bytes(warps);
-        default: return 0;
-    }
-}
-template <int MODEL>
-int batch_tmem(int NZ, int warps) {
-    switch (NZ) {
-        case 16: return StageKind<16, MODEL, true, BatchStaging<16>::ON>::SM::tmem_cols(warps);
-        case 32: return StageKind<32, MODEL, true, BatchStaging<32>::ON>::SM::tmem_cols(warps);
-        case 64: return StageKind<64, MODEL, true, BatchStaging<64>::ON>::SM::tmem_cols(warps);
-        case 128: return StageKind<128, MODEL, true, BatchStaging<128>::ON>::SM::tmem_cols(warps);
-        case 256: return StageKind<256, MODEL, true, BatchStaging<256>::ON>::SM::tmem_cols(warps);
+        case 16: return wide::WG<16, MODEL>::bytes(warps);
+        case 32: return wide::WG<32, MODEL>::bytes(warps);
+        case 64: return wide::WG<64, MODEL>::bytes(warps);
+        case 128: return wide::WG<128, MODEL>::bytes(warps);
+        case 256: return wide::WG<256, MODEL>::bytes(warps);
         default: return 0;
     }
 }
 template <int MODEL, int INTEG>
-bool make_batch_kernel(bool wide, BatchKernel* out) {
-    out->launch = wide ? &batch_launch<MODEL, INTEG, 256> : &batch_launch<MODEL, INTEG, 64>;
-    out->kernel = wide ? &batch_ptr<MODEL, INTEG, 256> : &batch_ptr<MODEL, INTEG, 64>;
+bool make_batch_kernel(BatchKernel* out) {
+    out->launch = &batch_launch<MODEL, INTEG>;
+    out->kernel = &batch_ptr<MODEL, INTEG>;
     out->smem = &batch_smem<MODEL>;
-    out->tmem = &batch_tmem<MODEL>;
-    out->max_nz = wide ? 256 : 64;
-    out->max_warps = (wide ? BatchOcc<256>::MAX_THREADS : BatchOcc<64>::MAX_THREADS) / 32;
+    out->max_warps = wide::MAX_WARPS;
     return true;
 }
 

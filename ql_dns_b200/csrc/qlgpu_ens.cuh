@@ -51,6 +51,7 @@
 
 #include "qlgpu_batch.cuh"
 #include "qlgpu_debug.cuh"
+#include "qlgpu_xform.cuh"
 
 namespace qlgpu {
 namespace ens {
@@ -101,79 +102,6 @@ struct EG {
     static constexpr size_t WARP_BYTES = 16 * (X_OFF + X_CPLX);
     static constexpr size_t BYTES = o_warp + WARPS * WARP_BYTES;
 };
-
-// Real-space / spectral register classes: index t + T r is in the dealiasing
-// gap for every t (dead), stored for every t, or stored for some t.
-template <class E>
-__device__ __forceinline__ int sidx(int t, int r) {
-    const int k = t + E::T * r;
-    if (k <= E::H) return k;
-    if (k >= E::NZ - E::H) return k - (E::NZ - E::nz);
-    return -1;
-}
-template <class E>
-__host__ __device__ constexpr bool rdead(int r) {
-    return E::T * r > E::H && E::T * r + E::T - 1 < E::NZ - E::H;
-}
-
-// cos / sin (2 pi i / 16)
-__device__ __forceinline__ constexpr double c16(int i) {
-    return i == 0 ? 1.0 : i == 1 ? QLGPU_C1 : i == 2 ? QLGPU_RSQRT2 : i == 3 ? QLGPU_S1 : i == 4 ? 0.0
-         : i == 5 ? -QLGPU_S1 : i == 6 ? -QLGPU_RSQRT2 : -QLGPU_C1;
-}
-__device__ __forceinline__ constexpr double s16(int i) {
-    return i == 0 ? 0.0 : i == 1 ? QLGPU_S1 : i == 2 ? QLGPU_RSQRT2 : i == 3 ? QLGPU_C1 : i == 4 ? 1.0
-         : i == 5 ? QLGPU_C1 : i == 6 ? QLGPU_RSQRT2 : QLGPU_S1;
-}
-
-// Exchange-buffer slot of (row q, column t) in group g's buffer (cplx units).
-template <class E>
-__device__ __forceinline__ int xslot(int g, int q, int t) {
-    return g * 8 * E::T + E::T * (q ^ (g & E::SWZ)) + ((t + q) & (E::T - 1));
-}
-
-// Backward DFT of one column: x[r] = X[t + T r] in, x[r] = y[t + T r] out,
-// y[n] = sum_k X[k] exp(+2 pi i n k / NZ).  xg = the warp's exchange buffers,
-// g = this thread's group in the warp, tw[q T + t] = exp(2 pi i q t / NZ).
-// Warp-collective (every lane of the warp calls it together).
-template <class E>
-__device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, int g, int t) {
-    constexpr int T = E::T;
-    dft8<+1>(x);
-#pragma unroll
-    for (int q = 1; q < 8; ++q) x[q] = cmul(x[q], tw[q * T + t]);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) xg[xslot<E>(g, q, t)] = x[q];
-    __syncwarp();
-    if constexpr (T <= 8) {
-        constexpr int J = 8 / T;
-#pragma unroll
-        for (int j = 0; j < J; ++j) {
-            const int q = t + T * j;
-            cplx v[T];
-#pragma unroll
-            for (int s = 0; s < T; ++s) v[s] = xg[xslot<E>(g, q, s)];
-            dft<T, +1>(v);
-#pragma unroll
-            for (int m = 0; m < T; ++m) x[j + J * m] = v[m];
-        }
-    } else {
-        // T = 16: thread (q, h) = (t % 8, t / 8) takes the outputs of parity h of the
-        // 16-point transforms over the columns of row q: a radix-2 step then a DFT-8.
-        const int q = t & 7, h = t >> 3;
-        const double sg = h ? -1.0 : 1.0;
-#pragma unroll
-        for (int s = 0; s < 8; ++s) {
-            const cplx za = xg[xslot<E>(g, q, s)];
-            const cplx zb = xg[xslot<E>(g, q, s + 8)];
-            cplx w = mk(fma(sg, zb.x, za.x), fma(sg, zb.y, za.y));
-            if (s != 0) w = cmul(w, mk(h ? c16(s) : 1.0, h ? s16(s) : 0.0));
-            x[s] = w;
-        }
-        dft8<+1>(x);
-    }
-    __syncwarp();
-}
 
 // A store of the new state or right-hand side: read again one stage later, after
 // the whole ensemble has streamed through L2, so it is marked evict-first
@@ -302,19 +230,18 @@ struct ChunkHdr {
 };
 
 // ---------------------------------------------------------------------------
-// Mean-field side of a stage, on the whole CTA (rare: once per case and stage).
-// The transforms use the 16-point geometry of qlgpu_fft.cuh; kept out of line
-// so that the chunk pipeline's registers are not shared with it.
+// Mean-field side of a stage, on the whole CTA (rare: once per case and stage),
+// kept out of line so that the chunk pipeline's registers are not shared with it.
 // ---------------------------------------------------------------------------
 // Real-space By, dz By, dz^2 By [3][NZ] of the header's mean field into prof.
 template <int NZ>
-__device__ __noinline__ void profiles_of(const ChunkHdr& hd, double* prof, cplx* scratch) {
-    using G = Geom<NZ>;
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int go = tid / G::T, to = tid % G::T;
-    const unsigned gm = (G::T == 32 ? 0xffffffffu : (((1u << G::T) - 1u) << ((lane / G::T) * G::T)));
-    if (go < 3) mean_profiles<G, MODEL_BQLIN>(hd.P, hd.A.mf, prof, scratch + (size_t)go * G::XSIZE, hd.A.tw, go, 3, to,
-                                              gm);
+__device__ __noinline__ void profiles_of(const ChunkHdr& hd, double* prof, cplx* scratch, const cplx* tw) {
+    using W = wide::WG<NZ, MODEL_BQLIN>;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 3)
+        wide::mean_profiles8<W, true>(
+            hd.P, [&](int m, int s) { return ldc_cg(hd.A.mf + m * W::nz + s); }, prof, scratch + 256 * warp, tw, warp,
+            3, lane);
 }
 
 // The CTA that completed case c's stage r: chunk partials summed in slot order,
@@ -322,14 +249,12 @@ __device__ __noinline__ void profiles_of(const ChunkHdr& hd, double* prof, cplx*
 // the next stage's real-space profiles, and the release of stage r + 1.
 template <int NZ, int INTEG>
 __device__ __noinline__ void top_stage(const EnsLaunch& L, ChunkHdr& hd, int c, int r, int nch, double* scratch,
-                                       double tclock, double t_new, bool last, bool diag_due) {
-    using G = Geom<NZ>;
+                                       const cplx* tw, double tclock, double t_new, bool last, bool diag_due) {
+    using W = wide::WG<NZ, MODEL_BQLIN>;
     using E = EG<NZ>;
-    const int tid = threadIdx.x, lane = tid & 31;
+    const int tid = threadIdx.x;
     double* tot = scratch;                     // [PL]
-    double* spec = tot + ((E::PL + 1) & ~1);   // [2 NEMF (H+1)]
-    cplx* xo = reinterpret_cast<cplx*>(spec + ((2 * NEMF * (G::H + 1) + 1) & ~1));
-    double* mfr = reinterpret_cast<double*>(xo + 3 * G::XSIZE);
+    cplx* xch = reinterpret_cast<cplx*>(scratch) + W::TOP_BYTES / 16 + 1;  // four exchange buffers
     // chunk slots in slot order; 32 loads in flight per thread (this sum is on the case's
     // critical path: every CTA waits for the stage it releases)
     constexpr int U = 32;
@@ -347,20 +272,8 @@ __device__ __noinline__ void top_stage(const EnsLaunch& L, ChunkHdr& hd, int c, 
         tot[idx] = sum;
     }
     __syncthreads();
-    const int go = tid / G::T, to = tid % G::T;
-    const unsigned gm = (G::T == 32 ? 0xffffffffu : (((1u << G::T) - 1u) << ((lane / G::T) * G::T)));
-    constexpr int NGO = 3;  // groups taking part in the mean-field transforms
-    cplx* xg_o = xo + (size_t)(go < NGO ? go : 0) * G::XSIZE;
-    mean_field_stage<G, MODEL_BQLIN, INTEG, NEMF>(hd.A, hd.P, tot, spec, xg_o, hd.A.tw, go < NGO ? go : NGO, NGO, to,
-                                                  gm, tclock, t_new, last, diag_due);
-    __syncthreads();
-    if (go < NGO) mean_profiles<G, MODEL_BQLIN>(hd.P, hd.A.mf, mfr, xg_o, hd.A.tw, go, NGO, to, gm);
-    __syncthreads();
-    for (int i = tid; i < 3 * NZ; i += THREADS) hd.A.mfr_cache[i] = mfr[i];
-    __threadfence();
-    __syncthreads();
+    wide::top_stage<W, MODEL_BQLIN, INTEG>(hd.A, hd.P, tot, xch, tw, tclock, t_new, last, diag_due);
     if (tid == 0) {
-        hd.A.clk->mfr_valid = 1;
         __threadfence();
         if (r == L.nrounds - 1) L.case_end[c] = gtimer();
         st_release_u32(L.epoch + (size_t)c * BATCH_EPOCH_STRIDE, (unsigned)(r + 1));
@@ -496,7 +409,7 @@ __device__ __noinline__ void run_chunk(const EnsLaunch& L, ChunkHdr& hd, const R
             // warp 0's exchange buffers and warp 1's K buffers, which no staged copy writes
             __syncthreads();
             profiles_of<NZ>(hd, prof,
-                            reinterpret_cast<cplx*>(smem_raw + E::o_warp) + E::X_OFF);
+                            reinterpret_cast<cplx*>(smem_raw + E::o_warp) + E::X_OFF, tw);
         }
     }
     __syncthreads();
@@ -1037,8 +950,8 @@ __device__ __noinline__ void run_chunk(const EnsLaunch& L, ChunkHdr& hd, const R
     if (!hd.top) return;
     __threadfence();
     const unsigned long long t0 = (L.trace && tid == 0) ? gtimer() : 0ull;
-    top_stage<NZ, INTEG>(L, hd, c, r, ec.nch, reinterpret_cast<double*>(smem_raw + E::o_warp), tclock, t_new, last,
-                         diag_due);
+    top_stage<NZ, INTEG>(L, hd, c, r, ec.nch, reinterpret_cast<double*>(smem_raw + E::o_warp), tw, tclock, t_new,
+                         last, diag_due);
     if (L.trace && tid == 0) L.trace[4 * (size_t)blockIdx.x + 2] += gtimer() - t0;
 }
 

@@ -41,7 +41,6 @@ struct qlgpu_handle {
     double* d_out15 = nullptr;
     double* d_linop = nullptr;
     double* d_ilap2 = nullptr;
-    int tmem_cols = 0;
     int per_sm = 0;
     unsigned long long* d_trace = nullptr;
     double* d_mfr = nullptr;  // [8][NZ] mean-field profile cache

@@ -27,61 +27,53 @@ constexpr double a0_ = 8.0 / 15.0, a1_ = 5.0 / 12.0, a2_ = 3.0 / 4.0, b1_ = -17.
 constexpr double p1_ = 8.0 / 15.0, p2_ = 2.0 / 3.0;
 
 typedef void (*stage_launch_fn)(const StageArgs&, const DevParams&, int grid, int block, size_t smem, cudaStream_t);
-typedef void (*diag_launch_fn)(const cplx*, const cplx*, const double*, const double*, const int*, const int*,
-                               const DevParams&, double, double*, cudaStream_t);
 typedef size_t (*smem_fn)(int warps);
-typedef int (*tmem_fn)(int warps);
 typedef const void* (*kptr_fn)();
 
-// One compiled stage kernel (NZ x model x integrator x private-store backing).
+// One compiled stage kernel (NZ x model x integrator).
 struct Variant {
     stage_launch_fn launch;
     kptr_fn kernel;
     smem_fn smem;
-    tmem_fn tmem;
-    diag_launch_fn diag;
-    int T;          // threads per transform group
+    int T;          // threads per transform group of the adjoint's layout (Geom)
     int PL;         // partial vector length (doubles)
     int max_warps;  // widest CTA the kernel is compiled for
 };
 
 // Defined in qlgpu_nz<NZ>.cu, one translation unit per NZ.
-bool make_variant_nz16(int model, int integ, bool tm, Variant* out);
-bool make_variant_nz32(int model, int integ, bool tm, Variant* out);
-bool make_variant_nz64(int model, int integ, bool tm, Variant* out);
-bool make_variant_nz128(int model, int integ, bool tm, Variant* out);
-bool make_variant_nz256(int model, int integ, bool tm, Variant* out);
+bool make_variant_nz16(int model, int integ, Variant* out);
+bool make_variant_nz32(int model, int integ, Variant* out);
+bool make_variant_nz64(int model, int integ, Variant* out);
+bool make_variant_nz128(int model, int integ, Variant* out);
+bool make_variant_nz256(int model, int integ, Variant* out);
 
-inline bool pick_variant(int NZ, int model, int integ, bool tm, Variant* out) {
+inline bool pick_variant(int NZ, int model, int integ, Variant* out) {
     switch (NZ) {
-        case 16: return make_variant_nz16(model, integ, tm, out);
-        case 32: return make_variant_nz32(model, integ, tm, out);
-        case 64: return make_variant_nz64(model, integ, tm, out);
-        case 128: return make_variant_nz128(model, integ, tm, out);
-        case 256: return make_variant_nz256(model, integ, tm, out);
+        case 16: return make_variant_nz16(model, integ, out);
+        case 32: return make_variant_nz32(model, integ, out);
+        case 64: return make_variant_nz64(model, integ, out);
+        case 128: return make_variant_nz128(model, integ, out);
+        case 256: return make_variant_nz256(model, integ, out);
         default: return false;
     }
 }
 
-// The persistent batch kernel of one model x integrator (qlgpu_batch_<model>_<integ>.cu),
-// in two builds: NZ <= 64 only (128 registers, two 8-warp CTAs per SM) and all NZ.
+// The persistent batch kernel of one model x integrator (qlgpu_batch_<model>_<integ>.cu).
 struct BatchKernel {
     cudaError_t (*launch)(const BatchLaunch& L, int grid, int block, size_t smem, cudaStream_t st);
     const void* (*kernel)();
     size_t (*smem)(int NZ, int warps);  // dynamic shared memory of one NZ class
-    int (*tmem)(int NZ, int warps);     // TMEM columns of one NZ class
-    int max_nz;                         // largest NZ class the build steps
     int max_warps;                      // widest CTA the build is compiled for
 };
-bool batch_kernel_bq_exp(bool wide, BatchKernel* out);
-bool batch_kernel_bq_cn(bool wide, BatchKernel* out);
-bool batch_kernel_fq_exp(bool wide, BatchKernel* out);
-bool batch_kernel_fq_cn(bool wide, BatchKernel* out);
+bool batch_kernel_bq_exp(BatchKernel* out);
+bool batch_kernel_bq_cn(BatchKernel* out);
+bool batch_kernel_fq_exp(BatchKernel* out);
+bool batch_kernel_fq_cn(BatchKernel* out);
 
-inline bool pick_batch_kernel(int model, int integ, bool wide, BatchKernel* out) {
+inline bool pick_batch_kernel(int model, int integ, BatchKernel* out) {
     if (model == MODEL_BQLIN)
-        return integ == INTEG_EXP ? batch_kernel_bq_exp(wide, out) : batch_kernel_bq_cn(wide, out);
-    return integ == INTEG_EXP ? batch_kernel_fq_exp(wide, out) : batch_kernel_fq_cn(wide, out);
+        return integ == INTEG_EXP ? batch_kernel_bq_exp(out) : batch_kernel_bq_cn(out);
+    return integ == INTEG_EXP ? batch_kernel_fq_exp(out) : batch_kernel_fq_cn(out);
 }
 
 // The dynamic shared memory limit is an attribute of the kernel function, shared
@@ -112,6 +104,33 @@ inline int group_threads(int NZ) {
         case 256: return 16;
         default: return 0;
     }
+}
+
+// Modes a team of the stage kernel steps at once and the teams of a CTA (qlgpu_wide.cuh WG).
+inline int block_modes(int NZ) { return 256 / NZ; }
+inline int stage_teams(int model, int warps) {
+    const int n = warps / (model == MODEL_BQLIN ? 5 : 8);
+    return n > 1 ? n : 1;
+}
+
+// CTA width and grid of a single case's stage kernel: one CTA per SM.  When every team can
+// have its own SM a team gets as many warps as it has inverse transforms (one round of tasks);
+// otherwise a CTA holds the teams that the case has blocks for.
+struct StageGeom {
+    int warps, grid;
+};
+inline StageGeom stage_geometry(int model, int NZ, int nxy, int sms, int max_grid) {
+    const int blocks = (nxy + block_modes(NZ) - 1) / block_modes(NZ);
+    const bool bq = model == MODEL_BQLIN;
+    const int per_sm = (blocks + sms - 1) / sms;
+    StageGeom g;
+    g.warps = bq ? (per_sm <= 1 ? 9 : per_sm == 2 ? 14 : 15) : (per_sm <= 1 ? 10 : 16);
+    const int teams = stage_teams(model, g.warps);
+    g.grid = (blocks + teams - 1) / teams;
+    if (g.grid > sms) g.grid = sms;
+    if (g.grid > max_grid) g.grid = max_grid;
+    if (g.grid < 1) g.grid = 1;
+    return g;
 }
 
 inline int stored_nz(int NZ) { return 1 + 2 * int(NZ / 3.0); }                   // Model.h:34
@@ -228,6 +247,16 @@ inline std::vector<double> twiddles(int NZ, int T) {
         }
     return tw;
 }
+// The table of a case: the adjoint's layout [P][T], then the 8-point layout [8][NZ/8].
+inline std::vector<double> stage_twiddles(int NZ) {
+    std::vector<double> tw = twiddles(NZ, group_threads(NZ));
+    const std::vector<double> t8 = twiddles(NZ, NZ / 8);
+    tw.insert(tw.end(), t8.begin(), t8.end());
+    return tw;
+}
+// Diagnostics of a state in one launch (qlgpu_diag.cu): the 15-column record at time t into out.
+void launch_diag(const cplx* lin, const cplx* mf, const double* kx0, const double* ky, const int* kyi,
+                 const DevParams& P, double t, double* out, cudaStream_t st);
 
 // 1/lap2 per (ky index, stored kz), Kdata.cpp:100-119
 inline std::vector<double> ilap2_table(const qlgpu_params& p, int nz) {

@@ -1,62 +1,47 @@
 // qlgpu_inst.cuh -- the stage-variant table for one NZ: launch wrappers and
-// sizes of stage_kernel<NZ, model, integrator, TMEM|smem>.  Included by one
-// translation unit per NZ (qlgpu_nz<NZ>.cu) so the variants compile in parallel.
+// sizes of stage_kernel<NZ, model, integrator>.  Included by one translation
+// unit per NZ (qlgpu_nz<NZ>.cu) so the variants compile in parallel.
 #pragma once
-#include <type_traits>
-
 #include "qlgpu_host.h"
-#include "qlgpu_kernel.cuh"
+#include "qlgpu_wide.cuh"
 
 namespace qlgpu {
 
-template <int NZ, int MODEL, int INTEG, bool TM>
+template <int NZ, int MODEL, int INTEG>
 void launch_stage(const StageArgs& A, const DevParams& P, int grid, int block, size_t smem, cudaStream_t st) {
-    stage_kernel<NZ, MODEL, INTEG, TM><<<grid, block, smem, st>>>(A, P);
+    stage_kernel<NZ, MODEL, INTEG><<<grid, block, smem, st>>>(A, P);
 }
-template <int NZ, int MODEL, int INTEG, bool TM>
+template <int NZ, int MODEL, int INTEG>
 const void* stage_ptr() {
-    return reinterpret_cast<const void*>(&stage_kernel<NZ, MODEL, INTEG, TM>);
+    return reinterpret_cast<const void*>(&stage_kernel<NZ, MODEL, INTEG>);
 }
-template <int NZ, int MODEL, bool TM>
+template <int NZ, int MODEL>
 size_t stage_smem(int warps) {
-    return StageKind<NZ, MODEL, TM>::SM::bytes(warps);
-}
-template <int NZ, int MODEL, bool TM>
-int stage_tmem(int warps) {
-    return StageKind<NZ, MODEL, TM>::SM::tmem_cols(warps);
-}
-template <int NZ>
-void launch_diag(const cplx* lin, const cplx* mf, const double* kx0, const double* ky, const int* kxi, const int* kyi,
-                 const DevParams& P, double t, double* out, cudaStream_t st) {
-    diag_kernel<NZ><<<1, 128, 0, st>>>(lin, mf, kx0, ky, kxi, kyi, P, t, out);
+    return wide::WG<NZ, MODEL>::bytes(warps);
 }
 
-template <int NZ, int MODEL, int INTEG, bool TM>
+template <int NZ, int MODEL, int INTEG>
 Variant make_variant() {
     Variant v;
-    v.launch = &launch_stage<NZ, MODEL, INTEG, TM>;
-    v.kernel = &stage_ptr<NZ, MODEL, INTEG, TM>;
-    v.smem = &stage_smem<NZ, MODEL, TM>;
-    v.tmem = &stage_tmem<NZ, MODEL, TM>;
-    v.diag = &launch_diag<NZ>;
+    v.launch = &launch_stage<NZ, MODEL, INTEG>;
+    v.kernel = &stage_ptr<NZ, MODEL, INTEG>;
+    v.smem = &stage_smem<NZ, MODEL>;
     v.T = Geom<NZ>::T;
-    v.PL = StageKind<NZ, MODEL, TM>::SM::PL;
-    v.max_warps = StageOcc<NZ>::MAX_THREADS / 32;
+    v.PL = wide::WG<NZ, MODEL>::PL;
+    v.max_warps = wide::MAX_WARPS;
     return v;
 }
 
 template <int NZ>
-bool make_variant_for(int model, int integ, bool tm, Variant* out) {
+bool make_variant_for(int model, int integ, Variant* out) {
     if (model == MODEL_BQLIN && integ == INTEG_EXP)
-        *out = tm ? make_variant<NZ, MODEL_BQLIN, INTEG_EXP, true>() : make_variant<NZ, MODEL_BQLIN, INTEG_EXP, false>();
+        *out = make_variant<NZ, MODEL_BQLIN, INTEG_EXP>();
     else if (model == MODEL_BQLIN && integ == INTEG_CN)
-        *out = tm ? make_variant<NZ, MODEL_BQLIN, INTEG_CN, true>() : make_variant<NZ, MODEL_BQLIN, INTEG_CN, false>();
+        *out = make_variant<NZ, MODEL_BQLIN, INTEG_CN>();
     else if (model == MODEL_FULLQLIN && integ == INTEG_EXP)
-        *out = tm ? make_variant<NZ, MODEL_FULLQLIN, INTEG_EXP, true>()
-                  : make_variant<NZ, MODEL_FULLQLIN, INTEG_EXP, false>();
+        *out = make_variant<NZ, MODEL_FULLQLIN, INTEG_EXP>();
     else if (model == MODEL_FULLQLIN && integ == INTEG_CN)
-        *out = tm ? make_variant<NZ, MODEL_FULLQLIN, INTEG_CN, true>()
-                  : make_variant<NZ, MODEL_FULLQLIN, INTEG_CN, false>();
+        *out = make_variant<NZ, MODEL_FULLQLIN, INTEG_CN>();
     else
         return false;
     return true;
@@ -64,9 +49,9 @@ bool make_variant_for(int model, int integ, bool tm, Variant* out) {
 
 }  // namespace qlgpu
 
-#define QLGPU_DEFINE_NZ(NZV)                                                 \
-    namespace qlgpu {                                                        \
-    bool make_variant_nz##NZV(int model, int integ, bool tm, Variant* out) { \
-        return make_variant_for<NZV>(model, integ, tm, out);                 \
-    }                                                                        \
+#define QLGPU_DEFINE_NZ(NZV)                                        \
+    namespace qlgpu {                                               \
+    bool make_variant_nz##NZV(int model, int integ, Variant* out) { \
+        return make_variant_for<NZV>(model, integ, out);            \
+    }                                                               \
     }

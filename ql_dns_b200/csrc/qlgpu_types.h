@@ -94,7 +94,7 @@ struct StageArgs {
     const double* ky;
     const int* kxi;
     const int* kyi;
-    const cplx* tw;         // twiddles exp(2 pi i n2 t/NZ), [P][T]
+    const cplx* tw;         // twiddles exp(2 pi i n2 t/NZ): [P][T] (Geom), then [8][NZ/8]
     const double* ilap2;    // [Ny/2][nz] 1/lap2 table (Kdata.cpp:100-119)
     double* partials;       // [grid][PL]
     double* gpartials;      // [ngroups][PL]
@@ -103,7 +103,7 @@ struct StageArgs {
     int diag_cap;
     int rhs_only;           // Model::rhs: write F (and linop) only, no update
     double* linop_out;      // rhs_only: [nxy][4][nz]
-    unsigned long long* trace;  // optional %globaltimer trace (null: off), see qlgpu_kernel.cuh
+    unsigned long long* trace;  // optional %globaltimer trace (null: off), see stage_body (qlgpu_wide.cuh)
     double* mfr_cache;      // [NMFR][NZ] real-space mean-field profiles written by the top CTA
     const double* ekz_tab;  // [2][nz] exp(linC nu kz2), exp(linC eta kz2) for this stage (null: compute)
     // optional record of the stage input (null: off): the fields [nxy][4][nz], the mean
@@ -147,8 +147,7 @@ struct BatchSlot {
 // The work list of one CTA of the persistent launch.
 struct BatchCta {
     int nslots;
-    int tcols;  // TMEM columns the CTA allocates (the largest of its slots' needs)
-    int pad[2];
+    int pad[3];
     BatchSlot slot[BATCH_MAX_SLOTS];
 };
 

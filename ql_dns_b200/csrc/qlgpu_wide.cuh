@@ -1,0 +1,858 @@
+// qlgpu_wide.cuh -- one RK3 stage of the quasi-linear models with a mode's
+// transforms side by side (sm_100a): MHD_BQlin and MHD_FullQlin, RK3CN_Elin and
+// RK3CN, NZ = 16 ... 256.
+//
+// What bounds it.  A case of a few thousand modes gives an SM a handful of modes
+// per stage, so a stage is latency: the chain of transforms one mode walks.  A
+// pair of groups that took the mode's transforms one after another walked 5
+// inverse and 4 forward transforms with the pointwise work between them, about
+// 31 us whatever NZ is.  Here a mode's inverse transforms are independent tasks
+// of the warps of a TEAM, and so are its forward transforms: two transforms
+// deep, two team barriers, and code that is one loop over tasks around one
+// transform instead of 9 unrolled steps (the instruction cache is cold at every
+// launch).
+//
+// Team.  `tw` warps (any count) share one block of GPW = 32/T modes: a warp-task
+// transforms one field of all GPW modes, group g of the warp (T = NZ/8 lanes,
+// 8 points each) the field of mode g.  Every task uses the same (lane, register)
+// map, index t + T r of mode g, in spectral and in real space, so a task's result
+// lies in shared memory at [r][lane] and its readers use their own lane: no bank
+// conflicts, no index math.
+//
+//   MHD_BQlin   (MHD_BQlin.cpp:135-257; 14 transforms, the reference does 22)
+//     inverse   R_uz R_bz R_u R_b R_zeta R_eta R_{i kz uz} R_uy R_by
+//     forward   S = i ky By R_b, then 2 kx ky dBy R_bz      -> u
+//               i ky By R_zeta - i kx dBy R_u - 2 dBy R_{i kz uz} - ddBy R_uz -> eta
+//               i ky By R_eta - i kx dBy R_b + ddBy R_bz     -> zeta
+//               i ky By R_u                                  -> b
+//     stress    Ex += Re(R_bz R_u* - R_uz R_b*), Ey += Re(R_bz R_uy* - R_uz R_by*)
+//   MHD_FullQlin (MHD_FullQlin.cpp:209-381; 16 transforms, the reference does 32)
+//     inverse   Ux Uy Uz Bx By Bz dzUx dzUy dzBx dzBy
+//     forward   T1 T2 T3 S1 S2 S3 (formulas at fq_input)
+//     stress    EMF x, y and the two velocity drives
+//     update    u, zeta, b, eta from the six spectra (a third barrier)
+//
+// A CTA holds teams = max(1, warps / TS) teams (TS = 5 / 8: the forward tasks of
+// a model), each with its own named barrier and its own blocks.  Partial sums of
+// the stresses are lane-private in shared memory; per-CTA sums go through the
+// fixed-order two-level reduction and the CTA that arrives last runs the
+// mean-field stage, its loads issued before the sums are waited for and its
+// transforms on the same 8-point layout.
+#pragma once
+#include "qlgpu_debug.cuh"
+#include "qlgpu_kernel.cuh"
+#include "qlgpu_noise.cuh"
+#include "qlgpu_stage.cuh"
+#include "qlgpu_xform.cuh"
+
+namespace qlgpu {
+namespace wide {
+
+constexpr int MAX_WARPS = 16;
+
+// Geometry and shared-memory layout of one NZ class and model.
+template <int NZ_, int MODEL>
+struct WG {
+    static constexpr int NZ = NZ_;
+    static constexpr int T = NZ_ / 8;                  // lanes per group
+    static constexpr int nz = 1 + 2 * (NZ_ / 3);       // Model.h:34
+    static constexpr int H = (nz - 1) / 2;
+    static constexpr int GPW = 32 / T;                 // modes per block
+    static constexpr int SWZ = T == 4 ? 1 : (T == 2 ? 3 : 0);
+    static constexpr bool BQ = MODEL == MODEL_BQLIN;
+    static constexpr int TS = BQ ? 5 : 8;              // warps of a full team
+    static constexpr int NINV = BQ ? 9 : 10;           // inverse tasks
+    static constexpr int NX = BQ ? 3 : 6;              // exchange buffers of the forward tasks
+    static constexpr int NE = BQ ? 2 : 4;              // stress profiles
+    static constexpr int NPROF = BQ ? 3 : 8;           // real-space mean-field profiles
+    static constexpr int PL = NE * NZ_ + 8;            // partial vector (doubles)
+    static constexpr int NZE = (nz + 1) & ~1;
+    static constexpr size_t o_tw = 0;                                  // [8][T] cplx
+    static constexpr size_t o_prof = o_tw + 16 * (size_t)NZ_;          // [NPROF][NZ]
+    static constexpr size_t o_kz = o_prof + 8 * (size_t)NPROF * NZ_;   // kz per spectral slot
+    static constexpr size_t o_ekz = o_kz + 8 * (size_t)NZ_;            // [2][NZE]
+    static constexpr size_t o_dred = o_ekz + 16 * (size_t)NZE;         // [MAX_WARPS][6] diagnostic sums
+    static constexpr size_t o_team = (o_dred + 8 * 6 * MAX_WARPS + 15) & ~(size_t)15;
+    // per team: results / exchange buffers [NINV + NX][8][32] cplx, staged fields [GPW][4][nz]
+    // cplx, stress sums [NE][8][32]
+    static constexpr size_t TM_STG = 16 * 256 * (size_t)(NINV + NX);
+    static constexpr size_t TM_ACC = TM_STG + 16 * (size_t)GPW * 4 * nz;
+    static constexpr size_t TEAM_BYTES = TM_ACC + 8 * 256 * (size_t)NE;
+    // the mean-field stage's scratch overlays the teams' buffers
+    static constexpr size_t TOP_BYTES = 8 * ((size_t)PL + 2) + 16 * (size_t)NE * (H + 1) + 16 * 4 * (size_t)nz;
+    static_assert(TOP_BYTES <= 16 * 256 * (size_t)(NINV + NX - 4), "mean-field scratch below its exchange buffers");
+    __host__ __device__ static constexpr int teams(int warps) { return warps / TS > 1 ? warps / TS : 1; }
+    __host__ __device__ static constexpr size_t bytes(int warps) {
+        return o_team + TEAM_BYTES * (size_t)teams(warps);
+    }
+};
+
+__device__ __forceinline__ void team_sync(int id, int threads) {
+    asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Mean-field side on the 8-point layout.  A warp transforms GPW profiles.
+// ---------------------------------------------------------------------------
+// Real-space profiles of the mean fields mf[][nz] (MHD_BQlin.cpp:122-127: By, dz
+// By, dz^2 By; MHD_FullQlin.cpp:180-198: Bx, By, Ux, Uy and dz of each) into
+// out[NPROF][NZ]; xg = the warp's exchange buffer.  Ends without a barrier.
+template <class W, bool BQ, class Load>
+__device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, double* out, cplx* xg, const cplx* tw,
+                                               int warp, int nwarps, int lane) {
+    const int g = lane / W::T, t = lane % W::T;
+    for (int base = warp * W::GPW; base < W::NPROF; base += nwarps * W::GPW) {
+        const int arr = base + g;
+        const int src = BQ ? 1 : arr / 2, deriv = BQ ? arr : arr % 2;
+        cplx x[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+            cplx v = mk(0.0, 0.0);
+            if (s >= 0 && arr < W::NPROF) {
+                v = cscale(mf(src, s), P.fac);
+                const int k = t + W::T * r;
+                const double c = kzval(k <= W::H ? k : k - W::NZ, P.kzL);
+                if (deriv == 1) v = imul(v, c);
+                if (deriv == 2) v = cscale(v, kz2val(c));
+            }
+            x[r] = v;
+        }
+        xform<W>(x, xg, tw, g, t);
+        if (arr < W::NPROF) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) out[arr * W::NZ + t + W::T * r] = x[r].x;
+        }
+    }
+}
+
+// Mean-field stage of the CTA that arrived last: tot[PL] holds the stress
+// profiles summed over the modes and the diagnostic sums.  Stress spectra
+// (MHD_BQlin.cpp:228-240 after the sum over modes; the transform is linear), the
+// mean-field update and clock (mean_field_update) and the next stage's profiles.
+template <class W, int MODEL, int INTEG>
+__device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P, double* tot, cplx* xch,
+                                          const cplx* tw, double tclock, double t_new, bool last, bool diag_due) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+    const int g = lane / W::T, t = lane % W::T;
+    double* spec = tot + W::PL + (W::PL & 1);
+    cplx* mfs = reinterpret_cast<cplx*>(spec + 2 * W::NE * (W::H + 1));
+    // at most four warps transform (their exchange buffers)
+    constexpr int NT = (W::NPROF + W::GPW - 1) / W::GPW < 4 ? (W::NPROF + W::GPW - 1) / W::GPW : 4;
+    const int ntw = nwarps < NT ? nwarps : NT;
+    cplx* xg = xch + (size_t)(warp < ntw ? warp : 0) * 256;
+    if (warp < ntw) {
+        for (int base = warp * W::GPW; base < W::NE; base += ntw * W::GPW) {
+            const int e = base + g;
+            cplx x[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) x[r] = mk(e < W::NE ? tot[e * W::NZ + t + W::T * r] : 0.0, 0.0);
+            xform<W>(x, xg, tw, g, t);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int k = t + W::T * r;
+                if (e < W::NE && k <= W::H) {
+                    cplx v = cscale(conjc(x[r]), P.rs_fac);
+                    if (MODEL == MODEL_BQLIN || e < 2) v = imul(v, kzval(k, P.kzL));  // times kz (z derivative)
+                    spec[(e * (W::H + 1) + k) * 2 + 0] = v.x;
+                    spec[(e * (W::H + 1) + k) * 2 + 1] = v.y;
+                }
+            }
+        }
+    }
+    __syncthreads();
+    mean_field_update<W, MODEL, INTEG, W::NE>(A, P, tot, spec, mfs, tclock, t_new, last, diag_due);
+    if (A.mfr_cache && !A.rhs_only && warp < ntw)
+        mean_profiles8<W, W::BQ>(
+            P, [&](int m, int s) { return mfs[m * W::nz + s]; }, A.mfr_cache, xg, tw, warp, ntw, lane);
+    __threadfence();
+    __syncthreads();
+    if (tid == 0 && A.mfr_cache && !A.rhs_only) A.clk->mfr_valid = 1;
+}
+
+// ---------------------------------------------------------------------------
+// Per-block constants of one lane: its mode's wavenumbers at the stage.
+// ---------------------------------------------------------------------------
+struct LaneMode {
+    int m, kyi, kxi;
+    bool valid, zero;
+    double kx0, a, b, kxe, kxo, mult;
+};
+
+// The stage update of one coefficient of field f (RK3CN_Elin.cpp:102-104 /
+// RK3CN.cpp:105-107), or F and the operator in rhs-only mode.
+template <class W, int MODEL, int INTEG>
+__device__ __forceinline__ void put_coef(const StageArgs& A, const DevParams& P, const LaneMode& M, const CnOld& cn,
+                                         const double* ekz, double em, int f, int s, double c, cplx F, cplx uin,
+                                         cplx fpv, bool has_fp) {
+    const StageConst& S = A.sc;
+    const int nzd = W::nz;
+    const size_t at = ((size_t)M.m * 4 + f) * nzd + QLGPU_CHECK_STORED(s, nzd, &A.clk->status);
+    const double kz2 = kz2val(c);
+    if (A.rhs_only) {
+        stc(A.lin_out + at, F);
+        if (A.linop_out) A.linop_out[at] = linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f);
+        return;
+    }
+    cplx nv;
+    if (INTEG == INTEG_EXP) {
+        double e;
+        if (MODEL == MODEL_BQLIN || P.factored) e = em * ekz[(f < 2 ? 0 : W::NZE) + s];
+        else e = exp(__dmul_rn(S.linC, linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f)));
+        const cplx acc = has_fp ? cadd(cadd(cscale(F, S.n1), cscale(fpv, S.n2)), uin) : cadd(cscale(F, S.n1), uin);
+        nv = cscale(acc, e);
+    } else {
+        const bool z0 = (M.kyi == 0 && s == 0);
+        const double L = linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f);
+        const double lo = cn.old_init ? lap_init<MODEL>(P, M.kxo, lap2val(M.b, kz2, z0))
+                                      : lap_end<MODEL>(P, M.kxo, M.b, kz2);
+        nv = rk_update<INTEG_CN>(S, L, linop_f<MODEL>(P, lo, f), F, fpv, uin, has_fp);
+    }
+    if (A.Fout) stc(A.Fout + at, F);
+    stc(A.lin_out + at, M.zero ? mk(0.0, 0.0) : nv);
+}
+
+// Integrating-factor scalar exp(linC c (-kx^2 - ky^2)) of field f's side.
+template <int MODEL, int INTEG>
+__device__ __forceinline__ double em_of(const StageArgs& A, const DevParams& P, const LaneMode& M, int f) {
+    if (INTEG != INTEG_EXP || A.rhs_only || !(MODEL == MODEL_BQLIN || P.factored)) return 1.0;
+    const double hxy = __dsub_rn(-__dmul_rn(M.kxe, M.kxe), __dmul_rn(M.b, M.b));
+    return exp(A.sc.linC * (f < 2 ? P.nu : P.cb) * hxy);
+}
+
+// Spectral input of an inverse task for this lane's mode, scaled by 1/NZ:
+// kind 0 the field, 1 z-component, 2 i kz z-component, 3 y-component
+// (MHD_BQlin.cpp:143-146), 4 i kz field, 5 i kz y-component.
+template <class W>
+__device__ __forceinline__ void inv_input(cplx (&x)[8], const cplx* g0, const double* __restrict__ il2, int kind,
+                                          double a, double b, double fac, const double* kzc, int t) {
+    const cplx* g1 = g0 + W::nz;
+    if (kind == 0 || kind == 4) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+            cplx v = mk(0.0, 0.0);
+            if (s >= 0) {
+                v = g0[s];
+                v = kind == 0 ? cscale(v, fac) : imul(v, kzc[t + W::T * r] * fac);
+            }
+            x[r] = v;
+        }
+        return;
+    }
+    const double ab = __dmul_rn(a, b);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+        cplx v = mk(0.0, 0.0);
+        if (s >= 0) {
+            const double c = kzc[t + W::T * r];
+            const cplx u = g0[s], z = g1[s];
+            const double sc = __ldg(il2 + s) * fac;
+            // y: (a b) u + i c z;  z: (a c) u - i b z
+            const double p = (kind == 3 || kind == 5) ? ab : __dmul_rn(a, c);
+            const double q = (kind == 3 || kind == 5) ? c : -b;
+            v = mk(fma(p, u.x, -q * z.y), fma(p, u.y, q * z.x));
+            v = (kind == 2 || kind == 5) ? imul(v, sc * c) : cscale(v, sc);
+        }
+        x[r] = v;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// MHD_BQlin: result buffers and the forward / stress tasks of one block
+// ---------------------------------------------------------------------------
+enum { R_UZ = 0, R_BZ, R_U, R_B, R_ZE, R_ET, R_DUZ, R_UY, R_BY };
+
+template <class W, int INTEG>
+__device__ __forceinline__ void bq_forward(const StageArgs& A, const DevParams& P, const LaneMode& M, const CnOld& cn,
+                                           int task, cplx* R, const cplx* stg, const double* ekz, const double* prof,
+                                           const double* kzc, const cplx* tw, int lane, int g, int t) {
+    constexpr int T = W::T, nzd = W::nz;
+    const StageConst& S = A.sc;
+    const double *By = prof, *dBy = prof + W::NZ, *ddBy = prof + 2 * W::NZ;
+    auto buf = [&](int i) { return R + (size_t)i * 256; };
+    const double a = M.a, b = M.b;
+    // field updated, its exchange buffer (one that no other task still reads)
+    const int f = task == 0 ? 0 : task == 1 ? 3 : task == 2 ? 1 : 2;
+    cplx* xg = task == 1 ? buf(R_ZE) : task == 2 ? buf(R_ET) : buf(W::NINV + (task == 0 ? 0 : 2));
+    cplx* Sb = buf(W::NINV + 1) + lane;  // task 0: S, this lane's entries
+    const cplx* Fp = (A.Fprev && S.has_prev) ? A.Fprev + ((size_t)M.m * 4 + f) * nzd : nullptr;
+    cplx x[8];
+    for (int sub = task == 0 ? 0 : 1; sub < 2; ++sub) {
+        if (task == 0) {
+            const cplx* p = buf(sub ? R_BZ : R_B) + lane;
+            const double ab2 = 2.0 * __dmul_rn(a, b);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int z = t + T * r;
+                const cplx v = p[32 * r];
+                const double w = ab2 * dBy[z], y = b * By[z];
+                // conj(2 kx ky dBy R_bz) or conj(i ky By R_b)
+                x[r] = sub ? mk(w * v.x, -w * v.y) : mk(-y * v.y, -y * v.x);
+            }
+        } else if (task == 3) {
+            const cplx* p = buf(R_U) + lane;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const cplx v = p[32 * r];
+                const double y = b * By[t + T * r];
+                x[r] = mk(-y * v.y, -y * v.x);  // conj(i ky By R_u)
+            }
+        } else {
+            // eta: i ky By R_zeta - i kx dBy R_u - 2 dBy R_{i kz uz} - ddBy R_uz (MHD_BQlin.cpp:189-198)
+            // zeta: i ky By R_eta - i kx dBy R_b + ddBy R_bz (MHD_BQlin.cpp:170-178)
+            const cplx* p0 = buf(task == 1 ? R_ZE : R_ET) + lane;
+            const cplx* p1 = buf(task == 1 ? R_U : R_B) + lane;
+            const cplx* p2 = buf(task == 1 ? R_UZ : R_BZ) + lane;
+            const cplx* p3 = buf(R_DUZ) + lane;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int z = t + T * r;
+                const cplx v0 = p0[32 * r], v1 = p1[32 * r], v2 = p2[32 * r];
+                const double y = b * By[z], d = a * dBy[z], e = task == 1 ? -ddBy[z] : ddBy[z];
+                double re = fma(-y, v0.y, fma(d, v1.y, e * v2.x));
+                double im = fma(y, v0.x, fma(-d, v1.x, e * v2.y));
+                if (task == 1) {
+                    const cplx v3 = p3[32 * r];
+                    const double d2 = -2.0 * dBy[z];
+                    re = fma(d2, v3.x, re);
+                    im = fma(d2, v3.y, im);
+                }
+                x[r] = mk(re, -im);
+            }
+        }
+        __syncwarp();  // the exchange buffer may be one of those just read
+        xform<W>(x, xg, tw, g, t);
+        if (sub == 0) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) Sb[32 * r] = conjc(x[r]);
+        }
+    }
+    if (!M.valid) return;
+    const double em = em_of<MODEL_BQLIN, INTEG>(A, P, M, f);
+    const double Om2 = __dmul_rn(2.0, P.Omega);
+    const double cl = f == 3 ? -P.q : (f == 1 ? (P.q - Om2) : 0.0);
+    const double rl = __dmul_rn(__dmul_rn(2.0, __dmul_rn(a, b)), P.q);
+    const cplx* fin = stg + f * nzd;
+    const cplx* l0 = stg + (f == 3 ? 2 : 0) * nzd;
+    cplx fpv[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+        fpv[r] = (Fp && s >= 0) ? ldc(Fp + s) : mk(0.0, 0.0);
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (rdead<W>(r)) continue;
+        const int s = sidx<W>(t, r);
+        if (s < 0) continue;
+        const double c = kzc[t + T * r];
+        cplx F = conjc(x[r]);
+        if (f == 0) {
+            // S + ilapF ((2 kx ky q) u + 2 Omega i kz zeta + fwd(...)) (MHD_BQlin.cpp:162)
+            const bool z0 = (M.kyi == 0 && s == 0);
+            const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2val(c), z0));
+            const double ilapF = (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF);
+            const cplx lin = cadd(cadd(F, cscale(stg[s], rl)), imul(stg[nzd + s], Om2 * c));
+            F = cadd(Sb[32 * r], cscale(lin, ilapF));
+        } else if (f != 2) {
+            F = cadd(F, imul(l0[s], cl * c));  // MHD_BQlin.cpp:178,201
+        }
+        put_coef<W, MODEL_BQLIN, INTEG>(A, P, M, cn, ekz, em, f, s, c, F, fin[s], fpv[r], Fp != nullptr);
+    }
+}
+
+template <class W>
+__device__ __forceinline__ void bq_stress(const LaneMode& M, const cplx* R, double* acc, int lane) {
+    auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const cplx uz = rd(R_UZ, r), bz = rd(R_BZ, r), u = rd(R_U, r), bb = rd(R_B, r), uy = rd(R_UY, r),
+                   by = rd(R_BY, r);
+        // MHD_BQlin.cpp:212-241
+        const double ex = fma(bz.x, u.x, bz.y * u.y) - fma(uz.x, bb.x, uz.y * bb.y);
+        const double ey = fma(bz.x, uy.x, bz.y * uy.y) - fma(uz.x, by.x, uz.y * by.y);
+        double* ax = acc + 32 * r + lane;
+        ax[0] = fma(M.mult, ex, ax[0]);
+        ax[256] = fma(M.mult, ey, ax[256]);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// MHD_FullQlin.  With aU = i(kx MUx + ky MUy), aB = i(kx MBx + ky MBy)
+// (MHD_FullQlin.cpp:271-299):
+//   T1 = aU Ux + Uz dMUx - aB Bx - Bz dMBx    S1 = aU Bx + Uz dMBx - aB Ux - Bz dMUx
+//   T2 = aU Uy + Uz dMUy - aB By - Bz dMBy    S2 = aU By + Uz dMBy - aB Uy - Bz dMUy
+//   T3 = aU Uz - aB Bz                        S3 = aU Bz - aB Uz
+// ---------------------------------------------------------------------------
+enum { Q_UX = 0, Q_UY, Q_UZ, Q_BX, Q_BY, Q_BZ, Q_DUX, Q_DUY, Q_DBX, Q_DBY };
+
+// conj of forward input n (0-2: T1..T3, 3-5: S1..S3)
+template <class W>
+__device__ __forceinline__ void fq_input(cplx (&x)[8], const LaneMode& M, int n, const cplx* R, const double* prof,
+                                         int lane, int t) {
+    constexpr int NZ = W::NZ;
+    auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+    const int k = n % 3;
+    const bool sside = n >= 3;
+    const int own = sside ? Q_BX + k : Q_UX + k, oth = sside ? Q_UX + k : Q_BX + k;
+    // dz profiles of the mean x (k = 0) or y (k = 1) components: prof = Bx, dBx, By, dBy, Ux, dUx, Uy, dUy
+    const double* d1 = prof + (sside ? 1 + 2 * k : 5 + 2 * k) * NZ;
+    const double* d2 = prof + (sside ? 5 + 2 * k : 1 + 2 * k) * NZ;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int z = t + W::T * r;
+        const double aU = M.a * prof[4 * NZ + z] + M.b * prof[6 * NZ + z];  // times i
+        const double aB = M.a * prof[z] + M.b * prof[2 * NZ + z];
+        const cplx F = rd(own, r), G = rd(oth, r);
+        cplx v = csub(imul(F, aU), imul(G, aB));
+        if (k < 2) v = csub(cadd(v, cscale(rd(Q_UZ, r), d1[z])), cscale(rd(Q_BZ, r), d2[z]));
+        x[r] = conjc(v);
+    }
+}
+
+// Stress sums: half 0 the EMFs and the x drive of u, half 1 the rest (MHD_FullQlin.cpp:314-362)
+template <class W>
+__device__ __forceinline__ void fq_stress(const LaneMode& M, int half, const cplx* R, double* acc, int lane) {
+    auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+    auto rc = [](cplx p, cplx q) { return p.x * q.x + p.y * q.y; };  // Re(p conj q)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        double* ax = acc + 32 * r + lane;
+        const cplx Ux = rd(Q_UX, r), Uy = rd(Q_UY, r), Uz = rd(Q_UZ, r);
+        const cplx Bx = rd(Q_BX, r), By = rd(Q_BY, r), Bz = rd(Q_BZ, r);
+        if (half == 0) {
+            // EMF x (:322) and the x drive (:342-343): Re(Fx (i kx Fx)*) + Re(Fy (i ky Fx)*) + Re(Fz (dz Fx)*)
+            const double ex = rc(Bz, Ux) - rc(Uz, Bx);
+            const double du = rc(Ux, imul(Ux, M.a)) + rc(Uy, imul(Ux, M.b)) + rc(Uz, rd(Q_DUX, r));
+            const double db = rc(Bx, imul(Bx, M.a)) + rc(By, imul(Bx, M.b)) + rc(Bz, rd(Q_DBX, r));
+            ax[0] = fma(M.mult, ex, ax[0]);
+            ax[512] = fma(M.mult, db - du, ax[512]);
+        } else {
+            // EMF y (:330) and the y drive (:357-358)
+            const double ey = rc(Bz, Uy) - rc(Uz, By);
+            const double du = rc(Ux, imul(Uy, M.a)) + rc(Uy, imul(Uy, M.b)) + rc(Uz, rd(Q_DUY, r));
+            const double db = rc(Bx, imul(By, M.a)) + rc(By, imul(By, M.b)) + rc(Bz, rd(Q_DBY, r));
+            ax[256] = fma(M.mult, ey, ax[256]);
+            ax[768] = fma(M.mult, db - du, ax[768]);
+        }
+    }
+}
+
+// Update of field f from the six spectra in X[n][r][lane] (MHD_FullQlin.cpp:283-305)
+template <class W, int INTEG>
+__device__ __forceinline__ void fq_update(const StageArgs& A, const DevParams& P, const LaneMode& M, const CnOld& cn,
+                                          int f, const cplx* X, const cplx* stg, const double* ekz, const double* kzc,
+                                          int lane, int t) {
+    constexpr int nzd = W::nz;
+    if (!M.valid) return;
+    const StageConst& S = A.sc;
+    const double a = M.a, b = M.b, ab = __dmul_rn(a, b), Om2 = __dmul_rn(2.0, P.Omega);
+    const double em = em_of<MODEL_FULLQLIN, INTEG>(A, P, M, f);
+    const cplx* Fp = (A.Fprev && S.has_prev) ? A.Fprev + ((size_t)M.m * 4 + f) * nzd : nullptr;
+    auto X_ = [&](int n, int r) { return X[(size_t)n * 256 + 32 * r + lane]; };
+    cplx fpv[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+        fpv[r] = (Fp && s >= 0) ? ldc(Fp + s) : mk(0.0, 0.0);
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (rdead<W>(r)) continue;
+        const int s = sidx<W>(t, r);
+        if (s < 0) continue;
+        const double c = kzc[t + W::T * r];
+        cplx F, uin;
+        if (f == 0) {
+            const cplx u0 = stg[s], ze = stg[nzd + s], t1 = X_(0, r), t2 = X_(1, r), t3 = X_(2, r);
+            const bool z0 = (M.kyi == 0 && s == 0);
+            const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2val(c), z0));
+            const double ilapF = (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF);
+            // (2 kx ky q) u + 2 Om i kz zeta - kx^2 t1 - kx ky t2 - kx kz t3
+            cplx inner = cadd(cscale(u0, __dmul_rn(__dmul_rn(2.0, ab), P.q)), imul(ze, Om2 * c));
+            inner = csub(inner, cadd(cadd(cscale(t1, a * a), cscale(t2, ab)), cscale(t3, a * c)));
+            F = csub(cadd(cscale(inner, ilapF), imul(stg[2 * nzd + s], P.B0z * c)), t1);
+            uin = u0;
+        } else if (f == 1) {
+            // (q - 2 Om) kz u + B0z kz eta - (kz t2 - ky t3)
+            F = csub(cadd(imul(stg[s], (P.q - Om2) * c), imul(stg[3 * nzd + s], P.B0z * c)),
+                     csub(imul(X_(1, r), c), imul(X_(2, r), b)));
+            uin = stg[nzd + s];
+        } else if (f == 2) {
+            F = csub(imul(stg[s], P.B0z * c), X_(3, r));  // B0z kz u - s1
+            uin = stg[2 * nzd + s];
+        } else {
+            // -q kz b + B0z kz zeta - (kz s2 - ky s3)
+            uin = stg[3 * nzd + s];
+            F = csub(cadd(imul(stg[2 * nzd + s], -P.q * c), imul(stg[nzd + s], P.B0z * c)),
+                     csub(imul(X_(4, r), c), imul(X_(5, r), b)));
+        }
+        put_coef<W, MODEL_FULLQLIN, INTEG>(A, P, M, cn, ekz, em, f, s, c, F, uin, fpv[r], Fp != nullptr);
+    }
+}
+
+// Per-mode diagnostic sums of one side (0 velocity, 1 magnetic) from the new
+// state just stored (MHD_BQlin.cpp:365-407): energy, stress, dissipation.
+template <class W>
+__device__ __forceinline__ void side_diag(const DevParams& P, const LaneMode& M, int side, const cplx* uo,
+                                          double t_new, const double* kzc, int t, double (&v)[3]) {
+    const double an = kx_at(M.kx0, P.q, t_new, M.b);
+    const double ab = __dmul_rn(an, M.b);
+    const double md = M.b == 0.0 ? 1.0 : 2.0;
+    const double vis = side ? P.eta : P.nu;
+    const cplx* f0 = uo + (size_t)(2 * side) * W::nz;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        if (rdead<W>(r)) continue;
+        const int s = sidx<W>(t, r);
+        if (s < 0) continue;
+        const double c = kzc[t + W::T * r];
+        const bool z0 = (M.kyi == 0 && s == 0);
+        const double lap2 = lap2val(M.b, kz2val(c), z0);
+        const double il2 = ilap2val(lap2, z0);
+        const double lapF = __dadd_rn(-__dmul_rn(an, an), lap2);
+        const double l2 = __dmul_rn(lapF, il2);
+        const cplx p = ldc(f0 + s), q = ldc(f0 + W::nz + s);
+        const double e = l2 * (p.x * p.x + p.y * p.y) - il2 * (q.x * q.x + q.y * q.y);
+        const cplx y = cscale(cadd(cscale(p, ab), imul(q, c)), il2);  // (MHD_BQlin.cpp:388-392)
+        v[0] += md * e;
+        v[1] += md * (p.x * y.x + p.y * y.y);
+        v[2] += md * vis * (-lapF * e);
+    }
+}
+
+}  // namespace wide
+
+// Static shared words of a stage: the last-arriver flag.
+struct StageShared {
+    int last;
+    int pad[3];
+};
+
+// One stage over the modes of one case, executed by one CTA that is number
+// `cta` of the `ncta` CTAs working on that case.  Returns true in the one CTA
+// that arrived last and ran the mean-field stage; every other CTA returns as
+// soon as its partial sums are published.
+template <int NZ, int MODEL, int INTEG>
+__device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& P, const int cta, const int ncta,
+                                           unsigned char* smem_raw, StageShared& ss) {
+    using namespace wide;
+    using W = WG<NZ, MODEL>;
+    constexpr int T = W::T, nzd = W::nz, GPW = W::GPW;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+    const int g = lane / T, t = lane % T;
+    const StageConst& S = A.sc;
+    cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
+    double* prof = reinterpret_cast<double*>(smem_raw + W::o_prof);
+    double* kzc = reinterpret_cast<double*>(smem_raw + W::o_kz);
+    double* ekz = reinterpret_cast<double*>(smem_raw + W::o_ekz);
+    double* dred = reinterpret_cast<double*>(smem_raw + W::o_dred);
+    const int nteams = W::teams(warps), tws = warps / nteams;  // teams, warps per team
+    const int team = warp / tws, wt = warp - team * tws;
+    const bool in_team = team < nteams;
+    unsigned char* tbase = smem_raw + W::o_team + W::TEAM_BYTES * (size_t)(in_team ? team : 0);
+    cplx* R = reinterpret_cast<cplx*>(tbase);
+    cplx* stg_all = reinterpret_cast<cplx*>(tbase + W::TM_STG);
+    double* acc = reinterpret_cast<double*>(tbase + W::TM_ACC);
+    const int bar = 1 + team, bthreads = 32 * tws;
+    const bool tr = A.trace && cta == 0 && tid == 0;
+    if (tr) A.trace[0] = gtimer();
+
+    // ---- first block's fields requested, then the tables and the cleared sums
+    const int step = ncta * nteams * GPW;
+    const int first = (cta * nteams + team) * GPW;
+    auto stage_block = [&](int base) {
+        const int n = min(GPW, P.nxy - base) * 4 * nzd;
+        const cplx* src = A.lin_in + (size_t)base * 4 * nzd;
+        for (int i = wt * 32 + lane; i < n; i += bthreads) cp_async16(stg_all + i, src + i);
+        cp_async_commit();
+    };
+    if (in_team && first < P.nxy) stage_block(first);
+    for (int i = tid; i < NZ; i += blockDim.x) {
+        tw[i] = ldc_cg(A.tw + NZ + i);
+        kzc[i] = kzval(i <= W::H ? i : i - NZ, P.kzL);
+    }
+    const double tclock = __ldcg(&A.clk->t);
+    CnOld cn;
+    cn.t_old = __ldcg(&A.clk->t_old);
+    cn.dtlin_old = __ldcg(&A.clk->dtlin_old);
+    cn.old_init = __ldcg(&A.clk->old_init);
+    const double timevar = __ldcg(&A.clk->timevar);
+    const bool cached = A.mfr_cache && !A.rhs_only && __ldcg(&A.clk->mfr_valid);
+    if (INTEG == INTEG_EXP) {
+        // factored integrating factor: exp(linC c kz2) per stored kz
+        for (int s = tid; s < nzd; s += blockDim.x) {
+            if (A.ekz_tab) {
+                ekz[s] = __ldg(A.ekz_tab + s);
+                ekz[W::NZE + s] = __ldg(A.ekz_tab + nzd + s);
+            } else {
+                const double kz2 = kz2val(kzval(s <= W::H ? s : s - nzd, P.kzL));
+                ekz[s] = exp(S.linC * P.nu * kz2);
+                ekz[W::NZE + s] = exp(S.linC * P.cb * kz2);
+            }
+        }
+    }
+    if (cached)
+        for (int i = tid; i < W::NPROF * NZ; i += blockDim.x) prof[i] = __ldcg(A.mfr_cache + i);
+    if (in_team)
+        for (int i = wt * 32 + lane; i < 256 * W::NE; i += bthreads) acc[i] = 0.0;
+    for (int i = tid; i < 6 * MAX_WARPS; i += blockDim.x) dred[i] = 0.0;
+    __syncthreads();
+    if (!cached) {
+        // scratch: the result buffers of the first team, which nothing uses yet
+        cplx* r0 = reinterpret_cast<cplx*>(smem_raw + W::o_team);
+        const int nw = warps < 8 ? warps : 8;
+        if (warp < nw)
+            mean_profiles8<W, W::BQ>(
+                P, [&](int m, int s) { return ldc_cg(A.mf + m * nzd + s); }, prof, r0 + 256 * (warp & 7), tw, warp, nw,
+                lane);
+        __syncthreads();
+    }
+    if (tr) A.trace[1] = gtimer();
+
+    // Last-stage bookkeeping identical in every CTA (main.cpp:111-130)
+    const double t_new = __dadd_rn(tclock, P.dt);
+    const bool last = S.last && !A.rhs_only;
+    bool diag_due = false;
+    if (last && P.tv_interval > 0.0)
+        diag_due = __dsub_rn(__dadd_rn(timevar, P.dt), P.tv_interval) > -1e-8;
+    const double qt = __dmul_rn(P.q, t_new);
+    const double ts = S.abs_time ? S.t_off : __dadd_rn(tclock, S.t_off);
+
+    // ---- optional record of the stage input (the adjoint's window recompute): CTA 0 of the
+    // case copies the mean fields and, in a step's first stage, kx0 and the clock; stable
+    // here because the previous stage (and its remap) completed before any CTA started this one
+    if (A.rec_mf && cta == 0) {
+        const int nmfe = P.nmf * nzd;
+        for (int i = tid; i < nmfe; i += blockDim.x) A.rec_mf[i] = ldc(A.mf + i);
+        if (A.rec_kx)
+            for (int i = tid; i < P.nxy; i += blockDim.x) A.rec_kx[i] = __ldcg(A.kx0 + i);
+        if (A.rec_t && tid == 0) A.rec_t[0] = tclock;
+        if (A.rec_cn && tid == 0) {
+            A.rec_cn->t_old = cn.t_old;
+            A.rec_cn->dtlin_old = cn.dtlin_old;
+            A.rec_cn->old_init = cn.old_init;
+        }
+    }
+
+    // ---- the team's blocks of GPW modes
+    const bool has_prev = A.Fprev && S.has_prev;
+    for (int base = first; in_team && base < P.nxy; base += step) {
+        const int nv = min(GPW, P.nxy - base);
+        LaneMode M;
+        M.valid = g < nv;
+        M.m = QLGPU_CHECK_INDEX(base + min(g, nv - 1), P.nxy, &A.clk->status);
+        const cplx* stg = stg_all + (size_t)min(g, nv - 1) * 4 * nzd;
+        M.b = __ldg(A.ky + M.m);
+        M.kx0 = __ldcg(A.kx0 + M.m);
+        M.kyi = __ldg(A.kyi + M.m);
+        M.kxi = __ldg(A.kxi + M.m);
+        if (base != first) stage_block(base);
+        if (wt == 0 && lane == 0) {
+            // the next block's fields and this and the next block's previous rhs into L2
+            const size_t nb = (size_t)base + step;
+            if (nb < (size_t)P.nxy) {
+                const unsigned bytes = 64u * nzd * (unsigned)min(GPW, P.nxy - (int)nb);
+                l2_prefetch(A.lin_in + nb * 4 * nzd, bytes);
+                if (has_prev) l2_prefetch(A.Fprev + nb * 4 * nzd, bytes);
+            }
+        }
+        M.a = kx_at(M.kx0, P.q, ts, M.b);  // kx(t_s), MHD_BQlin.cpp:498
+        M.mult = M.valid ? (M.b == 0.0 ? 1.0 : 2.0) : 0.0;
+        M.kxe = __dadd_rn(M.a, __dmul_rn(__dmul_rn(P.q, S.dt_lin), M.b));  // MHD_BQlin.cpp:248
+        M.kxo = 0.0;
+        if (INTEG == INTEG_CN) {
+            if (cn.old_init) M.kxo = kx_at(M.kx0, P.q, tclock, M.b);
+            else M.kxo = __dadd_rn(kx_at(M.kx0, P.q, cn.t_old, M.b), __dmul_rn(__dmul_rn(P.q, cn.dtlin_old), M.b));
+        }
+        // ShearingBox_Remap(q t) after t += dt (main.cpp:122-123, MHD_BQlin.cpp:319-329)
+        M.zero = last && P.remap && __dadd_rn(M.kx0, __dmul_rn(qt, M.b)) > P.remap_thresh;
+        const double* __restrict__ il2 = A.ilap2 + (size_t)M.kyi * nzd;
+        cp_async_wait_all();
+        team_sync(bar, bthreads);
+        if (A.rec_lin) {  // record the block's input fields
+            cplx* dst = A.rec_lin + (size_t)base * 4 * nzd;
+            for (int i = wt * 32 + lane; i < nv * 4 * nzd; i += bthreads) dst[i] = stg_all[i];
+        }
+        // ---- inverse transforms
+#pragma unroll 1
+        for (int task = wt; task < W::NINV; task += tws) {
+            int kind, side;
+            if (W::BQ) {
+                side = (task == R_BZ || task == R_B || task == R_ET || task == R_BY);
+                kind = (task == R_UZ || task == R_BZ) ? 1 : task == R_DUZ ? 2 : (task == R_UY || task == R_BY) ? 3 : 0;
+            } else {
+                side = (task >= Q_BX && task <= Q_BZ) || task >= Q_DBX;
+                kind = (task == Q_UX || task == Q_BX) ? 0 : (task == Q_UY || task == Q_BY) ? 3
+                     : (task == Q_UZ || task == Q_BZ) ? 1 : (task == Q_DUX || task == Q_DBX) ? 4 : 5;
+            }
+            const int f0 = 2 * side + (W::BQ && (task == R_ZE || task == R_ET) ? 1 : 0);
+            cplx x[8];
+            inv_input<W>(x, stg + f0 * nzd, il2, kind, M.a, M.b, P.fac, kzc, t);
+            cplx* xb = R + (size_t)task * 256;
+            xform<W>(x, xb, tw, g, t);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) xb[32 * r + lane] = x[r];
+        }
+        team_sync(bar, bthreads);
+        // ---- products, forward transforms, stresses
+        if constexpr (W::BQ) {
+#pragma unroll 1
+            for (int task = wt; task < 5; task += tws) {
+                if (task == 4) bq_stress<W>(M, R, acc, lane);
+                else bq_forward<W, INTEG>(A, P, M, cn, task, R, stg, ekz, prof, kzc, tw, lane, g, t);
+            }
+        } else {
+#pragma unroll 1
+            for (int task = wt; task < 8; task += tws) {
+                if (task >= 6) {
+                    fq_stress<W>(M, task - 6, R, acc, lane);
+                    continue;
+                }
+                cplx x[8];
+                fq_input<W>(x, M, task, R, prof, lane, t);
+                cplx* xb = R + (size_t)(W::NINV + task) * 256;
+                xform<W>(x, xb, tw, g, t);
+#pragma unroll
+                for (int r = 0; r < 8; ++r) xb[32 * r + lane] = conjc(x[r]);
+            }
+            team_sync(bar, bthreads);
+#pragma unroll 1
+            for (int f = wt; f < 4; f += tws)
+                fq_update<W, INTEG>(A, P, M, cn, f, R + (size_t)W::NINV * 256, stg, ekz, kzc, lane, t);
+        }
+        team_sync(bar, bthreads);  // the block's stores are done; its buffers are free
+        if (last) {
+            if (M.zero && M.valid && wt == 0 && t == 0) A.kx0[M.m] = __dsub_rn(M.kx0, P.remap_shift);
+            cplx* uo = A.lin_out + (size_t)M.m * 4 * nzd;
+            if (A.noise) {
+                // Model::DrivingNoise after the step (main.cpp:111-113), before the diagnostics see it
+                if (M.valid && !M.zero)
+                    noise_mode(A.noise, __ldcg(&A.clk->nstep), uo, nzd, wt * T + t, tws * T, M.m, M.kx0, M.b, M.kxi,
+                               M.kyi, P.q, tclock, P.kzL);
+                team_sync(bar, bthreads);
+            }
+            if (diag_due) {
+                for (int side = wt; side < 2; side += tws) {
+                    double v[3] = {0.0, 0.0, 0.0};
+                    if (M.valid && !M.zero) side_diag<W>(P, M, side, uo, t_new, kzc, t, v);
+#pragma unroll
+                    for (int q = 0; q < 3; ++q) {
+#pragma unroll
+                        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+                        if (lane == 0) dred[team * 6 + 2 * q + side] += v[q];
+                    }
+                }
+            }
+        }
+    }
+
+    // ---- CTA sums of the stress profiles and diagnostics (fixed order)
+    __syncthreads();
+    if (tr) A.trace[2] = gtimer();
+    double* part = A.partials + (size_t)cta * W::PL;
+    for (int idx = tid; idx < W::NE * NZ; idx += blockDim.x) {
+        const int e = idx / NZ, z = idx % NZ, r = z / T, tt = z % T;
+        double s = 0.0;
+        for (int tm = 0; tm < nteams; ++tm) {
+            const double* ac = reinterpret_cast<const double*>(smem_raw + W::o_team + W::TEAM_BYTES * (size_t)tm +
+                                                               W::TM_ACC) + 256 * e + 32 * r + tt;
+#pragma unroll
+            for (int gg = 0; gg < GPW; ++gg) s += ac[gg * T];
+        }
+        part[idx] = s;
+    }
+    if (tid < 6) {
+        double s = 0.0;
+        for (int tm = 0; tm < nteams; ++tm) s += dred[tm * 6 + tid];
+        part[W::NE * NZ + tid] = s;
+    }
+
+    // ---- two-level last-arriver reduction
+    __threadfence();
+    __syncthreads();
+    if (tr) A.trace[3] = gtimer();
+    const int ngroups = (ncta + RED_GROUP - 1) / RED_GROUP;
+    const int grp = QLGPU_CHECK_INDEX(cta / RED_GROUP, 64, &A.clk->status);  // DevClock::cnt_group
+    const int c0 = grp * RED_GROUP;
+    const int cn_in = min(RED_GROUP, ncta - c0);
+    if (tid == 0) {
+        unsigned tk = atomicAdd(&A.clk->cnt_group[grp], 1u);
+        ss.last = (tk == (unsigned)(cn_in - 1));
+    }
+    __syncthreads();
+    if (!ss.last) return false;
+    __threadfence();
+    double* tot = reinterpret_cast<double*>(smem_raw + W::o_team);
+    if (ngroups > 1) {
+        double* gpart = A.gpartials + (size_t)grp * W::PL;
+        for (int idx = tid; idx < W::PL; idx += blockDim.x) {
+            // CTAs in order, all their loads in flight
+            double v[RED_GROUP], s = 0.0;
+#pragma unroll
+            for (int u = 0; u < RED_GROUP; ++u)
+                v[u] = u < cn_in ? __ldcg(A.partials + (size_t)(c0 + u) * W::PL + idx) : 0.0;
+#pragma unroll
+            for (int u = 0; u < RED_GROUP; ++u)
+                if (u < cn_in) s += v[u];
+            gpart[idx] = s;
+        }
+        if (tid == 0) atomicExch(&A.clk->cnt_group[grp], 0u);
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            unsigned tk = atomicAdd(&A.clk->cnt_top, 1u);
+            ss.last = (tk == (unsigned)(ngroups - 1));
+        }
+        __syncthreads();
+        if (!ss.last) return false;
+        __threadfence();
+        for (int idx = tid; idx < W::PL; idx += blockDim.x) {
+            double s = 0.0;
+            for (int q = 0; q < ngroups; q += 16) {
+                double v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    v[u] = q + u < ngroups ? __ldcg(A.gpartials + (size_t)(q + u) * W::PL + idx) : 0.0;
+#pragma unroll
+                for (int u = 0; u < 16; ++u)
+                    if (q + u < ngroups) s += v[u];
+            }
+            tot[idx] = s;
+        }
+        if (tid == 0) atomicExch(&A.clk->cnt_top, 0u);
+    } else {
+        // one group: its last CTA is the last of all
+        for (int idx = tid; idx < W::PL; idx += blockDim.x) {
+            double v[RED_GROUP], s = 0.0;
+#pragma unroll
+            for (int u = 0; u < RED_GROUP; ++u)
+                v[u] = u < cn_in ? __ldcg(A.partials + (size_t)u * W::PL + idx) : 0.0;
+#pragma unroll
+            for (int u = 0; u < RED_GROUP; ++u)
+                if (u < cn_in) s += v[u];
+            tot[idx] = s;
+        }
+        if (tid == 0) atomicExch(&A.clk->cnt_group[0], 0u);
+    }
+    if (A.trace && tid == 0) A.trace[4] = gtimer();
+    __syncthreads();
+    // exchange buffers of the mean-field transforms: the last four result buffers of the first team
+    cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team) + 256 * (size_t)(W::NINV + W::NX - 4);
+    wide::top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, tclock, t_new, last, diag_due);
+    if (A.trace && tid == 0) A.trace[5] = gtimer();
+    return true;
+}
+
+// One stage launch of a single case.
+template <int NZ, int MODEL, int INTEG>
+__global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) stage_kernel(const __grid_constant__ StageArgs A,
+                                                                       const __grid_constant__ DevParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ StageShared ss;
+    stage_body<NZ, MODEL, INTEG>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss);
+}
+
+}  // namespace qlgpu

@@ -1,0 +1,106 @@
+// qlgpu_xform.cuh -- the z transforms with 8 points per thread (sm_100a).
+//
+// A group of T = NZ/8 threads (2 ... 32) holds one length-NZ column; thread t
+// register r holds index t + T r in spectral AND in real space.  One routine
+// (xform) computes the backward (FFTW_BACKWARD, fftwPlans.cpp:48-51) transform;
+// the forward one is conj(xform(conj(x))), and the conjugations are folded into
+// the pointwise code around it.  A transform is one register DFT-8, a twiddle,
+// one shared-memory exchange and 8/T register DFT-T (T = 16 / 32: a radix-2 / 4
+// step on the exchanged values and a DFT-8).
+#pragma once
+#include "qlgpu_fft.cuh"
+
+namespace qlgpu {
+
+// Real-space / spectral register classes: index t + T r is in the dealiasing
+// gap for every t (dead), stored for every t, or stored for some t.
+template <class E>
+__device__ __forceinline__ int sidx(int t, int r) {
+    const int k = t + E::T * r;
+    if (k <= E::H) return k;
+    if (k >= E::NZ - E::H) return k - (E::NZ - E::nz);
+    return -1;
+}
+template <class E>
+__host__ __device__ constexpr bool rdead(int r) {
+    return E::T * r > E::H && E::T * r + E::T - 1 < E::NZ - E::H;
+}
+
+// cos / sin (2 pi i / 16)
+__device__ __forceinline__ constexpr double c16(int i) {
+    return i == 0 ? 1.0 : i == 1 ? QLGPU_C1 : i == 2 ? QLGPU_RSQRT2 : i == 3 ? QLGPU_S1 : i == 4 ? 0.0
+         : i == 5 ? -QLGPU_S1 : i == 6 ? -QLGPU_RSQRT2 : -QLGPU_C1;
+}
+__device__ __forceinline__ constexpr double s16(int i) {
+    return i == 0 ? 0.0 : i == 1 ? QLGPU_S1 : i == 2 ? QLGPU_RSQRT2 : i == 3 ? QLGPU_C1 : i == 4 ? 1.0
+         : i == 5 ? QLGPU_C1 : i == 6 ? QLGPU_RSQRT2 : QLGPU_S1;
+}
+
+// Exchange-buffer slot of (row q, column t) in group g's buffer (cplx units).
+template <class E>
+__device__ __forceinline__ int xslot(int g, int q, int t) {
+    return g * 8 * E::T + E::T * (q ^ (g & E::SWZ)) + ((t + q) & (E::T - 1));
+}
+
+// Backward DFT of one column: x[r] = X[t + T r] in, x[r] = y[t + T r] out,
+// y[n] = sum_k X[k] exp(+2 pi i n k / NZ).  xg = the warp's exchange buffers,
+// g = this thread's group in the warp, tw[q T + t] = exp(2 pi i q t / NZ).
+// Warp-collective (every lane of the warp calls it together).
+template <class E>
+__device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, int g, int t) {
+    constexpr int T = E::T;
+    dft8<+1>(x);
+#pragma unroll
+    for (int q = 1; q < 8; ++q) x[q] = cmul(x[q], tw[q * T + t]);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) xg[xslot<E>(g, q, t)] = x[q];
+    __syncwarp();
+    if constexpr (T <= 8) {
+        constexpr int J = 8 / T;
+#pragma unroll
+        for (int j = 0; j < J; ++j) {
+            const int q = t + T * j;
+            cplx v[T];
+#pragma unroll
+            for (int s = 0; s < T; ++s) v[s] = xg[xslot<E>(g, q, s)];
+            dft<T, +1>(v);
+#pragma unroll
+            for (int m = 0; m < T; ++m) x[j + J * m] = v[m];
+        }
+    } else if constexpr (T == 16) {
+        // thread (q, h) = (t % 8, t / 8) takes the outputs of parity h of the 16-point
+        // transforms over the columns of row q: a radix-2 step then a DFT-8.
+        const int q = t & 7, h = t >> 3;
+        const double sg = h ? -1.0 : 1.0;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const cplx za = xg[xslot<E>(g, q, s)];
+            const cplx zb = xg[xslot<E>(g, q, s + 8)];
+            cplx w = mk(fma(sg, zb.x, za.x), fma(sg, zb.y, za.y));
+            if (s != 0) w = cmul(w, mk(h ? c16(s) : 1.0, h ? s16(s) : 0.0));
+            x[s] = w;
+        }
+        dft8<+1>(x);
+    } else {
+        static_assert(T == 32, "8 points per thread, NZ <= 256");
+        // thread (q, h) = (t % 8, t / 8) takes the outputs n = h + 4 m of the 32-point transforms
+        // over the columns of row q: w_s = exp(2 pi i s h / 32) sum_j i^(j h) z[s + 8 j], then a DFT-8.
+        const int q = t & 7, h = t >> 3;
+        const double s1 = (h & 1) ? -1.0 : 1.0, s2 = (h & 2) ? -1.0 : 1.0;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+            const cplx z0 = xg[xslot<E>(g, q, s)], z1 = xg[xslot<E>(g, q, s + 8)];
+            const cplx z2 = xg[xslot<E>(g, q, s + 16)], z3 = xg[xslot<E>(g, q, s + 24)];
+            const cplx a = mk(fma(s1, z2.x, z0.x), fma(s1, z2.y, z0.y));
+            const cplx b = mk(fma(s1, z3.x, z1.x), fma(s1, z3.y, z1.y));
+            const cplx ib = (h & 1) ? mk(-b.y, b.x) : b;  // i^h b up to the sign s2
+            cplx w = mk(fma(s2, ib.x, a.x), fma(s2, ib.y, a.y));
+            if (s != 0) w = cmul(w, tw[s * T + 8 * h]);  // exp(2 pi i 8 s h / 256)
+            x[s] = w;
+        }
+        dft8<+1>(x);
+    }
+    __syncwarp();
+}
+
+}  // namespace qlgpu
