@@ -105,9 +105,61 @@ void qlgpu_enqueue_step(qlgpu_t* h, cudaEvent_t* ev, const std::function<void(in
     }
 }
 
+// n steps in one cooperative launch (run_kernel), the stage inputs recorded where rec is set.
+cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec) {
+    cplx* Fbuf[3] = {h->d_F1, h->d_F2, nullptr};
+    const cplx* Fprev[3] = {nullptr, h->d_F1, h->d_F2};
+    cplx* Fmf[3] = {h->d_Fmf1, h->d_Fmf2, nullptr};
+    const cplx* Fmfp[3] = {nullptr, h->d_Fmf1, h->d_Fmf2};
+    RunArgs R;
+    std::memset(&R, 0, sizeof(R));
+    for (int s = 0; s < 3; ++s) {
+        StageArgs& A = R.A[s];
+        A = base_args(h);
+        A.Fprev = Fprev[s];
+        A.Fout = Fbuf[s];
+        A.Fmf_prev = Fmfp[s];
+        A.Fmf_out = Fmf[s];
+        A.sc = h->sc[s];
+        if (A.trace) A.trace += 32 * s;
+        A.ekz_tab = h->d_ekz + (size_t)s * 2 * h->nz;
+    }
+    R.P = h->dp;
+    R.lin[0] = h->d_lin[0];
+    R.lin[1] = h->d_lin[1];
+    R.cur = h->cur;
+    R.nsteps = n;
+    R.wait_ns = 2000000000LL;
+    if (rec) {
+        R.rec_lin = rec->lin;
+        R.rec_mf = rec->mf;
+        R.rec_kx = rec->kx;
+        R.rec_t = rec->t;
+        R.rec_cn = rec->cn;
+    }
+    const cudaError_t e = h->var.run(R, h->grid + 1, h->block, h->smem, h->stream);
+    if (e == cudaSuccess) h->cur ^= n & 1;  // three stages per step
+    return e;
+}
+
+// After a launch whose waits gave up: its counters are cleared, so that the handle is usable
+// again once a state is set.
+cudaError_t qlgpu_clear_abort(qlgpu_t* h) {
+    DevClock* c = h->d_clk;
+    cudaError_t e = cudaMemsetAsync(&c->cnt_top, 0, sizeof(unsigned), h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->cnt_group, 0, sizeof(c->cnt_group), h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(&c->abort, 0, sizeof(int), h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(&c->arrive, 0, sizeof(unsigned), h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(&c->epoch, 0, sizeof(unsigned), h->stream);
+    return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
+}
+
 namespace {
 
 void enqueue_step(qlgpu_t* h, cudaEvent_t* ev = nullptr) { qlgpu_enqueue_step(h, ev, nullptr); }
+
+// Steps per launch: short enough that a long run stays a sequence of launches of some 10 ms.
+constexpr int RUN_STEPS = 256;
 
 int ensure_diag(qlgpu_t* h, int cap) {
     if (cap <= h->diag_cap) return QLGPU_OK;
@@ -206,13 +258,14 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
         h->err = "cudaGetDeviceProperties failed";
         return bail(QLGPU_ERR_CUDA);
     }
-    const StageGeom sg = stage_geometry(p.model, p.NZ, h->nxy, prop.multiProcessorCount, 64 * RED_GROUP);
+    const StageGeom sg = stage_geometry(p.model, p.NZ, h->nxy, prop.multiProcessorCount - 1, 64 * RED_GROUP);
     h->warps = sg.warps;
     h->block = 32 * h->warps;
     h->smem = var.smem(h->warps);
     h->grid = sg.grid;
     h->per_sm = 1;
-    if (h->smem > (size_t)prop.sharedMemPerBlockOptin || ensure_smem_attr(var.kernel(), h->smem) != cudaSuccess) {
+    if (h->smem > (size_t)prop.sharedMemPerBlockOptin || ensure_smem_attr(var.kernel(), h->smem) != cudaSuccess ||
+        ensure_smem_attr(var.run_kernel(), h->smem) != cudaSuccess) {
         h->err = "shared memory request too large";
         return bail(QLGPU_ERR_CUDA);
     }
@@ -519,18 +572,18 @@ int qlgpu_step(qlgpu_t* h, int nsteps, int diag_every, double* diag_out, int max
         int zero = 0;
         QLGPU_CK(cudaMemcpyAsync(&h->d_clk->ndiag, &zero, sizeof(int), cudaMemcpyHostToDevice, h->stream));
     }
-    for (int n = 0; n < nsteps; ++n) {
-        enqueue_step(h);
-        if ((n & 63) == 63) {
-            int rc = check_launch(h);
-            if (rc) return rc;
-        }
+    for (int n = 0; n < nsteps; n += RUN_STEPS) {
+        QLGPU_CK(qlgpu_enqueue_run(h, std::min(RUN_STEPS, nsteps - n), nullptr));
     }
     int rc = check_launch(h);
     if (rc) return rc;
     DevClock c;
     QLGPU_CK(cudaMemcpyAsync(&c, h->d_clk, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
     QLGPU_CK(cudaStreamSynchronize(h->stream));
+    if (c.status & QLGPU_STATUS_TIMEOUT) {
+        QLGPU_CK(qlgpu_clear_abort(h));
+        return fail(h, QLGPU_ERR_STATUS, "step: a CTA gave up waiting for the other CTAs of the case");
+    }
     int nrec = 0;
     if (diag_every > 0) {
         nrec = c.ndiag < max_diag ? c.ndiag : max_diag;

@@ -162,6 +162,8 @@ struct AdjJob {
     cplx *lamU[2] = {nullptr, nullptr}, *lamB[2] = {nullptr, nullptr};
     cplx *lamF[2] = {nullptr, nullptr}, *lamG[2] = {nullptr, nullptr};
     double *prof = nullptr, *bpart = nullptr, *bsum = nullptr;
+    int* rec_status = nullptr;  // status bits of the window recomputes
+    int rec_status_host = 0;
     int iu = 0, ib = 0;
     double J = 0.0;
     // full-window graphs (replayed for every window of C steps when C is even)
@@ -224,8 +226,9 @@ int adj_checkpoint(AdjJob& j, int c) {
     return QLGPU_OK;
 }
 
-int adj_forward_step(AdjJob& j, int) {
-    qlgpu_enqueue_step(j.h, nullptr, nullptr);
+int adj_forward_window(AdjJob& j, int steps) {
+    qlgpu_t* h = j.h;
+    QA_CK(qlgpu_enqueue_run(h, steps, nullptr));
     return QLGPU_OK;
 }
 
@@ -250,6 +253,10 @@ int adj_alloc_backward(AdjJob& j);
 int adj_forward_finish(AdjJob& j) {
     qlgpu_t* h = j.h;
     h->dp.tv_interval = 0.0;
+    if (j.cend.status & QLGPU_STATUS_TIMEOUT) {
+        QA_CK(qlgpu_clear_abort(h));
+        return afail(h, QLGPU_ERR_STATUS, "forward run: a CTA gave up waiting for the other CTAs of the case");
+    }
     if (j.cend.status & (QLGPU_STATUS_NONFINITE | QLGPU_STATUS_UNSTABLE))
         return afail(h, QLGPU_ERR_STATUS, "forward run: non-finite or unstable solution");
     if (j.cend.ndiag != j.N) return afail(h, QLGPU_ERR_STATUS, "forward run: missing diagnostic records");
@@ -277,6 +284,7 @@ int adj_alloc_backward(AdjJob& j) {
     QA_CK(j.pool.get(&j.prof, (size_t)5 * h->NZ));
     QA_CK(j.pool.get(&j.bpart, (size_t)3 * h->NZ * j.nxy));
     QA_CK(j.pool.get(&j.bsum, (size_t)3 * h->NZ));
+    QA_CK(j.pool.get(&j.rec_status, 1));
     return QLGPU_OK;
 }
 
@@ -297,30 +305,20 @@ int adj_window_begin(AdjJob& j, int w) {
     return QLGPU_OK;
 }
 
-// recompute step n of the window, recording every stage's input
-int adj_recompute_step(AdjJob& j, int n) {
+// recompute a window, recording every stage's input
+int adj_recompute_window(AdjJob& j, int steps) {
     qlgpu_t* h = j.h;
-    cudaStream_t st = h->stream;
-    QA_CK(cudaMemcpyAsync(j.kx_pre + n * j.nxy, h->d_kx0, j.nxy * sizeof(double), cudaMemcpyDeviceToDevice, st));
-    QA_CK(cudaMemcpyAsync(j.t_pre + n, &h->d_clk->t, sizeof(double), cudaMemcpyDeviceToDevice, st));
-    cudaError_t herr = cudaSuccess;
-    qlgpu_enqueue_step(h, nullptr, [&](int s) {
-        const cudaError_t e1 = cudaMemcpyAsync(j.stU + ((size_t)n * 3 + s) * j.nlin, h->d_lin[h->cur],
-                                               j.nlin * sizeof(cplx), cudaMemcpyDeviceToDevice, st);
-        const cudaError_t e2 = cudaMemcpyAsync(j.stB + ((size_t)n * 3 + s) * j.nmfe, h->d_mf, j.nmfe * sizeof(cplx),
-                                               cudaMemcpyDeviceToDevice, st);
-        // t_old, dtlin_old, old_init of the clock (the layout of CnRec)
-        const cudaError_t e3 = cudaMemcpyAsync(j.cn_pre + (size_t)n * 3 + s, &h->d_clk->t_old, sizeof(CnRec),
-                                               cudaMemcpyDeviceToDevice, st);
-        if (herr == cudaSuccess) herr = e1 != cudaSuccess ? e1 : (e2 != cudaSuccess ? e2 : e3);
-    });
-    QA_CK(herr);
+    const RunRecord r{j.stU, j.stB, j.kx_pre, j.t_pre, j.cn_pre};
+    QA_CK(qlgpu_enqueue_run(h, steps, &r));
     return QLGPU_OK;
 }
+
+__global__ void adj_or_status_kernel(const DevClock* c, int* out) { *out |= c->status; }
 
 int adj_window_end(AdjJob& j, int w) {
     qlgpu_t* h = j.h;
     cudaStream_t st = h->stream;
+    adj_or_status_kernel<<<1, 1, 0, st>>>(h->d_clk, j.rec_status);
     const int steps = window_steps(j, w);
     QA_CK(cudaMemcpyAsync(j.postU, h->d_lin[h->cur], j.nlin * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
     QA_CK(cudaMemcpyAsync(j.kx_post, h->d_kx0, j.nxy * sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -448,6 +446,7 @@ int adj_finish(AdjJob& j, double* grad_lin, double* grad_mf) {
     cudaStream_t st = h->stream;
     QA_CK(cudaMemcpyAsync(grad_lin, j.lamU[j.iu], j.nlin * sizeof(cplx), cudaMemcpyDeviceToHost, st));
     if (grad_mf) QA_CK(cudaMemcpyAsync(grad_mf, j.lamB[j.ib], j.nmfe * sizeof(cplx), cudaMemcpyDeviceToHost, st));
+    QA_CK(cudaMemcpyAsync(&j.rec_status_host, j.rec_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     h->cur = j.fin_cur;
     QA_CK(cudaMemcpyAsync(h->d_lin[h->cur], j.fin_lin, j.nlin * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
     QA_CK(cudaMemcpyAsync(h->d_mf, j.fin_mf, j.nmfe * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
@@ -459,6 +458,10 @@ int adj_finish(AdjJob& j, double* grad_lin, double* grad_mf) {
 int sync_job(AdjJob& j) {
     qlgpu_t* h = j.h;
     QA_CK(cudaStreamSynchronize(h->stream));
+    if (j.rec_status_host & QLGPU_STATUS_TIMEOUT) {
+        QA_CK(qlgpu_clear_abort(h));
+        return afail(h, QLGPU_ERR_STATUS, "window recompute: a CTA gave up waiting for the other CTAs of the case");
+    }
     return QLGPU_OK;
 }
 
@@ -753,19 +756,9 @@ int run_jobs(std::vector<AdjJob>& jobs, double* J, double* const* grad_lin, doub
         int rc_ = (expr);                               \
         if (rc_) return rc_;                            \
     }
-    auto fwd_window = [&](AdjJob& j, int steps) -> int {
-        for (int n = 0; n < steps; ++n) {
-            int rc = adj_forward_step(j, n);
-            if (rc) return rc;
-        }
-        return QLGPU_OK;
-    };
     auto rec_window = [&](AdjJob& j, int w, int steps) -> int {
-        for (int n = 0; n < steps; ++n) {
-            int rc = adj_recompute_step(j, n);
-            if (rc) return rc;
-        }
-        return adj_window_end(j, w);
+        int rc = adj_recompute_window(j, steps);
+        return rc ? rc : adj_window_end(j, w);
     };
     auto bwd_window = [&](AdjJob& j, int steps) -> int {
         for (int n = steps - 1; n >= 0; --n) {
@@ -778,10 +771,10 @@ int run_jobs(std::vector<AdjJob>& jobs, double* J, double* const* grad_lin, doub
         const int steps = std::min(N, w * C + C) - w * C;
         QA_ALL(adj_checkpoint(jj, w));
         if (graphs && steps == C) {
-            QA_ALL(jj.g_fwd ? QLGPU_OK : capture(jj, &jj.g_fwd, [&] { return fwd_window(jj, C); }));
+            QA_ALL(jj.g_fwd ? QLGPU_OK : capture(jj, &jj.g_fwd, [&] { return adj_forward_window(jj, C); }));
             QA_ALL(launch_graph(jj, jj.g_fwd));
         } else {
-            for (int n = 0; n < steps; ++n) QA_ALL(adj_forward_step(jj, n));
+            QA_ALL(adj_forward_window(jj, steps));
         }
     }
     QA_ALL(adj_forward_end(jj));
@@ -796,8 +789,7 @@ int run_jobs(std::vector<AdjJob>& jobs, double* J, double* const* grad_lin, doub
             QA_ALL(jj.g_bwd ? QLGPU_OK : capture(jj, &jj.g_bwd, [&] { return bwd_window(jj, C); }));
             QA_ALL(launch_graph(jj, jj.g_bwd));
         } else {
-            for (int n = 0; n < steps; ++n) QA_ALL(adj_recompute_step(jj, n));
-            QA_ALL(adj_window_end(jj, w));
+            QA_ALL(rec_window(jj, w, steps));
             for (int n = steps - 1; n >= 0; --n) QA_ALL(adj_backward_step(jj, steps, n));
         }
     }

@@ -8,27 +8,19 @@
 // index and count of the item in place of blockIdx / gridDim.  The last CTA of
 // a case to publish its partial sums runs the case's mean-field stage and then
 // releases the case's stage counter; the other CTAs of the case wait for that
-// counter before their next stage of the case.  There is no grid-wide barrier:
-// cases advance independently, each at the pace of its own CTAs.
+// counter in their next stage of the case, after its first inverse transforms.
+// There is no grid-wide barrier: cases advance independently, each at the pace of
+// its own CTAs.  No cycle: a CTA publishes stage k - 1 of all its items before it
+// starts stage k of any.
 //
 // Every wait is bounded (wait_ns, and an iteration cap): a CTA that gives up
 // sets QLGPU_STATUS_TIMEOUT and the abort word, and every CTA then leaves its
-// step loop, frees its TMEM and returns.  The host launches the kernel with the
+// step loop and returns.  The host launches the kernel with the
 // cooperative attribute, so all CTAs are co-resident or the launch fails.
 #pragma once
 #include "qlgpu_wide.cuh"
 
 namespace qlgpu {
-
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ int ld_volatile_i32(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 
 // Wait (one thread) until *epoch >= target.  False when the launch was aborted
 // or the wait exceeded wait_ns (then the abort word is set here).
@@ -66,18 +58,20 @@ __device__ __forceinline__ void cta_copy8(void* dst, const void* src, int n) {
 // shared-memory objects are declared here so that every access stays a
 // shared-space access.
 template <int NZ, int MODEL, int INTEG>
-__device__ __noinline__ bool batch_item_stage(const BatchCase* cs, int s, int swap, int cta, int ncta, int n) {
+__device__ __noinline__ StageResult batch_item_stage(const BatchLaunch& L, const BatchCase* cs, const BatchSlot it,
+                                                     int s, int n, LocalClock& lc, bool fresh) {
     static_assert(sizeof(StageArgs) % 8 == 0 && sizeof(DevParams) % 8 == 0, "8-byte copies");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StageShared ss;
     __shared__ __align__(16) StageArgs sA;
     __shared__ __align__(16) DevParams sP;
     __syncthreads();  // the previous item is done with sA / sP
-    cta_copy8(&sP, &cs->P, (int)sizeof(DevParams));
+    if (fresh) cta_copy8(&sP, &cs->P, (int)sizeof(DevParams));
     cta_copy8(&sA, &cs->A[s], (int)sizeof(StageArgs));
     __syncthreads();
+    const unsigned k = 3u * (unsigned)n + (unsigned)s;  // stages before this one in the launch
     if (threadIdx.x == 0) {
-        if (swap) {
+        if ((n + L.parity) & 1) {
             const cplx* in = sA.lin_in;
             sA.lin_in = sA.lin_out;
             sA.lin_out = const_cast<cplx*>(in);
@@ -85,69 +79,60 @@ __device__ __noinline__ bool batch_item_stage(const BatchCase* cs, int s, int sw
         cplx* rl = cs->rec_lin;
         if (rl) {
             const size_t nlin = (size_t)sP.nxy * 4 * sP.nz, nmfe = (size_t)sP.nmf * sP.nz;
-            sA.rec_lin = rl + ((size_t)n * 3 + s) * nlin;
-            sA.rec_mf = cs->rec_mf + ((size_t)n * 3 + s) * nmfe;
+            sA.rec_lin = rl + (size_t)k * nlin;
+            sA.rec_mf = cs->rec_mf + (size_t)k * nmfe;
             sA.rec_kx = s == 0 ? cs->rec_kx + (size_t)n * sP.nxy : nullptr;
             sA.rec_t = s == 0 ? cs->rec_t + n : nullptr;
-            sA.rec_cn = cs->rec_cn ? cs->rec_cn + (size_t)n * 3 + s : nullptr;
+            sA.rec_cn = cs->rec_cn ? cs->rec_cn + k : nullptr;
         }
     }
     __syncthreads();
-    return stage_body<NZ, MODEL, INTEG>(sA, sP, cta, ncta, smem_raw, ss);
+    return stage_body<NZ, MODEL, INTEG, false>(sA, sP, it.cta, it.ncta, smem_raw, ss, lc, fresh, nullptr,
+                                               [&]() -> bool {
+        return batch_wait(L.epoch + (size_t)it.c * BATCH_EPOCH_STRIDE, k, L.ctl, L.wait_ns, it.c, k);
+    });
 }
 
 template <int MODEL, int INTEG>
 __global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) batch_kernel(const __grid_constant__ BatchLaunch L) {
-    __shared__ int s_ok;
     __shared__ BatchSlot s_items[BATCH_MAX_SLOTS];
-    __shared__ int s_top[BATCH_MAX_SLOTS];
+    __shared__ LocalClock s_clk[BATCH_MAX_SLOTS];
     const int tid = threadIdx.x;
     const BatchCta* me = L.ctas + blockIdx.x;
     const int nitems = min(me->nslots, BATCH_MAX_SLOTS);
-    if (tid < nitems * 4) reinterpret_cast<int*>(s_items)[tid] = reinterpret_cast<const int*>(me->slot)[tid];
+    if (tid < nitems) {
+        BatchSlot it = me->slot[tid];
+        it.c = QLGPU_CHECK_INDEX(it.c, L.ncases, &L.ctl->status);
+        s_items[tid] = it;
+        load_clock(s_clk[tid], L.cases[it.c].A[0].clk);
+    }
     if (blockIdx.x == 0 && tid == 0) L.ctl->t_start = gtimer();
     __syncthreads();
-    bool ok = true;
-    unsigned k = 0;  // stages completed by every case in this launch
-    for (int n = 0; n < L.nsteps && ok; ++n) {
-        const int swap = (n + L.parity) & 1;
-        for (int s = 0; s < 3 && ok; ++s, ++k) {
-            // all items of this CTA publish stage k before the CTA waits for any of them
+    for (int n = 0; n < L.nsteps; ++n)
+        for (int s = 0; s < 3; ++s)
             for (int i = 0; i < nitems; ++i) {
                 const BatchSlot it = s_items[i];
-                const BatchCase* cs = L.cases + QLGPU_CHECK_INDEX(it.c, L.ncases, &L.ctl->status);
-                bool top = false;
+                const BatchCase* cs = L.cases + it.c;
+                // the tables of a CTA's only item stay in shared memory
+                const bool fresh = nitems > 1 || (n == 0 && s == 0);
+                StageResult r;
                 switch (it.NZ) {
-                    case 16: top = batch_item_stage<16, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
-                    case 32: top = batch_item_stage<32, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
-                    case 64: top = batch_item_stage<64, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
-                    case 128: top = batch_item_stage<128, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
-                    default: top = batch_item_stage<256, MODEL, INTEG>(cs, s, swap, it.cta, it.ncta, n); break;
+                    case 16: r = batch_item_stage<16, MODEL, INTEG>(L, cs, it, s, n, s_clk[i], fresh); break;
+                    case 32: r = batch_item_stage<32, MODEL, INTEG>(L, cs, it, s, n, s_clk[i], fresh); break;
+                    case 64: r = batch_item_stage<64, MODEL, INTEG>(L, cs, it, s, n, s_clk[i], fresh); break;
+                    case 128: r = batch_item_stage<128, MODEL, INTEG>(L, cs, it, s, n, s_clk[i], fresh); break;
+                    default: r = batch_item_stage<256, MODEL, INTEG>(L, cs, it, s, n, s_clk[i], fresh); break;
                 }
-                if (tid == 0) s_top[i] = top ? 1 : 0;
-                if (top) {
+                if (r == STAGE_ABORT) return;
+                if (r == STAGE_TOP) {
                     __syncthreads();
                     if (tid == 0) {
                         __threadfence();
                         if (n == L.nsteps - 1 && s == 2) L.case_end[it.c] = gtimer();
-                        st_release_u32(L.epoch + (size_t)it.c * BATCH_EPOCH_STRIDE, k + 1);
+                        st_release_u32(L.epoch + (size_t)it.c * BATCH_EPOCH_STRIDE, 3u * (unsigned)n + s + 1);
                     }
                 }
             }
-            __syncthreads();
-            if (tid == 0) {
-                s_ok = 1;
-                for (int i = 0; i < nitems && s_ok; ++i) {
-                    if (s_top[i]) continue;
-                    const int c = s_items[i].c;
-                    if (!batch_wait(L.epoch + (size_t)c * BATCH_EPOCH_STRIDE, k + 1, L.ctl, L.wait_ns, c, k)) s_ok = 0;
-                }
-                __threadfence();
-            }
-            __syncthreads();
-            ok = s_ok != 0;
-        }
-    }
 }
 
 }  // namespace qlgpu

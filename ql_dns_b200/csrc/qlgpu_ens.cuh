@@ -255,6 +255,7 @@ __device__ __noinline__ void top_stage(const EnsLaunch& L, ChunkHdr& hd, int c, 
     const int tid = threadIdx.x;
     double* tot = scratch;                     // [PL]
     cplx* xch = reinterpret_cast<cplx*>(scratch) + W::TOP_BYTES / 16 + 1;  // four exchange buffers
+    wide::top_prefetch<W>(hd.A, tot);
     // chunk slots in slot order; 32 loads in flight per thread (this sum is on the case's
     // critical path: every CTA waits for the stage it releases)
     constexpr int U = 32;

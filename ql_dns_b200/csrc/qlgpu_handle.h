@@ -72,6 +72,18 @@ struct qlgpu_handle {
 // when set, runs on the host before each stage launch with the stage index.
 void qlgpu_enqueue_step(qlgpu_t* h, cudaEvent_t* ev, const std::function<void(int)>& hook);
 
+// n steps of the handle's state in one launch; rec (optional) takes every stage's inputs
+// (RunArgs' record layout).
+struct RunRecord {
+    cplx* lin;
+    cplx* mf;
+    double* kx;
+    double* t;
+    CnRec* cn;
+};
+cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec);
+cudaError_t qlgpu_clear_abort(qlgpu_t* h);
+
 // Debug build: the index checks' status bits and the guard zones of the handle after a
 // call's launches (QLGPU_ERR_STATUS when one fired).  QLGPU_OK at once in a release build.
 int qlgpu_debug_verify(qlgpu_t* h);

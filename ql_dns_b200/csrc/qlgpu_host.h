@@ -27,6 +27,7 @@ constexpr double a0_ = 8.0 / 15.0, a1_ = 5.0 / 12.0, a2_ = 3.0 / 4.0, b1_ = -17.
 constexpr double p1_ = 8.0 / 15.0, p2_ = 2.0 / 3.0;
 
 typedef void (*stage_launch_fn)(const StageArgs&, const DevParams&, int grid, int block, size_t smem, cudaStream_t);
+typedef cudaError_t (*run_launch_fn)(const RunArgs&, int grid, int block, size_t smem, cudaStream_t);
 typedef size_t (*smem_fn)(int warps);
 typedef const void* (*kptr_fn)();
 
@@ -34,6 +35,8 @@ typedef const void* (*kptr_fn)();
 struct Variant {
     stage_launch_fn launch;
     kptr_fn kernel;
+    run_launch_fn run;  // many steps in one cooperative launch
+    kptr_fn run_kernel;
     smem_fn smem;
     int T;          // threads per transform group of the adjoint's layout (Geom)
     int PL;         // partial vector length (doubles)
@@ -113,7 +116,8 @@ inline int stage_teams(int model, int warps) {
     return n > 1 ? n : 1;
 }
 
-// CTA width and grid of a single case's stage kernel: one CTA per SM.  When every team can
+// CTA width and grid of a single case's stage kernel: one CTA per SM, one SM left for the CTA of
+// the mean-field side (run_kernel).  When every team can
 // have its own SM a team gets as many warps as it has inverse transforms (one round of tasks);
 // otherwise a CTA holds the teams that the case has blocks for.
 struct StageGeom {

@@ -15,6 +15,25 @@ template <int NZ, int MODEL, int INTEG>
 const void* stage_ptr() {
     return reinterpret_cast<const void*>(&stage_kernel<NZ, MODEL, INTEG>);
 }
+template <int NZ, int MODEL, int INTEG>
+cudaError_t launch_run(const RunArgs& R, int grid, int block, size_t smem, cudaStream_t st) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;  // all CTAs co-resident, or the launch fails
+    at[0].val.cooperative = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, run_kernel<NZ, MODEL, INTEG>, R);
+}
+template <int NZ, int MODEL, int INTEG>
+const void* run_ptr() {
+    return reinterpret_cast<const void*>(&run_kernel<NZ, MODEL, INTEG>);
+}
 template <int NZ, int MODEL>
 size_t stage_smem(int warps) {
     return wide::WG<NZ, MODEL>::bytes(warps);
@@ -25,6 +44,8 @@ Variant make_variant() {
     Variant v;
     v.launch = &launch_stage<NZ, MODEL, INTEG>;
     v.kernel = &stage_ptr<NZ, MODEL, INTEG>;
+    v.run = &launch_run<NZ, MODEL, INTEG>;
+    v.run_kernel = &run_ptr<NZ, MODEL, INTEG>;
     v.smem = &stage_smem<NZ, MODEL>;
     v.T = Geom<NZ>::T;
     v.PL = wide::WG<NZ, MODEL>::PL;

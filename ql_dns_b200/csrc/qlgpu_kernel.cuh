@@ -36,14 +36,15 @@ __device__ __forceinline__ void put_record(const DevParams& P, const double* ds,
 // ---------------------------------------------------------------------------
 // Mean-field update, run by the whole CTA that arrives last: the mean-field
 // right-hand side from the stress spectra spec[NEMF][H + 1] and its RK update
-// (new values to A.mf and to mfs[nmf][nz] in shared memory), then the time and
+// (mfs[nmf][nz] in shared memory, updated in place, and A.mf; fps: the previous
+// right-hand side), then the time and
 // diagnostic bookkeeping in the last warp.  tot[] holds the stress profiles
 // summed over all modes (real z) followed by the six fluctuation diagnostic sums.
 // ---------------------------------------------------------------------------
 template <class W, int MODEL, int INTEG, int NEMF>
 __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevParams& P, const double* tot,
-                                                  const double* spec, cplx* mfs, double tclock, double t_new,
-                                                  bool last, bool diag_due) {
+                                                  const double* spec, cplx* mfs, const cplx* fps, double tclock,
+                                                  double t_new, bool last, bool diag_due) {
     const StageConst& S = A.sc;
     const int tid = threadIdx.x, lane = tid & 31;
     const int nzd = P.nz;
@@ -62,7 +63,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
         cplx m[4], F[4];
 #pragma unroll
         for (int mm = 0; mm < 4; ++mm) {
-            m[mm] = (mm < P.nmf) ? ldc_cg(A.mf + mm * nzd + s) : mk(0.0, 0.0);
+            m[mm] = (mm < P.nmf) ? mfs[mm * nzd + s] : mk(0.0, 0.0);
             F[mm] = mk(0.0, 0.0);
         }
         if (MODEL == MODEL_BQLIN) {
@@ -86,7 +87,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
                 continue;
             }
             const double Lm = P.ql ? __dmul_rn((MODEL == MODEL_FULLQLIN && mm >= 2) ? P.nu : P.eta, kz2) : 0.0;
-            cplx fp = S.has_prev ? ldc_cg(A.Fmf_prev + mm * nzd + s) : mk(0.0, 0.0);
+            cplx fp = S.has_prev ? fps[mm * nzd + s] : mk(0.0, 0.0);
             cplx nv = rk_update<INTEG>(S, Lm, Lm, F[mm], fp, m[mm], S.has_prev);
             if (A.Fmf_out) stc(A.Fmf_out + mm * nzd + s, F[mm]);
             stc(A.mf + mm * nzd + s, nv);

@@ -47,6 +47,13 @@ struct DevClock {
     int mfr_valid;     // mean-field profiles cache holds the current mean field
     unsigned cnt_group[64];
     unsigned long long nstep;  // steps since the clock was set: the noise counter of the next step
+    int abort;         // a wait of the running launch gave up (run_kernel)
+    // counters of the running launch, each on a line of its own (0 between launches)
+    unsigned pad0[32];
+    unsigned arrive;   // CTAs that have published a stage's partial sums
+    unsigned pad1[32];
+    unsigned epoch;    // stages whose mean-field side is complete
+    unsigned pad2[31];
 };
 
 // Driving noise of one case (Model::DrivingNoise, MHD_BQlin.cpp:558-618 and
@@ -115,6 +122,22 @@ struct StageArgs {
     CnRec* rec_cn;          // the CN old-operator fields at the stage start (null: off)
     const NoiseSpec* noise;  // last stage of a driven batch case: noise after each mode's update (null: off)
     StageConst sc;
+};
+
+// Many steps of a single case in one launch (run_kernel of qlgpu_wide.cuh).
+struct RunArgs {
+    StageArgs A[3];   // the step's stages; lin_in / lin_out / rec_* are set per stage
+    DevParams P;
+    cplx* lin[2];     // the ping-pong fields, lin[cur] the current ones
+    int cur, nsteps;
+    long long wait_ns;  // bound on one wait for the other CTAs
+    // optional record of every stage input (null: off): step n, stage s at rec_lin + (3 n + s) nxy 4 nz,
+    // rec_mf + (3 n + s) nmf nz, rec_cn + 3 n + s, rec_kx + n nxy, rec_t + n
+    cplx* rec_lin;
+    cplx* rec_mf;
+    double* rec_kx;
+    double* rec_t;
+    CnRec* rec_cn;
 };
 
 // ---------------------------------------------------------------------------

@@ -79,7 +79,8 @@ struct WG {
     static constexpr size_t TM_ACC = TM_STG + 16 * (size_t)GPW * 4 * nz;
     static constexpr size_t TEAM_BYTES = TM_ACC + 8 * 256 * (size_t)NE;
     // the mean-field stage's scratch overlays the teams' buffers
-    static constexpr size_t TOP_BYTES = 8 * ((size_t)PL + 2) + 16 * (size_t)NE * (H + 1) + 16 * 4 * (size_t)nz;
+    static constexpr int NMF = BQ ? 2 : 4;             // mean fields
+    static constexpr size_t TOP_BYTES = 8 * ((size_t)PL + 2) + 16 * (size_t)NE * (H + 1) + 16 * 2 * NMF * (size_t)nz;
     static_assert(TOP_BYTES <= 16 * 256 * (size_t)(NINV + NX - 4), "mean-field scratch below its exchange buffers");
     __host__ __device__ static constexpr int teams(int warps) { return warps / TS > 1 ? warps / TS : 1; }
     __host__ __device__ static constexpr size_t bytes(int warps) {
@@ -126,6 +127,24 @@ __device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, do
     }
 }
 
+// The mean-field stage's scratch: tot[PL], spec, the mean fields and their previous
+// right-hand side.  top_prefetch requests the latter two before the sums are read.
+template <class W>
+__device__ __forceinline__ cplx* top_mfs(double* tot) {
+    return reinterpret_cast<cplx*>(tot + W::PL + (W::PL & 1) + 2 * W::NE * (W::H + 1));
+}
+template <class W>
+__device__ __forceinline__ void top_prefetch(const StageArgs& A, double* tot) {
+    cplx* mfs = top_mfs<W>(tot);
+    constexpr int n = W::NMF * W::nz;
+    const bool hp = A.sc.has_prev && !A.rhs_only;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        cp_async16(mfs + i, A.mf + i);
+        if (hp) cp_async16(mfs + n + i, A.Fmf_prev + i);
+    }
+    cp_async_commit();
+}
+
 // Mean-field stage of the CTA that arrived last: tot[PL] holds the stress
 // profiles summed over the modes and the diagnostic sums.  Stress spectra
 // (MHD_BQlin.cpp:228-240 after the sum over modes; the transform is linear), the
@@ -136,7 +155,7 @@ __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
     const int g = lane / W::T, t = lane % W::T;
     double* spec = tot + W::PL + (W::PL & 1);
-    cplx* mfs = reinterpret_cast<cplx*>(spec + 2 * W::NE * (W::H + 1));
+    cplx* mfs = top_mfs<W>(tot);
     // at most four warps transform (their exchange buffers)
     constexpr int NT = (W::NPROF + W::GPW - 1) / W::GPW < 4 ? (W::NPROF + W::GPW - 1) / W::GPW : 4;
     const int ntw = nwarps < NT ? nwarps : NT;
@@ -160,8 +179,10 @@ __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P
             }
         }
     }
+    cp_async_wait_all();
     __syncthreads();
-    mean_field_update<W, MODEL, INTEG, W::NE>(A, P, tot, spec, mfs, tclock, t_new, last, diag_due);
+    mean_field_update<W, MODEL, INTEG, W::NE>(A, P, tot, spec, mfs, mfs + W::NMF * W::nz, tclock, t_new, last,
+                                              diag_due);
     if (A.mfr_cache && !A.rhs_only && warp < ntw)
         mean_profiles8<W, W::BQ>(
             P, [&](int m, int s) { return mfs[m * W::nz + s]; }, A.mfr_cache, xg, tw, warp, ntw, lane);
@@ -525,19 +546,67 @@ __device__ __forceinline__ void side_diag(const DevParams& P, const LaneMode& M,
 
 }  // namespace wide
 
-// Static shared words of a stage: the last-arriver flag.
+// Static shared words of a stage: the last-arriver flag and the gate's answer.
 struct StageShared {
-    int last;
-    int pad[3];
+    int last, ok;
+    int pad[2];
 };
 
+// A case's clock as this CTA follows it through a launch: every CTA advances its own
+// copy by the same operations the mean-field stage applies to DevClock, so only the
+// mean-field profiles have to come from the CTA that ran the mean-field stage.
+struct LocalClock {
+    double t, timevar, t_old, dtlin_old;
+    unsigned long long nstep;
+    int old_init, mfr_valid;
+};
+__device__ __forceinline__ void load_clock(LocalClock& lc, const DevClock* c) {
+    lc.t = __ldcg(&c->t);
+    lc.timevar = __ldcg(&c->timevar);
+    lc.t_old = __ldcg(&c->t_old);
+    lc.dtlin_old = __ldcg(&c->dtlin_old);
+    lc.nstep = __ldcg(&c->nstep);
+    lc.old_init = __ldcg(&c->old_init);
+    lc.mfr_valid = __ldcg(&c->mfr_valid);
+}
+
+// The clock after stage S of a step that started at tclock (what mean_field_update does to DevClock).
+__device__ __forceinline__ void advance_clock(LocalClock& lc, const StageConst& S, const DevParams& P, bool last,
+                                              bool diag_due) {
+    lc.t_old = S.abs_time ? S.t_off : __dadd_rn(lc.t, S.t_off);
+    lc.dtlin_old = S.dt_lin;
+    lc.old_init = 0;
+    lc.mfr_valid = 1;
+    if (!last) return;
+    lc.t = __dadd_rn(lc.t, P.dt);
+    lc.timevar = __dadd_rn(lc.timevar, P.dt);
+    if (diag_due) lc.timevar = __dsub_rn(lc.timevar, P.tv_interval);
+    lc.nstep += 1;
+}
+// A record is due at the end of this stage (main.cpp:117,127-130).
+__device__ __forceinline__ bool record_due(const LocalClock& lc, const DevParams& P, bool last) {
+    return last && P.tv_interval > 0.0 && __dsub_rn(__dadd_rn(lc.timevar, P.dt), P.tv_interval) > -1e-8;
+}
+
+enum StageResult { STAGE_DONE = 0, STAGE_TOP = 1, STAGE_ABORT = 2 };
+
 // One stage over the modes of one case, executed by one CTA that is number
-// `cta` of the `ncta` CTAs working on that case.  Returns true in the one CTA
-// that arrived last and ran the mean-field stage; every other CTA returns as
-// soon as its partial sums are published.
-template <int NZ, int MODEL, int INTEG>
-__device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& P, const int cta, const int ncta,
-                                           unsigned char* smem_raw, StageShared& ss) {
+// `cta` of the `ncta` CTAs working on that case.  STAGE_TOP in the one CTA that
+// arrived last and ran the mean-field stage; every other CTA returns STAGE_DONE
+// as soon as its partial sums are published.
+//
+// A team steps the same blocks in every stage, so a stage's fields, previous
+// right-hand sides and kx0 come from the CTA's own last stage: only the mean-field
+// profiles wait for the other CTAs.  The first block's inverse transforms therefore
+// run before gate() (called by thread 0; false ends the launch), which in a
+// persistent launch waits for the case's previous stage.  fresh: the shared-memory
+// tables do not hold this case's yet.  REDUCER: the launch has a CTA of its own for the
+// mean-field side (reduce_stage); this one only counts itself in at `arrive`.
+template <int NZ, int MODEL, int INTEG, bool REDUCER, class Gate>
+__device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevParams& P, const int cta,
+                                                  const int ncta, unsigned char* smem_raw, StageShared& ss,
+                                                  LocalClock& lc, const bool fresh, unsigned* arrive,
+                                                  Gate&& gate) {
     using namespace wide;
     using W = WG<NZ, MODEL>;
     constexpr int T = W::T, nzd = W::nz, GPW = W::GPW;
@@ -570,17 +639,14 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
         cp_async_commit();
     };
     if (in_team && first < P.nxy) stage_block(first);
-    for (int i = tid; i < NZ; i += blockDim.x) {
-        tw[i] = ldc_cg(A.tw + NZ + i);
-        kzc[i] = kzval(i <= W::H ? i : i - NZ, P.kzL);
-    }
-    const double tclock = __ldcg(&A.clk->t);
-    CnOld cn;
-    cn.t_old = __ldcg(&A.clk->t_old);
-    cn.dtlin_old = __ldcg(&A.clk->dtlin_old);
-    cn.old_init = __ldcg(&A.clk->old_init);
-    const double timevar = __ldcg(&A.clk->timevar);
-    const bool cached = A.mfr_cache && !A.rhs_only && __ldcg(&A.clk->mfr_valid);
+    const double tclock = lc.t;
+    const CnOld cn{lc.t_old, lc.dtlin_old, lc.old_init};
+    const bool cached = A.mfr_cache && !A.rhs_only && lc.mfr_valid;
+    if (fresh)
+        for (int i = tid; i < NZ; i += blockDim.x) {
+            tw[i] = ldc_cg(A.tw + NZ + i);
+            kzc[i] = kzval(i <= W::H ? i : i - NZ, P.kzL);
+        }
     if (INTEG == INTEG_EXP) {
         // factored integrating factor: exp(linC c kz2) per stored kz
         for (int s = tid; s < nzd; s += blockDim.x) {
@@ -594,71 +660,33 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
             }
         }
     }
-    if (cached)
-        for (int i = tid; i < W::NPROF * NZ; i += blockDim.x) prof[i] = __ldcg(A.mfr_cache + i);
     if (in_team)
         for (int i = wt * 32 + lane; i < 256 * W::NE; i += bthreads) acc[i] = 0.0;
     for (int i = tid; i < 6 * MAX_WARPS; i += blockDim.x) dred[i] = 0.0;
-    __syncthreads();
-    if (!cached) {
-        // scratch: the result buffers of the first team, which nothing uses yet
-        cplx* r0 = reinterpret_cast<cplx*>(smem_raw + W::o_team);
-        const int nw = warps < 8 ? warps : 8;
-        if (warp < nw)
-            mean_profiles8<W, W::BQ>(
-                P, [&](int m, int s) { return ldc_cg(A.mf + m * nzd + s); }, prof, r0 + 256 * (warp & 7), tw, warp, nw,
-                lane);
-        __syncthreads();
-    }
+    if (fresh) __syncthreads();
     if (tr) A.trace[1] = gtimer();
 
     // Last-stage bookkeeping identical in every CTA (main.cpp:111-130)
     const double t_new = __dadd_rn(tclock, P.dt);
     const bool last = S.last && !A.rhs_only;
-    bool diag_due = false;
-    if (last && P.tv_interval > 0.0)
-        diag_due = __dsub_rn(__dadd_rn(timevar, P.dt), P.tv_interval) > -1e-8;
+    const bool diag_due = record_due(lc, P, last);
     const double qt = __dmul_rn(P.q, t_new);
     const double ts = S.abs_time ? S.t_off : __dadd_rn(tclock, S.t_off);
 
-    // ---- optional record of the stage input (the adjoint's window recompute): CTA 0 of the
-    // case copies the mean fields and, in a step's first stage, kx0 and the clock; stable
-    // here because the previous stage (and its remap) completed before any CTA started this one
-    if (A.rec_mf && cta == 0) {
-        const int nmfe = P.nmf * nzd;
-        for (int i = tid; i < nmfe; i += blockDim.x) A.rec_mf[i] = ldc(A.mf + i);
-        if (A.rec_kx)
-            for (int i = tid; i < P.nxy; i += blockDim.x) A.rec_kx[i] = __ldcg(A.kx0 + i);
-        if (A.rec_t && tid == 0) A.rec_t[0] = tclock;
-        if (A.rec_cn && tid == 0) {
-            A.rec_cn->t_old = cn.t_old;
-            A.rec_cn->dtlin_old = cn.dtlin_old;
-            A.rec_cn->old_init = cn.old_init;
-        }
-    }
-
     // ---- the team's blocks of GPW modes
     const bool has_prev = A.Fprev && S.has_prev;
-    for (int base = first; in_team && base < P.nxy; base += step) {
-        const int nv = min(GPW, P.nxy - base);
+    for (int base = first;; base += step) {
+        const bool active = in_team && base < P.nxy;
+        if (!active && base != first) break;
+        const int nv = active ? min(GPW, P.nxy - base) : 1;
         LaneMode M;
-        M.valid = g < nv;
-        M.m = QLGPU_CHECK_INDEX(base + min(g, nv - 1), P.nxy, &A.clk->status);
+        M.valid = active && g < nv;
+        M.m = QLGPU_CHECK_INDEX(active ? base + min(g, nv - 1) : 0, P.nxy, &A.clk->status);
         const cplx* stg = stg_all + (size_t)min(g, nv - 1) * 4 * nzd;
         M.b = __ldg(A.ky + M.m);
         M.kx0 = __ldcg(A.kx0 + M.m);
         M.kyi = __ldg(A.kyi + M.m);
         M.kxi = __ldg(A.kxi + M.m);
-        if (base != first) stage_block(base);
-        if (wt == 0 && lane == 0) {
-            // the next block's fields and this and the next block's previous rhs into L2
-            const size_t nb = (size_t)base + step;
-            if (nb < (size_t)P.nxy) {
-                const unsigned bytes = 64u * nzd * (unsigned)min(GPW, P.nxy - (int)nb);
-                l2_prefetch(A.lin_in + nb * 4 * nzd, bytes);
-                if (has_prev) l2_prefetch(A.Fprev + nb * 4 * nzd, bytes);
-            }
-        }
         M.a = kx_at(M.kx0, P.q, ts, M.b);  // kx(t_s), MHD_BQlin.cpp:498
         M.mult = M.valid ? (M.b == 0.0 ? 1.0 : 2.0) : 0.0;
         M.kxe = __dadd_rn(M.a, __dmul_rn(__dmul_rn(P.q, S.dt_lin), M.b));  // MHD_BQlin.cpp:248
@@ -669,34 +697,82 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
         }
         // ShearingBox_Remap(q t) after t += dt (main.cpp:122-123, MHD_BQlin.cpp:319-329)
         M.zero = last && P.remap && __dadd_rn(M.kx0, __dmul_rn(qt, M.b)) > P.remap_thresh;
-        const double* __restrict__ il2 = A.ilap2 + (size_t)M.kyi * nzd;
-        cp_async_wait_all();
-        team_sync(bar, bthreads);
-        if (A.rec_lin) {  // record the block's input fields
-            cplx* dst = A.rec_lin + (size_t)base * 4 * nzd;
-            for (int i = wt * 32 + lane; i < nv * 4 * nzd; i += bthreads) dst[i] = stg_all[i];
-        }
-        // ---- inverse transforms
-#pragma unroll 1
-        for (int task = wt; task < W::NINV; task += tws) {
-            int kind, side;
-            if (W::BQ) {
-                side = (task == R_BZ || task == R_B || task == R_ET || task == R_BY);
-                kind = (task == R_UZ || task == R_BZ) ? 1 : task == R_DUZ ? 2 : (task == R_UY || task == R_BY) ? 3 : 0;
-            } else {
-                side = (task >= Q_BX && task <= Q_BZ) || task >= Q_DBX;
-                kind = (task == Q_UX || task == Q_BX) ? 0 : (task == Q_UY || task == Q_BY) ? 3
-                     : (task == Q_UZ || task == Q_BZ) ? 1 : (task == Q_DUX || task == Q_DBX) ? 4 : 5;
+        if (active) {
+            if (base != first) stage_block(base);
+            if (wt == 0 && lane == 0) {
+                // the next block's fields and previous rhs into L2
+                const size_t nb = (size_t)base + step;
+                if (nb < (size_t)P.nxy) {
+                    const unsigned bytes = 64u * nzd * (unsigned)min(GPW, P.nxy - (int)nb);
+                    l2_prefetch(A.lin_in + nb * 4 * nzd, bytes);
+                    if (has_prev) l2_prefetch(A.Fprev + nb * 4 * nzd, bytes);
+                }
             }
-            const int f0 = 2 * side + (W::BQ && (task == R_ZE || task == R_ET) ? 1 : 0);
-            cplx x[8];
-            inv_input<W>(x, stg + f0 * nzd, il2, kind, M.a, M.b, P.fac, kzc, t);
-            cplx* xb = R + (size_t)task * 256;
-            xform<W>(x, xb, tw, g, t);
+            const double* __restrict__ il2 = A.ilap2 + (size_t)M.kyi * nzd;
+            cp_async_wait_all();
+            team_sync(bar, bthreads);
+            if (A.rec_lin) {  // record the block's input fields
+                cplx* dst = A.rec_lin + (size_t)base * 4 * nzd;
+                for (int i = wt * 32 + lane; i < nv * 4 * nzd; i += bthreads) dst[i] = stg_all[i];
+            }
+            // ---- inverse transforms
+#pragma unroll 1
+            for (int task = wt; task < W::NINV; task += tws) {
+                int kind, side;
+                if (W::BQ) {
+                    side = (task == R_BZ || task == R_B || task == R_ET || task == R_BY);
+                    kind = (task == R_UZ || task == R_BZ) ? 1 : task == R_DUZ ? 2
+                         : (task == R_UY || task == R_BY) ? 3 : 0;
+                } else {
+                    side = (task >= Q_BX && task <= Q_BZ) || task >= Q_DBX;
+                    kind = (task == Q_UX || task == Q_BX) ? 0 : (task == Q_UY || task == Q_BY) ? 3
+                         : (task == Q_UZ || task == Q_BZ) ? 1 : (task == Q_DUX || task == Q_DBX) ? 4 : 5;
+                }
+                const int f0 = 2 * side + (W::BQ && (task == R_ZE || task == R_ET) ? 1 : 0);
+                cplx x[8];
+                inv_input<W>(x, stg + f0 * nzd, il2, kind, M.a, M.b, P.fac, kzc, t);
+                cplx* xb = R + (size_t)task * 256;
+                xform<W>(x, xb, tw, g, t);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) xb[32 * r + lane] = x[r];
+                for (int r = 0; r < 8; ++r) xb[32 * r + lane] = x[r];
+            }
         }
-        team_sync(bar, bthreads);
+        if (base == first) {
+            // ---- the mean field of this stage
+            if (tid == 0) ss.ok = gate() ? 1 : 0;
+            __syncthreads();
+            if (!ss.ok) return STAGE_ABORT;
+            if (tr) A.trace[6] = gtimer();
+            if (cached) {
+                for (int i = tid; i < W::NPROF * NZ; i += blockDim.x) prof[i] = __ldcg(A.mfr_cache + i);
+            } else {
+                // scratch: the forward tasks' exchange buffers of the first team
+                cplx* r0 = reinterpret_cast<cplx*>(smem_raw + W::o_team) + 256 * W::NINV;
+                const int nw = warps < W::NX ? warps : W::NX;
+                if (warp < nw)
+                    mean_profiles8<W, W::BQ>(
+                        P, [&](int m, int s) { return ldc_cg(A.mf + m * nzd + s); }, prof, r0 + 256 * warp, tw, warp,
+                        nw, lane);
+            }
+            // optional record of the stage input (the adjoint's window recompute): CTA 0 of the case
+            // copies the mean fields and, in a step's first stage, kx0 and the clock
+            if (A.rec_mf && cta == 0) {
+                for (int i = tid; i < P.nmf * nzd; i += blockDim.x) A.rec_mf[i] = ldc(A.mf + i);
+                if (A.rec_kx)
+                    for (int i = tid; i < P.nxy; i += blockDim.x) A.rec_kx[i] = __ldcg(A.kx0 + i);
+                if (A.rec_t && tid == 0) A.rec_t[0] = tclock;
+                if (A.rec_cn && tid == 0) {
+                    A.rec_cn->t_old = cn.t_old;
+                    A.rec_cn->dtlin_old = cn.dtlin_old;
+                    A.rec_cn->old_init = cn.old_init;
+                }
+            }
+            __syncthreads();
+            if (tr) A.trace[7] = gtimer();
+            if (!active) break;
+        } else {
+            team_sync(bar, bthreads);
+        }
         // ---- products, forward transforms, stresses
         if constexpr (W::BQ) {
 #pragma unroll 1
@@ -730,8 +806,8 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
             if (A.noise) {
                 // Model::DrivingNoise after the step (main.cpp:111-113), before the diagnostics see it
                 if (M.valid && !M.zero)
-                    noise_mode(A.noise, __ldcg(&A.clk->nstep), uo, nzd, wt * T + t, tws * T, M.m, M.kx0, M.b, M.kxi,
-                               M.kyi, P.q, tclock, P.kzL);
+                    noise_mode(A.noise, lc.nstep, uo, nzd, wt * T + t, tws * T, M.m, M.kx0, M.b, M.kxi, M.kyi, P.q,
+                               tclock, P.kzL);
                 team_sync(bar, bthreads);
             }
             if (diag_due) {
@@ -770,10 +846,19 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
         part[W::NE * NZ + tid] = s;
     }
 
+    __syncthreads();
+    if (tr) A.trace[3] = gtimer();
+    if (tid == 0 && !A.rhs_only) advance_clock(lc, S, P, last, diag_due);
+    if (REDUCER) {
+        if (tid == 0) {
+            __threadfence();  // covers the CTA's stores, ordered before it by the barrier
+            atomicAdd(arrive, 1u);
+        }
+        return STAGE_DONE;
+    }
     // ---- two-level last-arriver reduction
     __threadfence();
     __syncthreads();
-    if (tr) A.trace[3] = gtimer();
     const int ngroups = (ncta + RED_GROUP - 1) / RED_GROUP;
     const int grp = QLGPU_CHECK_INDEX(cta / RED_GROUP, 64, &A.clk->status);  // DevClock::cnt_group
     const int c0 = grp * RED_GROUP;
@@ -783,9 +868,10 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
         ss.last = (tk == (unsigned)(cn_in - 1));
     }
     __syncthreads();
-    if (!ss.last) return false;
+    if (!ss.last) return STAGE_DONE;
     __threadfence();
     double* tot = reinterpret_cast<double*>(smem_raw + W::o_team);
+    top_prefetch<W>(A, tot);
     if (ngroups > 1) {
         double* gpart = A.gpartials + (size_t)grp * W::PL;
         for (int idx = tid; idx < W::PL; idx += blockDim.x) {
@@ -807,7 +893,11 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
             ss.last = (tk == (unsigned)(ngroups - 1));
         }
         __syncthreads();
-        if (!ss.last) return false;
+        if (!ss.last) {
+            cp_async_wait_all();  // the scratch is reused by the next stage
+            __syncthreads();
+            return STAGE_DONE;
+        }
         __threadfence();
         for (int idx = tid; idx < W::PL; idx += blockDim.x) {
             double s = 0.0;
@@ -843,16 +933,176 @@ __device__ __forceinline__ bool stage_body(const StageArgs& A, const DevParams& 
     cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team) + 256 * (size_t)(W::NINV + W::NX - 4);
     wide::top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, tclock, t_new, last, diag_due);
     if (A.trace && tid == 0) A.trace[5] = gtimer();
-    return true;
+    return STAGE_TOP;
 }
 
-// One stage launch of a single case.
+// One stage launch of a single case (Model::rhs, timed stages, host-controlled steps).
 template <int NZ, int MODEL, int INTEG>
 __global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) stage_kernel(const __grid_constant__ StageArgs A,
                                                                        const __grid_constant__ DevParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StageShared ss;
-    stage_body<NZ, MODEL, INTEG>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss);
+    __shared__ LocalClock lc;
+    if (threadIdx.x == 0) load_clock(lc, A.clk);
+    __syncthreads();
+    stage_body<NZ, MODEL, INTEG, false>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss, lc, true, nullptr,
+                                        [] { return true; });
+}
+
+// ---------------------------------------------------------------------------
+// Stage counters shared by the CTAs of one launch (a case's mean field)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ int ld_volatile_i32(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
+
+// Wait (one thread) until *p >= target.  False when the launch was aborted or the wait
+// exceeded wait_ns; the caller's CTA then leaves, and the abort word makes the others leave.
+__device__ __forceinline__ bool run_wait(const unsigned* p, unsigned target, DevClock* C, long long wait_ns) {
+    const unsigned long long t0 = gtimer();
+    // at least ~16 ns per iteration: the cap ends the wait even if the timer misbehaves
+    const long long max_iter = wait_ns / 16 + 1024;
+    for (long long it = 0; it < max_iter; ++it) {
+        if (ld_acquire_u32(p) >= target) return true;
+        if ((it & 63) == 63) {
+            if (ld_volatile_i32(&C->abort)) return false;
+            if ((long long)(gtimer() - t0) > wait_ns) break;
+        }
+    }
+    atomicOr(&C->status, QLGPU_STATUS_TIMEOUT);
+    atomicExch(&C->abort, 1);
+    return false;
+}
+
+// The mean-field side of one stage in the reducer CTA: the partial sums of all `ncta`
+// CTAs, in the order of the two-level reduction (CTAs within a group of RED_GROUP, then
+// the groups), then the mean-field stage.
+template <int NZ, int MODEL, int INTEG>
+__device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams& P, int ncta,
+                                             unsigned char* smem_raw, const cplx* tw, LocalClock& lc) {
+    using namespace wide;
+    using W = WG<NZ, MODEL>;
+    const int tid = threadIdx.x, nth = blockDim.x;
+    const bool last = A.sc.last != 0, diag_due = record_due(lc, P, last);
+    const double tclock = lc.t, t_new = __dadd_rn(tclock, P.dt);
+    double* tot = reinterpret_cast<double*>(smem_raw + W::o_team);
+    // group sums beside the scratch where they fit, else through L2
+    constexpr int MAXG = (int)((W::TEAM_BYTES - W::TOP_BYTES - 16) / (8 * (size_t)W::PL));
+    const int ngroups = (ncta + RED_GROUP - 1) / RED_GROUP;
+    double* gs = ngroups <= MAXG ? reinterpret_cast<double*>(smem_raw + W::o_team + ((W::TOP_BYTES + 15) & ~(size_t)15))
+                                 : A.gpartials;
+    if (ngroups == 1) gs = tot;
+    top_prefetch<W>(A, tot);
+    for (int i0 = tid; i0 < ngroups * W::PL; i0 += 2 * nth) {
+        // two (group, value) pairs at a time, all their loads in flight
+        double v[2][RED_GROUP];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = i0 + h * nth, q = i / W::PL, idx = i - q * W::PL;
+            const int n = i < ngroups * W::PL ? min(RED_GROUP, ncta - q * RED_GROUP) : 0;
+            const double* src = A.partials + (size_t)q * RED_GROUP * W::PL + idx;
+#pragma unroll
+            for (int u = 0; u < RED_GROUP; ++u) v[h][u] = u < n ? __ldcg(src + (size_t)u * W::PL) : 0.0;
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int i = i0 + h * nth;
+            if (i >= ngroups * W::PL) break;
+            const int n = min(RED_GROUP, ncta - i / W::PL * RED_GROUP);
+            double s = 0.0;
+#pragma unroll
+            for (int u = 0; u < RED_GROUP; ++u)
+                if (u < n) s += v[h][u];
+            gs[i] = s;
+        }
+    }
+    __syncthreads();
+    if (ngroups > 1) {
+        for (int idx = tid; idx < W::PL; idx += nth) {
+            double s = 0.0;
+            for (int q = 0; q < ngroups; ++q) s += gs[(size_t)q * W::PL + idx];
+            tot[idx] = s;
+        }
+        __syncthreads();
+    }
+    if (A.trace && tid == 0) A.trace[4] = gtimer();
+    cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team) + 256 * (size_t)(W::NINV + W::NX - 4);
+    top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, tclock, t_new, last, diag_due);
+    if (tid == 0) advance_clock(lc, A.sc, P, last, diag_due);
+    if (A.trace && tid == 0) A.trace[5] = gtimer();
+}
+
+// Many steps of a single case in one cooperative launch.  Worker CTAs step their blocks
+// stage after stage; the last CTA has no modes and runs the mean-field side, so that its
+// chain (sums, two transforms, update, profiles: 4 us) runs under the workers' first
+// inverse transforms of the next stage instead of in a worker that would then be the
+// last one to arrive again.  Against three launches per step this saves the launch gap,
+// the tables and the round trips of profiles and clock.  Every wait is bounded in time
+// and iterations; one that gives up sets QLGPU_STATUS_TIMEOUT and the abort word, and
+// every CTA leaves.
+template <int NZ, int MODEL, int INTEG>
+__global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) run_kernel(const __grid_constant__ RunArgs L) {
+    using W = wide::WG<NZ, MODEL>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ StageShared ss;
+    __shared__ LocalClock lc;
+    __shared__ __align__(16) StageArgs sA[3];
+    const int tid = threadIdx.x, ncta = (int)gridDim.x - 1;
+    const bool reducer = (int)blockIdx.x == ncta;
+    DevClock* C = L.A[0].clk;
+    for (int i = tid; i < (int)(sizeof(sA) / 8); i += blockDim.x)
+        reinterpret_cast<unsigned long long*>(sA)[i] = reinterpret_cast<const unsigned long long*>(L.A)[i];
+    if (tid == 0) load_clock(lc, C);
+    unsigned k = 0;  // stages before this one in the launch
+    if (reducer) {
+        cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
+        for (int i = tid; i < NZ; i += blockDim.x) tw[i] = ldc_cg(L.A[0].tw + NZ + i);
+        for (int n = 0; n < L.nsteps; ++n)
+            for (int s = 0; s < 3; ++s, ++k) {
+                __syncthreads();
+                if (tid == 0) ss.ok = run_wait(&C->arrive, (k + 1) * (unsigned)ncta, C, L.wait_ns) ? 1 : 0;
+                __syncthreads();
+                if (!ss.ok) return;
+                reduce_stage<NZ, MODEL, INTEG>(sA[s], L.P, ncta, smem_raw, tw, lc);
+                if (tid == 0) {
+                    __threadfence();
+                    // after the last stage nobody waits any more: ready for the next launch
+                    const bool end = n == L.nsteps - 1 && s == 2;
+                    if (end) C->arrive = 0;
+                    st_release_u32(&C->epoch, end ? 0u : k + 1);
+                }
+            }
+        return;
+    }
+    const size_t nlin = (size_t)L.P.nxy * 4 * L.P.nz, nmfe = (size_t)L.P.nmf * L.P.nz;
+    for (int n = 0; n < L.nsteps; ++n)
+        for (int s = 0; s < 3; ++s, ++k) {
+            __syncthreads();
+            if (tid == 0) {
+                StageArgs& A = sA[s];
+                const int in = (int)((k + (unsigned)L.cur) & 1u);
+                A.lin_in = L.lin[in];
+                A.lin_out = L.lin[in ^ 1];
+                if (L.rec_lin) {
+                    A.rec_lin = L.rec_lin + (size_t)k * nlin;
+                    A.rec_mf = L.rec_mf + (size_t)k * nmfe;
+                    A.rec_kx = s == 0 ? L.rec_kx + (size_t)n * L.P.nxy : nullptr;
+                    A.rec_t = s == 0 ? L.rec_t + n : nullptr;
+                    A.rec_cn = L.rec_cn ? L.rec_cn + k : nullptr;
+                }
+            }
+            __syncthreads();
+            const StageResult r = stage_body<NZ, MODEL, INTEG, true>(
+                sA[s], L.P, (int)blockIdx.x, ncta, smem_raw, ss, lc, k == 0, &C->arrive,
+                [&]() -> bool { return run_wait(&C->epoch, k, C, L.wait_ns); });
+            if (r == STAGE_ABORT) return;
+        }
 }
 
 }  // namespace qlgpu

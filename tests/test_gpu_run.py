@@ -1,0 +1,47 @@
+"""The stage kernel's warp teams and the many-steps launch at the edges of their layout.
+
+A team steps 256/NZ modes at once; a CTA holds one to three teams; the sums over CTAs run in
+groups of 16.  The mode counts below give one mode, a ragged block, one CTA more than a group,
+two teams per CTA and several blocks per team.  Tolerance against the oracle: the 1e-10 bar of
+the step (relative L2 of the state).  One launch of n steps and n launches of one step run the
+same kernel on the same sums, so their states agree bit for bit.
+"""
+import numpy as np
+import pytest
+
+from gpu_util import rel, require_gpu
+from oracle import oracle as O
+from ql_dns_b200.initial import initial_state
+from ql_dns_b200.params import QLParams
+from ql_dns_b200.solver import QLSolver
+
+pytestmark = pytest.mark.gpu
+
+# (nx, ny, NZ): (nx - 1) * ny / 2 modes
+EDGES = [(2, 2, 128), (4, 2, 128), (12, 6, 128), (36, 18, 128), (32, 40, 128), (2, 2, 16), (36, 2, 16), (34, 32, 16),
+         (18, 2, 256), (20, 34, 256), (10, 8, 32), (36, 34, 64)]
+
+
+@pytest.mark.parametrize("integ", [0, 1])
+@pytest.mark.parametrize("model", [0, 1])
+@pytest.mark.parametrize("nx,ny,NZ", EDGES)
+def test_layout_edges(nx, ny, NZ, model, integ):
+    require_gpu()
+    p = QLParams(model=model, integrator=integ, nx=nx, ny=ny, NZ=NZ, dt=0.02, B0z=0.02 if model else 0.0)
+    lin, mf, kx0 = initial_state(p, 3, sigma=0.2, B0=0.05, mean_u=0.02 if model else 0.0)
+    n = 3
+    with QLSolver(p) as s:
+        s.set_state(0.0, lin, mf, kx0)
+        rec = s.step(n, diag_every=1)
+        t, lo, mo, ko = s.get_state()
+        s.set_state(0.0, lin, mf, kx0)
+        for _ in range(n):
+            s.step(1)
+        t1, l1, m1, k1 = s.get_state()
+    assert t == t1 and np.array_equal(lo, l1) and np.array_equal(mo, m1) and np.array_equal(ko, k1)
+    t2, lo2, mo2, ko2, d2 = O.run(p, 0.0, lin, mf, kx0, n, diag_every=1)
+    assert t == t2 and np.array_equal(ko, ko2)
+    assert rel(mo, mo2) < 1e-10
+    assert rel(lo, lo2) < 1e-10 if np.linalg.norm(lo2) else not lo.any()
+    scale = np.abs(d2[1:, 1:13]).max(0)
+    assert np.all(np.abs(rec[:, 1:13] - d2[1:, 1:13]) <= 1e-10 * scale)
