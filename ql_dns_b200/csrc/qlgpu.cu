@@ -442,7 +442,7 @@ static int step_forced(qlgpu_t* h, int nsteps, int diag_every, double* diag_out,
     for (int n = 0; n < nsteps && rc == QLGPU_OK; ++n) {
         double dt = h->p.dt;
         if (h->cfl > 0) {
-            mf_absmax2_kernel<<<1, 256, 0, h->stream>>>(h->d_mf, 1, h->nz, h->NZ, fac, h->d_forcing + 4);
+            mf_absmax2_kernel<<<1, MF_THREADS, 0, h->stream>>>(h->d_mf, h->nz, h->NZ, fac, h->d_forcing + 4);
             double m[8];
             QLGPU_CK(cudaMemcpyAsync(m, h->d_forcing, sizeof(m), cudaMemcpyDeviceToHost, h->stream));
             QLGPU_CK(cudaStreamSynchronize(h->stream));
@@ -463,7 +463,7 @@ static int step_forced(qlgpu_t* h, int nsteps, int diag_every, double* diag_out,
         }
         qlgpu_enqueue_step(h, nullptr, [&](int s) {
             if (s == 2 && h->cfl > 0)
-                mf_absmax2_kernel<<<1, 256, 0, h->stream>>>(h->d_mf, h->nmf, h->nz, h->NZ, fac, h->d_forcing);
+                mf_absmax2_kernel<<<h->nmf, MF_THREADS, 0, h->stream>>>(h->d_mf, h->nz, h->NZ, fac, h->d_forcing);
         });
         if (h->noise_f != 0.0) {
             NoiseArgs a;

@@ -91,9 +91,11 @@ struct Item {
 };
 
 struct CostModel {
-    double alpha = 12.0;                              // us per stage, per launch
-    double beta = 2.5;                                // us per work item per stage
-    double r[NCLASS] = {4.0, 6.0, 14.0, 30.0, 70.0};  // us per pipeline pass, per NZ class
+    // defaults as fitted on a B200 (12 MHD_FullQlin or MHD_BQlin cases of the ensemble law: a pass
+    // is 256 points per team at every NZ, so its cost hardly depends on the class)
+    double alpha = 20.0;                               // us per stage, per launch
+    double beta = 8.0;                                 // us per work item per stage
+    double r[NCLASS] = {9.5, 9.5, 9.8, 12.5, 16.0};    // us per pipeline pass, per NZ class
 };
 
 // Zeroes the launch control words, the case stage counters and the reduction
