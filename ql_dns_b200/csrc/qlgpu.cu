@@ -344,7 +344,7 @@ int qlgpu_destroy(qlgpu_t* h) {
     void* bufs[] = {h->d_lin[0], h->d_lin[1], h->d_F1, h->d_F2, h->d_mf, h->d_Fmf1, h->d_Fmf2,
                     h->d_kx0, h->d_ky, h->d_kxi, h->d_kyi, h->d_tw, h->d_partials, h->d_gpartials,
                     h->d_clk, h->d_diag, h->d_out15, h->d_linop, h->d_ilap2, h->d_trace,
-                    h->d_mfr, h->d_ekz, h->d_forcing, h->d_kx0_prev, h->d_dbg};
+                    h->d_mfr, h->d_ekz, h->d_forcing, h->d_kx0_prev, h->d_dbg, h->adj_ws, h->adj_tab};
     for (void* b : bufs)
         if (b) cudaFree(b);
     for (cudaEvent_t e : h->ev)

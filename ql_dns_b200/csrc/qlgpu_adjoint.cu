@@ -23,70 +23,42 @@ using namespace qlgpu;
 namespace {
 
 struct AdjOps {
-    void (*mf_pre)(const AdjMfArgs&, const DevParams&, cudaStream_t);
-    void (*modes)(const AdjStageArgs&, const DevParams&, int nxy, cudaStream_t);
-    void (*mf_post)(const double*, const cplx*, const DevParams&, cplx*, cudaStream_t);
-    void (*jgrad)(const cplx*, const double*, const double*, const int*, const double*, const DevParams&, double,
-                  const double*, double, cplx*, cudaStream_t);
+    cudaError_t (*modes)(const AdjShared&, const DevParams&, const AdjPos&, int ns, int threads, cudaStream_t);
+    cudaError_t (*mf)(const AdjShared&, const DevParams&, const AdjPos&, const AdjPos&, int post, int pre, int ns,
+                      cudaStream_t);
     const void* modes_kernel;
     size_t modes_smem;
-    // one launch for all seeds of a batch (seed = blockIdx.y)
-    void (*mf_pre_s)(const AdjMfArgs&, const DevParams&, const AdjRevPos&, int, cudaStream_t);
-    void (*modes_s)(const AdjStageArgs&, const DevParams&, const AdjRevPos&, int nxy, int, cudaStream_t);
-    void (*mf_post_s)(const cplx*, const DevParams&, const AdjRevPos&, int, cudaStream_t);
-    void (*jgrad_s)(const double*, const int*, const double*, const DevParams&, const AdjRevPos&, int, cudaStream_t);
-    const void* modes_seeds_kernel;
 };
 
-template <int NZ>
-void ops_mf_pre(const AdjMfArgs& A, const DevParams& P, cudaStream_t st) {
-    adj_mf_pre_kernel<NZ><<<1, 128, 0, st>>>(A, P);
+// A launch that may start while the kernel before it runs (the kernels wait where they
+// need its results).
+template <class... KA, class... Args>
+cudaError_t launch_pdl(void (*kern)(KA...), dim3 grid, int block, size_t smem, cudaStream_t st, const Args&... args) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 template <int NZ>
-void ops_modes(const AdjStageArgs& A, const DevParams& P, int nxy, cudaStream_t st) {
-    adj_modes_kernel<NZ><<<nxy, AdjGeom<NZ>::THREADS, AdjGeom<NZ>::BYTES, st>>>(A, P);
+cudaError_t ops_modes(const AdjShared& H, const DevParams& P, const AdjPos& X, int ns, int threads, cudaStream_t st) {
+    return launch_pdl(adj_modes_kernel<NZ>, dim3((unsigned)H.nchunk, (unsigned)ns), threads, AG<NZ>::BYTES, st, H, P, X);
 }
 template <int NZ>
-void ops_mf_post(const double* bsum, const cplx* tw, const DevParams& P, cplx* lamB, cudaStream_t st) {
-    adj_mf_post_kernel<NZ><<<1, 64, 0, st>>>(bsum, tw, P, lamB);
-}
-template <int NZ>
-void ops_jgrad(const cplx* U, const double* kx0, const double* ky, const int* kyi, const double* il2,
-               const DevParams& P, double t, const double* t_dev, double w, cplx* lam, cudaStream_t st) {
-    adj_jgrad_kernel<NZ><<<148, 256, 0, st>>>(U, kx0, ky, kyi, il2, P, t, t_dev, w, lam);
-}
-template <int NZ>
-void ops_mf_pre_s(const AdjMfArgs& M, const DevParams& P, const AdjRevPos& X, int ns, cudaStream_t st) {
-    adj_mf_pre_seeds_kernel<NZ><<<dim3(1, ns), 128, 0, st>>>(M, P, X);
-}
-template <int NZ>
-void ops_modes_s(const AdjStageArgs& A, const DevParams& P, const AdjRevPos& X, int nxy, int ns, cudaStream_t st) {
-    adj_modes_seeds_kernel<NZ><<<dim3(nxy, ns), AdjGeom<NZ>::THREADS, AdjGeom<NZ>::BYTES, st>>>(A, P, X);
-}
-template <int NZ>
-void ops_mf_post_s(const cplx* tw, const DevParams& P, const AdjRevPos& X, int ns, cudaStream_t st) {
-    adj_mf_post_seeds_kernel<NZ><<<dim3(1, ns), 64, 0, st>>>(tw, P, X);
-}
-template <int NZ>
-void ops_jgrad_s(const double* ky, const int* kyi, const double* il2, const DevParams& P, const AdjRevPos& X, int ns,
-                 cudaStream_t st) {
-    adj_jgrad_seeds_kernel<NZ><<<dim3(148, ns), 256, 0, st>>>(ky, kyi, il2, P, X);
+cudaError_t ops_mf(const AdjShared& H, const DevParams& P, const AdjPos& X, const AdjPos& Y, int post, int pre, int ns,
+                   cudaStream_t st) {
+    return launch_pdl(adj_mf_kernel<NZ>, dim3(1, (unsigned)ns), ADJ_MF_THREADS, 0, st, H, P, X, Y, post, pre);
 }
 template <int NZ>
 AdjOps make_ops() {
-    AdjOps o;
-    o.mf_pre = &ops_mf_pre<NZ>;
-    o.modes = &ops_modes<NZ>;
-    o.mf_post = &ops_mf_post<NZ>;
-    o.jgrad = &ops_jgrad<NZ>;
-    o.modes_kernel = reinterpret_cast<const void*>(&adj_modes_kernel<NZ>);
-    o.modes_smem = AdjGeom<NZ>::BYTES;
-    o.mf_pre_s = &ops_mf_pre_s<NZ>;
-    o.modes_s = &ops_modes_s<NZ>;
-    o.mf_post_s = &ops_mf_post_s<NZ>;
-    o.jgrad_s = &ops_jgrad_s<NZ>;
-    o.modes_seeds_kernel = reinterpret_cast<const void*>(&adj_modes_seeds_kernel<NZ>);
-    return o;
+    return AdjOps{&ops_modes<NZ>, &ops_mf<NZ>, reinterpret_cast<const void*>(&adj_modes_kernel<NZ>), AG<NZ>::BYTES};
 }
 bool pick_ops(int NZ, AdjOps* o) {
     switch (NZ) {
@@ -117,25 +89,31 @@ static_assert(offsetof(DevClock, dtlin_old) == offsetof(DevClock, t_old) + 8 &&
         if (e_ != cudaSuccess) return afail(h, QLGPU_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// Device allocations of one call, freed on every exit path.
-struct Pool {
-    std::vector<void*> ptrs;
-    ~Pool() {
-        for (void* p : ptrs) cudaFree(p);
-    }
+// The workspace of a handle's adjoint calls: one device block as large as the checkpoints and
+// one window's records ask for, cut into the call's buffers in two passes, sizes first.  A
+// block of at most ADJ_KEEP_BYTES stays with the handle for its next call and is freed with
+// it (25 allocations, clears and frees per seed and call took more than half of a 100-step
+// call of 16 seeds); a larger one is given back at the end of the call.
+constexpr size_t ADJ_KEEP_BYTES = (size_t)512 << 20;
+
+void adj_trim(qlgpu_t* h) {
+    if (!h || h->adj_bytes <= ADJ_KEEP_BYTES) return;
+    cudaStreamSynchronize(h->stream);
+    cudaFree(h->adj_ws);
+    h->adj_ws = nullptr;
+    h->adj_bytes = 0;
+}
+
+struct Arena {
+    size_t used = 0;
+    unsigned char* base = nullptr;
     template <class T>
-    cudaError_t get(T** out, size_t count) {
-        void* p = nullptr;
-        cudaError_t e = cudaMalloc(&p, sizeof(T) * (count ? count : 1));
-        if (e == cudaSuccess) {
-            ptrs.push_back(p);
-            e = cudaMemset(p, 0, sizeof(T) * (count ? count : 1));
-        }
-        *out = static_cast<T*>(p);
-        return e;
+    void get(T** out, size_t count) {
+        used = (used + 255) & ~(size_t)255;
+        if (base) *out = reinterpret_cast<T*>(base + used);
+        used += sizeof(T) * count;
     }
 };
-
 
 // One seed's adjoint: the buffers and the position of its sweeps.  The phases
 // below only enqueue work on the handle's stream (except where a host copy is
@@ -146,7 +124,6 @@ struct AdjJob {
     AdjOps ops{};
     int N = 0, C = 0, NC = 0;
     size_t nlin = 0, nmfe = 0, nxy = 0;
-    Pool pool;
     cplx *ck_lin = nullptr, *ck_mf = nullptr;
     double* ck_kx0 = nullptr;
     DevClock* ck_clk = nullptr;
@@ -161,10 +138,12 @@ struct AdjJob {
     CnRec* cn_pre = nullptr;  // RK3CN: the old-operator clock fields at every stage start of the window
     cplx *lamU[2] = {nullptr, nullptr}, *lamB[2] = {nullptr, nullptr};
     cplx *lamF[2] = {nullptr, nullptr}, *lamG[2] = {nullptr, nullptr};
-    double *prof = nullptr, *bpart = nullptr, *bsum = nullptr;
+    double *prof = nullptr, *bpart = nullptr;
+    AdjSeedBufs* tab = nullptr;  // this seed's entry of the device table
+    AdjShared sh{};
     int* rec_status = nullptr;  // status bits of the window recomputes
     int rec_status_host = 0;
-    int iu = 0, ib = 0;
+    int par = 0;  // stages reversed so far, mod 2
     double J = 0.0;
     // full-window graphs (replayed for every window of C steps when C is even)
     cudaGraphExec_t g_fwd = nullptr, g_rec = nullptr, g_bwd = nullptr;
@@ -173,6 +152,56 @@ struct AdjJob {
             if (g) cudaGraphExecDestroy(g);
     }
 };
+
+// This call's buffers in the handle's workspace.
+void adj_layout(AdjJob& j, Arena& w) {
+    const qlgpu_t* h = j.h;
+    w.get(&j.ck_lin, (size_t)j.NC * j.nlin);
+    w.get(&j.ck_mf, (size_t)j.NC * j.nmfe);
+    w.get(&j.ck_kx0, (size_t)j.NC * j.nxy);
+    w.get(&j.ck_clk, (size_t)j.NC);
+    w.get(&j.fin_lin, j.nlin);
+    w.get(&j.fin_mf, j.nmfe);
+    w.get(&j.fin_kx0, j.nxy);
+    w.get(&j.fin_clk, 1);
+    w.get(&j.stU, (size_t)j.C * 3 * j.nlin);
+    w.get(&j.stB, (size_t)j.C * 3 * j.nmfe);
+    w.get(&j.postU, j.nlin);
+    w.get(&j.kx_pre, (size_t)j.C * j.nxy);
+    w.get(&j.kx_post, j.nxy);
+    w.get(&j.t_pre, (size_t)j.C + 1);
+    w.get(&j.cn_pre, (size_t)j.C * 3);
+    for (int i = 0; i < 2; ++i) {
+        w.get(&j.lamU[i], j.nlin);
+        w.get(&j.lamB[i], j.nmfe);
+        w.get(&j.lamF[i], j.nlin);
+        w.get(&j.lamG[i], j.nmfe);
+    }
+    w.get(&j.prof, (size_t)5 * h->NZ);
+    w.get(&j.bpart, (size_t)3 * h->NZ * j.sh.nchunk);
+    w.get(&j.tab, 1);
+    w.get(&j.rec_status, 1);
+}
+
+AdjSeedBufs adj_seed_bufs(const AdjJob& j) {
+    AdjSeedBufs e;
+    e.cn_pre = j.cn_pre;
+    e.stU = j.stU;
+    e.stB = j.stB;
+    e.postU = j.postU;
+    e.kx_pre = j.kx_pre;
+    e.kx_post = j.kx_post;
+    e.t_pre = j.t_pre;
+    for (int i = 0; i < 2; ++i) {
+        e.lamU[i] = j.lamU[i];
+        e.lamB[i] = j.lamB[i];
+        e.lamF[i] = j.lamF[i];
+        e.lamG[i] = j.lamG[i];
+    }
+    e.prof = j.prof;
+    e.bpart = j.bpart;
+    return e;
+}
 
 int adj_begin(AdjJob& j, qlgpu_t* h, double t0, const double* lin0, const double* mf0, const double* kx0, int nsteps,
               int checkpoint_every) {
@@ -185,7 +214,6 @@ int adj_begin(AdjJob& j, qlgpu_t* h, double t0, const double* lin0, const double
     if (!pick_ops(h->NZ, &j.ops)) return afail(h, QLGPU_ERR_UNSUPPORTED, "unsupported NZ");
     QA_CK(cudaSetDevice(h->device));
     QA_CK(ensure_smem_attr(j.ops.modes_kernel, j.ops.modes_smem));
-    QA_CK(ensure_smem_attr(j.ops.modes_seeds_kernel, j.ops.modes_smem));
     int rc = qlgpu_set_state(h, t0, lin0, mf0, kx0);
     if (rc) return rc;
     j.N = nsteps;
@@ -194,14 +222,43 @@ int adj_begin(AdjJob& j, qlgpu_t* h, double t0, const double* lin0, const double
     j.nlin = (size_t)h->nxy * 4 * h->nz;
     j.nmfe = (size_t)h->nmf * h->nz;
     j.nxy = (size_t)h->nxy;
-    QA_CK(j.pool.get(&j.ck_lin, (size_t)j.NC * j.nlin));
-    QA_CK(j.pool.get(&j.ck_mf, (size_t)j.NC * j.nmfe));
-    QA_CK(j.pool.get(&j.ck_kx0, (size_t)j.NC * j.nxy));
-    QA_CK(j.pool.get(&j.ck_clk, (size_t)j.NC));
-    QA_CK(j.pool.get(&j.fin_lin, j.nlin));
-    QA_CK(j.pool.get(&j.fin_mf, j.nmfe));
-    QA_CK(j.pool.get(&j.fin_kx0, j.nxy));
-    QA_CK(j.pool.get(&j.fin_clk, 1));
+    AdjShared& H = j.sh;
+    H.ky = h->d_ky;
+    H.kxi = h->d_kxi;
+    H.kyi = h->d_kyi;
+    H.ilap2 = h->d_ilap2;
+    H.ekz = h->d_ekz;
+    H.tw8 = h->d_tw + h->NZ;
+    H.status = h->d_dbg;
+    H.nlin = (long long)j.nlin;
+    H.nmfe = (long long)j.nmfe;
+    // at most 256 chunk sums per seed whatever the number of seeds, so that a seed's result does
+    // not depend on the seeds reversed with it
+    const int nblocks = (h->nxy + adj_block_modes(h->NZ) - 1) / adj_block_modes(h->NZ);
+    H.cblocks = (nblocks + 255) / 256;
+    H.nchunk = (nblocks + H.cblocks - 1) / H.cblocks;
+    H.integ = adj_integ(h);
+    H.weight = 1.0 / j.N;
+    Arena w;
+    adj_layout(j, w);
+    if (w.used > h->adj_bytes) {
+        QA_CK(cudaStreamSynchronize(h->stream));
+        if (h->adj_ws) cudaFree(h->adj_ws);
+        h->adj_ws = nullptr;
+        h->adj_bytes = 0;
+        QA_CK(cudaMalloc(&h->adj_ws, w.used));
+        h->adj_bytes = w.used;
+    }
+    w.used = 0;
+    w.base = static_cast<unsigned char*>(h->adj_ws);
+    adj_layout(j, w);
+    H.seeds = j.tab;
+    const AdjSeedBufs e = adj_seed_bufs(j);
+    QA_CK(cudaMemcpyAsync(j.tab, &e, sizeof(e), cudaMemcpyHostToDevice, h->stream));
+    // the adjoint of the final state is zero
+    QA_CK(cudaMemsetAsync(j.lamU[0], 0, j.nlin * sizeof(cplx), h->stream));
+    QA_CK(cudaMemsetAsync(j.lamB[0], 0, j.nmfe * sizeof(cplx), h->stream));
+    QA_CK(cudaMemsetAsync(j.rec_status, 0, sizeof(int), h->stream));
     if (h->diag_cap < j.N) {
         if (h->d_diag) cudaFree(h->d_diag);
         h->d_diag = nullptr;
@@ -247,9 +304,7 @@ int adj_forward_end(AdjJob& j) {
     return QLGPU_OK;
 }
 
-int adj_alloc_backward(AdjJob& j);
-
-// after the stream is synchronised: J and the backward buffers
+// after the stream is synchronised: J
 int adj_forward_finish(AdjJob& j) {
     qlgpu_t* h = j.h;
     h->dp.tv_interval = 0.0;
@@ -263,28 +318,6 @@ int adj_forward_finish(AdjJob& j) {
     double s = 0.0;
     for (int n = 0; n < j.N; ++n) s += j.rec[(size_t)15 * n + 8];  // AM_b (MHD_BQlin.cpp:459)
     j.J = s / j.N;
-    return adj_alloc_backward(j);
-}
-
-int adj_alloc_backward(AdjJob& j) {
-    qlgpu_t* h = j.h;
-    QA_CK(j.pool.get(&j.stU, (size_t)j.C * 3 * j.nlin));
-    QA_CK(j.pool.get(&j.stB, (size_t)j.C * 3 * j.nmfe));
-    QA_CK(j.pool.get(&j.postU, j.nlin));
-    QA_CK(j.pool.get(&j.kx_pre, (size_t)j.C * j.nxy));
-    QA_CK(j.pool.get(&j.kx_post, j.nxy));
-    QA_CK(j.pool.get(&j.t_pre, (size_t)j.C + 1));
-    QA_CK(j.pool.get(&j.cn_pre, (size_t)j.C * 3));
-    for (int i = 0; i < 2; ++i) {
-        QA_CK(j.pool.get(&j.lamU[i], j.nlin));
-        QA_CK(j.pool.get(&j.lamB[i], j.nmfe));
-        QA_CK(j.pool.get(&j.lamF[i], j.nlin));
-        QA_CK(j.pool.get(&j.lamG[i], j.nmfe));
-    }
-    QA_CK(j.pool.get(&j.prof, (size_t)5 * h->NZ));
-    QA_CK(j.pool.get(&j.bpart, (size_t)3 * h->NZ * j.nxy));
-    QA_CK(j.pool.get(&j.bsum, (size_t)3 * h->NZ));
-    QA_CK(j.pool.get(&j.rec_status, 1));
     return QLGPU_OK;
 }
 
@@ -326,126 +359,50 @@ int adj_window_end(AdjJob& j, int w) {
     return QLGPU_OK;
 }
 
-// the adjoint of step n of a window of `steps` steps (stream-ordered after
-// adj_window_end; the step times are read on the device from t_pre)
-int adj_backward_step(AdjJob& j, int steps, int n) {
-    qlgpu_t* h = j.h;
-    cudaStream_t st = h->stream;
-    const cplx* Upost = (n + 1 < steps) ? j.stU + (size_t)(n + 1) * 3 * j.nlin : j.postU;
-    const double* kxa = (n + 1 < steps) ? j.kx_pre + (n + 1) * j.nxy : j.kx_post;
+// The adjoint of a window of `steps` steps for the ns seeds of H.seeds, on one stream (the
+// step times are read on the device).  Every seed's arithmetic is the same for any ns.
+int adj_reverse_window(qlgpu_t* h, const AdjOps& ops, const AdjShared& H, int ns, int steps, int* par,
+                       cudaStream_t st) {
+    AdjPos X;
+    std::memset(&X, 0, sizeof(X));
+    X.steps = steps;
+    X.n = steps - 1;
+    X.s = 2;
+    X.par = *par;
+    X.sc = h->sc[2];
     // J = (1/N) sum AM_b(post-step state), recorded after the remap (main.cpp:122-130)
-    j.ops.jgrad(Upost, kxa, h->d_ky, h->d_kyi, h->d_ilap2, h->dp, 0.0, j.t_pre + n + 1, 1.0 / j.N, j.lamU[j.iu], st);
-    adj_remap_kernel<<<148, 256, 0, st>>>(j.kx_pre + n * j.nxy, kxa, h->nxy, h->nz, j.lamU[j.iu]);
-    for (int s = 2; s >= 0; --s) {
-        const StageConst& S = h->sc[s];
-        AdjMfArgs M;
-        std::memset(&M, 0, sizeof(M));
-        M.B = j.stB + ((size_t)n * 3 + s) * j.nmfe;
-        M.lamB_out = j.lamB[j.ib];
-        M.lamG_out = (s == 2) ? nullptr : j.lamG[0];
-        M.lamB_in = j.lamB[j.ib ^ 1];
-        M.lamGp = (s == 0) ? nullptr : j.lamG[1];
-        M.prof = j.prof;
-        M.tw = h->d_tw;
-        M.sc = S;
-        M.integ = adj_integ(h);
-        j.ops.mf_pre(M, h->dp, st);
-        AdjStageArgs A;
-        std::memset(&A, 0, sizeof(A));
-        A.status = h->d_dbg;
-        A.U = j.stU + ((size_t)n * 3 + s) * j.nlin;
-        A.lamU_out = j.lamU[j.iu];
-        A.lamF_out = (s == 2) ? nullptr : j.lamF[0];
-        A.lamU_in = j.lamU[j.iu ^ 1];
-        A.lamFp = (s == 0) ? nullptr : j.lamF[1];
-        A.kx0 = j.kx_pre + n * j.nxy;
-        A.ky = h->d_ky;
-        A.kxi = h->d_kxi;
-        A.kyi = h->d_kyi;
-        A.ilap2 = h->d_ilap2;
-        A.tw = h->d_tw;
-        A.prof = j.prof;
-        A.bpart = j.bpart;
-        A.t_dev = j.t_pre + n;
-        A.cn = j.cn_pre + (size_t)n * 3 + s;
-        A.integ = adj_integ(h);
-        A.sc = S;
-        j.ops.modes(A, h->dp, h->nxy, st);
-        const int nout = 3 * h->NZ;
-        adj_bsum_kernel<<<(nout + 7) / 8, 256, 0, st>>>(j.bpart, h->nxy, nout, j.bsum);
-        j.ops.mf_post(j.bsum, h->d_tw, h->dp, j.lamB[j.ib ^ 1], st);
-        j.iu ^= 1;
-        j.ib ^= 1;
-        std::swap(j.lamF[0], j.lamF[1]);
-        std::swap(j.lamG[0], j.lamG[1]);
-    }
+    adj_jgrad_kernel<<<dim3(148, ns), 256, 0, st>>>(H, h->dp, X);
     QA_CK(cudaGetLastError());
+    QA_CK(ops.mf(H, h->dp, X, X, 0, 1, ns, st));
+    int sms = 0;
+    QA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+    const int threads = (long long)H.nchunk * ns <= sms ? 512 : 256;
+    for (int left = 3 * steps; left > 0; --left) {
+        QA_CK(ops.modes(H, h->dp, X, ns, threads, st));
+        AdjPos Y = X;
+        Y.par ^= 1;
+        if (--Y.s < 0) {
+            Y.s = 2;
+            --Y.n;
+        }
+        Y.sc = h->sc[Y.s];
+        QA_CK(ops.mf(H, h->dp, X, Y, 1, left > 1, ns, st));
+        X = Y;
+    }
+    *par = X.par;
     return QLGPU_OK;
 }
 
-// The reverse sweep of all seeds of a batch on one stream: the same kernels as
-// adj_backward_step, each launched once with one grid row per seed.  Every
-// seed's arithmetic is that of adj_backward_step (results bit for bit equal).
-struct SeedReverse {
-    qlgpu_t* h = nullptr;  // the first seed's handle: tables, parameters, error text
-    AdjOps ops{};
-    const AdjSeedBufs* d_seeds = nullptr;
-    int nseeds = 0;
-    int par = 0;  // stages reversed so far, mod 2
-    size_t nlin = 0, nmfe = 0, nxy = 0;
-    double weight = 0.0;
-};
-
-int adj_backward_step_seeds(SeedReverse& R, cudaStream_t st, int steps, int n) {
-    qlgpu_t* h = R.h;
-    const int ns = R.nseeds;
-    AdjRevPos X;
-    X.seeds = R.d_seeds;
-    X.n = n;
-    X.steps = steps;
-    X.s = 2;
-    X.par = R.par;
-    X.nlin = (long long)R.nlin;
-    X.nmfe = (long long)R.nmfe;
-    X.nxy = (long long)R.nxy;
-    X.weight = R.weight;
-    R.ops.jgrad_s(h->d_ky, h->d_kyi, h->d_ilap2, h->dp, X, ns, st);
-    adj_remap_seeds_kernel<<<dim3(148, ns), 256, 0, st>>>(X, h->nz);
-    for (int s = 2; s >= 0; --s) {
-        X.s = s;
-        X.par = R.par;
-        AdjMfArgs M;
-        std::memset(&M, 0, sizeof(M));
-        M.tw = h->d_tw;
-        M.sc = h->sc[s];
-        M.integ = adj_integ(h);
-        R.ops.mf_pre_s(M, h->dp, X, ns, st);
-        AdjStageArgs A;
-        std::memset(&A, 0, sizeof(A));
-        A.status = h->d_dbg;
-        A.ky = h->d_ky;
-        A.kxi = h->d_kxi;
-        A.kyi = h->d_kyi;
-        A.ilap2 = h->d_ilap2;
-        A.tw = h->d_tw;
-        A.integ = adj_integ(h);
-        A.sc = h->sc[s];
-        R.ops.modes_s(A, h->dp, X, h->nxy, ns, st);
-        const int nout = 3 * h->NZ;
-        adj_bsum_seeds_kernel<<<dim3((nout + 7) / 8, ns), 256, 0, st>>>(X, nout);
-        R.ops.mf_post_s(h->d_tw, h->dp, X, ns, st);
-        R.par ^= 1;
-    }
-    QA_CK(cudaGetLastError());
-    return QLGPU_OK;
+int adj_backward_window(AdjJob& j, int steps) {
+    return adj_reverse_window(j.h, j.ops, j.sh, 1, steps, &j.par, j.h->stream);
 }
 
 // gradients out, and the handle left at the end of the forward run
 int adj_finish(AdjJob& j, double* grad_lin, double* grad_mf) {
     qlgpu_t* h = j.h;
     cudaStream_t st = h->stream;
-    QA_CK(cudaMemcpyAsync(grad_lin, j.lamU[j.iu], j.nlin * sizeof(cplx), cudaMemcpyDeviceToHost, st));
-    if (grad_mf) QA_CK(cudaMemcpyAsync(grad_mf, j.lamB[j.ib], j.nmfe * sizeof(cplx), cudaMemcpyDeviceToHost, st));
+    QA_CK(cudaMemcpyAsync(grad_lin, j.lamU[j.par], j.nlin * sizeof(cplx), cudaMemcpyDeviceToHost, st));
+    if (grad_mf) QA_CK(cudaMemcpyAsync(grad_mf, j.lamB[j.par], j.nmfe * sizeof(cplx), cudaMemcpyDeviceToHost, st));
     QA_CK(cudaMemcpyAsync(&j.rec_status_host, j.rec_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     h->cur = j.fin_cur;
     QA_CK(cudaMemcpyAsync(h->d_lin[h->cur], j.fin_lin, j.nlin * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
@@ -476,7 +433,7 @@ template <class F>
 int capture(AdjJob& j, cudaGraphExec_t* out, F body);
 int launch_graph(AdjJob& j, cudaGraphExec_t g);
 
-// The reverse sweep runs once for all seeds (adj_backward_step_seeds) when the
+// The reverse sweep runs once for all seeds (one adj_reverse_window) when the
 // seeds share every parameter and the device; otherwise per seed.
 bool same_setup(const qlgpu_t* a, const qlgpu_t* b) {
     const qlgpu_params &p = a->p, &r = b->p;
@@ -558,8 +515,6 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
         QA_CK(cudaMemcpyAsync(j.fin_clk, d.clk, sizeof(DevClock), cudaMemcpyDeviceToDevice, bs));
         j.fin_cur = 0;
         j.h->dp.tv_interval = 0.0;
-        rc = adj_alloc_backward(j);
-        if (rc) return rc;
     }
     // the reverse sweep: one launch per kernel for all seeds (default), or every seed on its
     // own stream (QLGPU_ADJ_REVERSE=streams, or seeds that differ in a parameter)
@@ -567,41 +522,22 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
     bool seeds_rev = !(renv && std::string(renv) == "streams");
     for (int q = 1; q < nj; ++q)
         if (!same_setup(jobs[q].h, h0)) seeds_rev = false;
-    Pool tab;
-    SeedReverse R;
+    AdjShared SH = jobs[0].sh;  // all seeds' entries, in the first handle's table
+    int spar = 0;
     if (seeds_rev) {
         std::vector<AdjSeedBufs> hb(nj);
-        for (int q = 0; q < nj; ++q) {
-            const AdjJob& j = jobs[q];
-            AdjSeedBufs& e = hb[q];
-            e.cn_pre = adj_integ(j.h) == INTEG_CN ? j.cn_pre : nullptr;
-            e.stU = j.stU;
-            e.stB = j.stB;
-            e.postU = j.postU;
-            e.kx_pre = j.kx_pre;
-            e.kx_post = j.kx_post;
-            e.t_pre = j.t_pre;
-            for (int i = 0; i < 2; ++i) {
-                e.lamU[i] = j.lamU[i];
-                e.lamB[i] = j.lamB[i];
-                e.lamF[i] = j.lamF[i];
-                e.lamG[i] = j.lamG[i];
-            }
-            e.prof = j.prof;
-            e.bpart = j.bpart;
-            e.bsum = j.bsum;
+        for (int q = 0; q < nj; ++q) hb[q] = adj_seed_bufs(jobs[q]);
+        if (h0->adj_tab_cap < nj) {
+            if (h0->adj_tab) cudaFree(h0->adj_tab);
+            h0->adj_tab = nullptr;
+            h0->adj_tab_cap = 0;
+            QA_CK(cudaMalloc(&h0->adj_tab, sizeof(AdjSeedBufs) * nj));
+            h0->adj_tab_cap = nj;
         }
-        AdjSeedBufs* d = nullptr;
-        QA_CK(tab.get(&d, (size_t)nj));
-        QA_CK(cudaMemcpy(d, hb.data(), sizeof(AdjSeedBufs) * nj, cudaMemcpyHostToDevice));
-        R.h = h0;
-        R.ops = jobs[0].ops;
-        R.d_seeds = d;
-        R.nseeds = nj;
-        R.nlin = nlin;
-        R.nmfe = nmfe;
-        R.nxy = nxy;
-        R.weight = 1.0 / N;
+        QA_CK(cudaMemcpy(h0->adj_tab, hb.data(), sizeof(AdjSeedBufs) * nj, cudaMemcpyHostToDevice));
+        SH.seeds = static_cast<const AdjSeedBufs*>(h0->adj_tab);
+        // the seeds' zeroed adjoints were enqueued on their own streams
+        for (int q = 0; q < nj; ++q) QA_CK(cudaStreamSynchronize(jobs[q].h->stream));
     }
     // ---- reverse sweep, window by window
     cudaEvent_t ev_b = nullptr;
@@ -653,10 +589,8 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
             QA_CK(cudaMemcpyAsync(j.t_pre + steps, &d.clk->t, sizeof(double), cudaMemcpyDeviceToDevice, bs));
         }
         if (seeds_rev) {
-            for (int n = steps - 1; n >= 0; --n) {
-                rc = adj_backward_step_seeds(R, bs, steps, n);
-                if (rc) return rc;
-            }
+            rc = adj_reverse_window(h0, jobs[0].ops, SH, nj, steps, &spar, bs);
+            if (rc) return rc;
             continue;
         }
         QA_CK(cudaEventRecord(ev_b, bs));
@@ -664,37 +598,25 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
             AdjJob& j = jobs[q];
             QA_CK(cudaStreamWaitEvent(j.h->stream, ev_b, 0));
             if (graphs && steps == C) {
-                // a full window's reverse steps: 14 small kernels per step, one graph launch
+                // a full window's reverse steps, one graph launch
                 if (!j.g_bwd) {
-                    rc = capture(j, &j.g_bwd, [&] {
-                        for (int n = C - 1; n >= 0; --n) {
-                            int r = adj_backward_step(j, C, n);
-                            if (r) return r;
-                        }
-                        return (int)QLGPU_OK;
-                    });
+                    rc = capture(j, &j.g_bwd, [&] { return adj_backward_window(j, C); });
                     if (rc) return rc;
                 }
                 rc = launch_graph(j, j.g_bwd);
                 if (rc) return rc;
                 continue;
             }
-            for (int n = steps - 1; n >= 0; --n) {
-                rc = adj_backward_step(j, steps, n);
-                if (rc) return rc;
-            }
+            rc = adj_backward_window(j, steps);
+            if (rc) return rc;
         }
     }
     if (seeds_rev) {
-        // every seed's buffers in the state adj_backward_step would have left them
+        // every seed's buffers in the state adj_backward_window would have left them
         QA_CK(cudaEventRecord(ev_b, bs));
         for (int q = 0; q < nj; ++q) {
             AdjJob& j = jobs[q];
-            j.iu = j.ib = R.par;
-            if (R.par) {
-                std::swap(j.lamF[0], j.lamF[1]);
-                std::swap(j.lamG[0], j.lamG[1]);
-            }
+            j.par = spar;
             QA_CK(cudaStreamWaitEvent(j.h->stream, ev_b, 0));
         }
     }
@@ -760,13 +682,6 @@ int run_jobs(std::vector<AdjJob>& jobs, double* J, double* const* grad_lin, doub
         int rc = adj_recompute_window(j, steps);
         return rc ? rc : adj_window_end(j, w);
     };
-    auto bwd_window = [&](AdjJob& j, int steps) -> int {
-        for (int n = steps - 1; n >= 0; --n) {
-            int rc = adj_backward_step(j, steps, n);
-            if (rc) return rc;
-        }
-        return QLGPU_OK;
-    };
     for (int w = 0; w < NC; ++w) {
         const int steps = std::min(N, w * C + C) - w * C;
         QA_ALL(adj_checkpoint(jj, w));
@@ -786,11 +701,11 @@ int run_jobs(std::vector<AdjJob>& jobs, double* J, double* const* grad_lin, doub
         if (graphs && steps == C) {
             QA_ALL(jj.g_rec ? QLGPU_OK : capture(jj, &jj.g_rec, [&] { return rec_window(jj, w, C); }));
             QA_ALL(launch_graph(jj, jj.g_rec));
-            QA_ALL(jj.g_bwd ? QLGPU_OK : capture(jj, &jj.g_bwd, [&] { return bwd_window(jj, C); }));
+            QA_ALL(jj.g_bwd ? QLGPU_OK : capture(jj, &jj.g_bwd, [&] { return adj_backward_window(jj, C); }));
             QA_ALL(launch_graph(jj, jj.g_bwd));
         } else {
             QA_ALL(rec_window(jj, w, steps));
-            for (int n = steps - 1; n >= 0; --n) QA_ALL(adj_backward_step(jj, steps, n));
+            QA_ALL(adj_backward_window(jj, steps));
         }
     }
     for (int q = 0; q < nj; ++q) {
@@ -812,10 +727,10 @@ extern "C" int qlgpu_adjoint_maxwell(qlgpu_t* h, double t0, const double* lin0, 
     if (!J || !grad_lin) return afail(h, QLGPU_ERR_ARG, "null argument");
     std::vector<AdjJob> jobs(1);
     int rc = adj_begin(jobs[0], h, t0, lin0, mf0, kx0, nsteps, checkpoint_every);
-    if (rc) return rc;
     double* gl[1] = {grad_lin};
     double* gm[1] = {grad_mf};
-    rc = run_jobs(jobs, J, gl, grad_mf ? gm : nullptr);
+    if (!rc) rc = run_jobs(jobs, J, gl, grad_mf ? gm : nullptr);
+    adj_trim(h);
     return rc ? rc : qlgpu_debug_verify(h);
 }
 
@@ -840,6 +755,7 @@ extern "C" int qlgpu_adjoint_maxwell_batch(qlgpu_t* const* handles, int nseeds, 
                            kx0 ? kx0 + q * (size_t)h0->nxy : nullptr, nsteps, checkpoint_every);
         if (rc) {
             if (handles[q] != h0) h0->err = handles[q]->err;
+            for (int r = 0; r <= q; ++r) adj_trim(handles[r]);
             return rc;
         }
         gl[q] = grad_lin + q * 2 * nlin;
@@ -853,6 +769,7 @@ extern "C" int qlgpu_adjoint_maxwell_batch(qlgpu_t* const* handles, int nseeds, 
     const bool streams = mode && std::string(mode) == "streams";
     int rc = streams ? run_jobs(jobs, J, gl.data(), grad_mf ? gm.data() : nullptr)
                      : run_jobs_persistent(jobs, t0, lin0, mf0, kx0, J, gl.data(), grad_mf ? gm.data() : nullptr);
+    for (int q = 0; q < nseeds; ++q) adj_trim(handles[q]);
     for (int q = 0; q < nseeds && !rc; ++q) rc = qlgpu_debug_verify(handles[q]);
     if (rc) {
         for (int q = 0; q < nseeds; ++q)

@@ -22,321 +22,27 @@
 // <x, y> = Re sum conj(x) y:  mu = E lamU', lamF = n1 mu + lamF_out,
 // lamU = mu + (dR/dU)^H lamF + (dEMF/dU)^H lamG, lamFprev = n2 mu, and the
 // mean-field part likewise (Crank-Nicolson: mu = D lamU' and the direct term
-// C lamU' in place of mu).  One CTA per mode: 14 inverse transforms (the nine
-// forward real-space fields and five back-propagated rhs fields W = P(lamF)),
-// a pointwise pass giving the nine real-space adjoints and the mode's
-// contribution to the adjoint of the mean-field profiles, nine forward
-// transforms, and the spectral chain back to (u, zeta, b, eta).
+// C lamU' in place of mu).
+//
+// Two kernels per stage, for one seed or many (seed = blockIdx.y):
+//   adj_modes_kernel  a team of warps (one CTA) per chunk of modes: 14 inverse transforms
+//                     (the nine forward real-space fields and five back-propagated rhs
+//                     fields W = P(lamF)), the pointwise adjoints formed as inputs of nine
+//                     forward transforms, and the spectral chain back to (u, zeta, b, eta);
+//                     the chunk's sum of the adjoint of the mean-field profiles.
+//   adj_mf_kernel     one CTA per seed: the sum of those over the chunks, the rest of the
+//                     mean-field adjoint of the stage, and the profiles of the next one.
+// Both are launched with programmatic dependent launch: a chunk's inverse transforms need
+// only the mode kernel before the running mean-field kernel, and the mean-field kernel's
+// forward profiles need neither, so each kernel's first half runs under the other.
 #pragma once
 #include "qlgpu_debug.cuh"
 #include "qlgpu_stage.cuh"
+#include "qlgpu_xform.cuh"
 
 namespace qlgpu {
 
-struct AdjStageArgs {
-    const cplx* U;         // stage input fluctuations [nxy][4][nz]
-    const cplx* lamU_out;  // adjoint of the stage output
-    const cplx* lamF_out;  // adjoint of this stage's rhs from the next stage (null: none)
-    cplx* lamU_in;         // adjoint of the stage input (written)
-    cplx* lamFp;           // n2 mu: adjoint of the previous stage's rhs (null: first stage)
-    const double* kx0;     // unsheared kx of every mode during the step
-    const double* ky;
-    const int* kxi;
-    const int* kyi;
-    const double* ilap2;   // [Ny/2][nz]
-    const cplx* tw;        // transform twiddles [NZ]
-    const double* prof;    // [5][NZ]: By, dBy, ddBy, px, py (real space)
-    double* bpart;         // [3][NZ][nxy] per-mode adjoint of the mean-field profiles
-    double t_s;            // stage time (when t_dev is null)
-    const double* t_dev;   // the step's start time on the device: stage time = *t_dev + sc.t_off
-    const CnRec* cn;       // RK3CN: the old-operator fields at the stage start
-    int integ;             // INTEG_EXP or INTEG_CN
-    int pad;
-    int* status;           // the handle's status word (debug-build index checks)
-    StageConst sc;
-};
-
-template <int NZ>
-struct AdjGeom {
-    using G = Geom<NZ>;
-    static constexpr int NG = 16;  // transform groups per CTA (14 inverse, 9 forward transforms)
-    static constexpr int THREADS = NG * G::T;
-    static constexpr size_t o_tw = 0;
-    static constexpr size_t o_prof = o_tw + sizeof(cplx) * NZ;
-    static constexpr size_t o_rw = o_prof + sizeof(double) * 5 * NZ;
-    static constexpr size_t o_xch = o_rw + sizeof(cplx) * 14 * NZ;
-    static constexpr size_t BYTES = o_xch + sizeof(cplx) * NG * G::XSIZE;
-    // E of the four fields at every stored index, [4][nz]: in the exchange buffers of
-    // groups 14 and 15, which no transform phase uses (14 inverse, 9 forward transforms)
-    static constexpr size_t o_etab = o_xch + sizeof(cplx) * 14 * G::XSIZE;
-    static_assert(sizeof(double) * 4 * G::nz <= sizeof(cplx) * 2 * G::XSIZE, "E table fits two exchange buffers");
-};
-
-// E = exp(linC L_f) of field f at stored index s (RK3CN_Elin.cpp:102-104), L at the stage
-// end; for RK3CN D = 1/(1 - linC L_f) (RK3CN.cpp:105).
-__device__ __forceinline__ double adj_efac(const DevParams& P, const StageConst& S, double kxe, double ky, double kz2,
-                                           int f, int integ) {
-    const double L = linop_f<MODEL_BQLIN>(P, lap_end<MODEL_BQLIN>(P, kxe, ky, kz2), f);
-    if (integ == INTEG_CN) return __drcp_rn(__dsub_rn(1.0, __dmul_rn(S.linC, L)));
-    return exp(__dmul_rn(S.linC, L));
-}
-
-// The stage adjoint of one mode (one CTA).  A may live in parameter space (one
-// seed per launch) or in shared memory (a launch over many seeds).
-template <int NZ>
-__device__ __forceinline__ void adj_modes_body(const AdjStageArgs& A, const DevParams& P, int mode) {
-    mode = QLGPU_CHECK_INDEX(mode, P.nxy, A.status);
-    using G = Geom<NZ>;
-    using AG = AdjGeom<NZ>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    cplx* tw_s = reinterpret_cast<cplx*>(smem_raw + AG::o_tw);
-    double* prof = reinterpret_cast<double*>(smem_raw + AG::o_prof);
-    cplx* RW = reinterpret_cast<cplx*>(smem_raw + AG::o_rw);  // [14][NZ]
-    const int tid = threadIdx.x;
-    const int g = tid / G::T, t = tid % G::T;
-    const int lane = tid & 31;
-    const unsigned gmask =
-        (G::T == 32 ? 0xffffffffu : (((1u << G::T) - 1u) << ((lane / G::T) * G::T)));
-    cplx* xch = reinterpret_cast<cplx*>(smem_raw + AG::o_xch) + (size_t)g * G::XSIZE;
-    const int nz = P.nz;
-    for (int i = tid; i < NZ; i += blockDim.x) tw_s[i] = A.tw[i];
-    for (int i = tid; i < 5 * NZ; i += blockDim.x) prof[i] = A.prof[i];
-    const StageConst& S = A.sc;
-    const double ky = A.ky[mode];
-    const double kx0 = A.kx0[mode];
-    const int kyi = A.kyi[mode], kxi = A.kxi[mode];
-    const double ts = A.t_dev ? __dadd_rn(*A.t_dev, S.t_off) : A.t_s;
-    const double a = kx_at(kx0, P.q, ts, ky);
-    const double b = ky;
-    const double ab = __dmul_rn(a, b);
-    const double kxe = __dadd_rn(a, __dmul_rn(__dmul_rn(P.q, S.dt_lin), ky));
-    const double fac = P.fac;
-    const double mult = (ky == 0.0) ? 1.0 : 2.0;
-    const double Om2 = __dmul_rn(2.0, P.Omega);
-    const cplx* u = A.U + (size_t)mode * 4 * nz;
-    const cplx* lo = A.lamU_out + (size_t)mode * 4 * nz;
-    const cplx* lf = A.lamF_out ? A.lamF_out + (size_t)mode * 4 * nz : nullptr;
-    const double* il2row = A.ilap2 + (size_t)kyi * nz;
-    double* etab = reinterpret_cast<double*>(smem_raw + AG::o_etab);
-    for (int i = tid; i < 4 * nz; i += blockDim.x) {
-        const int f = i / nz, s = i % nz;
-        const int kzi = s <= G::H ? s : s - nz;
-        etab[i] = adj_efac(P, S, kxe, ky, kz2val(kzval(kzi, P.kzL)), f, A.integ);
-    }
-    // RK3CN: kx where the previous stage's operator was evaluated (RK3CN.cpp:119-122;
-    // the init form at the run's start, RK3CN.cpp:57), as the forward stage computes it
-    double kxo = 0.0;
-    int old_init = 0;
-    if (A.integ == INTEG_CN) {
-        const double tclock = A.t_dev ? *A.t_dev : __dsub_rn(A.t_s, S.t_off);
-        old_init = A.cn->old_init;
-        if (old_init) kxo = kx_at(kx0, P.q, tclock, ky);
-        else kxo = __dadd_rn(kx_at(kx0, P.q, A.cn->t_old, ky), __dmul_rn(__dmul_rn(P.q, A.cn->dtlin_old), ky));
-    }
-    __syncthreads();
-
-    // lamF of field f at stored index s: n1 E lamU' + lamF_out
-    auto lamF = [&](int f, int s, double) -> cplx {
-        cplx r = cscale(lo[f * nz + s], __dmul_rn(S.n1, etab[f * nz + s]));
-        if (lf) r = cadd(r, lf[f * nz + s]);
-        return r;
-    };
-
-    // ---- phase 1: fourteen inverse transforms
-    if (g < 14) {
-        cplx x[G::P];
-#pragma unroll
-        for (int k2 = 0; k2 < G::P; ++k2) {
-            const int k = t + G::T * k2;
-            const int s = stored_index<G>(k);
-            cplx v = mk(0.0, 0.0);
-            if (s >= 0) {
-                const double c = kzval(kz_int<G>(k), P.kzL);
-                const double kz2 = kz2val(c);
-                const bool z0 = (kyi == 0 && s == 0);
-                const double il2 = il2row[s];
-                if (g < 4) {
-                    v = cscale(u[g * nz + s], fac);  // R_u, R_zeta, R_b, R_eta
-                } else if (g < 9) {
-                    const int f0 = (g == 5 || g == 8) ? 2 : 0;
-                    const cplx g0 = u[f0 * nz + s], g1 = u[(f0 + 1) * nz + s];
-                    if (g == 7 || g == 8) {
-                        v = cscale(cadd(cscale(g0, ab), imul(g1, c)), il2);  // uy, by
-                    } else {
-                        v = cscale(csub(cscale(g0, __dmul_rn(a, c)), imul(g1, b)), il2);  // uz, bz
-                        if (g == 6) v = imul(v, c);                                        // i c uz
-                    }
-                    v = cscale(v, fac);
-                } else if (g == 9) {
-                    v = lamF(2, s, kz2);  // W_b
-                } else if (g == 10) {
-                    v = lamF(1, s, kz2);  // W_zeta
-                } else if (g == 11) {
-                    v = lamF(3, s, kz2);  // W_eta
-                } else {
-                    v = lamF(0, s, kz2);  // W_S, W_u2 = P(ilapF lamF_u)
-                    if (g == 13) {
-                        const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(ky, kz2, z0));
-                        const double ilapF = (z0 && kxi == 0) ? 1.0 : __drcp_rn(lapF);
-                        v = cscale(v, ilapF);
-                    }
-                }
-            }
-            x[k2] = v;
-        }
-        inv_fft<G>(x, xch, tw_s, t, gmask);
-#pragma unroll
-        for (int j = 0; j < G::P; ++j) RW[g * NZ + zpos<G>(t, j)] = x[j];
-    }
-    __syncthreads();
-
-    // ---- phase 2: pointwise adjoints in real space (in place: slots 0..8 become lamR)
-    const double* By = prof;
-    const double* dBy = prof + NZ;
-    const double* ddBy = prof + 2 * NZ;
-    const double* px = prof + 3 * NZ;
-    const double* py = prof + 4 * NZ;
-    // lamR = sum of conj(multiplier) W over the terms a field enters (reads slots 0..13 at z)
-    auto lam_r = [&](int z, cplx* o) {
-        const cplx Ru = RW[0 * NZ + z], Rb = RW[2 * NZ + z];
-        const cplx Ruz = RW[4 * NZ + z], Rbz = RW[5 * NZ + z];
-        const cplx Ruy = RW[7 * NZ + z], Rby = RW[8 * NZ + z];
-        const cplx Wb = RW[9 * NZ + z], Wz = RW[10 * NZ + z], We = RW[11 * NZ + z];
-        const cplx WS = RW[12 * NZ + z], Wu2 = RW[13 * NZ + z];
-        const double by = By[z], dby = dBy[z], ddby = ddBy[z];
-        const double mx = mult * px[z], my = mult * py[z];
-        const double bBy = b * by, adBy = a * dby;
-        o[0] = cadd(cadd(imul(Wb, -bBy), imul(We, adBy)), cscale(Rbz, mx));
-        o[1] = imul(We, -bBy);
-        o[2] = csub(cadd(imul(Wz, adBy), imul(WS, -bBy)), cscale(Ruz, mx));
-        o[3] = imul(Wz, -bBy);
-        o[4] = csub(csub(cscale(We, -ddby), cscale(Rb, mx)), cscale(Rby, my));
-        o[5] = cadd(cadd(cscale(Wz, ddby), cscale(Wu2, 2.0 * ab * dby)), cadd(cscale(Ru, mx), cscale(Ruy, my)));
-        o[6] = cscale(We, -2.0 * dby);
-        o[7] = cscale(Rbz, my);
-        o[8] = cscale(Ruz, -my);
-    };
-    // adjoint of the mean-field profiles at z: Re(conj(multiplier * R) W) per term
-    auto prof_adj = [&](int z) {
-        const cplx Ru = RW[0 * NZ + z], Rz = RW[1 * NZ + z], Rb = RW[2 * NZ + z], Re_ = RW[3 * NZ + z];
-        const cplx Ruz = RW[4 * NZ + z], Rbz = RW[5 * NZ + z], Rik = RW[6 * NZ + z];
-        const cplx Wb = RW[9 * NZ + z], Wz = RW[10 * NZ + z], We = RW[11 * NZ + z];
-        const cplx WS = RW[12 * NZ + z], Wu2 = RW[13 * NZ + z];
-        auto re_cw = [](cplx r, cplx w) { return r.x * w.x + r.y * w.y; };  // Re(conj(r) w)
-        auto re_icw = [](cplx r, cplx w) { return r.y * w.x - r.x * w.y; };  // Re(i conj(r) w)
-        const double pBy = -b * (re_icw(Ru, Wb) + re_icw(Re_, Wz) + re_icw(Rz, We) + re_icw(Rb, WS));
-        const double pdBy = a * (re_icw(Rb, Wz) + re_icw(Ru, We)) - 2.0 * re_cw(Rik, We) + 2.0 * ab * re_cw(Rbz, Wu2);
-        const double pddBy = re_cw(Rbz, Wz) - re_cw(Ruz, We);
-        const size_t nxy = (size_t)P.nxy;
-        A.bpart[(0 * (size_t)NZ + z) * nxy + mode] = pBy;
-        A.bpart[(1 * (size_t)NZ + z) * nxy + mode] = pdBy;
-        A.bpart[(2 * (size_t)NZ + z) * nxy + mode] = pddBy;
-    };
-    if constexpr (AG::THREADS >= 2 * NZ) {
-        // two threads per z: lamR in the first NZ threads, the profile adjoints in the
-        // next NZ; slots 0..8 are overwritten only after both have read them
-        const int z = tid % NZ, part = tid / NZ;
-        cplx o[9];
-        if (part == 0) lam_r(z, o);
-        else if (part == 1) prof_adj(z);
-        __syncthreads();
-        if (part == 0) {
-#pragma unroll
-            for (int k = 0; k < 9; ++k) RW[k * NZ + z] = o[k];
-        }
-    } else {
-        for (int z = tid; z < NZ; z += blockDim.x) {
-            cplx o[9];
-            lam_r(z, o);
-            prof_adj(z);
-#pragma unroll
-            for (int k = 0; k < 9; ++k) RW[k * NZ + z] = o[k];
-        }
-    }
-    __syncthreads();
-
-    // ---- phase 3: nine forward transforms, spectral results back into slots 0..8
-    if (g < 9) {
-        cplx x[G::P];
-#pragma unroll
-        for (int j = 0; j < G::P; ++j) x[j] = RW[g * NZ + zpos<G>(t, j)];
-        fwd_fft<G>(x, xch, tw_s, t, gmask);
-#pragma unroll
-        for (int k2 = 0; k2 < G::P; ++k2) {
-            const int s = stored_index<G>(t + G::T * k2);
-            if (s >= 0) RW[g * NZ + s] = x[k2];
-        }
-    }
-    __syncthreads();
-
-    // ---- phase 4: spectral chain to (u, zeta, b, eta), linear terms, RK adjoint
-    for (int idx = tid; idx < 4 * nz; idx += blockDim.x) {
-        const int f = idx / nz, s = idx % nz;
-        const int kzi = s <= G::H ? s : s - nz;
-        const double c = kzval(kzi, P.kzL);
-        const double kz2 = kz2val(c);
-        const bool z0 = (kyi == 0 && s == 0);
-        const double il2 = il2row[s];
-        const cplx mu = cscale(lo[f * nz + s], etab[idx]);
-        cplx r = mu;
-        if (A.integ == INTEG_CN) {
-            // the direct term (1 + linC Lold) D lamU' (RK3CN.cpp:107)
-            const double lo_lap = old_init ? lap_init<MODEL_BQLIN>(P, kxo, lap2val(ky, kz2, z0))
-                                           : lap_end<MODEL_BQLIN>(P, kxo, ky, kz2);
-            const double Lold = linop_f<MODEL_BQLIN>(P, lo_lap, f);
-            r = cscale(mu, __dadd_rn(1.0, __dmul_rn(S.linC, Lold)));
-        }
-        if (f == 0 || f == 1) {
-            // uz = (a c u - i b zeta) il2, i c uz, uy = (a b u + i c zeta) il2
-            const cplx luz = cscale(csub(RW[4 * NZ + s], imul(RW[6 * NZ + s], c)), fac);
-            const cplx luy = cscale(RW[7 * NZ + s], fac);
-            if (f == 0) {
-                r = cadd(r, cscale(RW[0 * NZ + s], fac));
-                r = cadd(r, cscale(luz, __dmul_rn(a, c) * il2));
-                r = cadd(r, cscale(luy, ab * il2));
-                // linear terms of F_zeta ((q - 2 Omega) i c u) and F_u (ilapF 2 a b q u)
-                r = cadd(r, imul(lamF(1, s, kz2), -(P.q - Om2) * c));
-                const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(ky, kz2, z0));
-                const double ilapF = (z0 && kxi == 0) ? 1.0 : __drcp_rn(lapF);
-                r = cadd(r, cscale(lamF(0, s, kz2), ilapF * 2.0 * ab * P.q));
-            } else {
-                r = cadd(r, cscale(RW[1 * NZ + s], fac));
-                r = cadd(r, imul(luz, b * il2));
-                r = cadd(r, imul(luy, -c * il2));
-                // linear term of F_u: ilapF 2 Omega i c zeta
-                const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(ky, kz2, z0));
-                const double ilapF = (z0 && kxi == 0) ? 1.0 : __drcp_rn(lapF);
-                r = cadd(r, imul(lamF(0, s, kz2), -Om2 * c * ilapF));
-            }
-        } else {
-            const cplx lbz = cscale(RW[5 * NZ + s], fac);
-            const cplx lby = cscale(RW[8 * NZ + s], fac);
-            if (f == 2) {
-                r = cadd(r, cscale(RW[2 * NZ + s], fac));
-                r = cadd(r, cscale(lbz, __dmul_rn(a, c) * il2));
-                r = cadd(r, cscale(lby, ab * il2));
-                r = cadd(r, imul(lamF(3, s, kz2), P.q * c));  // linear term of F_eta: -q i c b
-            } else {
-                r = cadd(r, cscale(RW[3 * NZ + s], fac));
-                r = cadd(r, imul(lbz, b * il2));
-                r = cadd(r, imul(lby, -c * il2));
-            }
-        }
-        A.lamU_in[(size_t)mode * 4 * nz + f * nz + s] = r;
-        if (A.lamFp) A.lamFp[(size_t)mode * 4 * nz + f * nz + s] = cscale(mu, S.n2);
-    }
-}
-
-template <int NZ>
-__global__ void __launch_bounds__(AdjGeom<NZ>::THREADS, 6)
-    adj_modes_kernel(const __grid_constant__ AdjStageArgs A, const __grid_constant__ DevParams P) {
-    adj_modes_body<NZ>(A, P, blockIdx.x);
-}
-
-// ---- the reverse sweep of many seeds at once (same dimensions and parameters):
-// every kernel of a reverse step runs once for all seeds, seed = blockIdx.y.
-// The per-seed buffers are read from a device table; the position in the sweep
-// (step n of a window of `steps`, stage s, buffer parity) is a launch argument.
+// Per-seed buffers of the reverse sweep (a device table).
 struct AdjSeedBufs {
     const CnRec* cn_pre;   // [C][3] RK3CN old-operator fields at every stage start (null: RK3CN_Elin)
     const cplx* stU;       // [C][3] recorded stage inputs
@@ -349,286 +55,537 @@ struct AdjSeedBufs {
     cplx* lamB[2];
     cplx* lamF[2];
     cplx* lamG[2];
-    double* prof;
-    double* bpart;
-    double* bsum;
+    double* prof;          // [5][NZ]: By, dBy, ddBy, px, py (real space)
+    double* bpart;         // [nchunk][3][NZ] chunk sums of the adjoint of the mean-field profiles
 };
 
-struct AdjRevPos {
+// Tables and parameters the seeds share.
+struct AdjShared {
     const AdjSeedBufs* seeds;
-    int n, steps, s;
-    int par;  // stages already reversed, mod 2: lamU[par] is the current adjoint state
-    long long nlin, nmfe, nxy;
-    double weight;  // of AM_b in J
-};
-
-// the post-step state of step n and its kx0 (the window end for the last step)
-__device__ __forceinline__ const cplx* adj_upost(const AdjSeedBufs& B, const AdjRevPos& X) {
-    return X.n + 1 < X.steps ? B.stU + (size_t)(X.n + 1) * 3 * X.nlin : B.postU;
-}
-__device__ __forceinline__ const double* adj_kxpost(const AdjSeedBufs& B, const AdjRevPos& X) {
-    return X.n + 1 < X.steps ? B.kx_pre + (size_t)(X.n + 1) * X.nxy : B.kx_post;
-}
-
-template <int NZ>
-__global__ void __launch_bounds__(AdjGeom<NZ>::THREADS, 6)
-    adj_modes_seeds_kernel(const __grid_constant__ AdjStageArgs base, const __grid_constant__ DevParams P,
-                           const __grid_constant__ AdjRevPos X) {
-    __shared__ __align__(16) AdjStageArgs sA;
-    if (threadIdx.x == 0) {
-        const AdjSeedBufs& B = X.seeds[blockIdx.y];
-        const int p = X.par;
-        sA = base;
-        sA.U = B.stU + ((size_t)X.n * 3 + X.s) * X.nlin;
-        sA.lamU_out = B.lamU[p];
-        sA.lamF_out = X.s == 2 ? nullptr : B.lamF[p];
-        sA.lamU_in = B.lamU[p ^ 1];
-        sA.lamFp = X.s == 0 ? nullptr : B.lamF[p ^ 1];
-        sA.kx0 = B.kx_pre + (size_t)X.n * X.nxy;
-        sA.prof = B.prof;
-        sA.bpart = B.bpart;
-        sA.t_dev = B.t_pre + X.n;
-        sA.cn = B.cn_pre ? B.cn_pre + (size_t)X.n * 3 + X.s : nullptr;
-    }
-    __syncthreads();
-    adj_modes_body<NZ>(sA, P, blockIdx.x);
-}
-
-// Mean-field part before the mode pass: forward profiles of the stage input
-// mean field (By, dBy, ddBy; MHD_BQlin.cpp:122-127), the adjoint stress
-// profiles px, py, and the RK / mean-field-rhs adjoint of B:
-//   muB = E_B lamB', lamG = n1 muB + lamG_out, lamB = muB - q lamG_y e_x,
-//   lamGp = n2 muB,  p(z) = Re sum_{s=1..H} h_s e^{+i k_s z},
-//   h_s = rs_fac (-i kz_s) (lamEMF[s] + conj(lamEMF[nz-s])).
-// One CTA of 5 transform groups.
-struct AdjMfArgs {
-    const cplx* B;         // stage input mean field [nmf][nz]
-    const cplx* lamB_out;  // adjoint of the stage output mean field
-    const cplx* lamG_out;  // adjoint of this stage's mean-field rhs from the next stage (null: none)
-    cplx* lamB_in;         // partial adjoint of the stage input mean field (the mode pass adds to By)
-    cplx* lamGp;           // n2 muB (null: first stage)
-    double* prof;          // [5][NZ] out
-    const cplx* tw;
+    const double* ky;
+    const int* kxi;
+    const int* kyi;
+    const double* ilap2;   // [Ny/2][nz]
+    const double* ekz;     // [3][2][nz] integrating factors exp(linC c kz2) of the stages
+    const cplx* tw8;       // transform twiddles [8][NZ/8]
+    int* status;           // the first handle's status word (debug-build index checks)
+    long long nlin, nmfe;
+    int nchunk, cblocks;   // chunks per seed, blocks of 256/NZ modes per chunk
     int integ;             // INTEG_EXP or INTEG_CN
     int pad;
+    double weight;         // of AM_b in J
+};
+
+// Position in the sweep: stage s of step n of a window of `steps` steps.
+struct AdjPos {
+    int n, steps, s;
+    int par;  // stages already reversed, mod 2: lamU[par] is the current adjoint state
     StageConst sc;
 };
 
+// The programmatic-launch pair: the next kernel may start / the kernels before are complete.
+__device__ __forceinline__ void pdl_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+// Geometry of the team kernels: T = NZ/8 lanes per transform, GPW modes per block.
+template <int NZ_>
+struct AG {
+    static constexpr int NZ = NZ_;
+    static constexpr int T = NZ_ / 8;
+    static constexpr int nz = 1 + 2 * (NZ_ / 3);
+    static constexpr int H = (nz - 1) / 2;
+    static constexpr int GPW = 32 / T;
+    static constexpr int SWZ = T == 4 ? 1 : (T == 2 ? 3 : 0);
+    static constexpr int NZE = (nz + 1) & ~1;
+    static constexpr int NR = 16;  // 14 inverse results, 2 exchange buffers
+    static constexpr size_t o_tw = 0;                                    // [8][T] cplx
+    static constexpr size_t o_prof = o_tw + 16 * (size_t)NZ_;           // [5][NZ]
+    static constexpr size_t o_kz = o_prof + 8 * 5 * (size_t)NZ_;        // kz per spectral slot
+    static constexpr size_t o_ekz = o_kz + 8 * (size_t)NZ_;             // [2][NZE]
+    static constexpr size_t o_acc = o_ekz + 16 * (size_t)NZE;           // [3][8][32] profile sums
+    static constexpr size_t o_R = o_acc + 8 * 3 * 256;                  // [NR][8][32] cplx
+    static constexpr size_t o_stg = o_R + 16 * 256 * (size_t)NR;        // [GPW][4][nz] cplx
+    static constexpr size_t BYTES = o_stg + 16 * (size_t)GPW * 4 * nz;
+};
+inline int adj_block_modes(int NZ) { return 256 / NZ; }
+
+enum { A_RU = 0, A_RZ, A_RB, A_RE, A_RUZ, A_RBZ, A_RIK, A_RUY, A_RBY, A_WB, A_WZ, A_WE, A_WS, A_WU2, A_X0, A_X1 };
+
+// One lane's mode in the stage being reversed.
+struct AdjLane {
+    int m, kyi, kxi;
+    bool valid;
+    double a, b, kxe, kxo, mult, em_u, em_b;
+    int old_init;
+};
+
+// E (RK3CN_Elin: em exp(linC c kz2)) or D = 1/(1 - linC L) (RK3CN.cpp:105) of field f.
+template <class W>
+__device__ __forceinline__ double adj_e(const DevParams& P, const StageConst& S, const AdjLane& M, const double* ekz,
+                                        int f, int s, double kz2, int integ) {
+    if (integ == INTEG_CN)
+        return __drcp_rn(__dsub_rn(
+            1.0, __dmul_rn(S.linC, linop_f<MODEL_BQLIN>(P, lap_end<MODEL_BQLIN>(P, M.kxe, M.b, kz2), f))));
+    return f < 2 ? M.em_u * ekz[s] : M.em_b * ekz[W::NZE + s];
+}
+
+// The stage adjoint of the chunk's modes.  What bounds it: the transforms' chain of a block
+// (two deep) at one seed, the FP64 and shared-memory work at many.  A CTA of 8 warps leaves
+// room for a second one per SM, whose transforms run under the barriers of the first; with
+// at most one chunk per SM it has 16 warps, one round of the 14 inverse transforms.
 template <int NZ>
-__device__ __forceinline__ void adj_mf_pre_body(const AdjMfArgs& A, const DevParams& P) {
-    using G = Geom<NZ>;
-    __shared__ __align__(16) cplx tw_s[NZ];
-    __shared__ __align__(16) cplx lamG[2][G::nz];
-    __shared__ __align__(16) cplx xchs[5][G::XSIZE];
-    const int tid = threadIdx.x;
-    const int nz = P.nz;
-    const StageConst& S = A.sc;
-    for (int i = tid; i < NZ; i += blockDim.x) tw_s[i] = A.tw[i];
-    for (int i = tid; i < 2 * nz; i += blockDim.x) {
-        const int m = i / nz, s = i % nz;
-        const int kzi = s <= G::H ? s : s - nz;
-        const double kz2 = kz2val(kzval(kzi, P.kzL));
+__global__ void __launch_bounds__(512, 1)
+    adj_modes_kernel(const __grid_constant__ AdjShared H, const __grid_constant__ DevParams P,
+                     const __grid_constant__ AdjPos X) {
+    using W = AG<NZ>;
+    constexpr int T = W::T, nzd = W::nz, GPW = W::GPW;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
+    double* prof = reinterpret_cast<double*>(smem_raw + W::o_prof);
+    double* kzc = reinterpret_cast<double*>(smem_raw + W::o_kz);
+    double* ekz = reinterpret_cast<double*>(smem_raw + W::o_ekz);
+    double* acc = reinterpret_cast<double*>(smem_raw + W::o_acc);
+    cplx* R = reinterpret_cast<cplx*>(smem_raw + W::o_R);
+    cplx* stg_all = reinterpret_cast<cplx*>(smem_raw + W::o_stg);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5, nth = blockDim.x;
+    const int g = lane / T, t = lane % T;
+    const AdjSeedBufs& B = H.seeds[blockIdx.y];
+    const StageConst& S = X.sc;
+    const int par = X.par;
+    const cplx* U = B.stU + (size_t)(3 * X.n + X.s) * H.nlin;
+    const cplx* lo_all = B.lamU[par];
+    const cplx* lf_all = X.s == 2 ? nullptr : B.lamF[par];
+    cplx* lu_all = B.lamU[par ^ 1];
+    cplx* lp_all = X.s == 0 ? nullptr : B.lamF[par ^ 1];
+    const double* kx0 = B.kx_pre + (size_t)X.n * P.nxy;
+    const int first = (int)blockIdx.x * H.cblocks * GPW;
+    const int end = min(P.nxy, first + H.cblocks * GPW);
+    auto stage_block = [&](int base) {
+        const int n = min(GPW, P.nxy - base) * 4 * nzd;
+        for (int i = tid; i < n; i += nth) cp_async16(stg_all + i, U + (size_t)base * 4 * nzd + i);
+        cp_async_commit();
+    };
+    stage_block(first);
+    for (int i = tid; i < NZ; i += nth) {
+        tw[i] = ldc_cg(H.tw8 + i);
+        kzc[i] = kzval(i <= W::H ? i : i - NZ, P.kzL);
+    }
+    for (int i = tid; i < nzd; i += nth) {
+        ekz[i] = __ldg(H.ekz + (size_t)(2 * X.s) * nzd + i);
+        ekz[W::NZE + i] = __ldg(H.ekz + (size_t)(2 * X.s + 1) * nzd + i);
+    }
+    for (int i = tid; i < 3 * 256; i += nth) acc[i] = 0.0;
+    const double tclock = B.t_pre[X.n];
+    const double ts = __dadd_rn(tclock, S.t_off);
+    auto buf = [&](int i) { return R + (size_t)i * 256; };
+    const double Om2 = __dmul_rn(2.0, P.Omega), fac = P.fac;
+
+    for (int base = first; base < end; base += GPW) {
+        const int nv = min(GPW, end - base);
+        AdjLane M;
+        M.valid = g < nv;
+        M.m = QLGPU_CHECK_INDEX(base + min(g, nv - 1), P.nxy, H.status);
+        const cplx* stg = stg_all + (size_t)min(g, nv - 1) * 4 * nzd;
+        M.b = __ldg(H.ky + M.m);
+        M.kyi = __ldg(H.kyi + M.m);
+        M.kxi = __ldg(H.kxi + M.m);
+        const double k0 = kx0[M.m];
+        M.a = kx_at(k0, P.q, ts, M.b);
+        M.mult = M.valid ? (M.b == 0.0 ? 1.0 : 2.0) : 0.0;
+        M.kxe = __dadd_rn(M.a, __dmul_rn(__dmul_rn(P.q, S.dt_lin), M.b));
+        M.kxo = M.em_u = M.em_b = 0.0;
+        M.old_init = 0;
+        if (H.integ == INTEG_CN) {
+            // kx where the previous stage's operator was evaluated (RK3CN.cpp:119-122; the init form
+            // at the run's start, RK3CN.cpp:57), as the forward stage computes it
+            const CnRec* cn = B.cn_pre + (size_t)3 * X.n + X.s;
+            M.old_init = cn->old_init;
+            if (M.old_init) M.kxo = kx_at(k0, P.q, tclock, M.b);
+            else M.kxo = __dadd_rn(kx_at(k0, P.q, cn->t_old, M.b), __dmul_rn(__dmul_rn(P.q, cn->dtlin_old), M.b));
+        } else {
+            const double hxy = __dsub_rn(-__dmul_rn(M.kxe, M.kxe), __dmul_rn(M.b, M.b));
+            M.em_u = exp(S.linC * P.nu * hxy);
+            M.em_b = exp(S.linC * P.cb * hxy);
+        }
+        const double a = M.a, b = M.b, ab = __dmul_rn(a, b);
+        const double* __restrict__ il2row = H.ilap2 + (size_t)M.kyi * nzd;
+        const cplx* lo = lo_all + (size_t)M.m * 4 * nzd;
+        const cplx* lf = lf_all ? lf_all + (size_t)M.m * 4 * nzd : nullptr;
+        // lamF of field f at stored index s: n1 E lamU' + lamF_out
+        auto lamF = [&](int f, int s, double kz2) -> cplx {
+            cplx r = cscale(ldc(lo + f * nzd + s), __dmul_rn(S.n1, adj_e<W>(P, S, M, ekz, f, s, kz2, H.integ)));
+            if (lf) r = cadd(r, ldc(lf + f * nzd + s));
+            return r;
+        };
+        if (base != first) stage_block(base);
+        cp_async_wait_all();
+        __syncthreads();
+        // ---- fourteen inverse transforms
+#pragma unroll 1
+        for (int task = warp; task < 14; task += warps) {
+            cplx x[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int s = rdead<W>(r) ? -1 : QLGPU_CHECK_STORED(sidx<W>(t, r), nzd, H.status);
+                cplx v = mk(0.0, 0.0);
+                if (s >= 0) {
+                    const double c = kzc[t + T * r], kz2 = kz2val(c);
+                    if (task < 4) {
+                        v = cscale(stg[task * nzd + s], fac);  // R_u, R_zeta, R_b, R_eta
+                    } else if (task < 9) {
+                        const int f0 = (task == A_RBZ || task == A_RBY) ? 2 : 0;
+                        const cplx g0 = stg[f0 * nzd + s], g1 = stg[(f0 + 1) * nzd + s];
+                        const double sc = __ldg(il2row + s) * fac;
+                        const bool y = task >= A_RUY;
+                        // y: (a b) u + i c z;  z: (a c) u - i b z
+                        const double p = y ? ab : __dmul_rn(a, c), q = y ? c : -b;
+                        v = mk(fma(p, g0.x, -q * g1.y), fma(p, g0.y, q * g1.x));
+                        v = task == A_RIK ? imul(v, sc * c) : cscale(v, sc);
+                    } else {
+                        v = lamF(task == A_WB ? 2 : task == A_WZ ? 1 : task == A_WE ? 3 : 0, s, kz2);
+                        if (task == A_WU2) {
+                            const bool z0 = (M.kyi == 0 && s == 0);
+                            const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2, z0));
+                            v = cscale(v, (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF));
+                        }
+                    }
+                }
+                x[r] = v;
+            }
+            xform<W>(x, buf(task), tw, g, t);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) buf(task)[32 * r + lane] = x[r];
+        }
+        if (base == first) {
+            pdl_wait();  // the mean-field kernel of the stage
+            for (int i = tid; i < 5 * NZ; i += nth) prof[i] = __ldcg(B.prof + i);
+            pdl_next();
+        }
+        __syncthreads();
+        // ---- pointwise adjoints as inputs of nine forward transforms.  Inputs 0-6 go on in the
+        // buffers of results 0-6, so those are held in registers until every warp has read its
+        // own; inputs 7 and 8 have exchange buffers of their own.
+        const double *By = prof, *dBy = prof + NZ, *ddBy = prof + 2 * NZ, *px = prof + 3 * NZ, *py = prof + 4 * NZ;
+        auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+        auto small_task = [&](int task) {  // 7: mult py R_bz, 8: -mult py R_uz
+            cplx x[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const double my = M.mult * py[t + T * r];
+                x[r] = conjc(task == 7 ? cscale(rd(A_RBZ, r), my) : cscale(rd(A_RUZ, r), -my));
+            }
+            cplx* xb = buf(task == 7 ? A_X0 : A_X1);
+            xform<W>(x, xb, tw, g, t);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) xb[32 * r + lane] = conjc(x[r]);
+        };
+        if (warp == (warps > 8 ? 8 : 7)) small_task(7);
+        if (warp == (warps > 9 ? 9 : 6)) small_task(8);
+        cplx x[8];
+        if (warp < 7) {
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const int z = t + T * r;
+                const double bBy = b * By[z], adBy = a * dBy[z];
+                const double mx = M.mult * px[z], my = M.mult * py[z];
+                cplx o;
+                switch (warp) {
+                    case 0: o = cadd(cadd(imul(rd(A_WB, r), -bBy), imul(rd(A_WE, r), adBy)), cscale(rd(A_RBZ, r), mx)); break;
+                    case 1: o = imul(rd(A_WE, r), -bBy); break;
+                    case 2: o = csub(cadd(imul(rd(A_WZ, r), adBy), imul(rd(A_WS, r), -bBy)), cscale(rd(A_RUZ, r), mx)); break;
+                    case 3: o = imul(rd(A_WZ, r), -bBy); break;
+                    case 4:
+                        o = csub(csub(cscale(rd(A_WE, r), -ddBy[z]), cscale(rd(A_RB, r), mx)), cscale(rd(A_RBY, r), my));
+                        break;
+                    case 5:
+                        o = cadd(cadd(cscale(rd(A_WZ, r), ddBy[z]), cscale(rd(A_WU2, r), 2.0 * ab * dBy[z])),
+                                 cadd(cscale(rd(A_RU, r), mx), cscale(rd(A_RUY, r), my)));
+                        break;
+                    default: o = cscale(rd(A_WE, r), -2.0 * dBy[z]); break;
+                }
+                x[r] = conjc(o);
+            }
+        } else if (warp == 7 && M.valid) {
+            // adjoint of the mean-field profiles: Re(conj(multiplier * R) W) per term
+            auto re_cw = [](cplx p, cplx w) { return p.x * w.x + p.y * w.y; };   // Re(conj(p) w)
+            auto re_icw = [](cplx p, cplx w) { return p.y * w.x - p.x * w.y; };  // Re(i conj(p) w)
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const cplx Wb = rd(A_WB, r), Wz = rd(A_WZ, r), We = rd(A_WE, r), WS = rd(A_WS, r);
+                const cplx Ru = rd(A_RU, r), Rb = rd(A_RB, r), Rbz = rd(A_RBZ, r);
+                double* ac = acc + 32 * r + lane;
+                ac[0] += -b * (re_icw(Ru, Wb) + re_icw(rd(A_RE, r), Wz) + re_icw(rd(A_RZ, r), We) + re_icw(Rb, WS));
+                ac[256] += a * (re_icw(Rb, Wz) + re_icw(Ru, We)) - 2.0 * re_cw(rd(A_RIK, r), We) +
+                           2.0 * ab * re_cw(Rbz, rd(A_WU2, r));
+                ac[512] += re_cw(Rbz, Wz) - re_cw(rd(A_RUZ, r), We);
+            }
+        }
+        __syncthreads();
+        if (warp < 7) {
+            cplx* xb = buf(warp);
+            xform<W>(x, xb, tw, g, t);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) xb[32 * r + lane] = conjc(x[r]);
+        }
+        __syncthreads();
+        // ---- spectral chain to (u, zeta, b, eta), linear terms, RK adjoint: field f, half of the
+        // registers per task
+#pragma unroll 1
+        for (int task = warp; task < 8; task += warps) {
+            const int f = task >> 1, h = task & 1;
+            if (!M.valid) continue;
+            const size_t at = ((size_t)M.m * 4 + f) * nzd;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = 4 * h + i;
+                const int s = QLGPU_CHECK_STORED(sidx<W>(t, r), nzd, H.status);
+                if (s < 0) continue;
+                const int rl = 32 * r + lane;
+                const double c = kzc[t + T * r], kz2 = kz2val(c);
+                const bool z0 = (M.kyi == 0 && s == 0);
+                const double il2 = __ldg(il2row + s);
+                const cplx mu = cscale(ldc(lo + f * nzd + s), adj_e<W>(P, S, M, ekz, f, s, kz2, H.integ));
+                cplx v = mu;
+                if (H.integ == INTEG_CN) {
+                    // the direct term (1 + linC Lold) D lamU' (RK3CN.cpp:107)
+                    const double lo_lap = M.old_init ? lap_init<MODEL_BQLIN>(P, M.kxo, lap2val(b, kz2, z0))
+                                                     : lap_end<MODEL_BQLIN>(P, M.kxo, b, kz2);
+                    v = cscale(mu, __dadd_rn(1.0, __dmul_rn(S.linC, linop_f<MODEL_BQLIN>(P, lo_lap, f))));
+                }
+                v = cadd(v, cscale(buf(f)[rl], fac));
+                // uz = (a c u - i b zeta) il2, i c uz, uy = (a b u + i c zeta) il2 (b, eta likewise)
+                const cplx lz = f < 2 ? cscale(csub(buf(4)[rl], imul(buf(6)[rl], c)), fac) : cscale(buf(5)[rl], fac);
+                const cplx ly = cscale(buf(f < 2 ? A_X0 : A_X1)[rl], fac);
+                if (f == 0 || f == 2) {
+                    v = cadd(v, cscale(lz, __dmul_rn(a, c) * il2));
+                    v = cadd(v, cscale(ly, ab * il2));
+                } else {
+                    v = cadd(v, imul(lz, b * il2));
+                    v = cadd(v, imul(ly, -c * il2));
+                }
+                if (f < 2) {
+                    const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2, z0));
+                    const double ilapF = (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF);
+                    const cplx l0 = lamF(0, s, kz2);
+                    if (f == 0) {
+                        // linear terms of F_zeta ((q - 2 Omega) i c u) and F_u (ilapF 2 a b q u)
+                        v = cadd(v, imul(lamF(1, s, kz2), -(P.q - Om2) * c));
+                        v = cadd(v, cscale(l0, ilapF * 2.0 * ab * P.q));
+                    } else {
+                        v = cadd(v, imul(l0, -Om2 * c * ilapF));  // linear term of F_u: ilapF 2 Omega i c zeta
+                    }
+                } else if (f == 2) {
+                    v = cadd(v, imul(lamF(3, s, kz2), P.q * c));  // linear term of F_eta: -q i c b
+                }
+                if (X.s == 0 && X.n > 0) {
+                    // this stage's input is the post-step state of step n - 1: the remap's adjoint (the
+                    // fields of a remapped mode were set to zero, MHD_BQlin.cpp:319-329) and J's gradient
+                    // there, d/db = 2 a b_y il2 b + i c il2 eta, d/deta = -i c il2 b (MHD_BQlin.cpp:388-392,424)
+                    const bool remapped = B.kx_pre[(size_t)(X.n - 1) * P.nxy + M.m] != kx0[M.m];
+                    const double w = H.weight * P.divfac * M.mult;
+                    if (f == 2)
+                        v = cadd(v, cscale(cadd(cscale(stg[2 * nzd + s], 2.0 * ab * il2),
+                                                imul(stg[3 * nzd + s], c * il2)), w));
+                    if (f == 3) v = cadd(v, cscale(imul(stg[2 * nzd + s], -c * il2), w));
+                    if (remapped) v = mk(0.0, 0.0);
+                }
+                stc(lu_all + at + s, v);
+                if (lp_all) stc(lp_all + at + s, cscale(mu, S.n2));
+            }
+        }
+        __syncthreads();
+    }
+    // ---- the chunk's sum of the profile adjoints (modes of a block in order, then blocks)
+    double* out = B.bpart + (size_t)blockIdx.x * 3 * NZ;
+    for (int i = tid; i < 3 * NZ; i += nth) {
+        const int e = i / NZ, z = i % NZ;
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < GPW; ++q) s += acc[256 * e + 32 * (z / T) + q * T + z % T];
+        out[i] = s;
+    }
+}
+
+// Mean-field side of the adjoint, one CTA per seed.  post (the stage X just reversed):
+// lamB_y += fac (T(pBy) - i c T(pdBy) - c^2 T(pddBy)), the adjoint of the stage's
+// mean-field profiles (MHD_BQlin.cpp:122-127).  pre (the next stage Y): the forward
+// profiles By, dBy, ddBy of its input and the RK / mean-field-rhs adjoint of B:
+//   muB = E_B lamB', lamG = n1 muB + lamG_out, lamB = muB - q lamG_y e_x,
+//   lamGp = n2 muB,  p(z) = Re sum_{s=1..H} h_s e^{+i k_s z},
+//   h_s = rs_fac (-i kz_s) (lamEMF[s] + conj(lamEMF[nz-s])).
+constexpr int ADJ_MF_THREADS = 512;
+
+template <int NZ>
+__global__ void __launch_bounds__(ADJ_MF_THREADS, 1)
+    adj_mf_kernel(const __grid_constant__ AdjShared H, const __grid_constant__ DevParams P,
+                  const __grid_constant__ AdjPos X, const __grid_constant__ AdjPos Y, int post, int pre) {
+    using W = AG<NZ>;
+    constexpr int T = W::T, nzd = W::nz;
+    constexpr int SPLIT = NZ <= 128 ? 4 : 2;  // threads that share a sum over the chunks
+    __shared__ __align__(16) cplx tw[NZ];
+    __shared__ __align__(16) cplx xch[3][256];
+    __shared__ __align__(16) cplx lamB[2][nzd], lamG[2][nzd];
+    __shared__ double tot[3 * NZ];
+    __shared__ __align__(16) double psum[SPLIT][3 * NZ];  // then the spectra of the sums
+    static_assert(SPLIT >= 2, "the spectra take two doubles per value");
+    cplx(*spec)[NZ] = reinterpret_cast<cplx(*)[NZ]>(&psum[0][0]);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = blockDim.x;
+    const int g = lane / T, t = lane % T;
+    const AdjSeedBufs& B = H.seeds[blockIdx.y];
+    const int pp = post ? X.par ^ 1 : Y.par;  // the buffers the pre part reads
+    cplx* lamBg = B.lamB[pp];
+    for (int i = tid; i < NZ; i += nth) tw[i] = ldc_cg(H.tw8 + i);
+    for (int i = tid; i < 2 * nzd; i += nth) lamB[i / nzd][i % nzd] = ldc(lamBg + i);
+    __syncthreads();
+    // forward profiles of the next stage's input: warp w transforms profiles w GPW ... (they
+    // do not depend on the stage being reversed)
+    constexpr int PW = (3 + W::GPW - 1) / W::GPW;  // warps of the three profiles
+    cplx x[8];
+    const int arr = warp * W::GPW + g;
+    if (pre && warp < PW) {
+        const cplx* By = B.stB + (size_t)(3 * Y.n + Y.s) * H.nmfe + nzd;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+            cplx v = mk(0.0, 0.0);
+            if (s >= 0 && arr < 3) {
+                const int k = t + T * r;
+                const double c = kzval(k <= W::H ? k : k - NZ, P.kzL);
+                v = cscale(ldc(By + s), P.fac);
+                if (arr == 1) v = imul(v, c);
+                if (arr == 2) v = cscale(v, kz2val(c));
+            }
+            x[r] = v;
+        }
+        xform<W>(x, xch[warp], tw, g, t);
+    }
+    pdl_wait();
+    pdl_next();
+    if (pre && warp < PW && arr < 3) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) B.prof[arr * NZ + t + T * r] = x[r].x;
+    }
+    if (post) {
+        // chunk sums: SPLIT runs of consecutive chunks per value, each in order, then the runs
+        const int len = (H.nchunk + SPLIT - 1) / SPLIT;
+        for (int i = tid; i < 3 * NZ * SPLIT; i += nth) {
+            const int j = i / (3 * NZ), idx = i - j * (3 * NZ);
+            const int c0 = j * len, c1 = min(H.nchunk, c0 + len);
+            double s = 0.0;
+            for (int c = c0; c < c1; c += 16) {
+                double v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) v[u] = c + u < c1 ? __ldcg(B.bpart + (size_t)(c + u) * 3 * NZ + idx) : 0.0;
+#pragma unroll
+                for (int u = 0; u < 16; ++u) s += v[u];
+            }
+            psum[j][idx] = s;
+        }
+        __syncthreads();
+        for (int i = tid; i < 3 * NZ; i += nth) {
+            double s = 0.0;
+#pragma unroll
+            for (int j = 0; j < SPLIT; ++j) s += psum[j][i];
+            tot[i] = s;
+        }
+        __syncthreads();
+        if (warp < PW) {
+            cplx y[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) y[r] = mk(arr < 3 ? tot[arr * NZ + t + T * r] : 0.0, 0.0);
+            xform<W>(y, xch[warp], tw, g, t);
+            if (arr < 3) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) spec[arr][t + T * r] = conjc(y[r]);
+            }
+        }
+        __syncthreads();
+        for (int s = tid; s < nzd; s += nth) {
+            const int k = s <= W::H ? s : s + (NZ - nzd);
+            const double c = kzval(s <= W::H ? s : s - nzd, P.kzL);
+            const cplx v = cadd(cadd(spec[0][k], imul(spec[1][k], -c)), cscale(spec[2][k], kz2val(c)));
+            lamB[1][s] = cadd(lamB[1][s], cscale(v, P.fac));
+            stc(lamBg + nzd + s, lamB[1][s]);
+        }
+        __syncthreads();
+    }
+    if (!pre) return;
+    const StageConst& S = Y.sc;
+    const cplx* lamG_out = Y.s == 2 ? nullptr : B.lamG[Y.par];
+    cplx* lamGp = Y.s == 0 ? nullptr : B.lamG[Y.par ^ 1];
+    cplx* lamB_in = B.lamB[Y.par ^ 1];
+    for (int s = tid; s < nzd; s += nth) {
+        const double kz2 = kz2val(kzval(s <= W::H ? s : s - nzd, P.kzL));
         const double Lm = P.ql ? __dmul_rn(P.eta, kz2) : 0.0;
         // exp(linC Lm), or D = 1/(1 - linC Lm) and the direct term (1 + linC Lm) D for RK3CN
-        const double e = A.integ == INTEG_CN ? __drcp_rn(__dsub_rn(1.0, __dmul_rn(S.linC, Lm)))
+        const double e = H.integ == INTEG_CN ? __drcp_rn(__dsub_rn(1.0, __dmul_rn(S.linC, Lm)))
                                              : exp(__dmul_rn(S.linC, Lm));
-        const cplx muB = cscale(A.lamB_out[m * nz + s], e);
-        cplx lg = cscale(muB, S.n1);
-        if (A.lamG_out) lg = cadd(lg, A.lamG_out[m * nz + s]);
-        lamG[m][s] = lg;
-        if (A.lamGp) A.lamGp[m * nz + s] = cscale(muB, S.n2);
-        A.lamB_in[m * nz + s] =
-            A.integ == INTEG_CN ? cscale(muB, __dadd_rn(1.0, __dmul_rn(S.linC, Lm))) : muB;
-    }
-    __syncthreads();
-    if (tid < 2 * nz && P.ql) {
-        // G_By = -q Bx + EMF_y (MHD_BQlin.cpp:274-276)
-        if (tid < nz) A.lamB_in[tid] = csub(A.lamB_in[tid], cscale(lamG[1][tid], P.q));
-    }
-    const int g = tid / G::T, t = tid % G::T, lane = tid & 31;
-    const unsigned gmask = (G::T == 32 ? 0xffffffffu : (((1u << G::T) - 1u) << ((lane / G::T) * G::T)));
-    if (g < 5) {
-        cplx x[G::P];
+        cplx nb[2];
 #pragma unroll
-        for (int k2 = 0; k2 < G::P; ++k2) {
-            const int k = t + G::T * k2;
-            const int s = stored_index<G>(k);
-            cplx v = mk(0.0, 0.0);
-            if (s >= 0) {
-                const double c = kzval(kz_int<G>(k), P.kzL);
-                if (g < 3) {
-                    v = cscale(A.B[1 * nz + s], P.fac);
-                    if (g == 1) v = imul(v, c);
-                    if (g == 2) v = cscale(v, kz2val(c));
-                } else if (P.ql && s >= 1 && s <= G::H) {
-                    const cplx l = lamG[g - 3][s], lm = conjc(lamG[g - 3][nz - s]);
-                    v = imul(cadd(l, lm), -c * P.rs_fac);
-                }
-            }
-            x[k2] = v;
+        for (int m = 0; m < 2; ++m) {
+            const cplx muB = cscale(lamB[m][s], e);
+            cplx lg = cscale(muB, S.n1);
+            if (lamG_out) lg = cadd(lg, ldc(lamG_out + m * nzd + s));
+            lamG[m][s] = lg;
+            if (lamGp) stc(lamGp + m * nzd + s, cscale(muB, S.n2));
+            nb[m] = H.integ == INTEG_CN ? cscale(muB, __dadd_rn(1.0, __dmul_rn(S.linC, Lm))) : muB;
         }
-        inv_fft<G>(x, xchs[g], tw_s, t, gmask);
-#pragma unroll
-        for (int j = 0; j < G::P; ++j) A.prof[g * NZ + zpos<G>(t, j)] = x[j].x;
-    }
-}
-
-template <int NZ>
-__global__ void adj_mf_pre_kernel(const __grid_constant__ AdjMfArgs A, const __grid_constant__ DevParams P) {
-    adj_mf_pre_body<NZ>(A, P);
-}
-
-template <int NZ>
-__global__ void adj_mf_pre_seeds_kernel(const __grid_constant__ AdjMfArgs base, const __grid_constant__ DevParams P,
-                                        const __grid_constant__ AdjRevPos X) {
-    __shared__ __align__(16) AdjMfArgs sM;
-    if (threadIdx.x == 0) {
-        const AdjSeedBufs& B = X.seeds[blockIdx.y];
-        const int p = X.par;
-        sM = base;
-        sM.B = B.stB + ((size_t)X.n * 3 + X.s) * X.nmfe;
-        sM.lamB_out = B.lamB[p];
-        sM.lamG_out = X.s == 2 ? nullptr : B.lamG[p];
-        sM.lamB_in = B.lamB[p ^ 1];
-        sM.lamGp = X.s == 0 ? nullptr : B.lamG[p ^ 1];
-        sM.prof = B.prof;
+        // G_By = -q Bx + EMF_y (MHD_BQlin.cpp:274-276)
+        if (P.ql) nb[0] = csub(nb[0], cscale(lamG[1][s], P.q));
+        stc(lamB_in + s, nb[0]);
+        stc(lamB_in + nzd + s, nb[1]);
     }
     __syncthreads();
-    adj_mf_pre_body<NZ>(sM, P);
-}
-
-// Sum of the per-mode profile adjoints over modes, one warp per (profile, z),
-// fixed order (lane-strided partial sums, then a shuffle tree).
-__device__ __forceinline__ void adj_bsum_body(const double* bpart, int nxy, int n_out, double* bsum) {
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= n_out) return;
-    const double* row = bpart + (size_t)w * nxy;
-    double s = 0.0;
-    for (int m = lane; m < nxy; m += 32) s += row[m];
+    constexpr int QW = (2 + W::GPW - 1) / W::GPW;  // warps of px, py
+    if (warp < QW) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (lane == 0) bsum[w] = s;
-}
-
-__global__ void adj_bsum_kernel(const double* bpart, int nxy, int n_out, double* bsum) {
-    adj_bsum_body(bpart, nxy, n_out, bsum);
-}
-
-__global__ void adj_bsum_seeds_kernel(const __grid_constant__ AdjRevPos X, int n_out) {
-    const AdjSeedBufs& B = X.seeds[blockIdx.y];
-    adj_bsum_body(B.bpart, (int)X.nxy, n_out, B.bsum);
-}
-
-// lamB_y += fac (T(pBy) - i c T(pdBy) - c^2 T(pddBy)): the adjoint of the
-// mean-field profiles of the stage (MHD_BQlin.cpp:122-127).  One CTA.
-template <int NZ>
-__device__ __forceinline__ void adj_mf_post_body(const double* bsum, const cplx* tw, const DevParams& P,
-                                                 cplx* lamB_in) {
-    using G = Geom<NZ>;
-    __shared__ __align__(16) cplx tw_s[NZ];
-    __shared__ __align__(16) cplx xchs[3][G::XSIZE];
-    __shared__ __align__(16) cplx spec[3][NZ];
-    const int tid = threadIdx.x;
-    for (int i = tid; i < NZ; i += blockDim.x) tw_s[i] = tw[i];
-    __syncthreads();
-    const int g = tid / G::T, t = tid % G::T, lane = tid & 31;
-    const unsigned gmask = (G::T == 32 ? 0xffffffffu : (((1u << G::T) - 1u) << ((lane / G::T) * G::T)));
-    if (g < 3) {
-        cplx x[G::P];
+        for (int r = 0; r < 8; ++r) {
+            const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+            cplx v = mk(0.0, 0.0);
+            if (P.ql && arr < 2 && s >= 1 && s <= W::H) {
+                const double c = kzval(s, P.kzL);
+                v = imul(cadd(lamG[arr][s], conjc(lamG[arr][nzd - s])), -c * P.rs_fac);
+            }
+            x[r] = v;
+        }
+        xform<W>(x, xch[warp], tw, g, t);
+        if (arr < 2) {
 #pragma unroll
-        for (int j = 0; j < G::P; ++j) x[j] = mk(bsum[g * NZ + zpos<G>(t, j)], 0.0);
-        fwd_fft<G>(x, xchs[g], tw_s, t, gmask);
-#pragma unroll
-        for (int k2 = 0; k2 < G::P; ++k2) spec[g][t + G::T * k2] = x[k2];
-    }
-    __syncthreads();
-    const int nz = P.nz;
-    for (int s = tid; s < nz; s += blockDim.x) {
-        const int k = s <= G::H ? s : s + (NZ - nz);
-        const int kzi = s <= G::H ? s : s - nz;
-        const double c = kzval(kzi, P.kzL);
-        cplx v = cadd(cadd(spec[0][k], imul(spec[1][k], -c)), cscale(spec[2][k], kz2val(c)));
-        lamB_in[nz + s] = cadd(lamB_in[nz + s], cscale(v, P.fac));
+            for (int r = 0; r < 8; ++r) B.prof[(3 + arr) * NZ + t + T * r] = x[r].x;
+        }
     }
 }
 
-template <int NZ>
-__global__ void adj_mf_post_kernel(const double* bsum, const cplx* tw, const __grid_constant__ DevParams P,
-                                   cplx* lamB_in) {
-    adj_mf_post_body<NZ>(bsum, tw, P, lamB_in);
-}
-
-template <int NZ>
-__global__ void adj_mf_post_seeds_kernel(const cplx* tw, const __grid_constant__ DevParams P,
-                                         const __grid_constant__ AdjRevPos X) {
-    const AdjSeedBufs& B = X.seeds[blockIdx.y];
-    adj_mf_post_body<NZ>(B.bsum, tw, P, B.lamB[X.par ^ 1]);
-}
-
-// Gradient of (weight) * AM_b at a post-step state (MHD_BQlin.cpp:388-392,424):
-// AM_b = divfac sum mult Re(b conj(by)), by = (a b_y b + i c eta) il2 gives
-// d/db = 2 a b_y il2 b + i c il2 eta, d/deta = -i c il2 b.  Adds to lamU.
-template <int NZ>
-__device__ __forceinline__ void adj_jgrad_body(const cplx* U, const double* kx0, const double* ky, const int* kyi,
-                                               const double* ilap2, const DevParams& P, double t_host,
-                                               const double* t_dev, double weight, cplx* lamU) {
-    using G = Geom<NZ>;
-    const int nz = P.nz;
-    const double t = t_dev ? *t_dev : t_host;
+// The window's last step: J's gradient at the window's end state and the adjoint of the
+// last step's remap (the other steps' are part of adj_modes_kernel).
+__global__ void adj_jgrad_kernel(const __grid_constant__ AdjShared H, const __grid_constant__ DevParams P,
+                                 const __grid_constant__ AdjPos X) {
+    const AdjSeedBufs& B = H.seeds[blockIdx.y];
+    const int nz = P.nz, HH = (nz - 1) / 2;
+    const double t = B.t_pre[X.steps];
+    const double* kx_before = B.kx_pre + (size_t)(X.steps - 1) * P.nxy;
+    cplx* lamU = B.lamU[X.par];
     const size_t n = (size_t)P.nxy * nz;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const int mode = (int)(i / nz), s = (int)(i % nz);
-        const double kyv = ky[mode];
-        const double a = kx_at(kx0[mode], P.q, t, kyv);
+        const double kyv = H.ky[mode];
+        const double a = kx_at(B.kx_post[mode], P.q, t, kyv);
         const double ab = __dmul_rn(a, kyv);
-        const int kzi = s <= G::H ? s : s - nz;
-        const double c = kzval(kzi, P.kzL);
-        const double il2 = ilap2[(size_t)kyi[mode] * nz + s];
-        const double w = weight * P.divfac * (kyv == 0.0 ? 1.0 : 2.0);
-        const cplx* u = U + (size_t)mode * 4 * nz;
-        const cplx bb = u[2 * nz + s], ee = u[3 * nz + s];
+        const double c = kzval(s <= HH ? s : s - nz, P.kzL);
+        const double il2 = H.ilap2[(size_t)H.kyi[mode] * nz + s];
+        const double w = H.weight * P.divfac * (kyv == 0.0 ? 1.0 : 2.0);
+        const cplx* u = B.postU + (size_t)mode * 4 * nz;
         cplx* l = lamU + (size_t)mode * 4 * nz;
+        if (kx_before[mode] != B.kx_post[mode]) {
+            for (int f = 0; f < 4; ++f) l[f * nz + s] = mk(0.0, 0.0);
+            continue;
+        }
+        const cplx bb = u[2 * nz + s], ee = u[3 * nz + s];
         const cplx gb = cadd(cscale(bb, 2.0 * ab * il2), imul(ee, c * il2));
         const cplx ge = imul(bb, -c * il2);
         l[2 * nz + s] = cadd(l[2 * nz + s], cscale(gb, w));
         l[3 * nz + s] = cadd(l[3 * nz + s], cscale(ge, w));
     }
-}
-
-template <int NZ>
-__global__ void adj_jgrad_kernel(const cplx* U, const double* kx0, const double* ky, const int* kyi,
-                                 const double* ilap2, const __grid_constant__ DevParams P, double t_host,
-                                 const double* t_dev, double weight, cplx* lamU) {
-    adj_jgrad_body<NZ>(U, kx0, ky, kyi, ilap2, P, t_host, t_dev, weight, lamU);
-}
-
-// J's gradient at the post-step state of step n (seed = blockIdx.y)
-template <int NZ>
-__global__ void adj_jgrad_seeds_kernel(const double* ky, const int* kyi, const double* ilap2,
-                                       const __grid_constant__ DevParams P, const __grid_constant__ AdjRevPos X) {
-    const AdjSeedBufs& B = X.seeds[blockIdx.y];
-    adj_jgrad_body<NZ>(adj_upost(B, X), adj_kxpost(B, X), ky, kyi, ilap2, P, 0.0, B.t_pre + X.n + 1, X.weight,
-                       B.lamU[X.par]);
-}
-
-// Adjoint of the shearing-box remap (MHD_BQlin.cpp:319-329): the fields of a
-// remapped mode were set to zero, so their adjoint is zero.
-__device__ __forceinline__ void adj_remap_body(const double* kx0_before, const double* kx0_after, int nxy, int nz,
-                                               cplx* lamU) {
-    const size_t n = (size_t)nxy * 4 * nz;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const int mode = (int)(i / (4 * (size_t)nz));
-        if (kx0_before[mode] != kx0_after[mode]) lamU[i] = mk(0.0, 0.0);
-    }
-}
-
-__global__ void adj_remap_kernel(const double* kx0_before, const double* kx0_after, int nxy, int nz, cplx* lamU) {
-    adj_remap_body(kx0_before, kx0_after, nxy, nz, lamU);
-}
-
-__global__ void adj_remap_seeds_kernel(const __grid_constant__ AdjRevPos X, int nz) {
-    const AdjSeedBufs& B = X.seeds[blockIdx.y];
-    adj_remap_body(B.kx_pre + (size_t)X.n * X.nxy, adj_kxpost(B, X), (int)X.nxy, nz, B.lamU[X.par]);
 }
 
 }  // namespace qlgpu

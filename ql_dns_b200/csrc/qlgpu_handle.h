@@ -64,6 +64,11 @@ struct qlgpu_handle {
     unsigned long long steps_taken = 0;  // since set_state; the noise counter's step word
     double* d_forcing = nullptr;         // [0..3] last rhs mean-field maxima, [4..7] current, [8] step start time
     double* d_kx0_prev = nullptr;        // kx0 at the start of the step (noise)
+    // the adjoint's workspace and its table of seeds, kept for the next call and freed with the handle
+    void* adj_ws = nullptr;
+    size_t adj_bytes = 0;
+    void* adj_tab = nullptr;
+    int adj_tab_cap = 0;
     bool ekz_dynamic = false;            // stage exp(kz) factors computed in the kernel (variable dt)
 };
 
