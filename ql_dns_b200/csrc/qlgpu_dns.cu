@@ -25,26 +25,29 @@ namespace {
 
 using KernFn = void (*)(DnsArgs);
 
+template <int NZ, int MX>
+void set_zx(KernFn* inv, KernFn* fwd, size_t* s_zx) {
+    *inv = dns_inv_zx<NZ, MX>;
+    *fwd = dns_fwd_xz<MX, NZ>;
+    *s_zx = PlaneZX<NZ, MX>::BYTES;
+}
 template <int NZ>
-bool pick_zx(int MX, KernFn* inv, KernFn* fwd, size_t* s_inv, size_t* s_fwd, int ncol) {
+bool pick_zx(int MX, KernFn* inv, KernFn* fwd, size_t* s_zx) {
     switch (MX) {
-        case 16: *inv = dns_inv_zx<NZ, 16>; *fwd = dns_fwd_xz<16, NZ>;
-                 *s_inv = InvZX<NZ, 16>::smem(ncol); *s_fwd = FwdXZ<16, NZ>::smem(ncol); return true;
-        case 32: *inv = dns_inv_zx<NZ, 32>; *fwd = dns_fwd_xz<32, NZ>;
-                 *s_inv = InvZX<NZ, 32>::smem(ncol); *s_fwd = FwdXZ<32, NZ>::smem(ncol); return true;
-        case 64: *inv = dns_inv_zx<NZ, 64>; *fwd = dns_fwd_xz<64, NZ>;
-                 *s_inv = InvZX<NZ, 64>::smem(ncol); *s_fwd = FwdXZ<64, NZ>::smem(ncol); return true;
+        case 16: set_zx<NZ, 16>(inv, fwd, s_zx); return true;
+        case 32: set_zx<NZ, 32>(inv, fwd, s_zx); return true;
+        case 64: set_zx<NZ, 64>(inv, fwd, s_zx); return true;
         default: return false;
     }
 }
 
-bool pick_kernels(int NZ, int MX, int MY, int ncol, KernFn* inv, KernFn* fwd, KernFn* phys, size_t* s_inv,
-                  size_t* s_fwd, size_t* s_phys, int* zc, int* phys_threads) {
+bool pick_kernels(int NZ, int MX, int MY, KernFn* inv, KernFn* fwd, KernFn* phys, size_t* s_zx, size_t* s_phys,
+                  int* zc, int* phys_threads) {
     bool ok = false;
     switch (NZ) {
-        case 16: ok = pick_zx<16>(MX, inv, fwd, s_inv, s_fwd, ncol); break;
-        case 32: ok = pick_zx<32>(MX, inv, fwd, s_inv, s_fwd, ncol); break;
-        case 64: ok = pick_zx<64>(MX, inv, fwd, s_inv, s_fwd, ncol); break;
+        case 16: ok = pick_zx<16>(MX, inv, fwd, s_zx); break;
+        case 32: ok = pick_zx<32>(MX, inv, fwd, s_zx); break;
+        case 64: ok = pick_zx<64>(MX, inv, fwd, s_zx); break;
         default: return false;
     }
     if (!ok) return false;
@@ -71,7 +74,7 @@ struct qlgpu_dns {
     DnsArgs a{};
     DnsStage st[3]{};
     KernFn k_inv = nullptr, k_fwd = nullptr, k_phys = nullptr;
-    size_t s_inv = 0, s_fwd = 0, s_phys = 0;
+    size_t s_zx = 0, s_phys = 0;
     int zc = 16, phys_threads = 256;
     double t = 0.0;
     double divf = 0.0, kzmax = 0.0;
@@ -158,10 +161,10 @@ static cudaError_t launch_pdl(void (*k)(Args...), dim3 grid, int block, size_t s
 // Products of the current state: launches A, B, C.
 static cudaError_t enqueue_products(qlgpu_dns* h) {
     const DnsArgs& a = h->a;
-    cudaError_t e = launch_pdl(h->k_inv, dim3(h->Kyn, 6), BLOCK, h->s_inv, h->stream, a);
+    cudaError_t e = launch_pdl(h->k_inv, dim3(h->Kyn, 6), 32 * ZX_WARPS, h->s_zx, h->stream, a);
     if (e == cudaSuccess)
         e = launch_pdl(h->k_phys, dim3(h->p.Mx, h->p.NZ / h->zc), h->phys_threads, h->s_phys, h->stream, a);
-    if (e == cudaSuccess) e = launch_pdl(h->k_fwd, dim3(h->Kyn, NPROD), BLOCK, h->s_fwd, h->stream, a);
+    if (e == cudaSuccess) e = launch_pdl(h->k_fwd, dim3(h->Kyn, NPROD), 32 * ZX_WARPS, h->s_zx, h->stream, a);
     return e;
 }
 
@@ -173,9 +176,7 @@ static cudaError_t enqueue_step(qlgpu_dns* h) {
             e = launch_pdl(dns_update, dim3((n + BLOCK - 1) / BLOCK), BLOCK, 0, h->stream, h->a, h->st[s]);
         if (e != cudaSuccess) return e;
     }
-    cudaError_t e = launch_pdl(dns_remap_kx, dim3((h->nxy + 255) / 256), 256, 0, h->stream, h->a);
-    if (e == cudaSuccess) e = launch_pdl(dns_advance_clock, dim3(1), 32, 0, h->stream, h->a);
-    return e;
+    return launch_pdl(dns_end_step, dim3(1), 1024, 0, h->stream, h->a);
 }
 
 static cudaError_t enqueue_diag(qlgpu_dns* h) {
@@ -219,8 +220,8 @@ int qlgpu_dns_create(const qlgpu_dns_params* p, int device, qlgpu_dns_t** out) {
     h->ncol = qp.nx - 1;
     h->nxy = h->ncol * h->Kyn;
     h->nz = stored_nz(p->NZ);
-    if (!pick_kernels(p->NZ, p->Mx, p->My, h->ncol, &h->k_inv, &h->k_fwd, &h->k_phys, &h->s_inv, &h->s_fwd,
-                      &h->s_phys, &h->zc, &h->phys_threads)) {
+    if (!pick_kernels(p->NZ, p->Mx, p->My, &h->k_inv, &h->k_fwd, &h->k_phys, &h->s_zx, &h->s_phys, &h->zc,
+                      &h->phys_threads)) {
         delete h;
         return fail(nullptr, QLGPU_ERR_UNSUPPORTED, "grid combination not built");
     }
@@ -277,9 +278,9 @@ int qlgpu_dns_create(const qlgpu_dns_params* p, int device, qlgpu_dns_t** out) {
     DNS_AL(h->d_rec, 15 * sizeof(double));
 #undef DNS_AL
     if (rc == QLGPU_OK) {
-        std::vector<double> twz = twiddles(p->NZ, group_threads(p->NZ));
-        std::vector<double> twx = twiddles(p->Mx, group_threads(p->Mx));
-        std::vector<double> twy = twiddles(p->My, group_threads(p->My));
+        std::vector<double> twz = twiddles(p->NZ, p->NZ / 8);
+        std::vector<double> twx = twiddles(p->Mx, p->Mx / 8);
+        std::vector<double> twy = twiddles(p->My, p->My / 8);
         cudaError_t e3 = cudaSuccess;
         if (e3 == cudaSuccess) e3 = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
         if (e3 == cudaSuccess) e3 = cudaMemcpy((void*)a.ky, ky.data(), h->nxy * sizeof(double), cudaMemcpyHostToDevice);
@@ -293,8 +294,8 @@ int qlgpu_dns_create(const qlgpu_dns_params* p, int device, qlgpu_dns_t** out) {
         if (e3 == cudaSuccess) e3 = cudaMemset(a.F[1], 0, ns * sizeof(cplx));
         if (e3 == cudaSuccess) e3 = cudaMemset(a.clock, 0, 2 * sizeof(double));
         if (e3 == cudaSuccess) e3 = cudaMemset(a.status, 0, sizeof(int));
-        if (e3 == cudaSuccess) e3 = ensure_smem_attr((const void*)h->k_inv, h->s_inv);
-        if (e3 == cudaSuccess) e3 = ensure_smem_attr((const void*)h->k_fwd, h->s_fwd);
+        if (e3 == cudaSuccess) e3 = ensure_smem_attr((const void*)h->k_inv, h->s_zx);
+        if (e3 == cudaSuccess) e3 = ensure_smem_attr((const void*)h->k_fwd, h->s_zx);
         if (e3 == cudaSuccess) e3 = ensure_smem_attr((const void*)h->k_phys, h->s_phys);
         if (e3 == cudaSuccess) e3 = cudaEventCreate(&h->ev[0]);
         if (e3 == cudaSuccess) e3 = cudaEventCreate(&h->ev[1]);

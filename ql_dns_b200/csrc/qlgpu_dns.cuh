@@ -15,19 +15,20 @@
 //                         (RK3CN_Elin exponential or RK3CN Crank-Nicolson), the 2/3
 //                         mask in x at the next stage time, the divergence correction
 //                         and, at the last stage, the remap zeroing.
-// Transforms use the register/shared-memory FFT of qlgpu_fft.cuh (one group of
-// T threads per row).  Sign and scale: backward exp(+), forward exp(-), both
-// unnormalised; 1/(Mx My NZ) is applied when the state is loaded.
+// Transforms are the 8-points-per-thread ones of qlgpu_xform.cuh: a warp transforms
+// GPW = 256/N rows of length N at once, lane (g, t) register r holding index t + T r of
+// row g before and after.  Sign and scale: backward exp(+), forward exp(-) as
+// conj(xform(conj)), both unnormalised; 1/(Mx My NZ) is applied when the state is loaded.
 #pragma once
 #include <cuda_runtime.h>
 
 #include "qlgpu_debug.cuh"
-#include "qlgpu_fft.cuh"
+#include "qlgpu_xform.cuh"
 
 namespace qlgpu {
 namespace dns {
 
-constexpr int BLOCK = 256;
+constexpr int BLOCK = 128;  // dns_update: 5 CTAs per SM, one wave at 64 x 128 x 64
 constexpr int NPROD = 9;
 
 struct DnsArgs {
@@ -66,10 +67,19 @@ __device__ __forceinline__ void pdl_start() {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
-__device__ __forceinline__ unsigned group_mask(int T) {
-    const int lane = threadIdx.x & 31;
-    const unsigned m = (T == 32) ? 0xffffffffu : ((1u << T) - 1u);
-    return m << (lane / T * T);
+// Rows of length N: T lanes each, GPW rows per warp.
+template <int N>
+struct XG {
+    static constexpr int NZ = N;
+    static constexpr int T = N / 8;
+    static constexpr int GPW = 32 / T;
+    static constexpr int SWZ = T == 4 ? 1 : (T == 2 ? 3 : 0);
+};
+// stored kz index of spectral slot k of an NZ-point row (fftwPlans.h:66-97), -1 in the gap
+template <int NZ>
+__device__ __forceinline__ int zstored(int k) {
+    constexpr int H = NZ / 3;
+    return k <= H ? k : (k >= NZ - H ? k - (NZ - 2 * H - 1) : -1);
 }
 
 // kx(t) = kx0 + (q t) ky, rounded as the host restatement does (no contraction)
@@ -84,93 +94,127 @@ __device__ __forceinline__ int xbin(double kx0, double dkx, int M) {
 }
 
 // ---------------------------------------------------------------------------
-// A: z inverse + x inverse of one field on one ky plane
+// The ky plane of A and C in shared memory, [x][z] with the 16-byte entries of a row
+// permuted within 128 bytes by its x, so that the lanes of a transform along x or z read
+// different banks.  The transforms exchange in place, in the entries they transform, so
+// a 64 x 64 plane is 64 KB: three CTAs of 8 warps per SM, and every plane of
+// 64 x 128 x 64 (258 in A, 387 in C) is resident at once.
 // ---------------------------------------------------------------------------
-template <int NZ, int MX>
-struct InvZX {
-    using GZ = Geom<NZ>;
-    using GX = Geom<MX>;
-    static constexpr int SROW = NZ + 1;  // padded rows (bank spread)
-    static constexpr int XZ = (BLOCK / GZ::T) * GZ::XSIZE;
-    static constexpr int XX = (BLOCK / GX::T) * GX::XSIZE;
-    static constexpr int XCH = XZ > XX ? XZ : XX;
-    static size_t smem(int ncol) { return sizeof(cplx) * ((size_t)ncol * SROW + XCH) + sizeof(int) * MX; }
-};
+constexpr int ZX_WARPS = 8;
 
 template <int NZ, int MX>
-__global__ void __launch_bounds__(BLOCK, 2) dns_inv_zx(DnsArgs a) {
-    pdl_start();
-    using K = InvZX<NZ, MX>;
-    using GZ = typename K::GZ;
-    using GX = typename K::GX;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cplx* S = reinterpret_cast<cplx*>(smraw);
-    cplx* xch = S + (size_t)a.ncol * K::SROW;
-    int* bin2col = reinterpret_cast<int*>(xch + K::XCH);
-    const int ky = blockIdx.x, f = blockIdx.y, tid = threadIdx.x;
-    for (int b = tid; b < MX; b += BLOCK) bin2col[b] = -1;
-    __syncthreads();
-    for (int c = tid; c < a.ncol; c += BLOCK) bin2col[QLGPU_CHECK_INDEX(xbin(a.kx0[QLGPU_CHECK_INDEX(ky + a.Kyn * c, a.nxy, a.status)], a.dkx, MX), MX, a.status)] = c;
-    __syncthreads();
-    {  // z inverse of every column of the plane
-        constexpr int T = GZ::T, NG = BLOCK / T;
-        const int g = tid / T, t = tid % T;
-        const unsigned gm = group_mask(T);
-        cplx* xg = xch + g * GZ::XSIZE;
-        for (int c = g; c < a.ncol; c += NG) {
-            const cplx* src = a.lin + ((size_t)QLGPU_CHECK_INDEX(ky + a.Kyn * c, a.nxy, a.status) * 6 + f) * a.nz;
-            cplx x[GZ::P];
-#pragma unroll
-            for (int k2 = 0; k2 < GZ::P; ++k2) {
-                const int s = QLGPU_CHECK_STORED(stored_index<GZ>(t + T * k2), a.nz, a.status);
-                x[k2] = s >= 0 ? cscale(src[s], a.scale) : mk(0.0, 0.0);
-            }
-            inv_fft<GZ>(x, xg, a.twz, t, gm);
-#pragma unroll
-            for (int j = 0; j < GZ::P; ++j) S[c * K::SROW + zpos<GZ>(t, j)] = x[j];
-        }
-    }
-    __syncthreads();
-    {  // x inverse of every z row, stored to X[f][ky][x][z]: the groups of a warp take
-       // consecutive z, so each store instruction writes whole 32-byte sectors
-        constexpr int T = GX::T, NG = BLOCK / T;
-        const int g = tid / T, t = tid % T;
-        const unsigned gm = group_mask(T);
-        cplx* xg = xch + g * GX::XSIZE;
-        cplx* dst = a.X + ((size_t)f * a.Kyn + ky) * MX * NZ;
-        for (int z = g; z < NZ; z += NG) {
-            cplx x[GX::P];
-#pragma unroll
-            for (int k2 = 0; k2 < GX::P; ++k2) {
-                const int c = bin2col[t + T * k2];
-                x[k2] = c >= 0 ? S[c * K::SROW + z] : mk(0.0, 0.0);
-            }
-            inv_fft<GX>(x, xg, a.twx, t, gm);
-#pragma unroll
-            for (int j = 0; j < GX::P; ++j) dst[(size_t)zpos<GX>(t, j) * NZ + z] = x[j];
-        }
-    }
+struct PlaneZX {
+    static constexpr size_t BYTES = sizeof(cplx) * ((size_t)NZ * MX + NZ + MX) + sizeof(int) * MX;
+};
+template <int NZ>
+__device__ __forceinline__ int plane_at(int x, int z) {
+    return x * NZ + (z ^ (x & 7));
+}
+// x bin of every column of the plane (bin2col[b] = column or -1)
+template <int MX>
+__device__ __forceinline__ void plane_bins(const DnsArgs& a, int ky, int* bin2col) {
+    for (int c = threadIdx.x; c < a.ncol; c += blockDim.x)
+        bin2col[QLGPU_CHECK_INDEX(xbin(a.kx0[QLGPU_CHECK_INDEX(ky + a.Kyn * c, a.nxy, a.status)], a.dkx, MX), MX,
+                                  a.status)] = c;
 }
 
 // ---------------------------------------------------------------------------
-// B: y transforms and the products, per (x, chunk of z lines)
+// A: z inverse + x inverse of one field on one ky plane
+// ---------------------------------------------------------------------------
+template <int NZ, int MX>
+__global__ void __launch_bounds__(32 * ZX_WARPS, 3) dns_inv_zx(const __grid_constant__ DnsArgs a) {
+    using GZ = XG<NZ>;
+    using GX = XG<MX>;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cplx* S = reinterpret_cast<cplx*>(smraw);
+    cplx* twz = S + NZ * MX;
+    cplx* twx = twz + NZ;
+    int* bin2col = reinterpret_cast<int*>(twx + MX);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = blockDim.x;
+    const int ky = blockIdx.x, f = blockIdx.y;
+    for (int i = tid; i < NZ; i += nth) twz[i] = a.twz[i];
+    for (int i = tid; i < MX; i += nth) twx[i] = a.twx[i];
+    for (int b = tid; b < MX; b += nth) bin2col[b] = -1;
+    __syncthreads();
+    pdl_start();
+    plane_bins<MX>(a, ky, bin2col);
+    __syncthreads();
+    {  // z inverse of every x row (zero where no column has the bin)
+        constexpr int T = GZ::T;
+        const int g = lane / T, t = lane % T;
+        for (int x0 = warp * GZ::GPW; x0 < MX; x0 += ZX_WARPS * GZ::GPW) {
+            const int xr = x0 + g, c = bin2col[xr];
+            cplx x[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) x[r] = mk(0.0, 0.0);
+            if (c >= 0) {
+                const cplx* src =
+                    a.lin + ((size_t)QLGPU_CHECK_INDEX(ky + a.Kyn * c, a.nxy, a.status) * 6 + f) * a.nz;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const int s = QLGPU_CHECK_STORED(zstored<NZ>(t + T * r), a.nz, a.status);
+                    if (s >= 0) x[r] = cscale(src[s], a.scale);
+                }
+            }
+            xform_at<GZ>(
+                x, [&](int q, int s) -> cplx& { return S[plane_at<NZ>(xr, q * T + ((s + q) & (T - 1)))]; }, twz, t);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) S[plane_at<NZ>(xr, t + T * r)] = x[r];
+        }
+    }
+    __syncthreads();
+    {  // x inverse of every z column
+        constexpr int T = GX::T;
+        const int g = lane / T, t = lane % T;
+        for (int z0 = warp * GX::GPW; z0 < NZ; z0 += ZX_WARPS * GX::GPW) {
+            const int z = z0 + g;
+            cplx x[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) x[r] = S[plane_at<NZ>(t + T * r, z)];
+            __syncwarp();
+            xform_at<GX>(
+                x, [&](int q, int s) -> cplx& { return S[plane_at<NZ>(q * T + ((s + q) & (T - 1)), z)]; }, twx, t);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) S[plane_at<NZ>(t + T * r, z)] = x[r];
+        }
+    }
+    __syncthreads();
+    cplx* dst = a.X + ((size_t)f * a.Kyn + ky) * MX * NZ;
+    for (int i = tid; i < MX * NZ; i += nth) dst[i] = S[plane_at<NZ>(i / NZ, i % NZ)];
+}
+
+// ---------------------------------------------------------------------------
+// B: y transforms and the products, per (x, chunk of ZC z lines).
+//
+// Its chain of loads, transforms and stores bounds it, and the bytes: 17 MB in, 25 MB out
+// at 64 x 128 x 64.  The chunk's spectra come in as one tile of contiguous ZC-line rows
+// (each entry is used twice, for k and for its conjugate My - k) and the products' spectra
+// leave the same way; the two real fields of a complex transform stay in the buffer it was
+// exchanged in, where the products read them at the same lane and register.  82 KB and 8
+// warps: two CTAs per SM.
 // ---------------------------------------------------------------------------
 template <int MY>
 struct Phys {
-    using GY = Geom<MY>;
-    // 192 threads and 8 lines (4 at MY = 256) keep the shared memory near 105 KB, so two
-    // CTAs share an SM; the inverse phase (3 transforms per line) is one round of the groups
-    static constexpr int THREADS = 192;
-    static constexpr int ZC = MY >= 256 ? 4 : 8;
-    static constexpr int PY = MY + 1;
-    static constexpr int NG = THREADS / GY::T;
-    static constexpr int XS = GY::XSIZE > MY ? GY::XSIZE : MY;
-    static size_t smem() {
-        size_t ph = sizeof(double) * 6 * ZC * PY;
-        ph = (ph + 15) / 16 * 16;
-        return ph + sizeof(cplx) * (size_t)NG * XS;
-    }
+    using G = XG<MY>;
+    static constexpr int ZC = MY >= 256 ? 4 : (MY == 16 ? 16 : 8);
+    static constexpr int LT = ZC / G::GPW;              // warp-tasks per field pair
+    static constexpr int WARPS = MY >= 128 ? 8 : (MY == 64 ? 6 : 5);
+    static constexpr int THREADS = 32 * WARPS;
+    static constexpr int KYN = MY / 3 + 1;              // ky of the mode set
+    static constexpr int PPR = (WARPS + LT - 1) / LT;   // product pairs per round of the forward tasks
+    static_assert(WARPS % LT == 0, "a round of forward tasks holds whole pairs");
+    static constexpr size_t TILE = (size_t)6 * KYN * ZC, XCH = (size_t)256 * WARPS;
+    static constexpr size_t OUT = (size_t)2 * PPR * KYN * ZC;
+    static constexpr size_t WORK = TILE > XCH ? (TILE > OUT ? TILE : OUT) : (XCH > OUT ? XCH : OUT);
+    static_assert(THREADS % ZC == 0, "whole tile rows per pass");
+    static size_t smem() { return sizeof(cplx) * ((size_t)3 * ZC * MY + WORK + MY); }
 };
+// tile row (field or product, k), line l: 16-byte entries permuted within 128 bytes, so that a
+// transform's lanes (consecutive k, one line) read different banks
+template <int ZC>
+__device__ __forceinline__ int tile_at(int row, int l) {
+    return row * ZC + (l ^ (row & (ZC - 1) & 7));
+}
 
 __device__ __forceinline__ double product(int p, const double* v) {
     // v = ux, uy, uz, bx, by, bz
@@ -188,80 +232,113 @@ __device__ __forceinline__ double product(int p, const double* v) {
     }
 }
 
-template <int MY>
-__global__ void __launch_bounds__(Phys<MY>::THREADS, 2) dns_phys(DnsArgs a) {
-    pdl_start();
-    using K = Phys<MY>;
-    using GY = typename K::GY;
-    constexpr int T = GY::T, NG = K::NG, ZC = K::ZC, PY = K::PY;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    double* Ph = reinterpret_cast<double*>(smraw);
-    size_t phb = sizeof(double) * 6 * ZC * PY;
-    phb = (phb + 15) / 16 * 16;
-    cplx* xch = reinterpret_cast<cplx*>(smraw + phb);
-    const int x = blockIdx.x, z0 = blockIdx.y * ZC, tid = threadIdx.x;
-    const int g = tid / T, t = tid % T;
-    const unsigned gm = group_mask(T);
-    cplx* xg = xch + g * K::XS;
-    const int Kyn = a.Kyn, MX = a.Mx, NZ = a.NZ;
-    // inverse: three complex transforms per line carry (ux,uy), (uz,bx), (by,bz)
-    for (int task = g; task < 3 * ZC; task += NG) {
-        const int l = task % ZC, pr = task / ZC;
-        const int fa = 2 * pr, fb = 2 * pr + 1;
-        const size_t zoff = (size_t)x * NZ + z0 + l;
-        cplx v[GY::P];
+// conj of products 2 PP and 2 PP + 1 as one complex row, from the three field pairs of the lane
+template <int PP, int LT>
+__device__ __forceinline__ void product_pair(cplx (&x)[8], const cplx* ph) {
 #pragma unroll
-        for (int k2 = 0; k2 < GY::P; ++k2) {
-            const int k = t + T * k2;
+    for (int r = 0; r < 8; ++r) {
+        double f6[6];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const cplx v = ph[256 * q * LT + 32 * r];
+            f6[2 * q] = v.x;
+            f6[2 * q + 1] = v.y;
+        }
+        x[r] = mk(product(2 * PP, f6), 2 * PP + 1 < NPROD ? -product(2 * PP + 1, f6) : 0.0);
+    }
+}
+
+template <int MY>
+__global__ void __launch_bounds__(Phys<MY>::THREADS, 2) dns_phys(const __grid_constant__ DnsArgs a) {
+    using K = Phys<MY>;
+    using G = typename K::G;
+    constexpr int T = G::T, GPW = G::GPW, ZC = K::ZC, LT = K::LT, KYN = K::KYN;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cplx* Ph = reinterpret_cast<cplx*>(smraw);   // [3 LT warp-tasks][8][32]: the pairs (ux,uy), (uz,bx), (by,bz)
+    cplx* work = Ph + (size_t)3 * ZC * MY;       // input tile; then exchange buffers / output tile
+    cplx* tw = work + K::WORK;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = blockDim.x;
+    const int g = lane / T, t = lane % T;
+    const int x0 = blockIdx.x, z0 = blockIdx.y * ZC;
+    const size_t plane = (size_t)a.Mx * a.NZ;
+    const size_t off = (size_t)x0 * a.NZ + z0;
+    for (int i = tid; i < MY; i += nth) tw[i] = a.twy[i];
+    pdl_start();
+    for (int row = tid / ZC, l = tid % ZC; row < 6 * KYN; row += K::THREADS / ZC)
+        cp_async16(work + tile_at<ZC>(row, l), a.X + (size_t)row * plane + off + l);
+    cp_async_commit();
+    cp_async_wait_all();
+    __syncthreads();
+    // inverse: three complex transforms per line, c(k) = A + i B, c(My - k) = conj(A) + i conj(B)
+    for (int task = warp; task < 3 * LT; task += K::WARPS) {
+        const int pr = task / LT, l = (task % LT) * GPW + g;
+        const int ra = 2 * pr * KYN, rb = ra + KYN;  // the fields' first tile rows
+        cplx x[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int k = t + T * r;
             cplx c = mk(0.0, 0.0);
-            if (k < Kyn) {
-                cplx A = a.X[((size_t)fa * Kyn + k) * MX * NZ + zoff];
-                cplx B = a.X[((size_t)fb * Kyn + k) * MX * NZ + zoff];
+            if (k < KYN) {
+                cplx A = work[tile_at<ZC>(ra + k, l)], B = work[tile_at<ZC>(rb + k, l)];
                 if (k == 0) { A.y = 0.0; B.y = 0.0; }
                 c = mk(A.x - B.y, A.y + B.x);
-            } else if (k > MY - Kyn) {
+            } else if (k > MY - KYN) {
                 const int kk = MY - k;
-                const cplx A = a.X[((size_t)fa * Kyn + kk) * MX * NZ + zoff];
-                const cplx B = a.X[((size_t)fb * Kyn + kk) * MX * NZ + zoff];
+                const cplx A = work[tile_at<ZC>(ra + kk, l)], B = work[tile_at<ZC>(rb + kk, l)];
                 c = mk(A.x + B.y, B.x - A.y);
             }
-            v[k2] = c;
+            x[r] = c;
         }
-        inv_fft<GY>(v, xg, a.twy, t, gm);
+        cplx* xb = Ph + 256 * task;
+        xform<G>(x, xb, tw, g, t);
 #pragma unroll
-        for (int j = 0; j < GY::P; ++j) {
-            const int y = zpos<GY>(t, j);
-            Ph[(fa * ZC + l) * PY + y] = v[j].x;
-            Ph[(fb * ZC + l) * PY + y] = v[j].y;
-        }
+        for (int r = 0; r < 8; ++r) xb[32 * r + lane] = x[r];
     }
     __syncthreads();
-    // products and their forward transforms, two per complex transform
-    for (int task = g; task < 5 * ZC; task += NG) {
-        const int l = task % ZC, pp = task / ZC;
-        const int pa = 2 * pp, pb = 2 * pp + 1;
-        cplx v[GY::P];
-#pragma unroll
-        for (int j = 0; j < GY::P; ++j) {
-            const int y = zpos<GY>(t, j);
-            double f6[6];
-#pragma unroll
-            for (int f = 0; f < 6; ++f) f6[f] = Ph[(f * ZC + l) * PY + y];
-            v[j] = mk(product(pa, f6), pb < NPROD ? product(pb, f6) : 0.0);
+    // products and their forward transforms, two per complex transform: pair pp of the lines of
+    // warp-task lt is task pp LT + lt
+#pragma unroll 1
+    for (int base = 0; base < 5 * LT; base += K::WARPS) {
+        const int task = base + warp;
+        const bool on = task < 5 * LT;
+        const int pp = task / LT, lt = task % LT, l = lt * GPW + g;
+        cplx x[8];
+        if (on) {
+            const cplx* ph = Ph + 256 * lt + lane;
+            switch (pp) {
+                case 0: product_pair<0, LT>(x, ph); break;
+                case 1: product_pair<1, LT>(x, ph); break;
+                case 2: product_pair<2, LT>(x, ph); break;
+                case 3: product_pair<3, LT>(x, ph); break;
+                default: product_pair<4, LT>(x, ph); break;
+            }
+            xform<G>(x, work + 256 * warp, tw, g, t);
         }
-        fwd_fft<GY>(v, xg, a.twy, t, gm);
+        __syncthreads();  // the exchange buffers become the output tile
+        if (on) {
+            const int ra = 2 * (pp - base / LT) * KYN, rb = ra + KYN;
+            const int lm = g * T + ((T - t) & (T - 1));  // the lane of My - k
 #pragma unroll
-        for (int k2 = 0; k2 < GY::P; ++k2) xg[t + T * k2] = v[k2];
-        __syncwarp(gm);
-        const size_t zoff = (size_t)x * NZ + z0 + l;
-        for (int k = t; k < Kyn; k += T) {
-            const cplx c = xg[k];
-            const cplx cm = xg[(MY - k) & (MY - 1)];
-            a.P[((size_t)pa * Kyn + k) * MX * NZ + zoff] = mk(0.5 * (c.x + cm.x), 0.5 * (c.y - cm.y));
-            if (pb < NPROD)
-                a.P[((size_t)pb * Kyn + k) * MX * NZ + zoff] = mk(0.5 * (c.y + cm.y), -0.5 * (c.x - cm.x));
+            for (int r = 0; r < 8; ++r) {
+                if (T * r >= KYN) break;
+                // c(k) and c(My - k): register 8 - r of this lane for t = 0, 7 - r of lane T - t
+                const cplx c = conjc(x[r]);
+                cplx m = mk(__shfl_sync(0xffffffffu, x[7 - r].x, lm), __shfl_sync(0xffffffffu, x[7 - r].y, lm));
+                if (t == 0) m = x[(8 - r) & 7];
+                m.y = -m.y;
+                const int k = t + T * r;
+                if (k < KYN) {
+                    work[tile_at<ZC>(ra + k, l)] = mk(0.5 * (c.x + m.x), 0.5 * (c.y - m.y));
+                    work[tile_at<ZC>(rb + k, l)] = mk(0.5 * (c.y + m.y), -0.5 * (c.x - m.x));
+                }
+            }
         }
-        __syncwarp(gm);
+        __syncthreads();
+        // the round's products, whole rows of ZC lines
+        const int p0 = 2 * (base / LT), np = min(2 * K::PPR, NPROD - p0);
+        for (int row = tid / ZC, l2 = tid % ZC; row < np * KYN; row += K::THREADS / ZC)
+            a.P[((size_t)p0 * KYN + row) * plane + off + l2] = work[tile_at<ZC>(row, l2)];
+        __syncthreads();
     }
 }
 
@@ -269,66 +346,61 @@ __global__ void __launch_bounds__(Phys<MY>::THREADS, 2) dns_phys(DnsArgs a) {
 // C: x forward + z forward of one product on one ky plane
 // ---------------------------------------------------------------------------
 template <int MX, int NZ>
-struct FwdXZ {
-    using GZ = Geom<NZ>;
-    using GX = Geom<MX>;
-    static constexpr int SROW = NZ + 1;
-    static constexpr int XZ = (BLOCK / GZ::T) * GZ::XSIZE;
-    static constexpr int XX = (BLOCK / GX::T) * GX::XSIZE;
-    static constexpr int XCH = XZ > XX ? XZ : XX;
-    static size_t smem(int ncol) { return sizeof(cplx) * ((size_t)ncol * SROW + XCH) + sizeof(int) * MX; }
-};
-
-template <int MX, int NZ>
-__global__ void __launch_bounds__(BLOCK, 2) dns_fwd_xz(DnsArgs a) {
-    pdl_start();
-    using K = FwdXZ<MX, NZ>;
-    using GZ = typename K::GZ;
-    using GX = typename K::GX;
+__global__ void __launch_bounds__(32 * ZX_WARPS, 3) dns_fwd_xz(const __grid_constant__ DnsArgs a) {
+    using GZ = XG<NZ>;
+    using GX = XG<MX>;
     extern __shared__ __align__(16) unsigned char smraw[];
     cplx* S = reinterpret_cast<cplx*>(smraw);
-    cplx* xch = S + (size_t)a.ncol * K::SROW;
-    int* bin2col = reinterpret_cast<int*>(xch + K::XCH);
-    const int ky = blockIdx.x, p = blockIdx.y, tid = threadIdx.x;
-    for (int b = tid; b < MX; b += BLOCK) bin2col[b] = -1;
+    cplx* twz = S + NZ * MX;
+    cplx* twx = twz + NZ;
+    int* bin2col = reinterpret_cast<int*>(twx + MX);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = blockDim.x;
+    const int ky = blockIdx.x, p = blockIdx.y;
+    for (int i = tid; i < NZ; i += nth) twz[i] = a.twz[i];
+    for (int i = tid; i < MX; i += nth) twx[i] = a.twx[i];
+    for (int b = tid; b < MX; b += nth) bin2col[b] = -1;
+    __syncthreads();
+    pdl_start();
     const cplx* src = a.P + ((size_t)p * a.Kyn + ky) * MX * NZ;
+    for (int i = tid; i < MX * NZ; i += nth) cp_async16(S + plane_at<NZ>(i / NZ, i % NZ), src + i);
+    cp_async_commit();
+    plane_bins<MX>(a, ky, bin2col);
+    cp_async_wait_all();
     __syncthreads();
-    for (int c = tid; c < a.ncol; c += BLOCK) bin2col[QLGPU_CHECK_INDEX(xbin(a.kx0[QLGPU_CHECK_INDEX(ky + a.Kyn * c, a.nxy, a.status)], a.dkx, MX), MX, a.status)] = c;
-    __syncthreads();
-    {  // x forward of every z row (loads: consecutive z per warp, whole sectors), kept at
-       // the plane's column bins
-        constexpr int T = GX::T, NG = BLOCK / T;
-        const int g = tid / T, t = tid % T;
-        const unsigned gm = group_mask(T);
-        cplx* xg = xch + g * GX::XSIZE;
-        for (int z = g; z < NZ; z += NG) {
-            cplx x[GX::P];
+    {  // x forward of every z column (the conjugates are kept: the z transform takes them)
+        constexpr int T = GX::T;
+        const int g = lane / T, t = lane % T;
+        for (int z0 = warp * GX::GPW; z0 < NZ; z0 += ZX_WARPS * GX::GPW) {
+            const int z = z0 + g;
+            cplx x[8];
 #pragma unroll
-            for (int j = 0; j < GX::P; ++j) x[j] = src[(size_t)zpos<GX>(t, j) * NZ + z];
-            fwd_fft<GX>(x, xg, a.twx, t, gm);
+            for (int r = 0; r < 8; ++r) x[r] = conjc(S[plane_at<NZ>(t + T * r, z)]);
+            __syncwarp();
+            xform_at<GX>(
+                x, [&](int q, int s) -> cplx& { return S[plane_at<NZ>(q * T + ((s + q) & (T - 1)), z)]; }, twx, t);
 #pragma unroll
-            for (int k2 = 0; k2 < GX::P; ++k2) {
-                const int c = bin2col[t + T * k2];
-                if (c >= 0) S[c * K::SROW + z] = x[k2];
-            }
+            for (int r = 0; r < 8; ++r) S[plane_at<NZ>(t + T * r, z)] = x[r];
         }
     }
     __syncthreads();
-    {  // z forward of every column, truncated to the stored kz
-        constexpr int T = GZ::T, NG = BLOCK / T;
-        const int g = tid / T, t = tid % T;
-        const unsigned gm = group_mask(T);
-        cplx* xg = xch + g * GZ::XSIZE;
-        for (int c = g; c < a.ncol; c += NG) {
-            cplx x[GZ::P];
+    {  // z forward of every x row that is a column's bin, truncated to the stored kz
+        constexpr int T = GZ::T;
+        const int g = lane / T, t = lane % T;
+        for (int x0 = warp * GZ::GPW; x0 < MX; x0 += ZX_WARPS * GZ::GPW) {
+            const int xr = x0 + g, c = bin2col[xr];
+            cplx x[8];
 #pragma unroll
-            for (int j = 0; j < GZ::P; ++j) x[j] = S[c * K::SROW + zpos<GZ>(t, j)];
-            fwd_fft<GZ>(x, xg, a.twz, t, gm);
-            cplx* dst = a.T + ((size_t)p * a.nxy + QLGPU_CHECK_INDEX(ky + a.Kyn * c, a.nxy, a.status)) * a.nz;
+            for (int r = 0; r < 8; ++r) x[r] = S[plane_at<NZ>(xr, t + T * r)];
+            __syncwarp();
+            xform_at<GZ>(
+                x, [&](int q, int s) -> cplx& { return S[plane_at<NZ>(xr, q * T + ((s + q) & (T - 1)))]; }, twz, t);
+            if (c >= 0) {
+                cplx* dst = a.T + ((size_t)p * a.nxy + QLGPU_CHECK_INDEX(ky + a.Kyn * c, a.nxy, a.status)) * a.nz;
 #pragma unroll
-            for (int k2 = 0; k2 < GZ::P; ++k2) {
-                const int s = QLGPU_CHECK_STORED(stored_index<GZ>(t + T * k2), a.nz, a.status);
-                if (s >= 0) dst[s] = x[k2];
+                for (int r = 0; r < 8; ++r) {
+                    const int s = QLGPU_CHECK_STORED(zstored<NZ>(t + T * r), a.nz, a.status);
+                    if (s >= 0) dst[s] = conjc(x[r]);
+                }
             }
         }
     }
@@ -354,7 +426,8 @@ __device__ __forceinline__ double lap_order(const DnsArgs& a, double kx0, double
 
 __device__ __forceinline__ cplx cmuli(cplx a) { return mk(-a.y, a.x); }  // i a
 
-__global__ void __launch_bounds__(BLOCK) dns_update(DnsArgs a, DnsStage st) {
+__global__ void __launch_bounds__(BLOCK, 5)
+    dns_update(const __grid_constant__ DnsArgs a, const __grid_constant__ DnsStage st) {
     pdl_start();
     const int idx = blockIdx.x * BLOCK + threadIdx.x;
     if (idx >= a.nxy * a.nz) return;
@@ -468,20 +541,18 @@ __global__ void __launch_bounds__(BLOCK) dns_update(DnsArgs a, DnsStage st) {
     if (bad) atomicOr(a.status, 1);
 }
 
-// After the last stage: shift kx0 of the columns that left the box (their
-// fields were zeroed by dns_update), MHD_FullQlin.cpp:464-481.
-__global__ void dns_remap_kx(DnsArgs a) {
+// After the last stage, one CTA: shift kx0 of the columns that left the box (their
+// fields were zeroed by dns_update), MHD_FullQlin.cpp:464-481, and the clock.
+__global__ void __launch_bounds__(1024) dns_end_step(const __grid_constant__ DnsArgs a) {
     pdl_start();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.nxy || !a.remap) return;
     const double tn = a.clock[0] + a.dt;
-    const double kxt = kx_at(a.kx0[i], a.q, tn, a.ky[i]);
-    if (kxt > a.remap_thresh) a.kx0[i] = __dsub_rn(a.kx0[i], a.remap_shift);
-}
-
-__global__ void dns_advance_clock(DnsArgs a) {
-    pdl_start();
-    if (threadIdx.x == 0 && blockIdx.x == 0) a.clock[0] = a.clock[0] + a.dt;
+    __syncthreads();
+    if (threadIdx.x == 0) a.clock[0] = tn;
+    if (!a.remap) return;
+    for (int i = threadIdx.x; i < a.nxy; i += blockDim.x) {
+        const double kxt = kx_at(a.kx0[i], a.q, tn, a.ky[i]);
+        if (kxt > a.remap_thresh) a.kx0[i] = __dsub_rn(a.kx0[i], a.remap_shift);
+    }
 }
 
 // ---------------------------------------------------------------------------

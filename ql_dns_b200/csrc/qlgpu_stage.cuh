@@ -17,7 +17,7 @@
 // FP64.
 #pragma once
 #include "qlgpu_debug.cuh"
-#include "qlgpu_fft.cuh"
+#include "qlgpu_xform.cuh"
 #include "qlgpu_priv.cuh"
 #include "qlgpu_types.h"
 
@@ -54,18 +54,6 @@ __device__ __forceinline__ unsigned long long gtimer() {
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(v)::"memory");
     return v;
 }
-
-// Asynchronous global -> shared copies (cp.async), 16 or 8 bytes each
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
 // kx(t) = kx0 + (q t) ky, evaluated with the reference's rounding order
 // (MHD_BQlin.cpp:498: K->kx[i] + q_*t*kyctmp_)

@@ -12,6 +12,14 @@
 
 namespace qlgpu {
 
+// Asynchronous global -> shared copies (cp.async), 16 bytes each
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
 // Real-space / spectral register classes: index t + T r is in the dealiasing
 // gap for every t (dead), stored for every t, or stored for some t.
 template <class E>
@@ -43,17 +51,17 @@ __device__ __forceinline__ int xslot(int g, int q, int t) {
 }
 
 // Backward DFT of one column: x[r] = X[t + T r] in, x[r] = y[t + T r] out,
-// y[n] = sum_k X[k] exp(+2 pi i n k / NZ).  xg = the warp's exchange buffers,
-// g = this thread's group in the warp, tw[q T + t] = exp(2 pi i q t / NZ).
+// y[n] = sum_k X[k] exp(+2 pi i n k / NZ).  at(q, s) is the group's exchange slot of
+// (row q < 8, column s < T), tw[q T + t] = exp(2 pi i q t / NZ).
 // Warp-collective (every lane of the warp calls it together).
-template <class E>
-__device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, int g, int t) {
+template <class E, class At>
+__device__ __forceinline__ void xform_at(cplx (&x)[8], At&& at, const cplx* tw, int t) {
     constexpr int T = E::T;
     dft8<+1>(x);
 #pragma unroll
     for (int q = 1; q < 8; ++q) x[q] = cmul(x[q], tw[q * T + t]);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) xg[xslot<E>(g, q, t)] = x[q];
+    for (int q = 0; q < 8; ++q) at(q, t) = x[q];
     __syncwarp();
     if constexpr (T <= 8) {
         constexpr int J = 8 / T;
@@ -62,7 +70,7 @@ __device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, in
             const int q = t + T * j;
             cplx v[T];
 #pragma unroll
-            for (int s = 0; s < T; ++s) v[s] = xg[xslot<E>(g, q, s)];
+            for (int s = 0; s < T; ++s) v[s] = at(q, s);
             dft<T, +1>(v);
 #pragma unroll
             for (int m = 0; m < T; ++m) x[j + J * m] = v[m];
@@ -74,8 +82,8 @@ __device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, in
         const double sg = h ? -1.0 : 1.0;
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
-            const cplx za = xg[xslot<E>(g, q, s)];
-            const cplx zb = xg[xslot<E>(g, q, s + 8)];
+            const cplx za = at(q, s);
+            const cplx zb = at(q, s + 8);
             cplx w = mk(fma(sg, zb.x, za.x), fma(sg, zb.y, za.y));
             if (s != 0) w = cmul(w, mk(h ? c16(s) : 1.0, h ? s16(s) : 0.0));
             x[s] = w;
@@ -89,8 +97,8 @@ __device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, in
         const double s1 = (h & 1) ? -1.0 : 1.0, s2 = (h & 2) ? -1.0 : 1.0;
 #pragma unroll
         for (int s = 0; s < 8; ++s) {
-            const cplx z0 = xg[xslot<E>(g, q, s)], z1 = xg[xslot<E>(g, q, s + 8)];
-            const cplx z2 = xg[xslot<E>(g, q, s + 16)], z3 = xg[xslot<E>(g, q, s + 24)];
+            const cplx z0 = at(q, s), z1 = at(q, s + 8);
+            const cplx z2 = at(q, s + 16), z3 = at(q, s + 24);
             const cplx a = mk(fma(s1, z2.x, z0.x), fma(s1, z2.y, z0.y));
             const cplx b = mk(fma(s1, z3.x, z1.x), fma(s1, z3.y, z1.y));
             const cplx ib = (h & 1) ? mk(-b.y, b.x) : b;  // i^h b up to the sign s2
@@ -101,6 +109,11 @@ __device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, in
         dft8<+1>(x);
     }
     __syncwarp();
+}
+// The same with the warp's exchange buffers xg, g = this thread's group in the warp.
+template <class E>
+__device__ __forceinline__ void xform(cplx (&x)[8], cplx* xg, const cplx* tw, int g, int t) {
+    xform_at<E>(x, [&](int q, int s) -> cplx& { return xg[xslot<E>(g, q, s)]; }, tw, t);
 }
 
 }  // namespace qlgpu
