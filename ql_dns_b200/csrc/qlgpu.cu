@@ -258,7 +258,7 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
         h->err = "cudaGetDeviceProperties failed";
         return bail(QLGPU_ERR_CUDA);
     }
-    const StageGeom sg = stage_geometry(p.model, p.NZ, h->nxy, prop.multiProcessorCount - 1, 64 * RED_GROUP);
+    const StageGeom sg = stage_geometry(p.model, p.NZ, h->nxy, prop.multiProcessorCount - 1, 64 * RED_GROUP, var.max_warps);
     h->warps = sg.warps;
     h->block = 32 * h->warps;
     h->smem = var.smem(h->warps);
@@ -890,7 +890,7 @@ extern "C" int qlgpu_rhs_noalloc(const qlgpu_params* pp, double t, double dt_lin
     }
     void* base = nd.ptr;
     // Launch geometry: as in qlgpu_create.
-    const StageGeom sg = stage_geometry(p.model, p.NZ, nxy, nd.sms, QLGPU_NOALLOC_MAX_GRID);
+    const StageGeom sg = stage_geometry(p.model, p.NZ, nxy, nd.sms, QLGPU_NOALLOC_MAX_GRID, var.max_warps);
     const int warps = sg.warps, grid = sg.grid;
     const size_t smem = var.smem(warps);
     if (ensure_smem_attr(var.kernel(), smem) != cudaSuccess)

@@ -98,13 +98,15 @@ struct AG {
     static constexpr int SWZ = T == 4 ? 1 : (T == 2 ? 3 : 0);
     static constexpr int NZE = (nz + 1) & ~1;
     static constexpr int NR = 16;  // 14 inverse results, 2 exchange buffers
+    static constexpr bool PAD = T >= 8;
+    static constexpr int XW = PAD ? 8 * GPW * (T + 1) : 256;  // one of them (cplx)
     static constexpr size_t o_tw = 0;                                    // [8][T] cplx
     static constexpr size_t o_prof = o_tw + 16 * (size_t)NZ_;           // [5][NZ]
     static constexpr size_t o_kz = o_prof + 8 * 5 * (size_t)NZ_;        // kz per spectral slot
     static constexpr size_t o_ekz = o_kz + 8 * (size_t)NZ_;             // [2][NZE]
     static constexpr size_t o_acc = o_ekz + 16 * (size_t)NZE;           // [3][8][32] profile sums
-    static constexpr size_t o_R = o_acc + 8 * 3 * 256;                  // [NR][8][32] cplx
-    static constexpr size_t o_stg = o_R + 16 * 256 * (size_t)NR;        // [GPW][4][nz] cplx
+    static constexpr size_t o_R = o_acc + 8 * 3 * 256;                  // [NR][XW] cplx, a result at [8][32]
+    static constexpr size_t o_stg = o_R + 16 * XW * (size_t)NR;        // [GPW][4][nz] cplx
     static constexpr size_t BYTES = o_stg + 16 * (size_t)GPW * 4 * nz;
 };
 inline int adj_block_modes(int NZ) { return 256 / NZ; }
@@ -177,7 +179,7 @@ __global__ void __launch_bounds__(512, 1)
     for (int i = tid; i < 3 * 256; i += nth) acc[i] = 0.0;
     const double tclock = B.t_pre[X.n];
     const double ts = __dadd_rn(tclock, S.t_off);
-    auto buf = [&](int i) { return R + (size_t)i * 256; };
+    auto buf = [&](int i) { return R + i * W::XW; };
     const double Om2 = __dmul_rn(2.0, P.Omega), fac = P.fac;
 
     for (int base = first; base < end; base += GPW) {
@@ -266,7 +268,7 @@ __global__ void __launch_bounds__(512, 1)
         // buffers of results 0-6, so those are held in registers until every warp has read its
         // own; inputs 7 and 8 have exchange buffers of their own.
         const double *By = prof, *dBy = prof + NZ, *ddBy = prof + 2 * NZ, *px = prof + 3 * NZ, *py = prof + 4 * NZ;
-        auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+        auto rd = [&](int i, int r) { return R[i * W::XW + 32 * r + lane]; };
         auto small_task = [&](int task) {  // 7: mult py R_bz, 8: -mult py R_uz
             cplx x[8];
 #pragma unroll
@@ -423,7 +425,7 @@ __global__ void __launch_bounds__(ADJ_MF_THREADS, 1)
     constexpr int T = W::T, nzd = W::nz;
     constexpr int SPLIT = NZ <= 128 ? 4 : 2;  // threads that share a sum over the chunks
     __shared__ __align__(16) cplx tw[NZ];
-    __shared__ __align__(16) cplx xch[3][256];
+    __shared__ __align__(16) cplx xch[3][W::XW];
     __shared__ __align__(16) cplx lamB[2][nzd], lamG[2][nzd];
     __shared__ double tot[3 * NZ];
     __shared__ __align__(16) double psum[SPLIT][3 * NZ];  // then the spectra of the sums

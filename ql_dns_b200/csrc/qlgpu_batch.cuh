@@ -87,14 +87,14 @@ __device__ __noinline__ StageResult batch_item_stage(const BatchLaunch& L, const
         }
     }
     __syncthreads();
-    return stage_body<NZ, MODEL, INTEG, false>(sA, sP, it.cta, it.ncta, smem_raw, ss, lc, fresh, nullptr,
+    return stage_body<NZ, MODEL, INTEG, false, false>(sA, sP, it.cta, it.ncta, smem_raw, ss, lc, fresh, nullptr,
                                                [&]() -> bool {
         return batch_wait(L.epoch + (size_t)it.c * BATCH_EPOCH_STRIDE, k, L.ctl, L.wait_ns, it.c, k);
     });
 }
 
 template <int MODEL, int INTEG>
-__global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) batch_kernel(const __grid_constant__ BatchLaunch L) {
+__global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) batch_kernel(const __grid_constant__ BatchLaunch L) {
     __shared__ BatchSlot s_items[BATCH_MAX_SLOTS];
     __shared__ LocalClock s_clk[BATCH_MAX_SLOTS];
     const int tid = threadIdx.x;
@@ -127,7 +127,6 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) batch_kernel(const __
                 if (r == STAGE_TOP) {
                     __syncthreads();
                     if (tid == 0) {
-                        __threadfence();
                         if (n == L.nsteps - 1 && s == 2) L.case_end[it.c] = gtimer();
                         st_release_u32(L.epoch + (size_t)it.c * BATCH_EPOCH_STRIDE, 3u * (unsigned)n + s + 1);
                     }

@@ -73,6 +73,7 @@ struct XG {
     static constexpr int NZ = N;
     static constexpr int T = N / 8;
     static constexpr int GPW = 32 / T;
+    static constexpr bool PAD = false;  // rows of T + 1 cost the y pass 3 %
     static constexpr int SWZ = T == 4 ? 1 : (T == 2 ? 3 : 0);
 };
 // stored kz index of spectral slot k of an NZ-point row (fftwPlans.h:66-97), -1 in the gap
@@ -198,16 +199,17 @@ struct Phys {
     using G = XG<MY>;
     static constexpr int ZC = MY >= 256 ? 4 : (MY == 16 ? 16 : 8);
     static constexpr int LT = ZC / G::GPW;              // warp-tasks per field pair
+    static constexpr int BUF = XWARP<G>;                // a warp-task's result / exchange buffer
     static constexpr int WARPS = MY >= 128 ? 8 : (MY == 64 ? 6 : 5);
     static constexpr int THREADS = 32 * WARPS;
     static constexpr int KYN = MY / 3 + 1;              // ky of the mode set
     static constexpr int PPR = (WARPS + LT - 1) / LT;   // product pairs per round of the forward tasks
     static_assert(WARPS % LT == 0, "a round of forward tasks holds whole pairs");
-    static constexpr size_t TILE = (size_t)6 * KYN * ZC, XCH = (size_t)256 * WARPS;
+    static constexpr size_t TILE = (size_t)6 * KYN * ZC, XCH = (size_t)BUF * WARPS;
     static constexpr size_t OUT = (size_t)2 * PPR * KYN * ZC;
     static constexpr size_t WORK = TILE > XCH ? (TILE > OUT ? TILE : OUT) : (XCH > OUT ? XCH : OUT);
     static_assert(THREADS % ZC == 0, "whole tile rows per pass");
-    static size_t smem() { return sizeof(cplx) * ((size_t)3 * ZC * MY + WORK + MY); }
+    static size_t smem() { return sizeof(cplx) * ((size_t)3 * LT * BUF + WORK + MY); }
 };
 // tile row (field or product, k), line l: 16-byte entries permuted within 128 bytes, so that a
 // transform's lanes (consecutive k, one line) read different banks
@@ -233,14 +235,14 @@ __device__ __forceinline__ double product(int p, const double* v) {
 }
 
 // conj of products 2 PP and 2 PP + 1 as one complex row, from the three field pairs of the lane
-template <int PP, int LT>
+template <int PP, int LT, int BUF>
 __device__ __forceinline__ void product_pair(cplx (&x)[8], const cplx* ph) {
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         double f6[6];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            const cplx v = ph[256 * q * LT + 32 * r];
+            const cplx v = ph[BUF * q * LT + 32 * r];
             f6[2 * q] = v.x;
             f6[2 * q + 1] = v.y;
         }
@@ -252,10 +254,10 @@ template <int MY>
 __global__ void __launch_bounds__(Phys<MY>::THREADS, 2) dns_phys(const __grid_constant__ DnsArgs a) {
     using K = Phys<MY>;
     using G = typename K::G;
-    constexpr int T = G::T, GPW = G::GPW, ZC = K::ZC, LT = K::LT, KYN = K::KYN;
+    constexpr int T = G::T, GPW = G::GPW, ZC = K::ZC, LT = K::LT, KYN = K::KYN, BUF = K::BUF;
     extern __shared__ __align__(16) unsigned char smraw[];
-    cplx* Ph = reinterpret_cast<cplx*>(smraw);   // [3 LT warp-tasks][8][32]: the pairs (ux,uy), (uz,bx), (by,bz)
-    cplx* work = Ph + (size_t)3 * ZC * MY;       // input tile; then exchange buffers / output tile
+    cplx* Ph = reinterpret_cast<cplx*>(smraw);   // [3 LT warp-tasks][BUF], [8][32] each: the pairs (ux,uy), (uz,bx), (by,bz)
+    cplx* work = Ph + (size_t)3 * LT * BUF;       // input tile; then exchange buffers / output tile
     cplx* tw = work + K::WORK;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nth = blockDim.x;
     const int g = lane / T, t = lane % T;
@@ -289,7 +291,7 @@ __global__ void __launch_bounds__(Phys<MY>::THREADS, 2) dns_phys(const __grid_co
             }
             x[r] = c;
         }
-        cplx* xb = Ph + 256 * task;
+        cplx* xb = Ph + BUF * task;
         xform<G>(x, xb, tw, g, t);
 #pragma unroll
         for (int r = 0; r < 8; ++r) xb[32 * r + lane] = x[r];
@@ -304,15 +306,15 @@ __global__ void __launch_bounds__(Phys<MY>::THREADS, 2) dns_phys(const __grid_co
         const int pp = task / LT, lt = task % LT, l = lt * GPW + g;
         cplx x[8];
         if (on) {
-            const cplx* ph = Ph + 256 * lt + lane;
+            const cplx* ph = Ph + BUF * lt + lane;
             switch (pp) {
-                case 0: product_pair<0, LT>(x, ph); break;
-                case 1: product_pair<1, LT>(x, ph); break;
-                case 2: product_pair<2, LT>(x, ph); break;
-                case 3: product_pair<3, LT>(x, ph); break;
-                default: product_pair<4, LT>(x, ph); break;
+                case 0: product_pair<0, LT, BUF>(x, ph); break;
+                case 1: product_pair<1, LT, BUF>(x, ph); break;
+                case 2: product_pair<2, LT, BUF>(x, ph); break;
+                case 3: product_pair<3, LT, BUF>(x, ph); break;
+                default: product_pair<4, LT, BUF>(x, ph); break;
             }
-            xform<G>(x, work + 256 * warp, tw, g, t);
+            xform<G>(x, work + BUF * warp, tw, g, t);
         }
         __syncthreads();  // the exchange buffers become the output tile
         if (on) {

@@ -82,6 +82,7 @@ struct EG {
     static constexpr int H = (nz - 1) / 2;
     static constexpr int GPW = 32 / T;                // groups per warp
     static constexpr int PPW = GPW / 2;               // pairs (modes) per warp
+    static constexpr bool PAD = T >= 8;
     static constexpr int SWZ = T == 4 ? 1 : (T == 2 ? 3 : 0);  // row swizzle of small groups
     static constexpr int PL = NEMF * NZ_ + 8;         // partial vector (doubles)
     static_assert(8 * T == NZ_ && T >= 2 && T <= 16, "NZ = 16, 32, 64 or 128");
@@ -97,7 +98,7 @@ struct EG {
     static constexpr int KPAIR = 2 * NZ_ + T;
     static constexpr size_t K_CPLX = (size_t)PPW * KPAIR;                    // per warp: KU, KB of its pairs
     static constexpr size_t STG_CPLX = (size_t)PPW * 4 * nz;                 // staged mode fields
-    static constexpr size_t X_CPLX = (size_t)GPW * 8 * T;                    // exchange buffers
+    static constexpr size_t X_CPLX = PAD ? 8 * (size_t)GPW * (T + 1) : 256;  // exchange buffer
     static constexpr size_t X_OFF = K_CPLX + STG_CPLX;                        // per warp: [K | STG | X]
     static constexpr size_t WARP_BYTES = 16 * (X_OFF + X_CPLX);
     static constexpr size_t BYTES = o_warp + WARPS * WARP_BYTES;
@@ -240,7 +241,7 @@ __device__ __noinline__ void profiles_of(const ChunkHdr& hd, double* prof, cplx*
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp < 3)
         wide::mean_profiles8<W, true>(
-            hd.P, [&](int m, int s) { return ldc_cg(hd.A.mf + m * W::nz + s); }, prof, scratch + 256 * warp, tw, warp,
+            hd.P, [&](int m, int s) { return ldc_cg(hd.A.mf + m * W::nz + s); }, prof, scratch, tw, warp,
             3, lane);
 }
 
@@ -273,9 +274,8 @@ __device__ __noinline__ void top_stage(const EnsLaunch& L, ChunkHdr& hd, int c, 
         tot[idx] = sum;
     }
     __syncthreads();
-    wide::top_stage<W, MODEL_BQLIN, INTEG>(hd.A, hd.P, tot, xch, tw, tclock, t_new, last, diag_due);
+    wide::top_stage<W, MODEL_BQLIN, INTEG>(hd.A, hd.P, tot, xch, tw, nullptr, tclock, t_new, last, diag_due);
     if (tid == 0) {
-        __threadfence();
         if (r == L.nrounds - 1) L.case_end[c] = gtimer();
         st_release_u32(L.epoch + (size_t)c * BATCH_EPOCH_STRIDE, (unsigned)(r + 1));
     }
@@ -406,11 +406,11 @@ __device__ __noinline__ void run_chunk(const EnsLaunch& L, ChunkHdr& hd, const R
         if (cached) {
             for (int i = tid; i < 3 * NZ; i += THREADS) prof[i] = __ldcg(A.mfr_cache + i);
         } else {
-            // real-space By, dz By, dz^2 By of the stage input (MHD_BQlin.cpp:122-127); scratch:
-            // warp 0's exchange buffers and warp 1's K buffers, which no staged copy writes
+            // real-space By, dz By, dz^2 By of the stage input (MHD_BQlin.cpp:122-127), in the warps'
+            // exchange buffers, which no staged copy writes
             __syncthreads();
             profiles_of<NZ>(hd, prof,
-                            reinterpret_cast<cplx*>(smem_raw + E::o_warp) + E::X_OFF, tw);
+                            xg, tw);
         }
     }
     __syncthreads();

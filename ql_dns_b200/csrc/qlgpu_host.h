@@ -123,12 +123,13 @@ inline int stage_teams(int model, int warps) {
 struct StageGeom {
     int warps, grid;
 };
-inline StageGeom stage_geometry(int model, int NZ, int nxy, int sms, int max_grid) {
+inline StageGeom stage_geometry(int model, int NZ, int nxy, int sms, int max_grid, int max_warps) {
     const int blocks = (nxy + block_modes(NZ) - 1) / block_modes(NZ);
     const bool bq = model == MODEL_BQLIN;
     const int per_sm = (blocks + sms - 1) / sms;
     StageGeom g;
-    g.warps = bq ? (per_sm <= 1 ? 9 : per_sm == 2 ? 14 : 15) : (per_sm <= 1 ? 10 : 16);
+    g.warps = bq ? (per_sm <= 1 ? 9 : per_sm == 2 ? 14 : per_sm == 3 ? 15 : max_warps) : (per_sm <= 1 ? 10 : 16);
+    if (g.warps > max_warps) g.warps = max_warps;
     const int teams = stage_teams(model, g.warps);
     g.grid = (blocks + teams - 1) / teams;
     if (g.grid > sms) g.grid = sms;

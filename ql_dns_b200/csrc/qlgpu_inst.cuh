@@ -49,7 +49,7 @@ Variant make_variant() {
     v.smem = &stage_smem<NZ, MODEL>;
     v.T = Geom<NZ>::T;
     v.PL = wide::WG<NZ, MODEL>::PL;
-    v.max_warps = wide::MAX_WARPS;
+    v.max_warps = wide::MAX_WARPS<MODEL>;
     return v;
 }
 

@@ -37,14 +37,14 @@ __device__ __forceinline__ void put_record(const DevParams& P, const double* ds,
 // Mean-field update, run by the whole CTA that arrives last: the mean-field
 // right-hand side from the stress spectra spec[NEMF][H + 1] and its RK update
 // (mfs[nmf][nz] in shared memory, updated in place, and A.mf; fps: the previous
-// right-hand side), then the time and
+// right-hand side; emf: the integrating factors, null to compute them), then the time and
 // diagnostic bookkeeping in the last warp.  tot[] holds the stress profiles
 // summed over all modes (real z) followed by the six fluctuation diagnostic sums.
 // ---------------------------------------------------------------------------
 template <class W, int MODEL, int INTEG, int NEMF>
 __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevParams& P, const double* tot,
-                                                  const double* spec, cplx* mfs, const cplx* fps, double tclock,
-                                                  double t_new, bool last, bool diag_due) {
+                                                  const double* spec, cplx* mfs, const cplx* fps, const double* emf,
+                                                  double tclock, double t_new, bool last, bool diag_due) {
     const StageConst& S = A.sc;
     const int tid = threadIdx.x, lane = tid & 31;
     const int nzd = P.nz;
@@ -88,7 +88,16 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
             }
             const double Lm = P.ql ? __dmul_rn((MODEL == MODEL_FULLQLIN && mm >= 2) ? P.nu : P.eta, kz2) : 0.0;
             cplx fp = S.has_prev ? fps[mm * nzd + s] : mk(0.0, 0.0);
-            cplx nv = rk_update<INTEG>(S, Lm, Lm, F[mm], fp, m[mm], S.has_prev);
+            cplx nv;
+            if (INTEG == INTEG_EXP) {
+                const double e = emf ? emf[(MODEL == MODEL_FULLQLIN && mm >= 2 ? W::NZE : 0) + s]
+                                     : exp(__dmul_rn(S.linC, Lm));
+                const cplx acc = S.has_prev ? cadd(cadd(cscale(F[mm], S.n1), cscale(fp, S.n2)), m[mm])
+                                            : cadd(cscale(F[mm], S.n1), m[mm]);
+                nv = cscale(acc, e);
+            } else {
+                nv = rk_update<INTEG_CN>(S, Lm, Lm, F[mm], fp, m[mm], S.has_prev);
+            }
             if (A.Fmf_out) stc(A.Fmf_out + mm * nzd + s, F[mm]);
             stc(A.mf + mm * nzd + s, nv);
             mfs[mm * nzd + s] = nv;

@@ -21,7 +21,7 @@
 //
 //   MHD_BQlin   (MHD_BQlin.cpp:135-257; 14 transforms, the reference does 22)
 //     inverse   R_uz R_bz R_u R_b R_zeta R_eta R_{i kz uz} R_uy R_by
-//     forward   S = i ky By R_b, then 2 kx ky dBy R_bz      -> u
+//     forward   i ky By R_b (S) and 2 kx ky dBy R_bz        -> u
 //               i ky By R_zeta - i kx dBy R_u - 2 dBy R_{i kz uz} - ddBy R_uz -> eta
 //               i ky By R_eta - i kx dBy R_b + ddBy R_bz     -> zeta
 //               i ky By R_u                                  -> b
@@ -48,7 +48,10 @@
 namespace qlgpu {
 namespace wide {
 
-constexpr int MAX_WARPS = 16;
+// widest CTA: 3 teams of MHD_BQlin, 2 of MHD_FullQlin, at 128 registers a thread (4 teams of
+// MHD_BQlin at 96 registers spill: 8 % slower at 64x64 x NZ=128)
+template <int MODEL>
+constexpr int MAX_WARPS = MODEL == MODEL_BQLIN ? 15 : 16;
 
 // Geometry and shared-memory layout of one NZ class and model.
 template <int NZ_, int MODEL>
@@ -62,34 +65,47 @@ struct WG {
     static constexpr bool BQ = MODEL == MODEL_BQLIN;
     static constexpr int TS = BQ ? 5 : 8;              // warps of a full team
     static constexpr int NINV = BQ ? 9 : 10;           // inverse tasks
-    static constexpr int NX = BQ ? 3 : 6;              // exchange buffers of the forward tasks
+    static constexpr int NX = BQ ? 0 : 6;              // further buffers: the forward tasks' results
     static constexpr int NE = BQ ? 2 : 4;              // stress profiles
     static constexpr int NPROF = BQ ? 3 : 8;           // real-space mean-field profiles
     static constexpr int PL = NE * NZ_ + 8;            // partial vector (doubles)
     static constexpr int NZE = (nz + 1) & ~1;
+    static constexpr bool PAD = T >= 8;
+    static constexpr int XW = PAD ? 8 * GPW * (T + 1) : 256;  // a result / exchange buffer (cplx)
     static constexpr size_t o_tw = 0;                                  // [8][T] cplx
     static constexpr size_t o_prof = o_tw + 16 * (size_t)NZ_;          // [NPROF][NZ]
     static constexpr size_t o_kz = o_prof + 8 * (size_t)NPROF * NZ_;   // kz per spectral slot
     static constexpr size_t o_ekz = o_kz + 8 * (size_t)NZ_;            // [2][NZE]
-    static constexpr size_t o_dred = o_ekz + 16 * (size_t)NZE;         // [MAX_WARPS][6] diagnostic sums
-    static constexpr size_t o_team = (o_dred + 8 * 6 * MAX_WARPS + 15) & ~(size_t)15;
-    // per team: results / exchange buffers [NINV + NX][8][32] cplx, staged fields [GPW][4][nz]
-    // cplx, stress sums [NE][8][32]
-    static constexpr size_t TM_STG = 16 * 256 * (size_t)(NINV + NX);
-    static constexpr size_t TM_ACC = TM_STG + 16 * (size_t)GPW * 4 * nz;
+    static constexpr size_t o_dred = o_ekz + 16 * (size_t)NZE;         // [4 teams][6] diagnostic sums
+    static constexpr size_t o_team = (o_dred + 8 * 6 * 4 + 15) & ~(size_t)15;
+    // per team: results / exchange buffers [NINV + NX][XW] cplx, a result at [8][32], staged fields and
+    // (MHD_BQlin: MHD_FullQlin reads them in its update, 4 % faster there) previous right-hand sides
+    // [GPW][4][nz] cplx, 1/lap2 [GPW][nz], stress sums [NE][8][32]
+    static constexpr size_t TM_STG = 16 * XW * (size_t)(NINV + NX);
+    static constexpr size_t TM_FP = TM_STG + 16 * (size_t)GPW * 4 * nz;
+    static constexpr size_t TM_IL2 = TM_FP + (BQ ? 16 * (size_t)GPW * 4 * nz : 0);
+    static constexpr size_t TM_ACC = (TM_IL2 + 8 * (size_t)GPW * nz + 15) & ~(size_t)15;
     static constexpr size_t TEAM_BYTES = TM_ACC + 8 * 256 * (size_t)NE;
     // the mean-field stage's scratch overlays the teams' buffers
     static constexpr int NMF = BQ ? 2 : 4;             // mean fields
     static constexpr size_t TOP_BYTES = 8 * ((size_t)PL + 2) + 16 * (size_t)NE * (H + 1) + 16 * 2 * NMF * (size_t)nz;
-    static_assert(TOP_BYTES <= 16 * 256 * (size_t)(NINV + NX - 4), "mean-field scratch below its exchange buffers");
+    static_assert(TOP_BYTES + 16 * XW * 4 <= TEAM_BYTES, "mean-field scratch and its exchange buffers in a team's bytes");
+    static constexpr size_t TOP_XCH = (TOP_BYTES + 15) & ~(size_t)15;  // four exchange buffers of the scratch
+    // named barriers of team i: 1 + i the team, 5 + i its first inverse round, 9 + i its S spectrum
     __host__ __device__ static constexpr int teams(int warps) { return warps / TS > 1 ? warps / TS : 1; }
     __host__ __device__ static constexpr size_t bytes(int warps) {
-        return o_team + TEAM_BYTES * (size_t)teams(warps);
+        // MHD_BQlin teams of fewer than five warps run forward tasks one after another, which takes
+        // three buffers more
+        return o_team + TEAM_BYTES * (size_t)teams(warps) + (BQ && warps < TS ? 3 * 16 * XW : 0);
     }
 };
 
 __device__ __forceinline__ void team_sync(int id, int threads) {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
+}
+
+__device__ __forceinline__ void team_arrive(int id, int threads) {
+    asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
 
 // ---------------------------------------------------------------------------
@@ -146,12 +162,15 @@ __device__ __forceinline__ void top_prefetch(const StageArgs& A, double* tot) {
 }
 
 // Mean-field stage of the CTA that arrived last: tot[PL] holds the stress
-// profiles summed over the modes and the diagnostic sums.  Stress spectra
+// profiles summed over the modes and the diagnostic sums; emf (optional): the integrating
+// factors exp(linC eta kz2), exp(linC nu kz2) [2][NZE] of the stage.  Ends with a barrier;
+// what it wrote is published by the caller's release.  Stress spectra
 // (MHD_BQlin.cpp:228-240 after the sum over modes; the transform is linear), the
 // mean-field update and clock (mean_field_update) and the next stage's profiles.
 template <class W, int MODEL, int INTEG>
 __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P, double* tot, cplx* xch,
-                                          const cplx* tw, double tclock, double t_new, bool last, bool diag_due) {
+                                          const cplx* tw, const double* emf, double tclock, double t_new, bool last,
+                                          bool diag_due) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
     const int g = lane / W::T, t = lane % W::T;
     double* spec = tot + W::PL + (W::PL & 1);
@@ -159,7 +178,7 @@ __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P
     // at most four warps transform (their exchange buffers)
     constexpr int NT = (W::NPROF + W::GPW - 1) / W::GPW < 4 ? (W::NPROF + W::GPW - 1) / W::GPW : 4;
     const int ntw = nwarps < NT ? nwarps : NT;
-    cplx* xg = xch + (size_t)(warp < ntw ? warp : 0) * 256;
+    cplx* xg = xch + (size_t)(warp < ntw ? warp : 0) * W::XW;
     if (warp < ntw) {
         for (int base = warp * W::GPW; base < W::NE; base += ntw * W::GPW) {
             const int e = base + g;
@@ -181,14 +200,13 @@ __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P
     }
     cp_async_wait_all();
     __syncthreads();
-    mean_field_update<W, MODEL, INTEG, W::NE>(A, P, tot, spec, mfs, mfs + W::NMF * W::nz, tclock, t_new, last,
+    mean_field_update<W, MODEL, INTEG, W::NE>(A, P, tot, spec, mfs, mfs + W::NMF * W::nz, emf, tclock, t_new, last,
                                               diag_due);
     if (A.mfr_cache && !A.rhs_only && warp < ntw)
         mean_profiles8<W, W::BQ>(
             P, [&](int m, int s) { return mfs[m * W::nz + s]; }, A.mfr_cache, xg, tw, warp, ntw, lane);
-    __threadfence();
-    __syncthreads();
     if (tid == 0 && A.mfr_cache && !A.rhs_only) A.clk->mfr_valid = 1;
+    __syncthreads();
 }
 
 // ---------------------------------------------------------------------------
@@ -198,54 +216,84 @@ struct LaneMode {
     int m, kyi, kxi;
     bool valid, zero;
     double kx0, a, b, kxe, kxo, mult;
+    // the mode's part of the integrating factor, exp(linC c (-kx^2 - ky^2)), of the fields this warp
+    // updates: side 0 (u, zeta), 1 (b, eta); -1: not computed
+    double em;
+    int em_side;
+    __device__ __forceinline__ double em_of(const StageArgs& A, const DevParams& P, int side) const {
+        const double hxy = __dsub_rn(-__dmul_rn(kxe, kxe), __dmul_rn(b, b));
+        return exp(A.sc.linC * (side ? P.cb : P.nu) * hxy);
+    }
 };
 
-// The stage update of one coefficient of field f (RK3CN_Elin.cpp:102-104 /
-// RK3CN.cpp:105-107), or F and the operator in rhs-only mode.
-template <class W, int MODEL, int INTEG>
-__device__ __forceinline__ void put_coef(const StageArgs& A, const DevParams& P, const LaneMode& M, const CnOld& cn,
-                                         const double* ekz, double em, int f, int s, double c, cplx F, cplx uin,
-                                         cplx fpv, bool has_fp) {
-    const StageConst& S = A.sc;
-    const int nzd = W::nz;
-    const size_t at = ((size_t)M.m * 4 + f) * nzd + QLGPU_CHECK_STORED(s, nzd, &A.clk->status);
-    const double kz2 = kz2val(c);
-    if (A.rhs_only) {
-        stc(A.lin_out + at, F);
-        if (A.linop_out) A.linop_out[at] = linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f);
-        return;
+// The update of one field of a lane's mode: everything the stage arguments say about it, in
+// registers (the arguments may lie in shared memory, where every global store would make the
+// compiler read them again).
+template <class W, int MODEL, int INTEG, bool RHS>
+struct Put {
+    cplx *out, *fo;        // new values (rhs-only: F), F of this stage (null: not kept)
+    const cplx* fp;        // F of the previous stage (null: none), staged (BQ) or in global memory
+    double* linop;         // rhs-only: the operator (may be null)
+    const double* ekz;
+    double n1, n2, em;
+    int f;
+    bool rhs_only, zero;
+    __device__ __forceinline__ Put(const StageArgs& A, const DevParams& P, const LaneMode& M, int f_,
+                                   const cplx* fps, const double* ekz_) {
+        const size_t at = ((size_t)M.m * 4 + f_) * W::nz;
+        f = f_;
+        out = A.lin_out + at;
+        fo = A.Fout ? A.Fout + at : nullptr;
+        fp = fps ? fps + f_ * W::nz : nullptr;
+        rhs_only = RHS && A.rhs_only;
+        linop = rhs_only && A.linop_out ? A.linop_out + at : nullptr;
+        ekz = ekz_ + (f_ < 2 ? 0 : W::NZE);
+        n1 = A.sc.n1;
+        n2 = A.sc.n2;
+        zero = M.zero;
+        em = 1.0;
+        if (INTEG == INTEG_EXP && !rhs_only && (MODEL == MODEL_BQLIN || P.factored))
+            em = M.em_side == f_ / 2 ? M.em : M.em_of(A, P, f_ / 2);
     }
-    cplx nv;
-    if (INTEG == INTEG_EXP) {
-        double e;
-        if (MODEL == MODEL_BQLIN || P.factored) e = em * ekz[(f < 2 ? 0 : W::NZE) + s];
-        else e = exp(__dmul_rn(S.linC, linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f)));
-        const cplx acc = has_fp ? cadd(cadd(cscale(F, S.n1), cscale(fpv, S.n2)), uin) : cadd(cscale(F, S.n1), uin);
-        nv = cscale(acc, e);
-    } else {
+    // (RK3CN_Elin.cpp:102-104 / RK3CN.cpp:105-107)
+    __device__ __forceinline__ cplx value(const StageConst& S, const DevParams& P, const LaneMode& M, const CnOld& cn,
+                                          int s, double c, cplx F, cplx uin, cplx fpv) const {
+        const double kz2 = kz2val(c);
+        if (INTEG == INTEG_EXP) {
+            double e;
+            if (MODEL == MODEL_BQLIN || P.factored) e = em * ekz[s];
+            else e = exp(__dmul_rn(S.linC, linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f)));
+            const cplx acc = fp ? cadd(cadd(cscale(F, n1), cscale(fpv, n2)), uin) : cadd(cscale(F, n1), uin);
+            return cscale(acc, e);
+        }
         const bool z0 = (M.kyi == 0 && s == 0);
         const double L = linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f);
         const double lo = cn.old_init ? lap_init<MODEL>(P, M.kxo, lap2val(M.b, kz2, z0))
                                       : lap_end<MODEL>(P, M.kxo, M.b, kz2);
-        nv = rk_update<INTEG_CN>(S, L, linop_f<MODEL>(P, lo, f), F, fpv, uin, has_fp);
+        return rk_update<INTEG_CN>(S, L, linop_f<MODEL>(P, lo, f), F, fpv, uin, fp != nullptr);
     }
-    if (A.Fout) stc(A.Fout + at, F);
-    stc(A.lin_out + at, M.zero ? mk(0.0, 0.0) : nv);
-}
-
-// Integrating-factor scalar exp(linC c (-kx^2 - ky^2)) of field f's side.
-template <int MODEL, int INTEG>
-__device__ __forceinline__ double em_of(const StageArgs& A, const DevParams& P, const LaneMode& M, int f) {
-    if (INTEG != INTEG_EXP || A.rhs_only || !(MODEL == MODEL_BQLIN || P.factored)) return 1.0;
-    const double hxy = __dsub_rn(-__dmul_rn(M.kxe, M.kxe), __dmul_rn(M.b, M.b));
-    return exp(A.sc.linC * (f < 2 ? P.nu : P.cb) * hxy);
-}
+    // store(s): F and the new value
+    __device__ __forceinline__ void store(const StageArgs& A, const DevParams& P, const LaneMode& M, int s, double c,
+                                          cplx F, cplx nv) const {
+        s = QLGPU_CHECK_INDEX(s, W::nz, &A.clk->status);
+        if (RHS && rhs_only) {
+            stg(out + s, F);
+            if (linop) linop[s] = linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2val(c)), f);
+            return;
+        }
+        if (fo) stg(fo + s, F);
+        stg(out + s, zero ? mk(0.0, 0.0) : nv);
+    }
+    static __device__ __forceinline__ void stg(cplx* p, cplx v) {
+        __stcg(reinterpret_cast<double2*>(p), make_double2(v.x, v.y));
+    }
+};
 
 // Spectral input of an inverse task for this lane's mode, scaled by 1/NZ:
 // kind 0 the field, 1 z-component, 2 i kz z-component, 3 y-component
 // (MHD_BQlin.cpp:143-146), 4 i kz field, 5 i kz y-component.
 template <class W>
-__device__ __forceinline__ void inv_input(cplx (&x)[8], const cplx* g0, const double* __restrict__ il2, int kind,
+__device__ __forceinline__ void inv_input(cplx (&x)[8], const cplx* g0, const double* il2, int kind,
                                           double a, double b, double fac, const double* kzc, int t) {
     const cplx* g1 = g0 + W::nz;
     if (kind == 0 || kind == 4) {
@@ -261,20 +309,31 @@ __device__ __forceinline__ void inv_input(cplx (&x)[8], const cplx* g0, const do
         }
         return;
     }
-    const double ab = __dmul_rn(a, b);
+    if (kind == 3 || kind == 5) {  // (a b) u + i c z
+        const double ab = __dmul_rn(a, b);
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
+        for (int r = 0; r < 8; ++r) {
+            const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+            cplx v = mk(0.0, 0.0);
+            if (s >= 0) {
+                const double c = kzc[t + W::T * r], sc = il2[s] * fac;
+                const cplx u = g0[s], z = g1[s];
+                v = mk(fma(ab, u.x, -c * z.y), fma(ab, u.y, c * z.x));
+                v = kind == 5 ? imul(v, sc * c) : cscale(v, sc);
+            }
+            x[r] = v;
+        }
+        return;
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {  // (a c) u - i b z
         const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
         cplx v = mk(0.0, 0.0);
         if (s >= 0) {
-            const double c = kzc[t + W::T * r];
+            const double c = kzc[t + W::T * r], sc = il2[s] * fac, p = __dmul_rn(a, c);
             const cplx u = g0[s], z = g1[s];
-            const double sc = __ldg(il2 + s) * fac;
-            // y: (a b) u + i c z;  z: (a c) u - i b z
-            const double p = (kind == 3 || kind == 5) ? ab : __dmul_rn(a, c);
-            const double q = (kind == 3 || kind == 5) ? c : -b;
-            v = mk(fma(p, u.x, -q * z.y), fma(p, u.y, q * z.x));
-            v = (kind == 2 || kind == 5) ? imul(v, sc * c) : cscale(v, sc);
+            v = mk(fma(p, u.x, b * z.y), fma(p, u.y, -b * z.x));
+            v = kind == 2 ? imul(v, sc * c) : cscale(v, sc);
         }
         x[r] = v;
     }
@@ -285,118 +344,131 @@ __device__ __forceinline__ void inv_input(cplx (&x)[8], const cplx* g0, const do
 // ---------------------------------------------------------------------------
 enum { R_UZ = 0, R_BZ, R_U, R_B, R_ZE, R_ET, R_DUZ, R_UY, R_BY };
 
-template <class W, int INTEG>
-__device__ __forceinline__ void bq_forward(const StageArgs& A, const DevParams& P, const LaneMode& M, const CnOld& cn,
-                                           int task, cplx* R, const cplx* stg, const double* ekz, const double* prof,
-                                           const double* kzc, const cplx* tw, int lane, int g, int t) {
-    constexpr int T = W::T, nzd = W::nz;
-    const StageConst& S = A.sc;
+// Forward task 0: S = T(i ky By R_b), kept in its buffer, 1: T(2 kx ky dBy R_bz) -> u, 2: eta,
+// 3: zeta, 4: b.  The input of a task, conjugated.
+template <class W>
+__device__ __forceinline__ void bq_input(cplx (&x)[8], const LaneMode& M, int task, const cplx* R, const double* prof,
+                                         int lane, int t) {
+    constexpr int T = W::T;
     const double *By = prof, *dBy = prof + W::NZ, *ddBy = prof + 2 * W::NZ;
-    auto buf = [&](int i) { return R + (size_t)i * 256; };
+    auto buf = [&](int i) { return R + i * W::XW; };
     const double a = M.a, b = M.b;
-    // field updated, its exchange buffer (one that no other task still reads)
-    const int f = task == 0 ? 0 : task == 1 ? 3 : task == 2 ? 1 : 2;
-    cplx* xg = task == 1 ? buf(R_ZE) : task == 2 ? buf(R_ET) : buf(W::NINV + (task == 0 ? 0 : 2));
-    cplx* Sb = buf(W::NINV + 1) + lane;  // task 0: S, this lane's entries
-    const cplx* Fp = (A.Fprev && S.has_prev) ? A.Fprev + ((size_t)M.m * 4 + f) * nzd : nullptr;
-    cplx x[8];
-    for (int sub = task == 0 ? 0 : 1; sub < 2; ++sub) {
-        if (task == 0) {
-            const cplx* p = buf(sub ? R_BZ : R_B) + lane;
-            const double ab2 = 2.0 * __dmul_rn(a, b);
+    if (task == 1) {
+        const cplx* p = buf(R_BZ) + lane;
+        const double ab2 = 2.0 * __dmul_rn(a, b);
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int z = t + T * r;
-                const cplx v = p[32 * r];
-                const double w = ab2 * dBy[z], y = b * By[z];
-                // conj(2 kx ky dBy R_bz) or conj(i ky By R_b)
-                x[r] = sub ? mk(w * v.x, -w * v.y) : mk(-y * v.y, -y * v.x);
-            }
-        } else if (task == 3) {
-            const cplx* p = buf(R_U) + lane;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const cplx v = p[32 * r];
-                const double y = b * By[t + T * r];
-                x[r] = mk(-y * v.y, -y * v.x);  // conj(i ky By R_u)
-            }
-        } else {
-            // eta: i ky By R_zeta - i kx dBy R_u - 2 dBy R_{i kz uz} - ddBy R_uz (MHD_BQlin.cpp:189-198)
-            // zeta: i ky By R_eta - i kx dBy R_b + ddBy R_bz (MHD_BQlin.cpp:170-178)
-            const cplx* p0 = buf(task == 1 ? R_ZE : R_ET) + lane;
-            const cplx* p1 = buf(task == 1 ? R_U : R_B) + lane;
-            const cplx* p2 = buf(task == 1 ? R_UZ : R_BZ) + lane;
-            const cplx* p3 = buf(R_DUZ) + lane;
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const int z = t + T * r;
-                const cplx v0 = p0[32 * r], v1 = p1[32 * r], v2 = p2[32 * r];
-                const double y = b * By[z], d = a * dBy[z], e = task == 1 ? -ddBy[z] : ddBy[z];
-                double re = fma(-y, v0.y, fma(d, v1.y, e * v2.x));
-                double im = fma(y, v0.x, fma(-d, v1.x, e * v2.y));
-                if (task == 1) {
-                    const cplx v3 = p3[32 * r];
-                    const double d2 = -2.0 * dBy[z];
-                    re = fma(d2, v3.x, re);
-                    im = fma(d2, v3.y, im);
-                }
-                x[r] = mk(re, -im);
-            }
+        for (int r = 0; r < 8; ++r) {
+            const cplx v = p[32 * r];
+            const double w = ab2 * dBy[t + T * r];
+            x[r] = mk(w * v.x, -w * v.y);  // conj(2 kx ky dBy R_bz)
         }
-        __syncwarp();  // the exchange buffer may be one of those just read
-        xform<W>(x, xg, tw, g, t);
-        if (sub == 0) {
+    } else if (task == 0 || task == 4) {
+        const cplx* p = buf(task == 0 ? R_B : R_U) + lane;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) Sb[32 * r] = conjc(x[r]);
+        for (int r = 0; r < 8; ++r) {
+            const cplx v = p[32 * r];
+            const double y = -b * By[t + T * r];
+            x[r] = mk(y * v.y, y * v.x);  // conj(i ky By R)
+        }
+    } else {
+        // eta: i ky By R_zeta - i kx dBy R_u - 2 dBy R_{i kz uz} - ddBy R_uz (MHD_BQlin.cpp:189-198)
+        // zeta: i ky By R_eta - i kx dBy R_b + ddBy R_bz (MHD_BQlin.cpp:170-178)
+        const bool eta = task == 2;
+        const cplx* p0 = buf(eta ? R_ZE : R_ET) + lane;
+        const cplx* p1 = buf(eta ? R_U : R_B) + lane;
+        const cplx* p2 = buf(eta ? R_UZ : R_BZ) + lane;
+        const cplx* p3 = buf(R_DUZ) + lane;
+        const double sg = eta ? -1.0 : 1.0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int z = t + T * r;
+            const cplx v0 = p0[32 * r], v1 = p1[32 * r], v2 = p2[32 * r];
+            const double y = b * By[z], d = a * dBy[z], e = sg * ddBy[z];
+            double re = fma(-y, v0.y, fma(d, v1.y, e * v2.x));
+            double im = fma(y, v0.x, fma(-d, v1.x, e * v2.y));
+            if (eta) {
+                const cplx v3 = p3[32 * r];
+                const double d2 = -2.0 * dBy[z];
+                re = fma(d2, v3.x, re);
+                im = fma(d2, v3.y, im);
+            }
+            x[r] = mk(re, -im);
         }
     }
+}
+
+// Transform of a task's input in exchange buffer xg and, but for S, the update of its field.
+// wait_S() comes before task 1 reads S (in Sb), which another warp may have written.
+template <class W, int INTEG, bool RHS, class WaitS>
+__device__ __forceinline__ void bq_finish(cplx (&x)[8], const StageArgs& A, const DevParams& P, const LaneMode& M,
+                                          const CnOld& cn, int task, cplx* xg, const cplx* Sb, const cplx* stg,
+                                          const cplx* fps, const double* ekz, const double* kzc, const cplx* tw, int lane, int g, int t,
+                                          WaitS&& wait_S) {
+    constexpr int T = W::T, nzd = W::nz;
+    const double a = M.a, b = M.b;
+    xform<W>(x, xg, tw, g, t);
+    if (task == 0) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) xg[32 * r + lane] = conjc(x[r]);
+        return;
+    }
+    if (task == 1) wait_S();
     if (!M.valid) return;
-    const double em = em_of<MODEL_BQLIN, INTEG>(A, P, M, f);
+    const int f = task == 1 ? 0 : task == 2 ? 3 : task == 3 ? 1 : 2;
+    const Put<W, MODEL_BQLIN, INTEG, RHS> put(A, P, M, f, fps, ekz);
+    const StageConst& S = A.sc;
     const double Om2 = __dmul_rn(2.0, P.Omega);
     const double cl = f == 3 ? -P.q : (f == 1 ? (P.q - Om2) : 0.0);
     const double rl = __dmul_rn(__dmul_rn(2.0, __dmul_rn(a, b)), P.q);
     const cplx* fin = stg + f * nzd;
     const cplx* l0 = stg + (f == 3 ? 2 : 0) * nzd;
-    cplx fpv[8];
+    // four registers at a time: the values, then the stores
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
-        fpv[r] = (Fp && s >= 0) ? ldc(Fp + s) : mk(0.0, 0.0);
-    }
+    for (int h = 0; h < 2; ++h) {
+        cplx nv[4];
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-        if (rdead<W>(r)) continue;
-        const int s = sidx<W>(t, r);
-        if (s < 0) continue;
-        const double c = kzc[t + T * r];
-        cplx F = conjc(x[r]);
-        if (f == 0) {
-            // S + ilapF ((2 kx ky q) u + 2 Omega i kz zeta + fwd(...)) (MHD_BQlin.cpp:162)
-            const bool z0 = (M.kyi == 0 && s == 0);
-            const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2val(c), z0));
-            const double ilapF = (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF);
-            const cplx lin = cadd(cadd(F, cscale(stg[s], rl)), imul(stg[nzd + s], Om2 * c));
-            F = cadd(Sb[32 * r], cscale(lin, ilapF));
-        } else if (f != 2) {
-            F = cadd(F, imul(l0[s], cl * c));  // MHD_BQlin.cpp:178,201
+        for (int i = 0; i < 4; ++i) {
+            const int r = 4 * h + i;
+            const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
+            nv[i] = mk(0.0, 0.0);
+            if (s < 0) continue;
+            const double c = kzc[t + T * r];
+            cplx F = conjc(x[r]);
+            if (f == 0) {
+                // S + ilapF ((2 kx ky q) u + 2 Omega i kz zeta + fwd(...)) (MHD_BQlin.cpp:162)
+                const bool z0 = (M.kyi == 0 && s == 0);
+                const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2val(c), z0));
+                const double ilapF = (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF);
+                const cplx lin = cadd(cadd(F, cscale(stg[s], rl)), imul(stg[nzd + s], Om2 * c));
+                F = cadd(Sb[32 * r + lane], cscale(lin, ilapF));
+            } else if (f != 2) {
+                F = cadd(F, imul(l0[s], cl * c));  // MHD_BQlin.cpp:178,201
+            }
+            x[r] = F;
+            nv[i] = put.value(S, P, M, cn, s, c, F, fin[s], put.fp ? put.fp[s] : mk(0.0, 0.0));
         }
-        put_coef<W, MODEL_BQLIN, INTEG>(A, P, M, cn, ekz, em, f, s, c, F, fin[s], fpv[r], Fp != nullptr);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int r = 4 * h + i;
+            if (rdead<W>(r)) continue;
+            const int s = sidx<W>(t, r);
+            if (s >= 0) put.store(A, P, M, s, kzc[t + T * r], x[r], nv[i]);
+        }
     }
 }
 
+// Stress sums, half 0: Ex (from R_uz, R_bz, R_u, R_b), half 1: Ey (MHD_BQlin.cpp:212-241)
 template <class W>
-__device__ __forceinline__ void bq_stress(const LaneMode& M, const cplx* R, double* acc, int lane) {
-    auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+__device__ __forceinline__ void bq_stress(const LaneMode& M, int half, const cplx* R, double* acc, int lane) {
+    const cplx* p = R + W::XW * (half ? R_UY : R_U) + lane;
+    const cplx* q = R + W::XW * (half ? R_BY : R_B) + lane;
+    const cplx *pu = R + W::XW * R_UZ + lane, *pb = R + W::XW * R_BZ + lane;
+    double* ax = acc + 256 * half + lane;
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
-        const cplx uz = rd(R_UZ, r), bz = rd(R_BZ, r), u = rd(R_U, r), bb = rd(R_B, r), uy = rd(R_UY, r),
-                   by = rd(R_BY, r);
-        // MHD_BQlin.cpp:212-241
-        const double ex = fma(bz.x, u.x, bz.y * u.y) - fma(uz.x, bb.x, uz.y * bb.y);
-        const double ey = fma(bz.x, uy.x, bz.y * uy.y) - fma(uz.x, by.x, uz.y * by.y);
-        double* ax = acc + 32 * r + lane;
-        ax[0] = fma(M.mult, ex, ax[0]);
-        ax[256] = fma(M.mult, ey, ax[256]);
+        const cplx uz = pu[32 * r], bz = pb[32 * r], u = p[32 * r], bb = q[32 * r];
+        const double e = fma(bz.x, u.x, bz.y * u.y) - fma(uz.x, bb.x, uz.y * bb.y);
+        ax[32 * r] = fma(M.mult, e, ax[32 * r]);
     }
 }
 
@@ -414,7 +486,7 @@ template <class W>
 __device__ __forceinline__ void fq_input(cplx (&x)[8], const LaneMode& M, int n, const cplx* R, const double* prof,
                                          int lane, int t) {
     constexpr int NZ = W::NZ;
-    auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+    auto rd = [&](int i, int r) { return R[i * W::XW + 32 * r + lane]; };
     const int k = n % 3;
     const bool sside = n >= 3;
     const int own = sside ? Q_BX + k : Q_UX + k, oth = sside ? Q_UX + k : Q_BX + k;
@@ -436,7 +508,7 @@ __device__ __forceinline__ void fq_input(cplx (&x)[8], const LaneMode& M, int n,
 // Stress sums: half 0 the EMFs and the x drive of u, half 1 the rest (MHD_FullQlin.cpp:314-362)
 template <class W>
 __device__ __forceinline__ void fq_stress(const LaneMode& M, int half, const cplx* R, double* acc, int lane) {
-    auto rd = [&](int i, int r) { return R[(size_t)i * 256 + 32 * r + lane]; };
+    auto rd = [&](int i, int r) { return R[i * W::XW + 32 * r + lane]; };
     auto rc = [](cplx p, cplx q) { return p.x * q.x + p.y * q.y; };  // Re(p conj q)
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
@@ -462,22 +534,21 @@ __device__ __forceinline__ void fq_stress(const LaneMode& M, int half, const cpl
 }
 
 // Update of field f from the six spectra in X[n][r][lane] (MHD_FullQlin.cpp:283-305)
-template <class W, int INTEG>
+template <class W, int INTEG, bool RHS>
 __device__ __forceinline__ void fq_update(const StageArgs& A, const DevParams& P, const LaneMode& M, const CnOld& cn,
-                                          int f, const cplx* X, const cplx* stg, const double* ekz, const double* kzc,
-                                          int lane, int t) {
+                                          int f, const cplx* X, const cplx* stg, const cplx* fps, const double* ekz,
+                                          const double* kzc, int lane, int t) {
     constexpr int nzd = W::nz;
     if (!M.valid) return;
     const StageConst& S = A.sc;
     const double a = M.a, b = M.b, ab = __dmul_rn(a, b), Om2 = __dmul_rn(2.0, P.Omega);
-    const double em = em_of<MODEL_FULLQLIN, INTEG>(A, P, M, f);
-    const cplx* Fp = (A.Fprev && S.has_prev) ? A.Fprev + ((size_t)M.m * 4 + f) * nzd : nullptr;
-    auto X_ = [&](int n, int r) { return X[(size_t)n * 256 + 32 * r + lane]; };
+    const Put<W, MODEL_FULLQLIN, INTEG, RHS> put(A, P, M, f, fps, ekz);
+    auto X_ = [&](int n, int r) { return X[n * W::XW + 32 * r + lane]; };
     cplx fpv[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
         const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
-        fpv[r] = (Fp && s >= 0) ? ldc(Fp + s) : mk(0.0, 0.0);
+        fpv[r] = (put.fp && s >= 0) ? ldc(put.fp + s) : mk(0.0, 0.0);
     }
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
@@ -510,7 +581,7 @@ __device__ __forceinline__ void fq_update(const StageArgs& A, const DevParams& P
             F = csub(cadd(imul(stg[2 * nzd + s], -P.q * c), imul(stg[nzd + s], P.B0z * c)),
                      csub(imul(X_(4, r), c), imul(X_(5, r), b)));
         }
-        put_coef<W, MODEL_FULLQLIN, INTEG>(A, P, M, cn, ekz, em, f, s, c, F, uin, fpv[r], Fp != nullptr);
+        put.store(A, P, M, s, c, F, put.value(S, P, M, cn, s, c, F, uin, fpv[r]));
     }
 }
 
@@ -601,8 +672,9 @@ enum StageResult { STAGE_DONE = 0, STAGE_TOP = 1, STAGE_ABORT = 2 };
 // run before gate() (called by thread 0; false ends the launch), which in a
 // persistent launch waits for the case's previous stage.  fresh: the shared-memory
 // tables do not hold this case's yet.  REDUCER: the launch has a CTA of its own for the
-// mean-field side (reduce_stage); this one only counts itself in at `arrive`.
-template <int NZ, int MODEL, int INTEG, bool REDUCER, class Gate>
+// mean-field side (reduce_stage); this one only counts itself in at `arrive`.  RHS: the
+// launch may ask for the right-hand side instead of the update (A.rhs_only).
+template <int NZ, int MODEL, int INTEG, bool REDUCER, bool RHS, class Gate>
 __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevParams& P, const int cta,
                                                   const int ncta, unsigned char* smem_raw, StageShared& ss,
                                                   LocalClock& lc, const bool fresh, unsigned* arrive,
@@ -624,6 +696,8 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
     unsigned char* tbase = smem_raw + W::o_team + W::TEAM_BYTES * (size_t)(in_team ? team : 0);
     cplx* R = reinterpret_cast<cplx*>(tbase);
     cplx* stg_all = reinterpret_cast<cplx*>(tbase + W::TM_STG);
+    cplx* fp_all = reinterpret_cast<cplx*>(tbase + W::TM_FP);
+    double* il2_all = reinterpret_cast<double*>(tbase + W::TM_IL2);
     double* acc = reinterpret_cast<double*>(tbase + W::TM_ACC);
     const int bar = 1 + team, bthreads = 32 * tws;
     const bool tr = A.trace && cta == 0 && tid == 0;
@@ -631,11 +705,17 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
 
     // ---- first block's fields requested, then the tables and the cleared sums
     const int step = ncta * nteams * GPW;
-    const int first = (cta * nteams + team) * GPW;
+    // block b: CTA b mod ncta, so that a last, partial round leaves one team per SM, not full and idle CTAs
+    const int first = (team * ncta + cta) * GPW;
+    const bool has_prev = A.Fprev && S.has_prev;
+    // a block's fields and 1/lap2
     auto stage_block = [&](int base) {
-        const int n = min(GPW, P.nxy - base) * 4 * nzd;
-        const cplx* src = A.lin_in + (size_t)base * 4 * nzd;
-        for (int i = wt * 32 + lane; i < n; i += bthreads) cp_async16(stg_all + i, src + i);
+        const int nm = min(GPW, P.nxy - base), n = nm * 4 * nzd;
+        const size_t at = (size_t)base * 4 * nzd;
+        for (int i = wt * 32 + lane; i < n; i += bthreads) cp_async16(stg_all + i, A.lin_in + at + i);
+        // a team of one block keeps its 1/lap2 from stage to stage
+        for (int i = wt * 32 + lane; (fresh || first + step < P.nxy) && i < nm * nzd; i += bthreads)
+            cp_async8(il2_all + i, A.ilap2 + (size_t)__ldg(A.kyi + base + i / nzd) * nzd + i % nzd);
         cp_async_commit();
     };
     if (in_team && first < P.nxy) stage_block(first);
@@ -662,8 +742,17 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
     }
     if (in_team)
         for (int i = wt * 32 + lane; i < 256 * W::NE; i += bthreads) acc[i] = 0.0;
-    for (int i = tid; i < 6 * MAX_WARPS; i += blockDim.x) dred[i] = 0.0;
+    for (int i = tid; i < 6 * 4; i += blockDim.x) dred[i] = 0.0;
     if (fresh) __syncthreads();
+    if (!cached) {
+        // a launch's first stage (the gate does not wait then); scratch: the first team's buffers
+        const int nw = warps < 8 ? warps : 8;
+        if (warp < nw)
+            mean_profiles8<W, W::BQ>(
+                P, [&](int m, int s) { return ldc_cg(A.mf + m * nzd + s); }, prof,
+                reinterpret_cast<cplx*>(smem_raw + W::o_team) + W::XW * warp, tw, warp, nw, lane);
+        __syncthreads();
+    }
     if (tr) A.trace[1] = gtimer();
 
     // Last-stage bookkeeping identical in every CTA (main.cpp:111-130)
@@ -674,7 +763,6 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
     const double ts = S.abs_time ? S.t_off : __dadd_rn(tclock, S.t_off);
 
     // ---- the team's blocks of GPW modes
-    const bool has_prev = A.Fprev && S.has_prev;
     for (int base = first;; base += step) {
         const bool active = in_team && base < P.nxy;
         if (!active && base != first) break;
@@ -683,6 +771,9 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
         M.valid = active && g < nv;
         M.m = QLGPU_CHECK_INDEX(active ? base + min(g, nv - 1) : 0, P.nxy, &A.clk->status);
         const cplx* stg = stg_all + (size_t)min(g, nv - 1) * 4 * nzd;
+        const cplx* fps = !has_prev ? nullptr
+                        : W::BQ ? fp_all + (size_t)min(g, nv - 1) * 4 * nzd : A.Fprev + (size_t)M.m * 4 * nzd;
+        const double* il2 = il2_all + min(g, nv - 1) * nzd;
         M.b = __ldg(A.ky + M.m);
         M.kx0 = __ldcg(A.kx0 + M.m);
         M.kyi = __ldg(A.kyi + M.m);
@@ -690,7 +781,8 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
         M.a = kx_at(M.kx0, P.q, ts, M.b);  // kx(t_s), MHD_BQlin.cpp:498
         M.mult = M.valid ? (M.b == 0.0 ? 1.0 : 2.0) : 0.0;
         M.kxe = __dadd_rn(M.a, __dmul_rn(__dmul_rn(P.q, S.dt_lin), M.b));  // MHD_BQlin.cpp:248
-        M.kxo = 0.0;
+        M.kxo = M.em = 0.0;
+        M.em_side = -1;
         if (INTEG == INTEG_CN) {
             if (cn.old_init) M.kxo = kx_at(M.kx0, P.q, tclock, M.b);
             else M.kxo = __dadd_rn(kx_at(M.kx0, P.q, cn.t_old, M.b), __dmul_rn(__dmul_rn(P.q, cn.dtlin_old), M.b));
@@ -708,9 +800,18 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
                     if (has_prev) l2_prefetch(A.Fprev + nb * 4 * nzd, bytes);
                 }
             }
-            const double* __restrict__ il2 = A.ilap2 + (size_t)M.kyi * nzd;
+            // computed while the block's fields are on their way
+            M.em_side = W::BQ ? (wt == 1 || wt == 3 ? 0 : 1) : (wt < 2 ? 0 : 1);
+            if (INTEG == INTEG_EXP && !A.rhs_only && (W::BQ || P.factored) && wt < (W::BQ ? 5 : 4)) M.em = M.em_of(A, P, M.em_side);
+            else M.em_side = -1;
             cp_async_wait_all();
             team_sync(bar, bthreads);
+            // its previous right-hand sides, on their way under the inverse transforms
+            if (W::BQ && has_prev) {
+                for (int i = wt * 32 + lane; i < nv * 4 * nzd; i += bthreads)
+                    cp_async16(fp_all + i, A.Fprev + (size_t)base * 4 * nzd + i);
+                cp_async_commit();
+            }
             if (A.rec_lin) {  // record the block's input fields
                 cplx* dst = A.rec_lin + (size_t)base * 4 * nzd;
                 for (int i = wt * 32 + lane; i < nv * 4 * nzd; i += bthreads) dst[i] = stg_all[i];
@@ -731,29 +832,31 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
                 const int f0 = 2 * side + (W::BQ && (task == R_ZE || task == R_ET) ? 1 : 0);
                 cplx x[8];
                 inv_input<W>(x, stg + f0 * nzd, il2, kind, M.a, M.b, P.fac, kzc, t);
-                cplx* xb = R + (size_t)task * 256;
+                cplx* xb = R + task * W::XW;
                 xform<W>(x, xb, tw, g, t);
 #pragma unroll
                 for (int r = 0; r < 8; ++r) xb[32 * r + lane] = x[r];
+                // a team of five: its last warp has one task less and takes the Ex sums meanwhile,
+                // once R_uz, R_bz, R_u, R_b of the others' first round are there
+                if (W::BQ && tws == 5) {
+                    if (wt == 4) {
+                        team_sync(bar + 4, 160);
+                        bq_stress<W>(M, 0, R, acc, lane);
+                    } else if (task < 4) {
+                        team_arrive(bar + 4, 160);
+                    }
+                }
             }
         }
+        cp_async_wait_all();
         if (base == first) {
             // ---- the mean field of this stage
             if (tid == 0) ss.ok = gate() ? 1 : 0;
             __syncthreads();
             if (!ss.ok) return STAGE_ABORT;
             if (tr) A.trace[6] = gtimer();
-            if (cached) {
+            if (cached)
                 for (int i = tid; i < W::NPROF * NZ; i += blockDim.x) prof[i] = __ldcg(A.mfr_cache + i);
-            } else {
-                // scratch: the forward tasks' exchange buffers of the first team
-                cplx* r0 = reinterpret_cast<cplx*>(smem_raw + W::o_team) + 256 * W::NINV;
-                const int nw = warps < W::NX ? warps : W::NX;
-                if (warp < nw)
-                    mean_profiles8<W, W::BQ>(
-                        P, [&](int m, int s) { return ldc_cg(A.mf + m * nzd + s); }, prof, r0 + 256 * warp, tw, warp,
-                        nw, lane);
-            }
             // optional record of the stage input (the adjoint's window recompute): CTA 0 of the case
             // copies the mean fields and, in a step's first stage, kx0 and the clock
             if (A.rec_mf && cta == 0) {
@@ -775,10 +878,38 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
         }
         // ---- products, forward transforms, stresses
         if constexpr (W::BQ) {
+            auto buf = [&](int i) { return R + i * W::XW; };
+            cplx x[8];
+            if (tws >= 5) {
+                // one forward task per warp.  Once all inputs (and the Ex sums) are read, the buffers of
+                // R_b, R_{i kz uz}, R_zeta, R_eta, R_u are the tasks' exchange buffers; S -> u is a
+                // hand-over between two warps, so that no warp has two transforms
+                if (wt < 5) bq_input<W>(x, M, wt, R, prof, lane, t);
+                else if (wt == 5) bq_stress<W>(M, 0, R, acc, lane);
+                team_sync(bar, bthreads);
+                if (wt < 5) {
+                    cplx* xg = buf(wt == 0 ? R_B : wt == 1 ? R_DUZ : wt == 2 ? R_ZE : wt == 3 ? R_ET : R_U);
+                    bq_finish<W, INTEG, RHS>(x, A, P, M, cn, wt, xg, buf(R_B), stg, fps, ekz, kzc, tw, lane, g, t,
+                                        [&] { team_sync(bar + 8, 64); });
+                }
+                if (wt == 0) team_arrive(bar + 8, 64);
+                if (wt == (tws == 5 ? 0 : 5)) bq_stress<W>(M, 1, R, acc, lane);
+            } else {
+                // S and u by warp 0, the others' fields and the stresses by the warps in turn; exchange
+                // buffers that no other task still reads (R_zeta and R_eta have one reader each)
+                cplx* more = reinterpret_cast<cplx*>(tbase + W::TEAM_BYTES);
 #pragma unroll 1
-            for (int task = wt; task < 5; task += tws) {
-                if (task == 4) bq_stress<W>(M, R, acc, lane);
-                else bq_forward<W, INTEG>(A, P, M, cn, task, R, stg, ekz, prof, kzc, tw, lane, g, t);
+                for (int task = 0; task < 7; ++task) {
+                    if ((task < 2 ? 0 : (task - 1) % tws) != wt) continue;
+                    if (task >= 5) {
+                        bq_stress<W>(M, task - 5, R, acc, lane);
+                        continue;
+                    }
+                    bq_input<W>(x, M, task, R, prof, lane, t);
+                    __syncwarp();
+                    cplx* xg = task == 2 ? buf(R_ZE) : task == 3 ? buf(R_ET) : more + W::XW * (task == 4 ? 2 : task);
+                    bq_finish<W, INTEG, RHS>(x, A, P, M, cn, task, xg, more, stg, fps, ekz, kzc, tw, lane, g, t, [] {});
+                }
             }
         } else {
 #pragma unroll 1
@@ -789,7 +920,7 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
                 }
                 cplx x[8];
                 fq_input<W>(x, M, task, R, prof, lane, t);
-                cplx* xb = R + (size_t)(W::NINV + task) * 256;
+                cplx* xb = R + (W::NINV + task) * W::XW;
                 xform<W>(x, xb, tw, g, t);
 #pragma unroll
                 for (int r = 0; r < 8; ++r) xb[32 * r + lane] = conjc(x[r]);
@@ -797,7 +928,7 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
             team_sync(bar, bthreads);
 #pragma unroll 1
             for (int f = wt; f < 4; f += tws)
-                fq_update<W, INTEG>(A, P, M, cn, f, R + (size_t)W::NINV * 256, stg, ekz, kzc, lane, t);
+                fq_update<W, INTEG, RHS>(A, P, M, cn, f, R + W::NINV * W::XW, stg, fps, ekz, kzc, lane, t);
         }
         team_sync(bar, bthreads);  // the block's stores are done; its buffers are free
         if (last) {
@@ -930,22 +1061,22 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
     if (A.trace && tid == 0) A.trace[4] = gtimer();
     __syncthreads();
     // exchange buffers of the mean-field transforms: the last four result buffers of the first team
-    cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team) + 256 * (size_t)(W::NINV + W::NX - 4);
-    wide::top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, tclock, t_new, last, diag_due);
+    cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team + W::TOP_XCH);
+    wide::top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, nullptr, tclock, t_new, last, diag_due);
     if (A.trace && tid == 0) A.trace[5] = gtimer();
     return STAGE_TOP;
 }
 
 // One stage launch of a single case (Model::rhs, timed stages, host-controlled steps).
 template <int NZ, int MODEL, int INTEG>
-__global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) stage_kernel(const __grid_constant__ StageArgs A,
+__global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) stage_kernel(const __grid_constant__ StageArgs A,
                                                                        const __grid_constant__ DevParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StageShared ss;
     __shared__ LocalClock lc;
     if (threadIdx.x == 0) load_clock(lc, A.clk);
     __syncthreads();
-    stage_body<NZ, MODEL, INTEG, false>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss, lc, true, nullptr,
+    stage_body<NZ, MODEL, INTEG, false, true>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss, lc, true, nullptr,
                                         [] { return true; });
 }
 
@@ -985,7 +1116,7 @@ __device__ __forceinline__ bool run_wait(const unsigned* p, unsigned target, Dev
 // the groups), then the mean-field stage.
 template <int NZ, int MODEL, int INTEG>
 __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams& P, int ncta,
-                                             unsigned char* smem_raw, const cplx* tw, LocalClock& lc) {
+                                             unsigned char* smem_raw, const cplx* tw, const double* emf, LocalClock& lc) {
     using namespace wide;
     using W = WG<NZ, MODEL>;
     const int tid = threadIdx.x, nth = blockDim.x;
@@ -1032,8 +1163,8 @@ __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams
         __syncthreads();
     }
     if (A.trace && tid == 0) A.trace[4] = gtimer();
-    cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team) + 256 * (size_t)(W::NINV + W::NX - 4);
-    top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, tclock, t_new, last, diag_due);
+    cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team + W::TOP_XCH);
+    top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, emf, tclock, t_new, last, diag_due);
     if (tid == 0) advance_clock(lc, A.sc, P, last, diag_due);
     if (A.trace && tid == 0) A.trace[5] = gtimer();
 }
@@ -1047,7 +1178,7 @@ __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams
 // and iterations; one that gives up sets QLGPU_STATUS_TIMEOUT and the abort word, and
 // every CTA leaves.
 template <int NZ, int MODEL, int INTEG>
-__global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) run_kernel(const __grid_constant__ RunArgs L) {
+__global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(const __grid_constant__ RunArgs L) {
     using W = wide::WG<NZ, MODEL>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StageShared ss;
@@ -1062,16 +1193,24 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) run_kernel(const __gr
     unsigned k = 0;  // stages before this one in the launch
     if (reducer) {
         cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
+        double* emf = reinterpret_cast<double*>(smem_raw + W::o_ekz);
         for (int i = tid; i < NZ; i += blockDim.x) tw[i] = ldc_cg(L.A[0].tw + NZ + i);
         for (int n = 0; n < L.nsteps; ++n)
             for (int s = 0; s < 3; ++s, ++k) {
                 __syncthreads();
                 if (tid == 0) ss.ok = run_wait(&C->arrive, (k + 1) * (unsigned)ncta, C, L.wait_ns) ? 1 : 0;
+                if (INTEG == INTEG_EXP)  // under the wait (the last threads: the first one polls)
+                    for (int i = blockDim.x - 1 - tid; i < W::nz; i += blockDim.x) {
+                        const double kz2 = kz2val(kzval(i <= W::H ? i : i - W::nz, L.P.kzL));
+                        const double lc_ = sA[s].sc.linC;
+                        emf[i] = L.P.ql ? exp(__dmul_rn(lc_, __dmul_rn(L.P.eta, kz2))) : 1.0;
+                        emf[W::NZE + i] = L.P.ql ? exp(__dmul_rn(lc_, __dmul_rn(L.P.nu, kz2))) : 1.0;
+                    }
                 __syncthreads();
                 if (!ss.ok) return;
-                reduce_stage<NZ, MODEL, INTEG>(sA[s], L.P, ncta, smem_raw, tw, lc);
+                reduce_stage<NZ, MODEL, INTEG>(sA[s], L.P, ncta, smem_raw, tw, INTEG == INTEG_EXP ? emf : nullptr,
+                                               lc);
                 if (tid == 0) {
-                    __threadfence();
                     // after the last stage nobody waits any more: ready for the next launch
                     const bool end = n == L.nsteps - 1 && s == 2;
                     if (end) C->arrive = 0;
@@ -1098,7 +1237,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS, 1) run_kernel(const __gr
                 }
             }
             __syncthreads();
-            const StageResult r = stage_body<NZ, MODEL, INTEG, true>(
+            const StageResult r = stage_body<NZ, MODEL, INTEG, true, false>(
                 sA[s], L.P, (int)blockIdx.x, ncta, smem_raw, ss, lc, k == 0, &C->arrive,
                 [&]() -> bool { return run_wait(&C->epoch, k, C, L.wait_ns); });
             if (r == STAGE_ABORT) return;
