@@ -347,6 +347,8 @@ int qlgpu_destroy(qlgpu_t* h) {
                     h->d_mfr, h->d_ekz, h->d_forcing, h->d_kx0_prev, h->d_dbg, h->adj_ws, h->adj_tab};
     for (void* b : bufs)
         if (b) cudaFree(b);
+    if (h->adj_batch) qlgpu_batch_destroy(h->adj_batch);
+    if (h->h_pin) cudaFreeHost(h->h_pin);
     for (cudaEvent_t e : h->ev)
         if (e) cudaEventDestroy(e);
     guard_release(h->guards);
@@ -364,17 +366,49 @@ int qlgpu_dims(const qlgpu_t* h, int* nxy, int* nlin, int* nz, int* nmf) {
     return QLGPU_OK;
 }
 
+// Host arrays of a small state cross through one pinned block: four copies from or to pageable
+// memory each wait for the device (get_state of 16x16 x NZ=32 100 us, through the block 40 us).
+// Larger ones go directly, in the driver's own pieces.
+constexpr size_t PIN_MAX = (size_t)1 << 20;
+
+static size_t state_bytes(const qlgpu_t* h) {
+    return ((size_t)h->nxy * 4 * h->nz + (size_t)h->nmf * h->nz) * sizeof(cplx) + h->nxy * sizeof(double) +
+           sizeof(DevClock);
+}
+static bool pinned(qlgpu_t* h) {
+    const size_t n = state_bytes(h);
+    if (h->h_pin) return true;
+    if (n > PIN_MAX || cudaMallocHost(&h->h_pin, n) != cudaSuccess) {
+        cudaGetLastError();  // without the block the copies are direct
+        h->h_pin = nullptr;
+        return false;
+    }
+    h->pin_bytes = n;
+    return true;
+}
+
 static int set_state_impl(qlgpu_t* h, double t, const void* lin, const void* mf, const void* kx0, cudaMemcpyKind k) {
     if (!h || !lin || !mf) return fail(h, QLGPU_ERR_ARG, "null state pointer");
     QLGPU_CK(cudaSetDevice(h->device));
-    const size_t nlin = (size_t)h->nxy * 4 * h->nz, nmfe = (size_t)h->nmf * h->nz;
+    const size_t nl = (size_t)h->nxy * 4 * h->nz * sizeof(cplx), nm = (size_t)h->nmf * h->nz * sizeof(cplx),
+                 nk = h->nxy * sizeof(double);
     h->cur = 0;
-    QLGPU_CK(cudaMemcpyAsync(h->d_lin[0], lin, nlin * sizeof(cplx), k, h->stream));
-    QLGPU_CK(cudaMemcpyAsync(h->d_mf, mf, nmfe * sizeof(cplx), k, h->stream));
-    if (kx0) QLGPU_CK(cudaMemcpyAsync(h->d_kx0, kx0, h->nxy * sizeof(double), k, h->stream));
-    else
-        QLGPU_CK(cudaMemcpyAsync(h->d_kx0, h->kx_tab.data(), h->nxy * sizeof(double), cudaMemcpyHostToDevice,
-                                 h->stream));
+    if (!kx0) kx0 = h->kx_tab.data();
+    else if (k == cudaMemcpyDeviceToDevice) {
+        QLGPU_CK(cudaMemcpyAsync(h->d_kx0, kx0, nk, k, h->stream));
+        kx0 = nullptr;  // done
+    }
+    if (k == cudaMemcpyHostToDevice && pinned(h)) {
+        std::memcpy(h->h_pin, lin, nl);
+        std::memcpy(h->h_pin + nl, mf, nm);
+        std::memcpy(h->h_pin + nl + nm, kx0, nk);
+        lin = h->h_pin;
+        mf = h->h_pin + nl;
+        kx0 = h->h_pin + nl + nm;
+    }
+    QLGPU_CK(cudaMemcpyAsync(h->d_lin[0], lin, nl, k, h->stream));
+    QLGPU_CK(cudaMemcpyAsync(h->d_mf, mf, nm, k, h->stream));
+    if (kx0) QLGPU_CK(cudaMemcpyAsync(h->d_kx0, kx0, nk, cudaMemcpyHostToDevice, h->stream));
     int rc = reset_clock(h, t);
     if (rc) return rc;
     // the integrator and model start afresh: no steps, zero mean-field profiles of a previous rhs
@@ -388,13 +422,22 @@ static int set_state_impl(qlgpu_t* h, double t, const void* lin, const void* mf,
 static int get_state_impl(qlgpu_t* h, double* t, void* lin, void* mf, void* kx0, cudaMemcpyKind k) {
     if (!h) return QLGPU_ERR_ARG;
     QLGPU_CK(cudaSetDevice(h->device));
-    const size_t nlin = (size_t)h->nxy * 4 * h->nz, nmfe = (size_t)h->nmf * h->nz;
-    if (lin) QLGPU_CK(cudaMemcpyAsync(lin, h->d_lin[h->cur], nlin * sizeof(cplx), k, h->stream));
-    if (mf) QLGPU_CK(cudaMemcpyAsync(mf, h->d_mf, nmfe * sizeof(cplx), k, h->stream));
-    if (kx0) QLGPU_CK(cudaMemcpyAsync(kx0, h->d_kx0, h->nxy * sizeof(double), k, h->stream));
+    const size_t nl = (size_t)h->nxy * 4 * h->nz * sizeof(cplx), nm = (size_t)h->nmf * h->nz * sizeof(cplx),
+                 nk = h->nxy * sizeof(double);
+    const bool pin = k == cudaMemcpyDeviceToHost && pinned(h);
+    auto to = [&](void* p, size_t off) -> void* { return pin ? h->h_pin + off : p; };
+    if (lin) QLGPU_CK(cudaMemcpyAsync(to(lin, 0), h->d_lin[h->cur], nl, k, h->stream));
+    if (mf) QLGPU_CK(cudaMemcpyAsync(to(mf, nl), h->d_mf, nm, k, h->stream));
+    if (kx0) QLGPU_CK(cudaMemcpyAsync(to(kx0, nl + nm), h->d_kx0, nk, k, h->stream));
     double tt = 0;
-    QLGPU_CK(cudaMemcpyAsync(&tt, &h->d_clk->t, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    QLGPU_CK(cudaMemcpyAsync(to(&tt, nl + nm + nk), &h->d_clk->t, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     QLGPU_CK(cudaStreamSynchronize(h->stream));
+    if (pin) {
+        if (lin) std::memcpy(lin, h->h_pin, nl);
+        if (mf) std::memcpy(mf, h->h_pin + nl, nm);
+        if (kx0) std::memcpy(kx0, h->h_pin + nl + nm, nk);
+        std::memcpy(&tt, h->h_pin + nl + nm + nk, sizeof(double));
+    }
     if (t) *t = tt;
     return QLGPU_OK;
 }
@@ -578,8 +621,10 @@ int qlgpu_step(qlgpu_t* h, int nsteps, int diag_every, double* diag_out, int max
     int rc = check_launch(h);
     if (rc) return rc;
     DevClock c;
-    QLGPU_CK(cudaMemcpyAsync(&c, h->d_clk, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
+    void* cp = h->h_pin ? (void*)(h->h_pin + h->pin_bytes - sizeof(DevClock)) : (void*)&c;
+    QLGPU_CK(cudaMemcpyAsync(cp, h->d_clk, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
     QLGPU_CK(cudaStreamSynchronize(h->stream));
+    if (cp != &c) std::memcpy(&c, cp, sizeof(DevClock));
     if (c.status & QLGPU_STATUS_TIMEOUT) {
         QLGPU_CK(qlgpu_clear_abort(h));
         return fail(h, QLGPU_ERR_STATUS, "step: a CTA gave up waiting for the other CTAs of the case");

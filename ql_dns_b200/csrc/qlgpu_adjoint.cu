@@ -204,7 +204,7 @@ AdjSeedBufs adj_seed_bufs(const AdjJob& j) {
 }
 
 int adj_begin(AdjJob& j, qlgpu_t* h, double t0, const double* lin0, const double* mf0, const double* kx0, int nsteps,
-              int checkpoint_every) {
+              int checkpoint_every, bool load_state) {
     j.h = h;
     if (!lin0 || !mf0 || nsteps < 1 || checkpoint_every < 1)
         return afail(h, QLGPU_ERR_ARG, "null argument, nsteps < 1 or checkpoint_every < 1");
@@ -214,8 +214,15 @@ int adj_begin(AdjJob& j, qlgpu_t* h, double t0, const double* lin0, const double
     if (!pick_ops(h->NZ, &j.ops)) return afail(h, QLGPU_ERR_UNSUPPORTED, "unsupported NZ");
     QA_CK(cudaSetDevice(h->device));
     QA_CK(ensure_smem_attr(j.ops.modes_kernel, j.ops.modes_smem));
-    int rc = qlgpu_set_state(h, t0, lin0, mf0, kx0);
-    if (rc) return rc;
+    if (load_state) {
+        const int rc = qlgpu_set_state(h, t0, lin0, mf0, kx0);
+        if (rc) return rc;
+    } else {
+        // the forward sweep runs elsewhere; the handle gets its end state at the end of the call
+        h->cur = 0;
+        h->dt_sum = 0.0;
+        h->steps_taken = 0;
+    }
     j.N = nsteps;
     j.C = std::min(checkpoint_every, nsteps);
     j.NC = (j.N + j.C - 1) / j.C;
@@ -283,9 +290,11 @@ int adj_checkpoint(AdjJob& j, int c) {
     return QLGPU_OK;
 }
 
-int adj_forward_window(AdjJob& j, int steps) {
+// record: every stage's input too (the last window, which is reversed first)
+int adj_forward_window(AdjJob& j, int steps, bool record) {
     qlgpu_t* h = j.h;
-    QA_CK(qlgpu_enqueue_run(h, steps, nullptr));
+    const RunRecord r{j.stU, j.stB, j.kx_pre, j.t_pre, j.cn_pre};
+    QA_CK(qlgpu_enqueue_run(h, steps, record ? &r : nullptr));
     return QLGPU_OK;
 }
 
@@ -435,19 +444,37 @@ int launch_graph(AdjJob& j, cudaGraphExec_t g);
 
 // The reverse sweep runs once for all seeds (one adj_reverse_window) when the
 // seeds share every parameter and the device; otherwise per seed.
-bool same_setup(const qlgpu_t* a, const qlgpu_t* b) {
-    const qlgpu_params &p = a->p, &r = b->p;
-    return a->device == b->device && p.model == r.model && p.integrator == r.integrator && p.nx == r.nx &&
+bool same_params(const qlgpu_params& p, const qlgpu_params& r) {
+    return p.model == r.model && p.integrator == r.integrator && p.nx == r.nx &&
            p.ny == r.ny && p.NZ == r.NZ && p.L[0] == r.L[0] && p.L[1] == r.L[1] && p.L[2] == r.L[2] && p.q == r.q &&
            p.omega == r.omega && p.nu == r.nu && p.eta == r.eta && p.B0z == r.B0z &&
            p.viscosity_order == r.viscosity_order && p.dt == r.dt && p.remap == r.remap &&
            p.quasilinear == r.quasilinear;
 }
+bool same_setup(const qlgpu_t* a, const qlgpu_t* b) { return a->device == b->device && same_params(a->p, b->p); }
 
+// The batch that runs the seeds' forward sweep and recompute: the first handle's from its last
+// call when it was made for the same cases (creating and destroying one takes 9 ms at 16
+// seeds), else a new one.  It goes back to the handle when the call succeeds and its fields
+// take at most ADJ_KEEP_BYTES; the handle frees it.
 struct BatchGuard {
     qlgpu_batch_t* b = nullptr;
     ~BatchGuard() {
         if (b) qlgpu_batch_destroy(b);
+    }
+    int take(qlgpu_t* h, const std::vector<qlgpu_params>& ps) {
+        std::swap(b, h->adj_batch);
+        bool same = b && ps.size() == h->adj_batch_ps.size();
+        for (size_t i = 0; same && i < ps.size(); ++i) same = same_params(ps[i], h->adj_batch_ps[i]);
+        if (same) return QLGPU_OK;
+        if (b) qlgpu_batch_destroy(b);
+        b = nullptr;
+        return qlgpu_batch_create(ps.data(), (int)ps.size(), h->device, &b);
+    }
+    void give(qlgpu_t* h, const std::vector<qlgpu_params>& ps, size_t bytes) {
+        if (bytes > ADJ_KEEP_BYTES) return;
+        std::swap(b, h->adj_batch);
+        h->adj_batch_ps = ps;
     }
 };
 
@@ -460,7 +487,7 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
     std::vector<qlgpu_params> ps(nj);
     for (int q = 0; q < nj; ++q) ps[q] = jobs[q].h->p;
     BatchGuard g;
-    int rc = qlgpu_batch_create(ps.data(), nj, h0->device, &g.b);
+    int rc = g.take(h0, ps);
     if (rc) {
         char buf[256];
         qlgpu_batch_last_error(nullptr, buf, sizeof(buf));
@@ -493,6 +520,12 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
             QA_CK(cudaMemcpyAsync(j.ck_kx0 + w * nxy, d.kx0, nxy * sizeof(double), cudaMemcpyDeviceToDevice, bs));
             QA_CK(cudaMemcpyAsync(j.ck_clk + w, d.clk, sizeof(DevClock), cudaMemcpyDeviceToDevice, bs));
         }
+        // the last window is reversed first: its stage inputs are recorded right away
+        if (w == NC - 1)
+            for (int q = 0; q < nj; ++q) {
+                const AdjJob& j = jobs[q];
+                qlgpu_batch_set_record(b, q, j.stU, j.stB, j.kx_pre, j.t_pre, j.cn_pre);
+            }
         rc = qlgpu_batch_step(b, steps, 1, recs.data(), C, nd.data());
         if (rc) {
             char buf[256];
@@ -562,7 +595,7 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
                 QA_CK(cudaEventRecord(ev_h[q], jobs[q].h->stream));
                 QA_CK(cudaStreamWaitEvent(bs, ev_h[q], 0));
             }
-        for (int q = 0; q < nj; ++q) {
+        for (int q = 0; q < nj && w != NC - 1; ++q) {
             AdjJob& j = jobs[q];
             BatchCaseDev d;
             qlgpu_batch_case_dev(b, q, &d);
@@ -574,7 +607,7 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
             QA_CK(cudaMemcpyAsync(&d.clk->mfr_valid, &zero, sizeof(int), cudaMemcpyHostToDevice, bs));
             qlgpu_batch_set_record(b, q, j.stU, j.stB, j.kx_pre, j.t_pre, j.cn_pre);
         }
-        rc = qlgpu_batch_step(b, steps, 0, nullptr, 0, nullptr);
+        if (w != NC - 1) rc = qlgpu_batch_step(b, steps, 0, nullptr, 0, nullptr);
         if (rc) {
             char buf[256];
             qlgpu_batch_last_error(b, buf, sizeof(buf));
@@ -631,6 +664,7 @@ int run_jobs_persistent(std::vector<AdjJob>& jobs, double t0, const double* lin0
     }
     QA_CK(cudaStreamSynchronize(bs));
     for (int q = 0; q < nj; ++q) J[q] = jobs[q].J;
+    g.give(h0, ps, 4 * sizeof(cplx) * nlin * nj);
     return QLGPU_OK;
 }
 
@@ -685,26 +719,32 @@ int run_jobs(std::vector<AdjJob>& jobs, double* J, double* const* grad_lin, doub
     for (int w = 0; w < NC; ++w) {
         const int steps = std::min(N, w * C + C) - w * C;
         QA_ALL(adj_checkpoint(jj, w));
-        if (graphs && steps == C) {
-            QA_ALL(jj.g_fwd ? QLGPU_OK : capture(jj, &jj.g_fwd, [&] { return adj_forward_window(jj, C); }));
+        if (graphs && steps == C && w != NC - 1) {
+            QA_ALL(jj.g_fwd ? QLGPU_OK : capture(jj, &jj.g_fwd, [&] { return adj_forward_window(jj, C, false); }));
             QA_ALL(launch_graph(jj, jj.g_fwd));
         } else {
-            QA_ALL(adj_forward_window(jj, steps));
+            QA_ALL(adj_forward_window(jj, steps, w == NC - 1));
         }
     }
+    QA_ALL(adj_window_end(jj, NC - 1));
     QA_ALL(adj_forward_end(jj));
     QA_ALL(sync_job(jj));
     QA_ALL(adj_forward_finish(jj));
     for (int w = NC - 1; w >= 0; --w) {
         const int steps = std::min(N, w * C + C) - w * C;
-        QA_ALL(adj_window_begin(jj, w));
+        if (w != NC - 1) {
+            QA_ALL(adj_window_begin(jj, w));
+            if (graphs && steps == C) {
+                QA_ALL(jj.g_rec ? QLGPU_OK : capture(jj, &jj.g_rec, [&] { return rec_window(jj, w, C); }));
+                QA_ALL(launch_graph(jj, jj.g_rec));
+            } else {
+                QA_ALL(rec_window(jj, w, steps));
+            }
+        }
         if (graphs && steps == C) {
-            QA_ALL(jj.g_rec ? QLGPU_OK : capture(jj, &jj.g_rec, [&] { return rec_window(jj, w, C); }));
-            QA_ALL(launch_graph(jj, jj.g_rec));
             QA_ALL(jj.g_bwd ? QLGPU_OK : capture(jj, &jj.g_bwd, [&] { return adj_backward_window(jj, C); }));
             QA_ALL(launch_graph(jj, jj.g_bwd));
         } else {
-            QA_ALL(rec_window(jj, w, steps));
             QA_ALL(adj_backward_window(jj, steps));
         }
     }
@@ -726,7 +766,7 @@ extern "C" int qlgpu_adjoint_maxwell(qlgpu_t* h, double t0, const double* lin0, 
     if (!h) return QLGPU_ERR_ARG;
     if (!J || !grad_lin) return afail(h, QLGPU_ERR_ARG, "null argument");
     std::vector<AdjJob> jobs(1);
-    int rc = adj_begin(jobs[0], h, t0, lin0, mf0, kx0, nsteps, checkpoint_every);
+    int rc = adj_begin(jobs[0], h, t0, lin0, mf0, kx0, nsteps, checkpoint_every, true);
     double* gl[1] = {grad_lin};
     double* gm[1] = {grad_mf};
     if (!rc) rc = run_jobs(jobs, J, gl, grad_mf ? gm : nullptr);
@@ -748,11 +788,13 @@ extern "C" int qlgpu_adjoint_maxwell_batch(qlgpu_t* const* handles, int nseeds, 
             return afail(h0, QLGPU_ERR_ARG, "handles of a batch must have the same dimensions");
     }
     const size_t nlin = (size_t)h0->nxy * 4 * h0->nz, nmfe = (size_t)h0->nmf * h0->nz;
+    const char* mode = getenv("QLGPU_ADJ_BATCH");
+    const bool streams = mode && std::string(mode) == "streams";
     std::vector<AdjJob> jobs(nseeds);
     std::vector<double*> gl(nseeds), gm(nseeds);
     for (int q = 0; q < nseeds; ++q) {
         int rc = adj_begin(jobs[q], handles[q], t0, lin0 + q * 2 * nlin, mf0 + q * 2 * nmfe,
-                           kx0 ? kx0 + q * (size_t)h0->nxy : nullptr, nsteps, checkpoint_every);
+                           kx0 ? kx0 + q * (size_t)h0->nxy : nullptr, nsteps, checkpoint_every, streams);
         if (rc) {
             if (handles[q] != h0) h0->err = handles[q]->err;
             for (int r = 0; r <= q; ++r) adj_trim(handles[r]);
@@ -765,8 +807,6 @@ extern "C" int qlgpu_adjoint_maxwell_batch(qlgpu_t* const* handles, int nseeds, 
     // QLGPU_ADJ_BATCH=streams interleaves the single-case path of every seed on its stream
     // (results bit-identical to qlgpu_adjoint_maxwell) from one host thread (threads per
     // seed were slower: their launches contend in the driver)
-    const char* mode = getenv("QLGPU_ADJ_BATCH");
-    const bool streams = mode && std::string(mode) == "streams";
     int rc = streams ? run_jobs(jobs, J, gl.data(), grad_mf ? gm.data() : nullptr)
                      : run_jobs_persistent(jobs, t0, lin0, mf0, kx0, J, gl.data(), grad_mf ? gm.data() : nullptr);
     for (int q = 0; q < nseeds; ++q) adj_trim(handles[q]);

@@ -69,6 +69,11 @@ struct qlgpu_handle {
     size_t adj_bytes = 0;
     void* adj_tab = nullptr;
     int adj_tab_cap = 0;
+    qlgpu_batch_t* adj_batch = nullptr;  // of the last qlgpu_adjoint_maxwell_batch whose first handle this is
+    std::vector<qlgpu_params> adj_batch_ps;
+    // pinned block through which small states cross to and from host arrays, and the clock
+    unsigned char* h_pin = nullptr;
+    size_t pin_bytes = 0;
     bool ekz_dynamic = false;            // stage exp(kz) factors computed in the kernel (variable dt)
 };
 
