@@ -26,7 +26,7 @@ struct AdjOps {
     cudaError_t (*modes)(const AdjShared&, const DevParams&, const AdjPos&, int ns, int threads, cudaStream_t);
     cudaError_t (*mf)(const AdjShared&, const DevParams&, const AdjPos&, const AdjPos&, int post, int pre, int ns,
                       cudaStream_t);
-    const void* modes_kernel;
+    const void* modes_kernel[2];
     size_t modes_smem;
 };
 
@@ -49,7 +49,9 @@ cudaError_t launch_pdl(void (*kern)(KA...), dim3 grid, int block, size_t smem, c
 }
 template <int NZ>
 cudaError_t ops_modes(const AdjShared& H, const DevParams& P, const AdjPos& X, int ns, int threads, cudaStream_t st) {
-    return launch_pdl(adj_modes_kernel<NZ>, dim3((unsigned)H.nchunk, (unsigned)ns), threads, AG<NZ>::BYTES, st, H, P, X);
+    const dim3 grid((unsigned)H.nchunk, (unsigned)ns);
+    return threads == ADJ_FEW ? launch_pdl(adj_modes_kernel<NZ, ADJ_FEW>, grid, threads, AG<NZ>::BYTES, st, H, P, X)
+                              : launch_pdl(adj_modes_kernel<NZ, ADJ_MANY>, grid, threads, AG<NZ>::BYTES, st, H, P, X);
 }
 template <int NZ>
 cudaError_t ops_mf(const AdjShared& H, const DevParams& P, const AdjPos& X, const AdjPos& Y, int post, int pre, int ns,
@@ -58,7 +60,9 @@ cudaError_t ops_mf(const AdjShared& H, const DevParams& P, const AdjPos& X, cons
 }
 template <int NZ>
 AdjOps make_ops() {
-    return AdjOps{&ops_modes<NZ>, &ops_mf<NZ>, reinterpret_cast<const void*>(&adj_modes_kernel<NZ>), AG<NZ>::BYTES};
+    return AdjOps{&ops_modes<NZ>, &ops_mf<NZ>,
+                  {reinterpret_cast<const void*>(&adj_modes_kernel<NZ, ADJ_FEW>),
+                   reinterpret_cast<const void*>(&adj_modes_kernel<NZ, ADJ_MANY>)}, AG<NZ>::BYTES};
 }
 bool pick_ops(int NZ, AdjOps* o) {
     switch (NZ) {
@@ -213,7 +217,7 @@ int adj_begin(AdjJob& j, qlgpu_t* h, double t0, const double* lin0, const double
     if (h->noise_f != 0.0 || h->cfl > 0) return afail(h, QLGPU_ERR_UNSUPPORTED, "the adjoint runs at fixed dt, no noise");
     if (!pick_ops(h->NZ, &j.ops)) return afail(h, QLGPU_ERR_UNSUPPORTED, "unsupported NZ");
     QA_CK(cudaSetDevice(h->device));
-    QA_CK(ensure_smem_attr(j.ops.modes_kernel, j.ops.modes_smem));
+    for (const void* k : j.ops.modes_kernel) QA_CK(ensure_smem_attr(k, j.ops.modes_smem));
     if (load_state) {
         const int rc = qlgpu_set_state(h, t0, lin0, mf0, kx0);
         if (rc) return rc;
@@ -385,7 +389,7 @@ int adj_reverse_window(qlgpu_t* h, const AdjOps& ops, const AdjShared& H, int ns
     QA_CK(ops.mf(H, h->dp, X, X, 0, 1, ns, st));
     int sms = 0;
     QA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
-    const int threads = (long long)H.nchunk * ns <= sms ? 512 : 256;
+    const int threads = (long long)H.nchunk * ns <= sms ? ADJ_FEW : ADJ_MANY;
     for (int left = 3 * steps; left > 0; --left) {
         QA_CK(ops.modes(H, h->dp, X, ns, threads, st));
         AdjPos Y = X;

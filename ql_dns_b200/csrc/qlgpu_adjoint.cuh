@@ -106,8 +106,10 @@ struct AG {
     static constexpr size_t o_ekz = o_kz + 8 * (size_t)NZ_;             // [2][NZE]
     static constexpr size_t o_acc = o_ekz + 16 * (size_t)NZE;           // [3][8][32] profile sums
     static constexpr size_t o_R = o_acc + 8 * 3 * 256;                  // [NR][XW] cplx, a result at [8][32]
-    static constexpr size_t o_stg = o_R + 16 * XW * (size_t)NR;        // [GPW][4][nz] cplx
-    static constexpr size_t BYTES = o_stg + 16 * (size_t)GPW * 4 * nz;
+    static constexpr size_t o_stg = o_R + 16 * XW * (size_t)NR;        // [GPW][4][nz] cplx: U
+    static constexpr size_t o_lf = o_stg + 16 * (size_t)GPW * 4 * nz;   // [GPW][4][nz] cplx: lamF
+    static constexpr size_t o_il2 = o_lf + 16 * (size_t)GPW * 4 * nz;   // [GPW][nz] 1/lap2
+    static constexpr size_t BYTES = o_il2 + 8 * (size_t)GPW * nz;
 };
 inline int adj_block_modes(int NZ) { return 256 / NZ; }
 
@@ -132,11 +134,14 @@ __device__ __forceinline__ double adj_e(const DevParams& P, const StageConst& S,
 }
 
 // The stage adjoint of the chunk's modes.  What bounds it: the transforms' chain of a block
-// (two deep) at one seed, the FP64 and shared-memory work at many.  A CTA of 8 warps leaves
-// room for a second one per SM, whose transforms run under the barriers of the first; with
-// at most one chunk per SM it has 16 warps, one round of the 14 inverse transforms.
-template <int NZ>
-__global__ void __launch_bounds__(512, 1)
+// (two deep) at one seed, the instruction and barrier latency at many.  Eight warps at 128
+// registers leave room for a second CTA per SM, whose transforms run under the barriers of the
+// first (nine, one round of the forward transforms, would have 96 registers and spill); with at most one chunk per SM a CTA has 16 warps, one
+// round of the 14 inverse transforms too.
+constexpr int ADJ_FEW = 512, ADJ_MANY = 256;  // threads
+
+template <int NZ, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == ADJ_MANY ? 2 : 1)
     adj_modes_kernel(const __grid_constant__ AdjShared H, const __grid_constant__ DevParams P,
                      const __grid_constant__ AdjPos X) {
     using W = AG<NZ>;
@@ -149,7 +154,10 @@ __global__ void __launch_bounds__(512, 1)
     double* acc = reinterpret_cast<double*>(smem_raw + W::o_acc);
     cplx* R = reinterpret_cast<cplx*>(smem_raw + W::o_R);
     cplx* stg_all = reinterpret_cast<cplx*>(smem_raw + W::o_stg);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5, nth = blockDim.x;
+    cplx* lf_s = reinterpret_cast<cplx*>(smem_raw + W::o_lf);
+    double* il2_all = reinterpret_cast<double*>(smem_raw + W::o_il2);
+    constexpr int warps = THREADS / 32, nth = THREADS;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane / T, t = lane % T;
     const AdjSeedBufs& B = H.seeds[blockIdx.y];
     const StageConst& S = X.sc;
@@ -165,6 +173,8 @@ __global__ void __launch_bounds__(512, 1)
     auto stage_block = [&](int base) {
         const int n = min(GPW, P.nxy - base) * 4 * nzd;
         for (int i = tid; i < n; i += nth) cp_async16(stg_all + i, U + (size_t)base * 4 * nzd + i);
+        for (int i = tid; i < n / 4; i += nth)
+            cp_async8(il2_all + i, H.ilap2 + (size_t)__ldg(H.kyi + base + i / nzd) * nzd + i % nzd);
         cp_async_commit();
     };
     stage_block(first);
@@ -210,11 +220,12 @@ __global__ void __launch_bounds__(512, 1)
             M.em_b = exp(S.linC * P.cb * hxy);
         }
         const double a = M.a, b = M.b, ab = __dmul_rn(a, b);
-        const double* __restrict__ il2row = H.ilap2 + (size_t)M.kyi * nzd;
+        const double* il2row = il2_all + min(g, nv - 1) * nzd;
+        cplx* lfm = lf_s + (size_t)min(g, nv - 1) * 4 * nzd;  // this mode's lamF
         const cplx* lo = lo_all + (size_t)M.m * 4 * nzd;
         const cplx* lf = lf_all ? lf_all + (size_t)M.m * 4 * nzd : nullptr;
         // lamF of field f at stored index s: n1 E lamU' + lamF_out
-        auto lamF = [&](int f, int s, double kz2) -> cplx {
+        auto lam_F = [&](int f, int s, double kz2) -> cplx {
             cplx r = cscale(ldc(lo + f * nzd + s), __dmul_rn(S.n1, adj_e<W>(P, S, M, ekz, f, s, kz2, H.integ)));
             if (lf) r = cadd(r, ldc(lf + f * nzd + s));
             return r;
@@ -237,15 +248,18 @@ __global__ void __launch_bounds__(512, 1)
                     } else if (task < 9) {
                         const int f0 = (task == A_RBZ || task == A_RBY) ? 2 : 0;
                         const cplx g0 = stg[f0 * nzd + s], g1 = stg[(f0 + 1) * nzd + s];
-                        const double sc = __ldg(il2row + s) * fac;
+                        const double sc = il2row[s] * fac;
                         const bool y = task >= A_RUY;
                         // y: (a b) u + i c z;  z: (a c) u - i b z
                         const double p = y ? ab : __dmul_rn(a, c), q = y ? c : -b;
                         v = mk(fma(p, g0.x, -q * g1.y), fma(p, g0.y, q * g1.x));
                         v = task == A_RIK ? imul(v, sc * c) : cscale(v, sc);
                     } else {
-                        v = lamF(task == A_WB ? 2 : task == A_WZ ? 1 : task == A_WE ? 3 : 0, s, kz2);
-                        if (task == A_WU2) {
+                        const int f = task == A_WB ? 2 : task == A_WZ ? 1 : task == A_WE ? 3 : 0;
+                        v = lam_F(f, s, kz2);
+                        if (task != A_WU2) {
+                            if (M.valid) lfm[f * nzd + s] = v;  // kept for the spectral chain
+                        } else {
                             const bool z0 = (M.kyi == 0 && s == 0);
                             const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2, z0));
                             v = cscale(v, (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF));
@@ -264,25 +278,13 @@ __global__ void __launch_bounds__(512, 1)
             pdl_next();
         }
         __syncthreads();
-        // ---- pointwise adjoints as inputs of nine forward transforms.  Inputs 0-6 go on in the
-        // buffers of results 0-6, so those are held in registers until every warp has read its
-        // own; inputs 7 and 8 have exchange buffers of their own.
+        // ---- pointwise adjoints as inputs of nine forward transforms.  Inputs 0-6 are held in
+        // registers until every warp has read its own (and the profile adjoints are formed); then
+        // every result has a buffer of its own: 0-3 and 6 theirs, 4 and 5 the two spare ones, and 7
+        // and 8 transform in place of the R_bz and R_uz they are made of.
+        auto res = [&](int k) { return buf(k == 4 ? A_X1 : k == 5 ? A_X0 : k == 7 ? A_RBZ : k == 8 ? A_RUZ : k); };
         const double *By = prof, *dBy = prof + NZ, *ddBy = prof + 2 * NZ, *px = prof + 3 * NZ, *py = prof + 4 * NZ;
         auto rd = [&](int i, int r) { return R[i * W::XW + 32 * r + lane]; };
-        auto small_task = [&](int task) {  // 7: mult py R_bz, 8: -mult py R_uz
-            cplx x[8];
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const double my = M.mult * py[t + T * r];
-                x[r] = conjc(task == 7 ? cscale(rd(A_RBZ, r), my) : cscale(rd(A_RUZ, r), -my));
-            }
-            cplx* xb = buf(task == 7 ? A_X0 : A_X1);
-            xform<W>(x, xb, tw, g, t);
-#pragma unroll
-            for (int r = 0; r < 8; ++r) xb[32 * r + lane] = conjc(x[r]);
-        };
-        if (warp == (warps > 8 ? 8 : 7)) small_task(7);
-        if (warp == (warps > 9 ? 9 : 6)) small_task(8);
         cplx x[8];
         if (warp < 7) {
 #pragma unroll
@@ -307,7 +309,7 @@ __global__ void __launch_bounds__(512, 1)
                 }
                 x[r] = conjc(o);
             }
-        } else if (warp == 7 && M.valid) {
+        } else if (warp == (warps > 9 ? 9 : 7) && M.valid) {
             // adjoint of the mean-field profiles: Re(conj(multiplier * R) W) per term
             auto re_cw = [](cplx p, cplx w) { return p.x * w.x + p.y * w.y; };   // Re(conj(p) w)
             auto re_icw = [](cplx p, cplx w) { return p.y * w.x - p.x * w.y; };  // Re(i conj(p) w)
@@ -323,8 +325,18 @@ __global__ void __launch_bounds__(512, 1)
             }
         }
         __syncthreads();
-        if (warp < 7) {
-            cplx* xb = buf(warp);
+        // with eight warps the one that formed the profile adjoints takes both of 7 and 8
+#pragma unroll 1
+        for (int k = warp; k < 9; k += warps > 8 ? warps : (warp == 7 ? 1 : 9)) {
+            if (k >= 7) {  // 7: mult py R_bz, 8: -mult py R_uz
+#pragma unroll
+                for (int r = 0; r < 8; ++r) {
+                    const double my = M.mult * py[t + T * r];
+                    x[r] = conjc(k == 7 ? cscale(rd(A_RBZ, r), my) : cscale(rd(A_RUZ, r), -my));
+                }
+                __syncwarp();
+            }
+            cplx* xb = res(k);
             xform<W>(x, xb, tw, g, t);
 #pragma unroll
             for (int r = 0; r < 8; ++r) xb[32 * r + lane] = conjc(x[r]);
@@ -337,6 +349,12 @@ __global__ void __launch_bounds__(512, 1)
             const int f = task >> 1, h = task & 1;
             if (!M.valid) continue;
             const size_t at = ((size_t)M.m * 4 + f) * nzd;
+            cplx lov[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int s = sidx<W>(t, 4 * h + i);
+                lov[i] = s >= 0 ? ldc(lo + f * nzd + s) : mk(0.0, 0.0);
+            }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int r = 4 * h + i;
@@ -345,8 +363,8 @@ __global__ void __launch_bounds__(512, 1)
                 const int rl = 32 * r + lane;
                 const double c = kzc[t + T * r], kz2 = kz2val(c);
                 const bool z0 = (M.kyi == 0 && s == 0);
-                const double il2 = __ldg(il2row + s);
-                const cplx mu = cscale(ldc(lo + f * nzd + s), adj_e<W>(P, S, M, ekz, f, s, kz2, H.integ));
+                const double il2 = il2row[s];
+                const cplx mu = cscale(lov[i], adj_e<W>(P, S, M, ekz, f, s, kz2, H.integ));
                 cplx v = mu;
                 if (H.integ == INTEG_CN) {
                     // the direct term (1 + linC Lold) D lamU' (RK3CN.cpp:107)
@@ -354,10 +372,10 @@ __global__ void __launch_bounds__(512, 1)
                                                      : lap_end<MODEL_BQLIN>(P, M.kxo, b, kz2);
                     v = cscale(mu, __dadd_rn(1.0, __dmul_rn(S.linC, linop_f<MODEL_BQLIN>(P, lo_lap, f))));
                 }
-                v = cadd(v, cscale(buf(f)[rl], fac));
+                v = cadd(v, cscale(res(f)[rl], fac));
                 // uz = (a c u - i b zeta) il2, i c uz, uy = (a b u + i c zeta) il2 (b, eta likewise)
-                const cplx lz = f < 2 ? cscale(csub(buf(4)[rl], imul(buf(6)[rl], c)), fac) : cscale(buf(5)[rl], fac);
-                const cplx ly = cscale(buf(f < 2 ? A_X0 : A_X1)[rl], fac);
+                const cplx lz = f < 2 ? cscale(csub(res(4)[rl], imul(res(6)[rl], c)), fac) : cscale(res(5)[rl], fac);
+                const cplx ly = cscale(res(f < 2 ? 7 : 8)[rl], fac);
                 if (f == 0 || f == 2) {
                     v = cadd(v, cscale(lz, __dmul_rn(a, c) * il2));
                     v = cadd(v, cscale(ly, ab * il2));
@@ -368,16 +386,16 @@ __global__ void __launch_bounds__(512, 1)
                 if (f < 2) {
                     const double lapF = __dadd_rn(-__dmul_rn(a, a), lap2val(b, kz2, z0));
                     const double ilapF = (z0 && M.kxi == 0) ? 1.0 : __drcp_rn(lapF);
-                    const cplx l0 = lamF(0, s, kz2);
+                    const cplx l0 = lfm[s];
                     if (f == 0) {
                         // linear terms of F_zeta ((q - 2 Omega) i c u) and F_u (ilapF 2 a b q u)
-                        v = cadd(v, imul(lamF(1, s, kz2), -(P.q - Om2) * c));
+                        v = cadd(v, imul(lfm[nzd + s], -(P.q - Om2) * c));
                         v = cadd(v, cscale(l0, ilapF * 2.0 * ab * P.q));
                     } else {
                         v = cadd(v, imul(l0, -Om2 * c * ilapF));  // linear term of F_u: ilapF 2 Omega i c zeta
                     }
                 } else if (f == 2) {
-                    v = cadd(v, imul(lamF(3, s, kz2), P.q * c));  // linear term of F_eta: -q i c b
+                    v = cadd(v, imul(lfm[3 * nzd + s], P.q * c));  // linear term of F_eta: -q i c b
                 }
                 if (X.s == 0 && X.n > 0) {
                     // this stage's input is the post-step state of step n - 1: the remap's adjoint (the
