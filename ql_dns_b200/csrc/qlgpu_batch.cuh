@@ -94,7 +94,7 @@ __device__ __noinline__ StageResult batch_item_stage(const BatchLaunch& L, const
 }
 
 template <int MODEL, int INTEG>
-__global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) batch_kernel(const __grid_constant__ BatchLaunch L) {
+__global__ void __launch_bounds__(32 * BATCH_MAX_WARPS, 1) batch_kernel(const __grid_constant__ BatchLaunch L) {
     __shared__ BatchSlot s_items[BATCH_MAX_SLOTS];
     __shared__ LocalClock s_clk[BATCH_MAX_SLOTS];
     const int tid = threadIdx.x;

@@ -302,6 +302,13 @@ bool width_limits(qlgpu_batch_t* b, int warps, int* per_sm, size_t* smem) {
     return true;
 }
 
+// Width without warps that belong to no team (16 warps of MHD_BQlin are three teams of five and an
+// idle warp, which a caller may ask for but no plan takes).
+int whole_teams(const qlgpu_batch_t* b, int warps) {
+    const int teams = stage_teams(b->cs[0].p.model, warps);
+    return warps - warps % teams;
+}
+
 // Plan: CTAs per case and the packing of work items onto at most G CTAs.
 // fixed_k (optional) pins the CTA count of every case.
 bool plan(const qlgpu_batch_t* b, int warps, int G, const CostModel& cm, const int* fixed_k, std::vector<int>& k_out,
@@ -1054,7 +1061,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         b->err = "event create failed";
         return bail(QLGPU_ERR_CUDA);
     }
-    // initial mapping from the cost model: the widest CTA that fits
+    // initial mapping from the cost model: the widest CTA of whole teams that fits
     b->wide_warps = 0;
     for (int w = b->bk.max_warps; w >= 1 && !b->wide_warps; --w) {
         int ps = 0;
@@ -1065,7 +1072,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         b->err = "batch: no CTA width fits (shared memory / TMEM)";
         return bail(QLGPU_ERR_UNSUPPORTED);
     }
-    int rc = plan_and_apply(b, b->wide_warps, nullptr);
+    int rc = plan_and_apply(b, whole_teams(b, b->wide_warps), nullptr);
     if (rc) return bail(rc);
     rc = upload_descriptors(b);
     if (rc) return bail(rc);
@@ -1512,7 +1519,7 @@ int qlgpu_batch_tune(qlgpu_batch_t* b, int probe_steps, double* best_ms) {
             if (x[2 + j] > 0) cm.r[j] = x[2 + j];
     };
     int rc = QLGPU_OK;
-    for (int warps : {b->wide_warps, std::max(1, b->wide_warps / 2)}) {
+    for (int warps : {whole_teams(b, b->wide_warps), std::max(1, b->wide_warps / 2)}) {
         int per_sm = 0;
         size_t smem = 0;
         if (!width_limits(b, warps, &per_sm, &smem)) continue;

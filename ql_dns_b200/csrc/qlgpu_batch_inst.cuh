@@ -41,7 +41,7 @@ bool make_batch_kernel(BatchKernel* out) {
     out->launch = &batch_launch<MODEL, INTEG>;
     out->kernel = &batch_ptr<MODEL, INTEG>;
     out->smem = &batch_smem<MODEL>;
-    out->max_warps = wide::MAX_WARPS<MODEL>;
+    out->max_warps = BATCH_MAX_WARPS;
     return true;
 }
 

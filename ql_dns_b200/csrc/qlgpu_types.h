@@ -144,6 +144,7 @@ struct RunArgs {
 // Batched ensemble (persistent kernel, qlgpu_batch.cuh)
 // ---------------------------------------------------------------------------
 constexpr int BATCH_MAX_SLOTS = 8;      // work items (case, CTA index) per CTA
+constexpr int BATCH_MAX_WARPS = 16;     // widest CTA of a work item mapping
 constexpr int BATCH_EPOCH_STRIDE = 32;  // words between the per-case stage counters (one 128-byte line each)
 
 // One case of a batch in device memory: its run constants and the arguments of

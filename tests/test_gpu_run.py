@@ -11,6 +11,7 @@ import pytest
 
 from gpu_util import rel, require_gpu
 from oracle import oracle as O
+from ql_dns_b200.batch import QLBatch
 from ql_dns_b200.initial import initial_state
 from ql_dns_b200.params import QLParams
 from ql_dns_b200.solver import QLSolver
@@ -45,3 +46,20 @@ def test_layout_edges(nx, ny, NZ, model, integ):
     assert rel(lo, lo2) < 1e-10 if np.linalg.norm(lo2) else not lo.any()
     scale = np.abs(d2[1:, 1:13]).max(0)
     assert np.all(np.abs(rec[:, 1:13] - d2[1:, 1:13]) <= 1e-10 * scale)
+
+
+@pytest.mark.parametrize("model", [0, 1])
+@pytest.mark.parametrize("warps", [1, 3, 5, 8, 9, 14, 15, 16])
+def test_work_item_widths(warps, model):
+    """Work items of every kind of team: less than one, one wider than its tasks, several, idle warps."""
+    require_gpu()
+    p = QLParams(model=model, nx=6, ny=6, NZ=16, dt=0.02, B0z=0.02 if model else 0.0)
+    lin, mf, kx0 = initial_state(p, 3, sigma=0.2, B0=0.05, mean_u=0.02 if model else 0.0)
+    with QLBatch([p]) as b:
+        b.set_mapping(warps, [1])
+        b.set_state(0, 0.0, lin, mf, kx0)
+        b.step(3)
+        t, lo, mo, ko = b.get_state(0)
+    t2, lo2, mo2, ko2, _ = O.run(p, 0.0, lin, mf, kx0, 3)
+    assert t == t2 and np.array_equal(ko, ko2)
+    assert rel(mo, mo2) < 1e-10 and rel(lo, lo2) < 1e-10
