@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
-#include <functional>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -18,7 +17,6 @@
 #include "qlgpu_handle.h"
 #include "qlgpu_host.h"
 #include "qlgpu_kernel.cuh"
-#include "qlgpu_forcing.cuh"
 
 using namespace qlgpu;
 
@@ -73,15 +71,9 @@ StageArgs base_args(qlgpu_t* h) {
     return A;
 }
 
-// One RK3 step = three stage launches (RK3CN_Elin::Step / RK3CN::Step).
-// ev (optional): 4 events recorded before stage 1 and after each stage.
-}  // namespace
-
-// One RK3 step = three stage launches (RK3CN_Elin::Step / RK3CN::Step).  ev
-// (optional): 4 events recorded before stage 1 and after each stage.  hook
-// (optional) is called before each stage launch with the stage index (the
-// adjoint records the stage inputs there).
-void qlgpu_enqueue_step(qlgpu_t* h, cudaEvent_t* ev, const std::function<void(int)>& hook) {
+// One RK3 step = three stage launches (RK3CN_Elin::Step / RK3CN::Step), timed by 4 events recorded
+// before stage 1 and after each stage.
+void enqueue_step(qlgpu_t* h, cudaEvent_t* ev) {
     cplx* Fbuf[3] = {h->d_F1, h->d_F2, nullptr};
     const cplx* Fprev[3] = {nullptr, h->d_F1, h->d_F2};
     cplx* Fmf[3] = {h->d_Fmf1, h->d_Fmf2, h->d_Fmf1};
@@ -97,16 +89,17 @@ void qlgpu_enqueue_step(qlgpu_t* h, cudaEvent_t* ev, const std::function<void(in
         A.Fmf_out = (s < 2) ? Fmf[s] : nullptr;
         A.sc = h->sc[s];
         if (A.trace) A.trace += 32 * s;
-        A.ekz_tab = h->ekz_dynamic ? nullptr : h->d_ekz + (size_t)s * 2 * h->nz;
-        if (hook) hook(s);
+        A.ekz_tab = h->d_ekz + (size_t)s * 2 * h->nz;
         h->var.launch(A, h->dp, h->grid, h->block, h->smem, h->stream);
         if (ev) cudaEventRecord(ev[s + 1], h->stream);
         h->cur ^= 1;
     }
 }
 
+}  // namespace
+
 // n steps in one cooperative launch (run_kernel), the stage inputs recorded where rec is set.
-cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec) {
+cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec, const RunForcing* force) {
     cplx* Fbuf[3] = {h->d_F1, h->d_F2, nullptr};
     const cplx* Fprev[3] = {nullptr, h->d_F1, h->d_F2};
     cplx* Fmf[3] = {h->d_Fmf1, h->d_Fmf2, nullptr};
@@ -122,7 +115,7 @@ cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec) {
         A.Fmf_out = Fmf[s];
         A.sc = h->sc[s];
         if (A.trace) A.trace += 32 * s;
-        A.ekz_tab = h->d_ekz + (size_t)s * 2 * h->nz;
+        A.ekz_tab = force && force->cfl > 0 ? nullptr : h->d_ekz + (size_t)s * 2 * h->nz;
     }
     R.P = h->dp;
     R.lin[0] = h->d_lin[0];
@@ -137,7 +130,19 @@ cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec) {
         R.rec_t = rec->t;
         R.rec_cn = rec->cn;
     }
-    const cudaError_t e = h->var.run(R, h->grid + 1, h->block, h->smem, h->stream);
+    if (force) {
+        R.noise = force->noise;
+        R.noise_on = force->noise_on;
+        R.step0 = force->step0;
+        R.cfl = force->cfl;
+        R.dt_max = force->dt_max;
+        R.kmax = force->kmax;
+        R.forcing = h->d_forcing;
+        R.diag_every = force->diag_every;
+        R.diag_step0 = force->diag_step0;
+        R.diag_max = force->diag_max;
+    }
+    const cudaError_t e = h->var.run[force != nullptr](R, h->grid + 1, h->block, h->smem, h->stream);
     if (e == cudaSuccess) h->cur ^= n & 1;  // three stages per step
     return e;
 }
@@ -155,8 +160,6 @@ cudaError_t qlgpu_clear_abort(qlgpu_t* h) {
 }
 
 namespace {
-
-void enqueue_step(qlgpu_t* h, cudaEvent_t* ev = nullptr) { qlgpu_enqueue_step(h, ev, nullptr); }
 
 // Steps per launch: short enough that a long run stays a sequence of launches of some 10 ms.
 constexpr int RUN_STEPS = 256;
@@ -265,7 +268,8 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     h->grid = sg.grid;
     h->per_sm = 1;
     if (h->smem > (size_t)prop.sharedMemPerBlockOptin || ensure_smem_attr(var.kernel(), h->smem) != cudaSuccess ||
-        ensure_smem_attr(var.run_kernel(), h->smem) != cudaSuccess) {
+        ensure_smem_attr(var.run_kernel[0](), h->smem) != cudaSuccess ||
+        ensure_smem_attr(var.run_kernel[1](), h->smem) != cudaSuccess) {
         h->err = "shared memory request too large";
         return bail(QLGPU_ERR_CUDA);
     }
@@ -344,7 +348,7 @@ int qlgpu_destroy(qlgpu_t* h) {
     void* bufs[] = {h->d_lin[0], h->d_lin[1], h->d_F1, h->d_F2, h->d_mf, h->d_Fmf1, h->d_Fmf2,
                     h->d_kx0, h->d_ky, h->d_kxi, h->d_kyi, h->d_tw, h->d_partials, h->d_gpartials,
                     h->d_clk, h->d_diag, h->d_out15, h->d_linop, h->d_ilap2, h->d_trace,
-                    h->d_mfr, h->d_ekz, h->d_forcing, h->d_kx0_prev, h->d_dbg, h->adj_ws, h->adj_tab};
+                    h->d_mfr, h->d_ekz, h->d_forcing, h->d_dbg, h->adj_ws, h->adj_tab};
     for (void* b : bufs)
         if (b) cudaFree(b);
     if (h->adj_batch) qlgpu_batch_destroy(h->adj_batch);
@@ -414,7 +418,7 @@ static int set_state_impl(qlgpu_t* h, double t, const void* lin, const void* mf,
     // the integrator and model start afresh: no steps, zero mean-field profiles of a previous rhs
     h->dt_sum = 0.0;
     h->steps_taken = 0;
-    if (h->d_forcing) QLGPU_CK(cudaMemsetAsync(h->d_forcing, 0, 9 * sizeof(double), h->stream));
+    if (h->d_forcing) QLGPU_CK(cudaMemsetAsync(h->d_forcing, 0, 6 * sizeof(double), h->stream));
     QLGPU_CK(cudaStreamSynchronize(h->stream));
     return QLGPU_OK;
 }
@@ -456,95 +460,54 @@ int qlgpu_get_state_device(qlgpu_t* h, double* t, void* lin, void* mf, void* kx0
 }
 
 // Steps with driving noise and / or the CFL time step (main.cpp:108-133 with
-// RK3CN_Elin.cpp:76-80): per step the host reads the mean-field maxima, sets dt
-// and the stage constants, enqueues the three stages (the stage-3 input's
-// maxima are taken before stage 3: the profiles the last rhs computed), then
-// the noise; a record after every diag_every-th step through diag_kernel.
+// RK3CN_Elin.cpp:76-80): run_kernel adds the noise and sets dt; a record after every
+// diag_every-th step.
 static int step_forced(qlgpu_t* h, int nsteps, int diag_every, double* diag_out, int max_diag, int* ndiag) {
     if (!h->d_forcing) {
-        QLGPU_CK(cudaMalloc(&h->d_forcing, 9 * sizeof(double)));
-        QLGPU_CK(cudaMemsetAsync(h->d_forcing, 0, 9 * sizeof(double), h->stream));
+        QLGPU_CK(cudaMalloc(&h->d_forcing, 6 * sizeof(double)));
+        QLGPU_CK(cudaMemsetAsync(h->d_forcing, 0, 6 * sizeof(double), h->stream));
     }
-    if (h->noise_f != 0.0 && !h->d_kx0_prev) QLGPU_CK(cudaMalloc(&h->d_kx0_prev, h->nxy * sizeof(double)));
     if (diag_every > 0) {
         int rc = ensure_diag(h, max_diag > 0 ? max_diag : 1);
         if (rc) return rc;
+        int zero = 0;
+        QLGPU_CK(cudaMemcpyAsync(&h->d_clk->ndiag, &zero, sizeof(int), cudaMemcpyHostToDevice, h->stream));
     }
-    const double fac = 1.0 / h->NZ;  // fftwPlans.cpp:30
     const double Ns[3] = {(double)h->p.nx, (double)((h->p.ny / 2) * 2), (double)h->NZ};
     const double dealias[3] = {2.0, 2.0, 3.0};
-    double kmax = 0;  // MHD_BQlin.cpp:69-74
-    for (int i = 0; i < 3; ++i) kmax = std::max(kmax, 2 * kPI / h->p.L[i] * (Ns[i] / dealias[i]));
-    double t = 0;
-    QLGPU_CK(cudaMemcpyAsync(&t, &h->d_clk->t, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    QLGPU_CK(cudaStreamSynchronize(h->stream));
-    const double tv_saved = h->dp.tv_interval;
-    h->dp.tv_interval = 0.0;  // records come from diag_kernel here
-    h->ekz_dynamic = h->cfl > 0;
-    int nd = 0, rc = QLGPU_OK;
-    for (int n = 0; n < nsteps && rc == QLGPU_OK; ++n) {
-        double dt = h->p.dt;
-        if (h->cfl > 0) {
-            mf_absmax2_kernel<<<1, MF_THREADS, 0, h->stream>>>(h->d_mf, h->nz, h->NZ, fac, h->d_forcing + 4);
-            double m[8];
-            QLGPU_CK(cudaMemcpyAsync(m, h->d_forcing, sizeof(m), cudaMemcpyDeviceToHost, h->stream));
-            QLGPU_CK(cudaStreamSynchronize(h->stream));
-            const double c = h->p.model == QLGPU_MODEL_MHD_BQLIN
-                                 ? kmax * std::sqrt(m[1]) + kmax * std::sqrt(m[4]) + h->p.q
-                                 : kmax * (std::sqrt(m[1]) + std::sqrt(m[0]) + std::sqrt(m[2]) + std::sqrt(m[3])) +
-                                       h->p.q;
-            dt = h->cfl / c;  // RK3CN_Elin.cpp:77-79
-            if (dt > h->dt_max) dt = h->dt_max;
-        }
-        qlgpu_params pp = h->p;
-        pp.dt = dt;
-        h->dp.dt = dt;
-        for (int s = 0; s < 3; ++s) h->sc[s] = stage_const(pp, s);
-        if (h->noise_f != 0.0) {
-            QLGPU_CK(cudaMemcpyAsync(h->d_kx0_prev, h->d_kx0, h->nxy * sizeof(double), cudaMemcpyDeviceToDevice,
-                                     h->stream));
-        }
-        qlgpu_enqueue_step(h, nullptr, [&](int s) {
-            if (s == 2 && h->cfl > 0)
-                mf_absmax2_kernel<<<h->nmf, MF_THREADS, 0, h->stream>>>(h->d_mf, h->nz, h->NZ, fac, h->d_forcing);
-        });
-        if (h->noise_f != 0.0) {
-            NoiseArgs a;
-            a.lin = h->d_lin[h->cur];
-            a.kx0_prev = h->d_kx0_prev;
-            a.kx0_now = h->d_kx0;
-            a.ky = h->d_ky;
-            a.kxi = h->d_kxi;
-            a.kyi = h->d_kyi;
-            a.nxy = h->nxy;
-            a.nz = h->nz;
-            a.q = h->p.q;
-            a.t = t;
-            a.kzL = 2 * kPI / h->p.L[2];
-            a.step = h->steps_taken;
-            a.ns = noise_spec(h->p, h->NZ, dt, h->noise_f, h->noise_klo, h->noise_khi, h->noise_seed,
-                              h->noise_only_vel, h->noise_only_mag);
-            const int n_el = h->nxy * h->nz;
-            noise_kernel<<<(n_el + 255) / 256, 256, 0, h->stream>>>(a);
-        }
-        t = t + dt;  // main.cpp:116, the device clock's sum
-        h->dt_sum += dt;
-        ++h->steps_taken;
-        if (diag_every > 0 && (n + 1) % diag_every == 0 && nd < max_diag) {
-            launch_diag(h->d_lin[h->cur], h->d_mf, h->d_kx0, h->d_ky, h->d_kyi, h->dp, t,
-                        h->d_diag + 15 * (size_t)nd, h->stream);
-            ++nd;
-        }
-        rc = check_launch(h);
+    RunForcing f;
+    f.kmax = 0;  // MHD_BQlin.cpp:69-74
+    for (int i = 0; i < 3; ++i) f.kmax = std::max(f.kmax, 2 * kPI / h->p.L[i] * (Ns[i] / dealias[i]));
+    f.cfl = h->cfl;
+    f.dt_max = h->dt_max;
+    f.noise_on = h->noise_f != 0.0;
+    f.noise = noise_spec(h->p, h->NZ, h->p.dt, h->noise_f, h->noise_klo, h->noise_khi, h->noise_seed,
+                         h->noise_only_vel, h->noise_only_mag);
+    f.diag_every = diag_every > 0 ? diag_every : 0;
+    f.diag_max = max_diag;
+    h->dp.tv_interval = 0.0;
+    double* const d_dt_sum = h->d_forcing + 4;
+    if (f.cfl > 0) QLGPU_CK(cudaMemcpyAsync(d_dt_sum, &h->dt_sum, sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    for (int n = 0; n < nsteps; n += RUN_STEPS) {
+        f.diag_step0 = n;
+        f.step0 = h->steps_taken + n;
+        QLGPU_CK(qlgpu_enqueue_run(h, std::min(RUN_STEPS, nsteps - n), nullptr, &f));
     }
-    h->dp.tv_interval = tv_saved;
-    h->dp.dt = h->p.dt;
-    for (int s = 0; s < 3; ++s) h->sc[s] = stage_const(h->p, s);
-    h->ekz_dynamic = false;
+    int rc = check_launch(h);
     if (rc) return rc;
+    h->steps_taken += nsteps;
+    for (int n = 0; n < nsteps && !(f.cfl > 0); ++n) h->dt_sum += h->p.dt;
     DevClock c;
+    double sum = 0;
     QLGPU_CK(cudaMemcpyAsync(&c, h->d_clk, sizeof(DevClock), cudaMemcpyDeviceToHost, h->stream));
+    if (f.cfl > 0) QLGPU_CK(cudaMemcpyAsync(&sum, d_dt_sum, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     QLGPU_CK(cudaStreamSynchronize(h->stream));
+    if (f.cfl > 0) h->dt_sum = sum;
+    if (c.status & QLGPU_STATUS_TIMEOUT) {
+        QLGPU_CK(qlgpu_clear_abort(h));
+        return fail(h, QLGPU_ERR_STATUS, "step: a CTA gave up waiting for the other CTAs of the case");
+    }
+    const int nd = diag_every > 0 ? std::min(c.ndiag, max_diag) : 0;
     if (nd > 0) QLGPU_CK(cudaMemcpy(diag_out, h->d_diag, sizeof(double) * 15 * (size_t)nd, cudaMemcpyDeviceToHost));
     if (ndiag) *ndiag = nd;
     if (c.status & (QLGPU_STATUS_NONFINITE | QLGPU_STATUS_UNSTABLE))
@@ -616,7 +579,7 @@ int qlgpu_step(qlgpu_t* h, int nsteps, int diag_every, double* diag_out, int max
         QLGPU_CK(cudaMemcpyAsync(&h->d_clk->ndiag, &zero, sizeof(int), cudaMemcpyHostToDevice, h->stream));
     }
     for (int n = 0; n < nsteps; n += RUN_STEPS) {
-        QLGPU_CK(qlgpu_enqueue_run(h, std::min(RUN_STEPS, nsteps - n), nullptr));
+        QLGPU_CK(qlgpu_enqueue_run(h, std::min(RUN_STEPS, nsteps - n), nullptr, nullptr));
     }
     int rc = check_launch(h);
     if (rc) return rc;

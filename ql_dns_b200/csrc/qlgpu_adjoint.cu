@@ -298,7 +298,7 @@ int adj_checkpoint(AdjJob& j, int c) {
 int adj_forward_window(AdjJob& j, int steps, bool record) {
     qlgpu_t* h = j.h;
     const RunRecord r{j.stU, j.stB, j.kx_pre, j.t_pre, j.cn_pre};
-    QA_CK(qlgpu_enqueue_run(h, steps, record ? &r : nullptr));
+    QA_CK(qlgpu_enqueue_run(h, steps, record ? &r : nullptr, nullptr));
     return QLGPU_OK;
 }
 
@@ -355,7 +355,7 @@ int adj_window_begin(AdjJob& j, int w) {
 int adj_recompute_window(AdjJob& j, int steps) {
     qlgpu_t* h = j.h;
     const RunRecord r{j.stU, j.stB, j.kx_pre, j.t_pre, j.cn_pre};
-    QA_CK(qlgpu_enqueue_run(h, steps, &r));
+    QA_CK(qlgpu_enqueue_run(h, steps, &r, nullptr));
     return QLGPU_OK;
 }
 

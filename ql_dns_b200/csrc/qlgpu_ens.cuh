@@ -361,11 +361,11 @@ __device__ __noinline__ void run_chunk(const EnsLaunch& L, ChunkHdr& hd, const R
         hd.cn_t_old = __ldcg(&A.clk->t_old);
         hd.cn_dtlin_old = __ldcg(&A.clk->dtlin_old);
         hd.cn_old_init = __ldcg(&A.clk->old_init);
-        const double tn = __dadd_rn(tc, P.dt);
+        const double tn = __dadd_rn(tc, S.dt);
         hd.t_new = tn;
         int dd = 0;
         if (S.last && P.tv_interval > 0.0) {
-            const double tv = __dadd_rn(__ldcg(&A.clk->timevar), P.dt);
+            const double tv = __dadd_rn(__ldcg(&A.clk->timevar), S.dt);
             dd = __dsub_rn(tv, P.tv_interval) > -1e-8;
         }
         hd.diag_due = dd;

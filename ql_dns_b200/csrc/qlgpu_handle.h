@@ -3,7 +3,6 @@
 #pragma once
 #include <cuda_runtime.h>
 
-#include <functional>
 #include <string>
 #include <vector>
 
@@ -62,8 +61,7 @@ struct qlgpu_handle {
     double cfl = 0.0, dt_max = 0.0;
     double dt_sum = 0.0;                 // Integrator::mean_time_step accumulators
     unsigned long long steps_taken = 0;  // since set_state; the noise counter's step word
-    double* d_forcing = nullptr;         // [0..3] last rhs mean-field maxima, [4..7] current, [8] step start time
-    double* d_kx0_prev = nullptr;        // kx0 at the start of the step (noise)
+    double* d_forcing = nullptr;         // RunArgs::forcing
     // the adjoint's workspace and its table of seeds, kept for the next call and freed with the handle
     void* adj_ws = nullptr;
     size_t adj_bytes = 0;
@@ -74,13 +72,8 @@ struct qlgpu_handle {
     // pinned block through which small states cross to and from host arrays, and the clock
     unsigned char* h_pin = nullptr;
     size_t pin_bytes = 0;
-    bool ekz_dynamic = false;            // stage exp(kz) factors computed in the kernel (variable dt)
 };
 
-
-// One step of the handle's state on its stream (three stage launches); hook,
-// when set, runs on the host before each stage launch with the stage index.
-void qlgpu_enqueue_step(qlgpu_t* h, cudaEvent_t* ev, const std::function<void(int)>& hook);
 
 // n steps of the handle's state in one launch; rec (optional) takes every stage's inputs
 // (RunArgs' record layout).
@@ -91,7 +84,15 @@ struct RunRecord {
     double* t;
     CnRec* cn;
 };
-cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec);
+// Noise and time step of a launch (force, optional): RunArgs' fields of the same names.
+struct RunForcing {
+    NoiseSpec noise;
+    int noise_on;
+    unsigned long long step0;
+    double cfl, dt_max, kmax;
+    int diag_every, diag_step0, diag_max;
+};
+cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec, const RunForcing* force);
 cudaError_t qlgpu_clear_abort(qlgpu_t* h);
 
 // Debug build: the index checks' status bits and the guard zones of the handle after a

@@ -22,10 +22,6 @@ struct cplx;
 
 constexpr double kPI = 3.14159265358979323846;  // General_Definitions.h PI
 
-// RK3 coefficients (RK3CN_Elin.cpp:19-20, RK3CN.cpp:19-20)
-constexpr double a0_ = 8.0 / 15.0, a1_ = 5.0 / 12.0, a2_ = 3.0 / 4.0, b1_ = -17.0 / 60.0, b2_ = -5.0 / 12.0;
-constexpr double p1_ = 8.0 / 15.0, p2_ = 2.0 / 3.0;
-
 typedef void (*stage_launch_fn)(const StageArgs&, const DevParams&, int grid, int block, size_t smem, cudaStream_t);
 typedef cudaError_t (*run_launch_fn)(const RunArgs&, int grid, int block, size_t smem, cudaStream_t);
 typedef size_t (*smem_fn)(int warps);
@@ -35,8 +31,8 @@ typedef const void* (*kptr_fn)();
 struct Variant {
     stage_launch_fn launch;
     kptr_fn kernel;
-    run_launch_fn run;  // many steps in one cooperative launch
-    kptr_fn run_kernel;
+    run_launch_fn run[2];  // many steps in one cooperative launch: plain, with noise and / or the CFL time step
+    kptr_fn run_kernel[2];
     smem_fn smem;
     int T;          // threads per transform group of the adjoint's layout (Geom)
     int PL;         // partial vector length (doubles)
@@ -310,10 +306,10 @@ inline NoiseSpec noise_spec(const qlgpu_params& p, int NZ, double dt, double f_n
     std::memset(&n, 0, sizeof(n));
     const int Ny = (p.ny / 2) * 2;
     const double tot = (double)p.nx * (double)Ny * (double)NZ;
-    const double mult_noise_fac = (1.0 / (16 * 32 * 32)) * (1.0 / (16 * 32 * 32));
     n.lo2 = k_low * k_low;
     n.hi2 = k_high * k_high;
-    n.multfac = dt * (tot * tot) * mult_noise_fac;
+    n.tot2 = tot * tot;
+    n.multfac = noise_factor(dt, n.tot2);
     n.sd = f_noise / std::sqrt(2.0);
     n.seed = seed;
     n.pair_ky0 = p.model == QLGPU_MODEL_MHD_FULLQLIN;
@@ -324,38 +320,9 @@ inline NoiseSpec noise_spec(const qlgpu_params& p, int NZ, double dt, double f_n
     return n;
 }
 
-// Stage constants of RK3CN_Elin::Step / RK3CN::Step for stage s of a step
-// (RK3CN_Elin.cpp:89-91,122-125,155-158; RK3CN.cpp:92-94).
+// Stage constants of a case at its fixed time step.
 inline StageConst stage_const(const qlgpu_params& p, int s) {
-    const double dt = p.dt;
-    const bool cn = p.integrator == QLGPU_INTEG_RK3CN;
-    const double lcf = cn ? dt / 2 : dt;
-    StageConst c;
-    std::memset(&c, 0, sizeof(c));
-    if (s == 0) {
-        c.t_off = 0.0;
-        c.dt_lin = dt * p1_;
-        c.linC = lcf * a0_;
-        c.n1 = a0_ * dt;
-        c.n2 = 0.0;
-        c.has_prev = 0;
-    } else if (s == 1) {
-        c.t_off = dt * p1_;
-        c.dt_lin = dt * (p2_ - p1_);
-        c.linC = lcf * (a1_ + b1_);
-        c.n1 = a1_ * dt;
-        c.n2 = b1_ * dt;
-        c.has_prev = 1;
-    } else {
-        c.t_off = dt * p2_;
-        c.dt_lin = dt * (1.0 - p2_);
-        c.linC = lcf * (a2_ + b2_);
-        c.n1 = a2_ * dt;
-        c.n2 = b2_ * dt;
-        c.has_prev = 1;
-    }
-    c.last = (s == 2);
-    return c;
+    return stage_const(p.dt, p.integrator == QLGPU_INTEG_RK3CN, s);
 }
 
 }  // namespace qlgpu

@@ -15,7 +15,7 @@ template <int NZ, int MODEL, int INTEG>
 const void* stage_ptr() {
     return reinterpret_cast<const void*>(&stage_kernel<NZ, MODEL, INTEG>);
 }
-template <int NZ, int MODEL, int INTEG>
+template <int NZ, int MODEL, int INTEG, bool FORCED>
 cudaError_t launch_run(const RunArgs& R, int grid, int block, size_t smem, cudaStream_t st) {
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));
@@ -28,11 +28,11 @@ cudaError_t launch_run(const RunArgs& R, int grid, int block, size_t smem, cudaS
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, run_kernel<NZ, MODEL, INTEG>, R);
+    return cudaLaunchKernelEx(&cfg, run_kernel<NZ, MODEL, INTEG, FORCED>, R);
 }
-template <int NZ, int MODEL, int INTEG>
+template <int NZ, int MODEL, int INTEG, bool FORCED>
 const void* run_ptr() {
-    return reinterpret_cast<const void*>(&run_kernel<NZ, MODEL, INTEG>);
+    return reinterpret_cast<const void*>(&run_kernel<NZ, MODEL, INTEG, FORCED>);
 }
 template <int NZ, int MODEL>
 size_t stage_smem(int warps) {
@@ -44,8 +44,10 @@ Variant make_variant() {
     Variant v;
     v.launch = &launch_stage<NZ, MODEL, INTEG>;
     v.kernel = &stage_ptr<NZ, MODEL, INTEG>;
-    v.run = &launch_run<NZ, MODEL, INTEG>;
-    v.run_kernel = &run_ptr<NZ, MODEL, INTEG>;
+    v.run[0] = &launch_run<NZ, MODEL, INTEG, false>;
+    v.run[1] = &launch_run<NZ, MODEL, INTEG, true>;
+    v.run_kernel[0] = &run_ptr<NZ, MODEL, INTEG, false>;
+    v.run_kernel[1] = &run_ptr<NZ, MODEL, INTEG, true>;
     v.smem = &stage_smem<NZ, MODEL>;
     v.T = Geom<NZ>::T;
     v.PL = wide::WG<NZ, MODEL>::PL;

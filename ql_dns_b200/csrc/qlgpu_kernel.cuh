@@ -117,7 +117,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
         C->old_init = 0;
         if (last) {
             C->t = t_new;
-            C->timevar = __dadd_rn(C->timevar, P.dt);
+            C->timevar = __dadd_rn(C->timevar, S.dt);
             C->since += 1;
             C->nstep += 1;
         }

@@ -60,7 +60,8 @@ struct DevClock {
 // MHD_FullQlin.cpp:786-1045), added to every mode after its last-stage update.
 struct NoiseSpec {
     double lo2, hi2;     // noise_range_ bounds squared (MHD_FullQlin.cpp:51-52)
-    double multfac;      // dt (Nx Ny NZ)^2 mult_noise_fac_ (MHD_FullQlin.cpp:63-66,804)
+    double multfac;      // dt (Nx Ny NZ)^2 mult_noise_fac_ (MHD_FullQlin.cpp:63-66,804): noise_factor
+    double tot2;         // (Nx Ny NZ)^2
     double sd;           // f_noise/sqrt(2), the standard deviation of each part (:45)
     unsigned long long seed;
     int pair_ky0;        // MHD_FullQlin: ky = 0 modes driven in conjugate pairs (dont_drive_ky0_modes_ = 0)
@@ -87,7 +88,37 @@ struct StageConst {
     int last;         // last stage of the step: advance time, remap, diagnostics
     int abs_time;     // Model::rhs mode: stage time is t_off itself
     int pad;
+    double dt;        // of the step
 };
+
+// RK3 coefficients (RK3CN_Elin.cpp:19-20, RK3CN.cpp:19-20)
+constexpr double a0_ = 8.0 / 15.0, a1_ = 5.0 / 12.0, a2_ = 3.0 / 4.0, b1_ = -17.0 / 60.0, b2_ = -5.0 / 12.0;
+constexpr double p1_ = 8.0 / 15.0, p2_ = 2.0 / 3.0;
+
+// Stage constants of RK3CN_Elin::Step / RK3CN::Step for stage s of a step of dt
+// (RK3CN_Elin.cpp:89-91,122-125,155-158; RK3CN.cpp:92-94).  Products of two factors only:
+// the same numbers on the host and, where the CFL condition sets dt, on the device.
+__host__ __device__ inline StageConst stage_const(double dt, bool cn, int s) {
+    const double lcf = cn ? dt / 2 : dt;
+    StageConst c;
+    c.t_off = s == 0 ? 0.0 : dt * (s == 1 ? p1_ : p2_);
+    c.dt_lin = dt * (s == 0 ? p1_ : s == 1 ? p2_ - p1_ : 1.0 - p2_);
+    c.linC = lcf * (s == 0 ? a0_ : s == 1 ? a1_ + b1_ : a2_ + b2_);
+    c.n1 = dt * (s == 0 ? a0_ : s == 1 ? a1_ : a2_);
+    c.n2 = s == 0 ? 0.0 : dt * (s == 1 ? b1_ : b2_);
+    c.has_prev = s > 0;
+    c.last = s == 2;
+    c.abs_time = 0;
+    c.pad = 0;
+    c.dt = dt;
+    return c;
+}
+
+// The amplitude factor of driving noise of a step of dt (MHD_FullQlin.cpp:63-66,804).
+__host__ __device__ inline double noise_factor(double dt, double tot2) {
+    constexpr double mult_noise_fac = (1.0 / (16 * 32 * 32)) * (1.0 / (16 * 32 * 32));
+    return dt * tot2 * mult_noise_fac;
+}
 
 struct StageArgs {
     const cplx* lin_in;
@@ -138,6 +169,17 @@ struct RunArgs {
     double* rec_kx;
     double* rec_t;
     CnRec* rec_cn;
+    // driving noise after each step (noise_on), its counter on the first step of the launch
+    NoiseSpec noise;
+    int noise_on;
+    unsigned long long step0;
+    // CFL time step (cfl > 0): forcing = {largest |mean field|^2 in real space of up to four fields before
+    // the last stage, sum of the time steps taken, time step of the next step}
+    double cfl, dt_max, kmax;
+    double* forcing;
+    // with noise or the CFL condition: a record after every diag_every-th step of the call, of which
+    // diag_step0 lie before this launch, up to diag_max records (0: none)
+    int diag_every, diag_step0, diag_max;
 };
 
 // ---------------------------------------------------------------------------

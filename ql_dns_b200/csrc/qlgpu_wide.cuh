@@ -113,20 +113,25 @@ __device__ __forceinline__ void team_arrive(int id, int threads) {
 // ---------------------------------------------------------------------------
 // Real-space profiles of the mean fields mf[][nz] (MHD_BQlin.cpp:122-127: By, dz
 // By, dz^2 By; MHD_FullQlin.cpp:180-198: Bx, By, Ux, Uy and dz of each) into
-// out[NPROF][NZ]; xg = the warp's exchange buffer.  Ends without a barrier.
-template <class W, bool BQ, class Load>
+// out[NPROF][NZ]; xg = the warp's exchange buffer.  mx (MAXIMA; null: off) takes the
+// largest |profile|^2 of each mean field, what Calculate_CFL reads (MHD_BQlin.cpp:540-552,
+// MHD_FullQlin.cpp:769-780): MHD_BQlin's Bx is one transform more, in a group that is
+// otherwise idle (NZ <= 128).  Ends without a barrier.
+template <class W, bool BQ, bool MAXIMA = false, class Load>
 __device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, double* out, cplx* xg, const cplx* tw,
-                                               int warp, int nwarps, int lane) {
+                                               int warp, int nwarps, int lane, double* mx = nullptr) {
     const int g = lane / W::T, t = lane % W::T;
-    for (int base = warp * W::GPW; base < W::NPROF; base += nwarps * W::GPW) {
+    const int n = W::NPROF + (MAXIMA && BQ && mx ? 1 : 0);
+    for (int base = warp * W::GPW; base < n; base += nwarps * W::GPW) {
         const int arr = base + g;
-        const int src = BQ ? 1 : arr / 2, deriv = BQ ? arr : arr % 2;
+        const bool bx = MAXIMA && BQ && arr >= W::NPROF;
+        const int src = BQ ? (bx ? 0 : 1) : arr / 2, deriv = BQ ? (bx ? 0 : arr) : arr % 2;
         cplx x[8];
 #pragma unroll
         for (int r = 0; r < 8; ++r) {
             const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
             cplx v = mk(0.0, 0.0);
-            if (s >= 0 && arr < W::NPROF) {
+            if (s >= 0 && arr < n) {
                 v = cscale(mf(src, s), P.fac);
                 const int k = t + W::T * r;
                 const double c = kzval(k <= W::H ? k : k - W::NZ, P.kzL);
@@ -139,6 +144,14 @@ __device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, do
         if (arr < W::NPROF) {
 #pragma unroll
             for (int r = 0; r < 8; ++r) out[arr * W::NZ + t + W::T * r] = x[r].x;
+        }
+        if (MAXIMA && mx) {
+            double v = 0.0;
+#pragma unroll
+            for (int r = 0; r < 8; ++r) v = fmax(v, x[r].x * x[r].x + x[r].y * x[r].y);
+#pragma unroll
+            for (int o = W::T / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+            if (t == 0 && arr < n && deriv == 0) mx[src] = v;
         }
     }
 }
@@ -167,16 +180,17 @@ __device__ __forceinline__ void top_prefetch(const StageArgs& A, double* tot) {
 // what it wrote is published by the caller's release.  Stress spectra
 // (MHD_BQlin.cpp:228-240 after the sum over modes; the transform is linear), the
 // mean-field update and clock (mean_field_update) and the next stage's profiles.
-template <class W, int MODEL, int INTEG>
+template <class W, int MODEL, int INTEG, bool MAXIMA = false>
 __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P, double* tot, cplx* xch,
                                           const cplx* tw, const double* emf, double tclock, double t_new, bool last,
-                                          bool diag_due) {
+                                          bool diag_due, double* mx = nullptr) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
     const int g = lane / W::T, t = lane % W::T;
     double* spec = tot + W::PL + (W::PL & 1);
     cplx* mfs = top_mfs<W>(tot);
     // at most four warps transform (their exchange buffers)
-    constexpr int NT = (W::NPROF + W::GPW - 1) / W::GPW < 4 ? (W::NPROF + W::GPW - 1) / W::GPW : 4;
+    constexpr int NP = W::NPROF + (MAXIMA && W::BQ ? 1 : 0);
+    constexpr int NT = (NP + W::GPW - 1) / W::GPW < 4 ? (NP + W::GPW - 1) / W::GPW : 4;
     const int ntw = nwarps < NT ? nwarps : NT;
     cplx* xg = xch + (size_t)(warp < ntw ? warp : 0) * W::XW;
     if (warp < ntw) {
@@ -203,8 +217,8 @@ __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P
     mean_field_update<W, MODEL, INTEG, W::NE>(A, P, tot, spec, mfs, mfs + W::NMF * W::nz, emf, tclock, t_new, last,
                                               diag_due);
     if (A.mfr_cache && !A.rhs_only && warp < ntw)
-        mean_profiles8<W, W::BQ>(
-            P, [&](int m, int s) { return mfs[m * W::nz + s]; }, A.mfr_cache, xg, tw, warp, ntw, lane);
+        mean_profiles8<W, W::BQ, MAXIMA>(
+            P, [&](int m, int s) { return mfs[m * W::nz + s]; }, A.mfr_cache, xg, tw, warp, ntw, lane, mx);
     if (tid == 0 && A.mfr_cache && !A.rhs_only) A.clk->mfr_valid = 1;
     __syncthreads();
 }
@@ -630,6 +644,8 @@ struct LocalClock {
     double t, timevar, t_old, dtlin_old;
     unsigned long long nstep;
     int old_init, mfr_valid;
+    // forced steps: records after every `every` steps (0: none), step counter, limit of records
+    int every, step, max_rec;
 };
 __device__ __forceinline__ void load_clock(LocalClock& lc, const DevClock* c) {
     lc.t = __ldcg(&c->t);
@@ -642,6 +658,7 @@ __device__ __forceinline__ void load_clock(LocalClock& lc, const DevClock* c) {
 }
 
 // The clock after stage S of a step that started at tclock (what mean_field_update does to DevClock).
+template <bool FORCED>
 __device__ __forceinline__ void advance_clock(LocalClock& lc, const StageConst& S, const DevParams& P, bool last,
                                               bool diag_due) {
     lc.t_old = S.abs_time ? S.t_off : __dadd_rn(lc.t, S.t_off);
@@ -649,14 +666,22 @@ __device__ __forceinline__ void advance_clock(LocalClock& lc, const StageConst& 
     lc.old_init = 0;
     lc.mfr_valid = 1;
     if (!last) return;
-    lc.t = __dadd_rn(lc.t, P.dt);
-    lc.timevar = __dadd_rn(lc.timevar, P.dt);
+    const double dt = FORCED ? S.dt : P.dt;
+    lc.t = __dadd_rn(lc.t, dt);
+    lc.timevar = __dadd_rn(lc.timevar, dt);
     if (diag_due) lc.timevar = __dsub_rn(lc.timevar, P.tv_interval);
     lc.nstep += 1;
+    if (FORCED) lc.step += 1;
 }
 // A record is due at the end of this stage (main.cpp:117,127-130).
-__device__ __forceinline__ bool record_due(const LocalClock& lc, const DevParams& P, bool last) {
-    return last && P.tv_interval > 0.0 && __dsub_rn(__dadd_rn(lc.timevar, P.dt), P.tv_interval) > -1e-8;
+template <bool FORCED>
+__device__ __forceinline__ bool record_due(const LocalClock& lc, const DevParams& P, double dt, bool last) {
+    if (FORCED) {
+        if (lc.every <= 0) return false;
+        const int n = (lc.step + 1) / lc.every;
+        return last && n * lc.every == lc.step + 1 && n <= lc.max_rec;
+    }
+    return last && P.tv_interval > 0.0 && __dsub_rn(__dadd_rn(lc.timevar, dt), P.tv_interval) > -1e-8;
 }
 
 enum StageResult { STAGE_DONE = 0, STAGE_TOP = 1, STAGE_ABORT = 2 };
@@ -673,8 +698,9 @@ enum StageResult { STAGE_DONE = 0, STAGE_TOP = 1, STAGE_ABORT = 2 };
 // persistent launch waits for the case's previous stage.  fresh: the shared-memory
 // tables do not hold this case's yet.  REDUCER: the launch has a CTA of its own for the
 // mean-field side (reduce_stage); this one only counts itself in at `arrive`.  RHS: the
-// launch may ask for the right-hand side instead of the update (A.rhs_only).
-template <int NZ, int MODEL, int INTEG, bool REDUCER, bool RHS, class Gate>
+// launch may ask for the right-hand side instead of the update (A.rhs_only).  FORCED: driving
+// noise and records by step count (run_kernel; work items have the noise alone).
+template <int NZ, int MODEL, int INTEG, bool REDUCER, bool RHS, bool FORCED, class Gate>
 __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevParams& P, const int cta,
                                                   const int ncta, unsigned char* smem_raw, StageShared& ss,
                                                   LocalClock& lc, const bool fresh, unsigned* arrive,
@@ -756,9 +782,9 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
     if (tr) A.trace[1] = gtimer();
 
     // Last-stage bookkeeping identical in every CTA (main.cpp:111-130)
-    const double t_new = __dadd_rn(tclock, P.dt);
+    const double t_new = __dadd_rn(tclock, FORCED ? S.dt : P.dt);
     const bool last = S.last && !A.rhs_only;
-    const bool diag_due = record_due(lc, P, last);
+    const bool diag_due = record_due<FORCED>(lc, P, FORCED ? S.dt : P.dt, last);
     const double qt = __dmul_rn(P.q, t_new);
     const double ts = S.abs_time ? S.t_off : __dadd_rn(tclock, S.t_off);
 
@@ -934,7 +960,7 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
         if (last) {
             if (M.zero && M.valid && wt == 0 && t == 0) A.kx0[M.m] = __dsub_rn(M.kx0, P.remap_shift);
             cplx* uo = A.lin_out + (size_t)M.m * 4 * nzd;
-            if (A.noise) {
+            if ((FORCED || (!REDUCER && !RHS)) && A.noise) {
                 // Model::DrivingNoise after the step (main.cpp:111-113), before the diagnostics see it
                 if (M.valid && !M.zero)
                     noise_mode(A.noise, lc.nstep, uo, nzd, wt * T + t, tws * T, M.m, M.kx0, M.b, M.kxi, M.kyi, P.q,
@@ -979,7 +1005,7 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
 
     __syncthreads();
     if (tr) A.trace[3] = gtimer();
-    if (tid == 0 && !A.rhs_only) advance_clock(lc, S, P, last, diag_due);
+    if (tid == 0 && !A.rhs_only) advance_clock<FORCED>(lc, S, P, last, diag_due);
     if (REDUCER) {
         if (tid == 0) {
             __threadfence();  // covers the CTA's stores, ordered before it by the barrier
@@ -1076,7 +1102,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) stage_kernel(c
     __shared__ LocalClock lc;
     if (threadIdx.x == 0) load_clock(lc, A.clk);
     __syncthreads();
-    stage_body<NZ, MODEL, INTEG, false, true>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss, lc, true, nullptr,
+    stage_body<NZ, MODEL, INTEG, false, true, false>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss, lc, true, nullptr,
                                         [] { return true; });
 }
 
@@ -1114,14 +1140,15 @@ __device__ __forceinline__ bool run_wait(const unsigned* p, unsigned target, Dev
 // The mean-field side of one stage in the reducer CTA: the partial sums of all `ncta`
 // CTAs, in the order of the two-level reduction (CTAs within a group of RED_GROUP, then
 // the groups), then the mean-field stage.
-template <int NZ, int MODEL, int INTEG>
+template <int NZ, int MODEL, int INTEG, bool FORCED>
 __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams& P, int ncta,
-                                             unsigned char* smem_raw, const cplx* tw, const double* emf, LocalClock& lc) {
+                                             unsigned char* smem_raw, const cplx* tw, const double* emf, LocalClock& lc,
+                                             double* mx) {
     using namespace wide;
     using W = WG<NZ, MODEL>;
     const int tid = threadIdx.x, nth = blockDim.x;
-    const bool last = A.sc.last != 0, diag_due = record_due(lc, P, last);
-    const double tclock = lc.t, t_new = __dadd_rn(tclock, P.dt);
+    const bool last = A.sc.last != 0, diag_due = record_due<FORCED>(lc, P, FORCED ? A.sc.dt : P.dt, last);
+    const double tclock = lc.t, t_new = __dadd_rn(tclock, FORCED ? A.sc.dt : P.dt);
     double* tot = reinterpret_cast<double*>(smem_raw + W::o_team);
     // group sums beside the scratch where they fit, else through L2
     constexpr int MAXG = (int)((W::TEAM_BYTES - W::TOP_BYTES - 16) / (8 * (size_t)W::PL));
@@ -1164,9 +1191,24 @@ __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams
     }
     if (A.trace && tid == 0) A.trace[4] = gtimer();
     cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team + W::TOP_XCH);
-    top_stage<W, MODEL, INTEG>(A, P, tot, xch, tw, emf, tclock, t_new, last, diag_due);
-    if (tid == 0) advance_clock(lc, A.sc, P, last, diag_due);
+    top_stage<W, MODEL, INTEG, FORCED>(A, P, tot, xch, tw, emf, tclock, t_new, last, diag_due, mx);
+    if (tid == 0) advance_clock<FORCED>(lc, A.sc, P, last, diag_due);
     if (A.trace && tid == 0) A.trace[5] = gtimer();
+}
+
+// The CFL time step (RK3CN_Elin.cpp:76-80 with Calculate_CFL, MHD_BQlin.cpp:531-556,
+// MHD_FullQlin.cpp:760-784): m the largest |mean field|^2 before the previous step's last
+// stage, mx0 that of the first mean field now.
+template <int MODEL>
+__device__ __forceinline__ double cfl_step(const RunArgs& L, const double* m, double mx0) {
+    double c;
+    if (MODEL == MODEL_BQLIN)
+        c = __dadd_rn(__dadd_rn(__dmul_rn(L.kmax, sqrt(m[1])), __dmul_rn(L.kmax, sqrt(mx0))), L.P.q);
+    else
+        c = __dadd_rn(__dmul_rn(L.kmax, __dadd_rn(__dadd_rn(__dadd_rn(sqrt(m[1]), sqrt(m[0])), sqrt(m[2])), sqrt(m[3]))),
+                      L.P.q);
+    const double dt = __ddiv_rn(L.cfl, c);
+    return dt > L.dt_max ? L.dt_max : dt;
 }
 
 // Many steps of a single case in one cooperative launch.  Worker CTAs step their blocks
@@ -1177,27 +1219,68 @@ __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams
 // the tables and the round trips of profiles and clock.  Every wait is bounded in time
 // and iterations; one that gives up sets QLGPU_STATUS_TIMEOUT and the abort word, and
 // every CTA leaves.
-template <int NZ, int MODEL, int INTEG>
+//
+// FORCED, a kernel of its own (with its code in the plain one every launch is 2-3 %
+// slower): with the CFL condition (L.cfl > 0) the reducer sets each step's dt from the maxima of the
+// profiles that it has formed, in the launch's first wait and at the end of each step, and
+// the workers wait for it before a step's first stage.  Driving noise is added by the teams
+// after the last stage.  32x32 x NZ=64 with both: 95 us a step with the host setting dt and the
+// noise in a launch of its own, 44 us so.
+template <int NZ, int MODEL, int INTEG, bool FORCED>
 __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(const __grid_constant__ RunArgs L) {
     using W = wide::WG<NZ, MODEL>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StageShared ss;
     __shared__ LocalClock lc;
+    __shared__ NoiseSpec s_noise;
+    __shared__ double s_mx[4];
     __shared__ __align__(16) StageArgs sA[3];
     const int tid = threadIdx.x, ncta = (int)gridDim.x - 1;
     const bool reducer = (int)blockIdx.x == ncta;
+    const bool cfl = FORCED && L.cfl > 0.0;
+    const unsigned e0 = cfl ? 1 : 0;  // epoch 1: the first time step is set
     DevClock* C = L.A[0].clk;
     for (int i = tid; i < (int)(sizeof(sA) / 8); i += blockDim.x)
         reinterpret_cast<unsigned long long*>(sA)[i] = reinterpret_cast<const unsigned long long*>(L.A)[i];
-    if (tid == 0) load_clock(lc, C);
+    if (tid == 0) {
+        load_clock(lc, C);
+        if (FORCED) {
+            lc.every = L.diag_every;
+            lc.step = L.diag_step0;
+            lc.max_rec = L.diag_max;
+            s_noise = L.noise;
+        }
+    }
     unsigned k = 0;  // stages before this one in the launch
     if (reducer) {
         cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
         double* emf = reinterpret_cast<double*>(smem_raw + W::o_ekz);
         for (int i = tid; i < NZ; i += blockDim.x) tw[i] = ldc_cg(L.A[0].tw + NZ + i);
+        double m[4] = {0.0, 0.0, 0.0, 0.0}, dt_sum = 0.0;  // thread 0
+        if (cfl) {
+            __syncthreads();
+            cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team + W::TOP_XCH);
+            const int warp = tid >> 5, nw = blockDim.x >= 128 ? 4 : blockDim.x >> 5;
+            if (warp < nw)
+                wide::mean_profiles8<W, W::BQ, true>(
+                    L.P, [&](int f, int s) { return ldc_cg(L.A[0].mf + f * W::nz + s); },
+                    reinterpret_cast<double*>(smem_raw + W::o_prof), xch + W::XW * warp, tw, warp, nw, tid & 31, s_mx);
+            __syncthreads();
+            if (tid == 0) {
+#pragma unroll
+                for (int f = 0; f < 4; ++f) m[f] = __ldcg(L.forcing + f);
+                dt_sum = __ldcg(L.forcing + 4);
+                L.forcing[5] = cfl_step<MODEL>(L, m, s_mx[0]);
+                st_release_u32(&C->epoch, e0);
+            }
+        }
         for (int n = 0; n < L.nsteps; ++n)
             for (int s = 0; s < 3; ++s, ++k) {
                 __syncthreads();
+                if (cfl && s == 0) {
+                    if (tid < 3) sA[tid].sc = stage_const(L.forcing[5], INTEG == INTEG_CN, tid);
+                    __syncthreads();
+                }
                 if (tid == 0) ss.ok = run_wait(&C->arrive, (k + 1) * (unsigned)ncta, C, L.wait_ns) ? 1 : 0;
                 if (INTEG == INTEG_EXP)  // under the wait (the last threads: the first one polls)
                     for (int i = blockDim.x - 1 - tid; i < W::nz; i += blockDim.x) {
@@ -1208,21 +1291,46 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
                     }
                 __syncthreads();
                 if (!ss.ok) return;
-                reduce_stage<NZ, MODEL, INTEG>(sA[s], L.P, ncta, smem_raw, tw, INTEG == INTEG_EXP ? emf : nullptr,
-                                               lc);
+                reduce_stage<NZ, MODEL, INTEG, FORCED>(sA[s], L.P, ncta, smem_raw, tw, INTEG == INTEG_EXP ? emf : nullptr,
+                                               lc, cfl ? s_mx : nullptr);
                 if (tid == 0) {
+                    if (cfl && s == 1) {
+#pragma unroll
+                        for (int f = 0; f < W::NMF; ++f) L.forcing[f] = m[f] = s_mx[f];
+                    }
+                    if (cfl && s == 2) {
+                        L.forcing[4] = dt_sum = __dadd_rn(dt_sum, sA[0].sc.dt);
+                        L.forcing[5] = cfl_step<MODEL>(L, m, s_mx[0]);
+                    }
                     // after the last stage nobody waits any more: ready for the next launch
                     const bool end = n == L.nsteps - 1 && s == 2;
                     if (end) C->arrive = 0;
-                    st_release_u32(&C->epoch, end ? 0u : k + 1);
+                    st_release_u32(&C->epoch, end ? 0u : k + 1 + e0);
                 }
             }
         return;
     }
     const size_t nlin = (size_t)L.P.nxy * 4 * L.P.nz, nmfe = (size_t)L.P.nmf * L.P.nz;
+    if (FORCED) {
+        __syncthreads();
+        if (tid == 0 && L.noise_on) {
+            lc.nstep = L.step0;
+            sA[2].noise = &s_noise;
+        }
+    }
     for (int n = 0; n < L.nsteps; ++n)
         for (int s = 0; s < 3; ++s, ++k) {
             __syncthreads();
+            if (cfl && s == 0) {
+                if (tid == 0) {
+                    ss.ok = run_wait(&C->epoch, k + 1, C, L.wait_ns) ? 1 : 0;
+                    const double dt = __ldcg(L.forcing + 5);
+                    for (int i = 0; i < 3; ++i) sA[i].sc = stage_const(dt, INTEG == INTEG_CN, i);
+                    s_noise.multfac = noise_factor(dt, s_noise.tot2);
+                }
+                __syncthreads();
+                if (!ss.ok) return;
+            }
             if (tid == 0) {
                 StageArgs& A = sA[s];
                 const int in = (int)((k + (unsigned)L.cur) & 1u);
@@ -1237,9 +1345,9 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
                 }
             }
             __syncthreads();
-            const StageResult r = stage_body<NZ, MODEL, INTEG, true, false>(
+            const StageResult r = stage_body<NZ, MODEL, INTEG, true, false, FORCED>(
                 sA[s], L.P, (int)blockIdx.x, ncta, smem_raw, ss, lc, k == 0, &C->arrive,
-                [&]() -> bool { return run_wait(&C->epoch, k, C, L.wait_ns); });
+                [&]() -> bool { return run_wait(&C->epoch, k + e0, C, L.wait_ns); });
             if (r == STAGE_ABORT) return;
         }
 }

@@ -63,3 +63,53 @@ def test_work_item_widths(warps, model):
     t2, lo2, mo2, ko2, _ = O.run(p, 0.0, lin, mf, kx0, 3)
     assert t == t2 and np.array_equal(ko, ko2)
     assert rel(mo, mo2) < 1e-10 and rel(lo, lo2) < 1e-10
+
+
+@pytest.mark.parametrize("integ", [0, 1])
+@pytest.mark.parametrize("model", [0, 1])
+@pytest.mark.parametrize("nx,ny,NZ", [(2, 2, 128), (32, 40, 128), (18, 2, 256), (36, 34, 64), (8, 8, 16)])
+def test_forced_layout_edges(nx, ny, NZ, model, integ):
+    """Noise and the CFL time step inside the launch; a record every second step."""
+    require_gpu()
+    p = QLParams(model=model, integrator=integ, nx=nx, ny=ny, NZ=NZ, dt=0.02, B0z=0.02 if model else 0.0)
+    lin, mf, kx0 = initial_state(p, 3, sigma=0.02, B0=0.2, mean_u=0.05 if model else 0.0)
+    n, cfl, noise = 6, (0.3, 0.05), (0.02, 0.5, 50.0, 7)
+    with QLSolver(p) as s:
+        s.set_noise(*noise)
+        s.set_cfl(*cfl)
+        s.set_state(0.0, lin, mf, kx0)
+        rec = s.step(n, diag_every=2)
+        t, lo, mo, ko = s.get_state()
+        dtm = s.mean_time_step()
+        s.set_state(0.0, lin, mf, kx0)
+        for _ in range(n):
+            s.step(1)
+        t1, l1, m1, k1 = s.get_state()
+        assert dtm == s.mean_time_step()
+    assert t == t1 and np.array_equal(lo, l1) and np.array_equal(mo, m1) and np.array_equal(ko, k1)
+    t2, lo2, mo2, ko2, d2, dtm2 = O.run_forced(p, 0.0, lin, mf, kx0, n, diag_every=2, cfl=cfl[0], dt_max=cfl[1],
+                                              f_noise=noise[0], k_lo=noise[1], k_hi=noise[2], seed=noise[3])
+    assert abs(t - t2) <= 1e-13 * t2 and abs(dtm - dtm2) <= 1e-13 * dtm2 and np.array_equal(ko, ko2)
+    assert rel(mo, mo2) < 1e-10
+    assert rel(lo, lo2) < 1e-10 if np.linalg.norm(lo2) else not lo.any()
+    assert rec.shape[0] == 3
+    scale = np.abs(d2[1:, 1:13]).max(0)
+    assert np.all(np.abs(rec[:, 1:13] - d2[1:, 1:13]) <= 1e-10 * scale)
+
+
+def test_forced_across_launches():
+    """260 steps are two launches: noise counter, time step and its mean carry over."""
+    require_gpu()
+    p = QLParams(nx=8, ny=8, NZ=16, dt=0.02)
+    st = initial_state(p, 3, sigma=0.02, B0=0.2)
+    out = []
+    for parts in ((260,), (100, 160)):
+        with QLSolver(p) as s:
+            s.set_noise(0.02, 0.5, 50.0, 7)
+            s.set_cfl(0.3, 0.05)
+            s.set_state(0.0, *st)
+            for n in parts:
+                rec = s.step(n, diag_every=20)
+            out.append(s.get_state() + (s.mean_time_step(), rec[-1]))
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
