@@ -120,6 +120,7 @@ cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec, const Run
     R.P = h->dp;
     R.lin[0] = h->d_lin[0];
     R.lin[1] = h->d_lin[1];
+    R.mf_alt = h->d_mf_alt;
     R.cur = h->cur;
     R.nsteps = n;
     R.wait_ns = 2000000000LL;
@@ -142,7 +143,7 @@ cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec, const Run
         R.diag_step0 = force->diag_step0;
         R.diag_max = force->diag_max;
     }
-    const cudaError_t e = h->var.run[force != nullptr](R, h->grid + 1, h->block, h->smem, h->stream);
+    const cudaError_t e = h->var.run[force != nullptr](R, h->grid + h->nmf, h->block, h->smem, h->stream);
     if (e == cudaSuccess) h->cur ^= n & 1;  // three stages per step
     return e;
 }
@@ -154,8 +155,8 @@ cudaError_t qlgpu_clear_abort(qlgpu_t* h) {
     cudaError_t e = cudaMemsetAsync(&c->cnt_top, 0, sizeof(unsigned), h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(c->cnt_group, 0, sizeof(c->cnt_group), h->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(&c->abort, 0, sizeof(int), h->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&c->arrive, 0, sizeof(unsigned), h->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(&c->epoch, 0, sizeof(unsigned), h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->arrive, 0, sizeof(c->arrive), h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->epoch, 0, sizeof(c->epoch), h->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(h->stream) : e;
 }
 
@@ -261,7 +262,8 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
         h->err = "cudaGetDeviceProperties failed";
         return bail(QLGPU_ERR_CUDA);
     }
-    const StageGeom sg = stage_geometry(p.model, p.NZ, h->nxy, prop.multiProcessorCount - 1, 64 * RED_GROUP, var.max_warps);
+    const StageGeom sg = stage_geometry(p.model, p.NZ, h->nxy, prop.multiProcessorCount - h->nmf,
+                                         RUN_MAX_GROUPS * RED_GROUP, var.max_warps);
     h->warps = sg.warps;
     h->block = 32 * h->warps;
     h->smem = var.smem(h->warps);
@@ -293,6 +295,7 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     QLGPU_ALLOC(h->d_F1, nlin * sizeof(cplx));
     QLGPU_ALLOC(h->d_F2, nlin * sizeof(cplx));
     QLGPU_ALLOC(h->d_mf, nmfe * sizeof(cplx));
+    QLGPU_ALLOC(h->d_mf_alt, 2 * nmfe * sizeof(cplx));
     QLGPU_ALLOC(h->d_Fmf1, nmfe * sizeof(cplx));
     QLGPU_ALLOC(h->d_Fmf2, nmfe * sizeof(cplx));
     QLGPU_ALLOC(h->d_kx0, h->nxy * sizeof(double));
@@ -345,7 +348,7 @@ int qlgpu_destroy(qlgpu_t* h) {
     if (!h) return QLGPU_OK;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    void* bufs[] = {h->d_lin[0], h->d_lin[1], h->d_F1, h->d_F2, h->d_mf, h->d_Fmf1, h->d_Fmf2,
+    void* bufs[] = {h->d_lin[0], h->d_lin[1], h->d_F1, h->d_F2, h->d_mf, h->d_mf_alt, h->d_Fmf1, h->d_Fmf2,
                     h->d_kx0, h->d_ky, h->d_kxi, h->d_kyi, h->d_tw, h->d_partials, h->d_gpartials,
                     h->d_clk, h->d_diag, h->d_out15, h->d_linop, h->d_ilap2, h->d_trace,
                     h->d_mfr, h->d_ekz, h->d_forcing, h->d_dbg, h->adj_ws, h->adj_tab};

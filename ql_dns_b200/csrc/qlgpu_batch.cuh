@@ -88,8 +88,8 @@ __device__ __noinline__ StageResult batch_item_stage(const BatchLaunch& L, const
     }
     __syncthreads();
     return stage_body<NZ, MODEL, INTEG, false, false, false>(sA, sP, it.cta, it.ncta, smem_raw, ss, lc, fresh, nullptr,
-                                               [&]() -> bool {
-        return batch_wait(L.epoch + (size_t)it.c * BATCH_EPOCH_STRIDE, k, L.ctl, L.wait_ns, it.c, k);
+                                               [&](int lane) -> bool {
+        return lane > 0 || batch_wait(L.epoch + (size_t)it.c * BATCH_EPOCH_STRIDE, k, L.ctl, L.wait_ns, it.c, k);
     });
 }
 

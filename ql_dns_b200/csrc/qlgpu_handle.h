@@ -25,6 +25,7 @@ struct qlgpu_handle {
     cplx* d_F1 = nullptr;
     cplx* d_F2 = nullptr;
     cplx* d_mf = nullptr;
+    cplx* d_mf_alt = nullptr;  // RunArgs::mf_alt
     cplx* d_Fmf1 = nullptr;
     cplx* d_Fmf2 = nullptr;
     double* d_kx0 = nullptr;

@@ -112,8 +112,8 @@ inline int stage_teams(int model, int warps) {
     return n > 1 ? n : 1;
 }
 
-// CTA width and grid of a single case's stage kernel: one CTA per SM, one SM left for the CTA of
-// the mean-field side (run_kernel).  When every team can
+// CTA width and grid of a single case's stage kernel: one CTA per SM (sms: those left beside the
+// CTAs of the mean-field side, run_kernel).  When every team can
 // have its own SM a team gets as many warps as it has inverse transforms (one round of tasks);
 // otherwise a CTA holds the teams that the case has blocks for.
 struct StageGeom {

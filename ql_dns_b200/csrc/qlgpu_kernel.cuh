@@ -7,6 +7,7 @@
 namespace qlgpu {
 
 constexpr int RED_GROUP = 16;  // CTAs per first-level reduction group
+constexpr int RUN_MAX_GROUPS = 16;  // of a many-steps launch
 
 // Energy, stress and dissipation sums of one pair of mean fields at stored index s
 // (MHD_BQlin.cpp:408-447): v += {energy, stress, -k^2 energy}.
@@ -34,17 +35,49 @@ __device__ __forceinline__ void put_record(const DevParams& P, const double* ds,
 }
 
 // ---------------------------------------------------------------------------
+// The diagnostic record of a step (Calc_Energy_AM_Diss, MHD_BQlin.cpp:408-477) by one warp
+// from the fluctuation sums ds[6] and the mean fields mfs[nmf][nz]: lanes over kz, then a
+// fixed shuffle tree.
+// ---------------------------------------------------------------------------
+template <class W>
+__device__ __forceinline__ void step_record(const StageArgs& A, const DevParams& P, const double* ds, const cplx* mfs,
+                                            double t_new, int lane) {
+    const int nzd = P.nz;
+    DevClock* C = A.clk;
+    double v[6] = {0, 0, 0, 0, 0, 0};  // eMB, aMB, dMB, eMU, aMU, dMU
+    for (int s = lane; s < nzd; s += 32) {
+        const double kz2 = kz2val(kzval(s <= W::H ? s : s - nzd, P.kzL));
+        mf_sums(mfs, mfs + nzd, s, kz2, v);
+        if (P.nmf == 4) mf_sums(mfs + 2 * nzd, mfs + 3 * nzd, s, kz2, v + 3);
+    }
+#pragma unroll
+    for (int q = 0; q < 6; ++q)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
+    if (lane != 0) return;
+    const int r = C->ndiag;
+    if (r < A.diag_cap)
+        put_record(P, ds, v, t_new, A.diag_ring + (size_t)QLGPU_CHECK_INDEX(r, A.diag_cap, &C->status) * 15);
+    else
+        C->status |= QLGPU_STATUS_DIAG_FULL;
+    C->ndiag = r + 1;
+    C->timevar = __dsub_rn(C->timevar, P.tv_interval);
+    C->since = 0;
+}
+
+// ---------------------------------------------------------------------------
 // Mean-field update, run by the whole CTA that arrives last: the mean-field
 // right-hand side from the stress spectra spec[NEMF][H + 1] and its RK update
-// (mfs[nmf][nz] in shared memory, updated in place, and A.mf; fps: the previous
+// (mfs[nmf][nz] in shared memory, updated in place, and mfo; fps: the previous
 // right-hand side; emf: the integrating factors, null to compute them), then the time and
-// diagnostic bookkeeping in the last warp.  tot[] holds the stress profiles
+// diagnostic bookkeeping in the last warp.  only >= 0 (a reducer of run_kernel): that field
+// alone, and no record.  tot[] holds the stress profiles
 // summed over all modes (real z) followed by the six fluctuation diagnostic sums.
 // ---------------------------------------------------------------------------
 template <class W, int MODEL, int INTEG, int NEMF>
 __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevParams& P, const double* tot,
                                                   const double* spec, cplx* mfs, const cplx* fps, const double* emf,
-                                                  double tclock, double t_new, bool last, bool diag_due) {
+                                                  double tclock, double t_new, bool last, bool diag_due, int only, cplx* mfo) {
     const StageConst& S = A.sc;
     const int tid = threadIdx.x, lane = tid & 31;
     const int nzd = P.nz;
@@ -82,6 +115,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
             }
         }
         for (int mm = 0; mm < P.nmf; ++mm) {
+            if (only >= 0 && mm != only) continue;
             if (A.rhs_only) {
                 stc(A.Fmf_out + mm * nzd + s, F[mm]);
                 continue;
@@ -99,7 +133,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
                 nv = rk_update<INTEG_CN>(S, Lm, Lm, F[mm], fp, m[mm], S.has_prev);
             }
             if (A.Fmf_out) stc(A.Fmf_out + mm * nzd + s, F[mm]);
-            stc(A.mf + mm * nzd + s, nv);
+            stc(mfo + mm * nzd + s, nv);
             mfs[mm * nzd + s] = nv;
             const double mag = nv.x * nv.x + nv.y * nv.y;
             if (!(mag == mag) || isinf(mag)) atomicOr(&A.clk->status, QLGPU_STATUS_NONFINITE);
@@ -110,7 +144,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
     // the rest in the last warp: the first ones go on to the next stage's profiles
     if (A.rhs_only || (tid >> 5) != (int)(blockDim.x >> 5) - 1) return;
     DevClock* C = A.clk;
-    if (lane == 0) {
+    if (lane == 0 && only <= 0) {
         // CN bookkeeping: this stage's operator time becomes "old" (RK3CN.cpp:119-122)
         C->t_old = S.abs_time ? S.t_off : __dadd_rn(tclock, S.t_off);
         C->dtlin_old = S.dt_lin;
@@ -122,28 +156,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
             C->nstep += 1;
         }
     }
-    if (!last || !diag_due) return;
-    // Calc_Energy_AM_Diss (MHD_BQlin.cpp:408-477): lanes over kz, then a fixed shuffle tree
-    double v[6] = {0, 0, 0, 0, 0, 0};  // eMB, aMB, dMB, eMU, aMU, dMU
-    for (int s = lane; s < nzd; s += 32) {
-        const double kz2 = kz2val(kzval(s <= W::H ? s : s - nzd, P.kzL));
-        mf_sums(mfs, mfs + nzd, s, kz2, v);
-        if (P.nmf == 4) mf_sums(mfs + 2 * nzd, mfs + 3 * nzd, s, kz2, v + 3);
-    }
-#pragma unroll
-    for (int q = 0; q < 6; ++q)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], o);
-    if (lane != 0) return;
-    const int r = C->ndiag;
-    if (r < A.diag_cap)
-        put_record(P, tot + NEMF * W::NZ, v, t_new,
-                   A.diag_ring + (size_t)QLGPU_CHECK_INDEX(r, A.diag_cap, &C->status) * 15);
-    else
-        C->status |= QLGPU_STATUS_DIAG_FULL;
-    C->ndiag = r + 1;
-    C->timevar = __dsub_rn(C->timevar, P.tv_interval);
-    C->since = 0;
+    if (last && diag_due && only < 0) step_record<W>(A, P, tot + NEMF * W::NZ, mfs, t_new, lane);
 }
 
 }  // namespace qlgpu

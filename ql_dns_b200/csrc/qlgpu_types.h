@@ -50,10 +50,8 @@ struct DevClock {
     int abort;         // a wait of the running launch gave up (run_kernel)
     // counters of the running launch, each on a line of its own (0 between launches)
     unsigned pad0[32];
-    unsigned arrive;   // CTAs that have published a stage's partial sums
-    unsigned pad1[32];
-    unsigned epoch;    // stages whose mean-field side is complete
-    unsigned pad2[31];
+    unsigned arrive[32 * 4];  // per reducer CTA: CTAs that have published a stage's partial sums
+    unsigned epoch[32 * 4];   // per reducer CTA: stages whose mean field of that reducer is complete
 };
 
 // Driving noise of one case (Model::DrivingNoise, MHD_BQlin.cpp:558-618 and
@@ -160,6 +158,7 @@ struct RunArgs {
     StageArgs A[3];   // the step's stages; lin_in / lin_out / rec_* are set per stage
     DevParams P;
     cplx* lin[2];     // the ping-pong fields, lin[cur] the current ones
+    cplx* mf_alt;     // [2][nmf][nz]: the mean fields between the first stage's input and the last one's result
     int cur, nsteps;
     long long wait_ns;  // bound on one wait for the other CTAs
     // optional record of every stage input (null: off): step n, stage s at rec_lin + (3 n + s) nxy 4 nz,

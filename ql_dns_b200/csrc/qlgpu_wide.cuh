@@ -115,14 +115,14 @@ __device__ __forceinline__ void team_arrive(int id, int threads) {
 // By, dz^2 By; MHD_FullQlin.cpp:180-198: Bx, By, Ux, Uy and dz of each) into
 // out[NPROF][NZ]; xg = the warp's exchange buffer.  mx (MAXIMA; null: off) takes the
 // largest |profile|^2 of each mean field, what Calculate_CFL reads (MHD_BQlin.cpp:540-552,
-// MHD_FullQlin.cpp:769-780): MHD_BQlin's Bx is one transform more, in a group that is
-// otherwise idle (NZ <= 128).  Ends without a barrier.
+// MHD_FullQlin.cpp:769-780); number NPROF of MHD_BQlin is Bx, for its maximum alone.  lo, hi:
+// the profiles taken.  Ends without a barrier.
 template <class W, bool BQ, bool MAXIMA = false, class Load>
 __device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, double* out, cplx* xg, const cplx* tw,
-                                               int warp, int nwarps, int lane, double* mx = nullptr) {
+                                               int warp, int nwarps, int lane, double* mx = nullptr, int lo = 0,
+                                               int hi = W::NPROF) {
     const int g = lane / W::T, t = lane % W::T;
-    const int n = W::NPROF + (MAXIMA && BQ && mx ? 1 : 0);
-    for (int base = warp * W::GPW; base < n; base += nwarps * W::GPW) {
+    for (int base = lo + warp * W::GPW; base < hi; base += nwarps * W::GPW) {
         const int arr = base + g;
         const bool bx = MAXIMA && BQ && arr >= W::NPROF;
         const int src = BQ ? (bx ? 0 : 1) : arr / 2, deriv = BQ ? (bx ? 0 : arr) : arr % 2;
@@ -131,7 +131,7 @@ __device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, do
         for (int r = 0; r < 8; ++r) {
             const int s = rdead<W>(r) ? -1 : sidx<W>(t, r);
             cplx v = mk(0.0, 0.0);
-            if (s >= 0 && arr < n) {
+            if (s >= 0 && arr < hi) {
                 v = cscale(mf(src, s), P.fac);
                 const int k = t + W::T * r;
                 const double c = kzval(k <= W::H ? k : k - W::NZ, P.kzL);
@@ -141,7 +141,7 @@ __device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, do
             x[r] = v;
         }
         xform<W>(x, xg, tw, g, t);
-        if (arr < W::NPROF) {
+        if (arr < hi && !bx) {
 #pragma unroll
             for (int r = 0; r < 8; ++r) out[arr * W::NZ + t + W::T * r] = x[r].x;
         }
@@ -151,7 +151,7 @@ __device__ __forceinline__ void mean_profiles8(const DevParams& P, Load&& mf, do
             for (int r = 0; r < 8; ++r) v = fmax(v, x[r].x * x[r].x + x[r].y * x[r].y);
 #pragma unroll
             for (int o = W::T / 2; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-            if (t == 0 && arr < n && deriv == 0) mx[src] = v;
+            if (t == 0 && arr < hi && deriv == 0) mx[src] = v;
         }
     }
 }
@@ -177,25 +177,26 @@ __device__ __forceinline__ void top_prefetch(const StageArgs& A, double* tot) {
 // Mean-field stage of the CTA that arrived last: tot[PL] holds the stress
 // profiles summed over the modes and the diagnostic sums; emf (optional): the integrating
 // factors exp(linC eta kz2), exp(linC nu kz2) [2][NZE] of the stage.  Ends with a barrier;
-// what it wrote is published by the caller's release.  Stress spectra
+// what it wrote is published by the caller's release.  ONE: a reducer of run_kernel, which
+// takes the mean field `only` and its stress, and has the new field in mfo.  Stress spectra
 // (MHD_BQlin.cpp:228-240 after the sum over modes; the transform is linear), the
 // mean-field update and clock (mean_field_update) and the next stage's profiles.
-template <class W, int MODEL, int INTEG, bool MAXIMA = false>
+template <class W, int MODEL, int INTEG, bool ONE = false, bool MAXIMA = false>
 __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P, double* tot, cplx* xch,
                                           const cplx* tw, const double* emf, double tclock, double t_new, bool last,
-                                          bool diag_due, double* mx = nullptr) {
+                                          bool diag_due, double* mx = nullptr, int only = -1, cplx* mfo = nullptr) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
     const int g = lane / W::T, t = lane % W::T;
     double* spec = tot + W::PL + (W::PL & 1);
     cplx* mfs = top_mfs<W>(tot);
     // at most four warps transform (their exchange buffers)
-    constexpr int NP = W::NPROF + (MAXIMA && W::BQ ? 1 : 0);
+    constexpr int NP = !ONE ? W::NPROF : W::BQ ? 3 : 2;
     constexpr int NT = (NP + W::GPW - 1) / W::GPW < 4 ? (NP + W::GPW - 1) / W::GPW : 4;
     const int ntw = nwarps < NT ? nwarps : NT;
     cplx* xg = xch + (size_t)(warp < ntw ? warp : 0) * W::XW;
     if (warp < ntw) {
-        for (int base = warp * W::GPW; base < W::NE; base += ntw * W::GPW) {
-            const int e = base + g;
+        for (int base = warp * W::GPW; base < (ONE ? 1 : W::NE); base += ntw * W::GPW) {
+            const int e = !ONE ? base + g : g == 0 ? only : W::NE;
             cplx x[8];
 #pragma unroll
             for (int r = 0; r < 8; ++r) x[r] = mk(e < W::NE ? tot[e * W::NZ + t + W::T * r] : 0.0, 0.0);
@@ -215,10 +216,13 @@ __device__ __forceinline__ void top_stage(const StageArgs& A, const DevParams& P
     cp_async_wait_all();
     __syncthreads();
     mean_field_update<W, MODEL, INTEG, W::NE>(A, P, tot, spec, mfs, mfs + W::NMF * W::nz, emf, tclock, t_new, last,
-                                              diag_due);
+                                              diag_due, ONE ? only : -1, ONE ? mfo : A.mf);
+    // MHD_BQlin needs the profiles of By alone, the reducer of Bx at most its largest value
+    const int lo = !ONE ? 0 : !W::BQ ? 2 * only : only == 1 ? 0 : W::NPROF;
+    const int hi = !ONE ? W::NPROF : !W::BQ ? lo + 2 : only == 1 || (MAXIMA && mx) ? lo + (only == 1 ? 3 : 1) : lo;
     if (A.mfr_cache && !A.rhs_only && warp < ntw)
         mean_profiles8<W, W::BQ, MAXIMA>(
-            P, [&](int m, int s) { return mfs[m * W::nz + s]; }, A.mfr_cache, xg, tw, warp, ntw, lane, mx);
+            P, [&](int m, int s) { return mfs[m * W::nz + s]; }, A.mfr_cache, xg, tw, warp, ntw, lane, mx, lo, hi);
     if (tid == 0 && A.mfr_cache && !A.rhs_only) A.clk->mfr_valid = 1;
     __syncthreads();
 }
@@ -694,10 +698,10 @@ enum StageResult { STAGE_DONE = 0, STAGE_TOP = 1, STAGE_ABORT = 2 };
 // A team steps the same blocks in every stage, so a stage's fields, previous
 // right-hand sides and kx0 come from the CTA's own last stage: only the mean-field
 // profiles wait for the other CTAs.  The first block's inverse transforms therefore
-// run before gate() (called by thread 0; false ends the launch), which in a
+// run before gate(lane) (called by the first warp; false ends the launch), which in a
 // persistent launch waits for the case's previous stage.  fresh: the shared-memory
-// tables do not hold this case's yet.  REDUCER: the launch has a CTA of its own for the
-// mean-field side (reduce_stage); this one only counts itself in at `arrive`.  RHS: the
+// tables do not hold this case's yet.  REDUCER: the launch has CTAs of their own for the
+// mean-field side (reduce_stage); this one only counts itself in at their `arrive`.  RHS: the
 // launch may ask for the right-hand side instead of the update (A.rhs_only).  FORCED: driving
 // noise and records by step count (run_kernel; work items have the noise alone).
 template <int NZ, int MODEL, int INTEG, bool REDUCER, bool RHS, bool FORCED, class Gate>
@@ -877,7 +881,10 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
         cp_async_wait_all();
         if (base == first) {
             // ---- the mean field of this stage
-            if (tid == 0) ss.ok = gate() ? 1 : 0;
+            if (warp == 0) {
+                const int ok = __all_sync(0xffffffffu, gate(lane));
+                if (lane == 0) ss.ok = ok;
+            }
             __syncthreads();
             if (!ss.ok) return STAGE_ABORT;
             if (tr) A.trace[6] = gtimer();
@@ -1007,9 +1014,9 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
     if (tr) A.trace[3] = gtimer();
     if (tid == 0 && !A.rhs_only) advance_clock<FORCED>(lc, S, P, last, diag_due);
     if (REDUCER) {
-        if (tid == 0) {
+        if (tid < W::NMF) {
             __threadfence();  // covers the CTA's stores, ordered before it by the barrier
-            atomicAdd(arrive, 1u);
+            atomicAdd(arrive + 32 * tid, 1u);
         }
         return STAGE_DONE;
     }
@@ -1103,7 +1110,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) stage_kernel(c
     if (threadIdx.x == 0) load_clock(lc, A.clk);
     __syncthreads();
     stage_body<NZ, MODEL, INTEG, false, true, false>(A, P, (int)blockIdx.x, (int)gridDim.x, smem_raw, ss, lc, true, nullptr,
-                                        [] { return true; });
+                                        [](int) { return true; });
 }
 
 // ---------------------------------------------------------------------------
@@ -1137,71 +1144,77 @@ __device__ __forceinline__ bool run_wait(const unsigned* p, unsigned target, Dev
     return false;
 }
 
-// The mean-field side of one stage in the reducer CTA: the partial sums of all `ncta`
-// CTAs, in the order of the two-level reduction (CTAs within a group of RED_GROUP, then
-// the groups), then the mean-field stage.
+// The mean-field side of one stage in the reducer CTA of mean field `e`: the partial sums of
+// stress profile e over all `ncta` CTAs, in the order of the two-level reduction (CTAs within
+// a group of RED_GROUP, then the groups), then the field's part of the mean-field stage, the
+// result in mfo.  What bounds it is one SM's reading of the sums (8-byte loads, 32 a thread in
+// flight): 147 CTAs x NZ = 128 take 5.8 us for both profiles of MHD_BQlin, 3.8 us for one.
 template <int NZ, int MODEL, int INTEG, bool FORCED>
-__device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams& P, int ncta,
+__device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams& P, int e, int ncta,
                                              unsigned char* smem_raw, const cplx* tw, const double* emf, LocalClock& lc,
-                                             double* mx) {
+                                             double* mx, cplx* mfo) {
     using namespace wide;
     using W = WG<NZ, MODEL>;
     const int tid = threadIdx.x, nth = blockDim.x;
     const bool last = A.sc.last != 0, diag_due = record_due<FORCED>(lc, P, FORCED ? A.sc.dt : P.dt, last);
     const double tclock = lc.t, t_new = __dadd_rn(tclock, FORCED ? A.sc.dt : P.dt);
     double* tot = reinterpret_cast<double*>(smem_raw + W::o_team);
-    // group sums beside the scratch where they fit, else through L2
-    constexpr int MAXG = (int)((W::TEAM_BYTES - W::TOP_BYTES - 16) / (8 * (size_t)W::PL));
+    // group sums beside the scratch
+    static_assert((size_t)RUN_MAX_GROUPS * 8 * (NZ + 8) + W::TOP_BYTES + 16 <= W::TEAM_BYTES, "group sums fit");
+    double* gs = reinterpret_cast<double*>(smem_raw + W::o_team + ((W::TOP_BYTES + 15) & ~(size_t)15));
     const int ngroups = (ncta + RED_GROUP - 1) / RED_GROUP;
-    double* gs = ngroups <= MAXG ? reinterpret_cast<double*>(smem_raw + W::o_team + ((W::TOP_BYTES + 15) & ~(size_t)15))
-                                 : A.gpartials;
-    if (ngroups == 1) gs = tot;
-    top_prefetch<W>(A, tot);
-    for (int i0 = tid; i0 < ngroups * W::PL; i0 += 2 * nth) {
-        // two (group, value) pairs at a time, all their loads in flight
-        double v[2][RED_GROUP];
+    // columns [col, col + NC) of all rows
+    auto sum = [&](auto nc_, int col) {
+        constexpr int NC = decltype(nc_)::value;
+        const double* p0 = A.partials + col;
+        for (int i0 = tid; i0 < ngroups * NC; i0 += 2 * nth) {
+            // two (group, value) pairs at a time, all their loads in flight
+            double v[2][RED_GROUP];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = i0 + h * nth, q = i / W::PL, idx = i - q * W::PL;
-            const int n = i < ngroups * W::PL ? min(RED_GROUP, ncta - q * RED_GROUP) : 0;
-            const double* src = A.partials + (size_t)q * RED_GROUP * W::PL + idx;
+            for (int h = 0; h < 2; ++h) {
+                const int i = i0 + h * nth, q = i / NC, idx = i - q * NC;
+                const int n = i < ngroups * NC ? min(RED_GROUP, ncta - q * RED_GROUP) : 0;
+                const double* src = p0 + (size_t)q * RED_GROUP * W::PL + idx;
 #pragma unroll
-            for (int u = 0; u < RED_GROUP; ++u) v[h][u] = u < n ? __ldcg(src + (size_t)u * W::PL) : 0.0;
-        }
+                for (int u = 0; u < RED_GROUP; ++u) v[h][u] = u < n ? __ldcg(src + (size_t)u * W::PL) : 0.0;
+            }
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int i = i0 + h * nth;
-            if (i >= ngroups * W::PL) break;
-            const int n = min(RED_GROUP, ncta - i / W::PL * RED_GROUP);
-            double s = 0.0;
+            for (int h = 0; h < 2; ++h) {
+                const int i = i0 + h * nth;
+                if (i >= ngroups * NC) break;
+                const int n = min(RED_GROUP, ncta - i / NC * RED_GROUP);
+                double s = 0.0;
 #pragma unroll
-            for (int u = 0; u < RED_GROUP; ++u)
-                if (u < n) s += v[h][u];
-            gs[i] = s;
-        }
-    }
-    __syncthreads();
-    if (ngroups > 1) {
-        for (int idx = tid; idx < W::PL; idx += nth) {
-            double s = 0.0;
-            for (int q = 0; q < ngroups; ++q) s += gs[(size_t)q * W::PL + idx];
-            tot[idx] = s;
+                for (int u = 0; u < RED_GROUP; ++u)
+                    if (u < n) s += v[h][u];
+                gs[i] = s;
+            }
         }
         __syncthreads();
-    }
-    if (A.trace && tid == 0) A.trace[4] = gtimer();
+        for (int idx = tid; idx < NC; idx += nth) {
+            double s = ngroups > 1 ? 0.0 : gs[idx];
+            for (int q = 0; q < ngroups && ngroups > 1; ++q) s += gs[(size_t)q * NC + idx];
+            tot[col + idx] = s;
+        }
+        __syncthreads();
+    };
+    sum(std::integral_constant<int, NZ>{}, e * NZ);
+    if (e == 0 && diag_due) sum(std::integral_constant<int, 8>{}, W::NE * NZ);
+    if (A.trace && tid == 0 && e == 0) A.trace[4] = gtimer();
     cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team + W::TOP_XCH);
-    top_stage<W, MODEL, INTEG, FORCED>(A, P, tot, xch, tw, emf, tclock, t_new, last, diag_due, mx);
+    top_stage<W, MODEL, INTEG, true, FORCED>(A, P, tot, xch, tw, emf, tclock, t_new, last, diag_due, mx, e, mfo);
     if (tid == 0) advance_clock<FORCED>(lc, A.sc, P, last, diag_due);
-    if (A.trace && tid == 0) A.trace[5] = gtimer();
+    if (A.trace && tid == 0 && e == 0) A.trace[5] = gtimer();
 }
 
 // The CFL time step (RK3CN_Elin.cpp:76-80 with Calculate_CFL, MHD_BQlin.cpp:531-556,
-// MHD_FullQlin.cpp:760-784): m the largest |mean field|^2 before the previous step's last
+// MHD_FullQlin.cpp:760-784) from the largest |mean field|^2 before the previous step's last
 // stage, mx0 that of the first mean field now.
 template <int MODEL>
-__device__ __forceinline__ double cfl_step(const RunArgs& L, const double* m, double mx0) {
-    double c;
+__device__ __forceinline__ double cfl_step(const RunArgs& L, double mx0) {
+    double c, m[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) m[f] = __ldcg(L.forcing + f);
     if (MODEL == MODEL_BQLIN)
         c = __dadd_rn(__dadd_rn(__dmul_rn(L.kmax, sqrt(m[1])), __dmul_rn(L.kmax, sqrt(mx0))), L.P.q);
     else
@@ -1212,31 +1225,34 @@ __device__ __forceinline__ double cfl_step(const RunArgs& L, const double* m, do
 }
 
 // Many steps of a single case in one cooperative launch.  Worker CTAs step their blocks
-// stage after stage; the last CTA has no modes and runs the mean-field side, so that its
-// chain (sums, two transforms, update, profiles: 4 us) runs under the workers' first
-// inverse transforms of the next stage instead of in a worker that would then be the
-// last one to arrive again.  Against three launches per step this saves the launch gap,
-// the tables and the round trips of profiles and clock.  Every wait is bounded in time
-// and iterations; one that gives up sets QLGPU_STATUS_TIMEOUT and the abort word, and
-// every CTA leaves.
+// stage after stage; the last NMF CTAs have no modes and run the mean-field side, one mean
+// field each, so that its chain (sums, two transforms, update, profiles) runs under the
+// workers' first inverse transforms of the next stage instead of in a worker that would then
+// be the last one to arrive again.  A reducer reads all fields of the stage's start, so the
+// fields alternate between two buffers.  Against three launches per step this saves the launch
+// gap, the tables and the round trips of profiles and clock.  One reducer for all fields:
+// 29.5 us a stage at 64x64 x NZ=128, 15.2 at 22x18 x NZ=256, 14.7 at 48x48 x NZ=64 of
+// MHD_FullQlin; one per field: 27.0, 13.2, 12.0.  Every wait is bounded in time and iterations; one
+// that gives up sets QLGPU_STATUS_TIMEOUT and the abort word, and every CTA leaves.
 //
 // FORCED, a kernel of its own (with its code in the plain one every launch is 2-3 %
-// slower): with the CFL condition (L.cfl > 0) the reducer sets each step's dt from the maxima of the
-// profiles that it has formed, in the launch's first wait and at the end of each step, and
-// the workers wait for it before a step's first stage.  Driving noise is added by the teams
-// after the last stage.  32x32 x NZ=64 with both: 95 us a step with the host setting dt and the
-// noise in a launch of its own, 44 us so.
+// slower): with the CFL condition (L.cfl > 0) the first reducer sets each step's dt from the
+// maxima of the profiles that the reducers form, in the launch's first wait and at the end of
+// each step, and the others wait for it before a step's first stage.  Driving noise is added
+// by the teams after the last stage.  32x32 x NZ=64 with both: 95 us a step with the host setting
+// dt and the noise in a launch of its own, 41 us so.
 template <int NZ, int MODEL, int INTEG, bool FORCED>
 __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(const __grid_constant__ RunArgs L) {
     using W = wide::WG<NZ, MODEL>;
+    constexpr int NR = W::NMF;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StageShared ss;
     __shared__ LocalClock lc;
     __shared__ NoiseSpec s_noise;
     __shared__ double s_mx[4];
     __shared__ __align__(16) StageArgs sA[3];
-    const int tid = threadIdx.x, ncta = (int)gridDim.x - 1;
-    const bool reducer = (int)blockIdx.x == ncta;
+    const int tid = threadIdx.x, lane = tid & 31, ncta = (int)gridDim.x - NR;
+    const int e = (int)blockIdx.x - ncta;  // >= 0: reducer of field e
     const bool cfl = FORCED && L.cfl > 0.0;
     const unsigned e0 = cfl ? 1 : 0;  // epoch 1: the first time step is set
     DevClock* C = L.A[0].clk;
@@ -1251,37 +1267,59 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
             s_noise = L.noise;
         }
     }
+    __syncthreads();
+    const size_t nlin = (size_t)L.P.nxy * 4 * L.P.nz, nmfe = (size_t)L.P.nmf * L.P.nz;
+    const unsigned nstages = 3u * (unsigned)L.nsteps;
+    // the mean fields at the start of stage k of the launch
+    auto mf_in = [&](unsigned k) {
+        return k == 0 || k == nstages ? L.A[0].mf : L.mf_alt + (size_t)((k - 1) & 1u) * nmfe;
+    };
     unsigned k = 0;  // stages before this one in the launch
-    if (reducer) {
+    if (e >= 0) {
         cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
         double* emf = reinterpret_cast<double*>(smem_raw + W::o_ekz);
+        double* tot = reinterpret_cast<double*>(smem_raw + W::o_team);
         for (int i = tid; i < NZ; i += blockDim.x) tw[i] = ldc_cg(L.A[0].tw + NZ + i);
-        double m[4] = {0.0, 0.0, 0.0, 0.0}, dt_sum = 0.0;  // thread 0
+        // wait by the first warp's lanes for the other reducers' `target` (lane: its reducer)
+        auto wait_others = [&](unsigned target, int r) -> bool {
+            return r >= NR || r == e || run_wait(C->epoch + 32 * r, target, C, L.wait_ns);
+        };
+        double dt_sum = 0.0;  // thread 0 of the first reducer
         if (cfl) {
             __syncthreads();
-            cplx* xch = reinterpret_cast<cplx*>(smem_raw + W::o_team + W::TOP_XCH);
-            const int warp = tid >> 5, nw = blockDim.x >= 128 ? 4 : blockDim.x >> 5;
-            if (warp < nw)
+            if (e == 0 && tid < 32 && W::BQ)
                 wide::mean_profiles8<W, W::BQ, true>(
-                    L.P, [&](int f, int s) { return ldc_cg(L.A[0].mf + f * W::nz + s); },
-                    reinterpret_cast<double*>(smem_raw + W::o_prof), xch + W::XW * warp, tw, warp, nw, tid & 31, s_mx);
+                    L.P, [&](int f, int s) { return ldc_cg(L.A[0].mf + f * W::nz + s); }, nullptr,
+                    reinterpret_cast<cplx*>(smem_raw + W::o_team + W::TOP_XCH), tw, 0, 1, tid, s_mx, W::NPROF,
+                    W::NPROF + 1);
             __syncthreads();
             if (tid == 0) {
-#pragma unroll
-                for (int f = 0; f < 4; ++f) m[f] = __ldcg(L.forcing + f);
-                dt_sum = __ldcg(L.forcing + 4);
-                L.forcing[5] = cfl_step<MODEL>(L, m, s_mx[0]);
-                st_release_u32(&C->epoch, e0);
+                if (e == 0) {
+                    dt_sum = __ldcg(L.forcing + 4);
+                    L.forcing[5] = cfl_step<MODEL>(L, s_mx[0]);
+                }
+                st_release_u32(C->epoch + 32 * e, e0);
             }
         }
         for (int n = 0; n < L.nsteps; ++n)
             for (int s = 0; s < 3; ++s, ++k) {
                 __syncthreads();
-                if (cfl && s == 0) {
-                    if (tid < 3) sA[tid].sc = stage_const(L.forcing[5], INTEG == INTEG_CN, tid);
-                    __syncthreads();
+                // the fields at the stage's start, complete once all reducers are (at the launch's start they are)
+                if (tid < 32) {
+                    const int ok = __all_sync(0xffffffffu, k + e0 == 0 || wait_others(k + e0, lane));
+                    if (lane == 0) {
+                        ss.ok = ok;
+                        sA[s].mf = mf_in(k);
+                        if (cfl && s == 0)
+                            for (int i = 0; i < 3; ++i)
+                                sA[i].sc = stage_const(__ldcg(L.forcing + 5), INTEG == INTEG_CN, i);
+                    }
                 }
-                if (tid == 0) ss.ok = run_wait(&C->arrive, (k + 1) * (unsigned)ncta, C, L.wait_ns) ? 1 : 0;
+                __syncthreads();
+                if (!ss.ok) return;
+                wide::top_prefetch<W>(sA[s], tot);
+                if (tid == 0)
+                    ss.ok = run_wait(C->arrive + 32 * e, (k + 1) * (unsigned)ncta, C, L.wait_ns) ? 1 : 0;
                 if (INTEG == INTEG_EXP)  // under the wait (the last threads: the first one polls)
                     for (int i = blockDim.x - 1 - tid; i < W::nz; i += blockDim.x) {
                         const double kz2 = kz2val(kzval(i <= W::H ? i : i - W::nz, L.P.kzL));
@@ -1291,39 +1329,50 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
                     }
                 __syncthreads();
                 if (!ss.ok) return;
-                reduce_stage<NZ, MODEL, INTEG, FORCED>(sA[s], L.P, ncta, smem_raw, tw, INTEG == INTEG_EXP ? emf : nullptr,
-                                               lc, cfl ? s_mx : nullptr);
+                const bool rec = e == 0 && record_due<FORCED>(lc, L.P, FORCED ? sA[s].sc.dt : L.P.dt, s == 2);
+                reduce_stage<NZ, MODEL, INTEG, FORCED>(sA[s], L.P, e, ncta, smem_raw, tw,
+                                                       INTEG == INTEG_EXP ? emf : nullptr, lc, cfl ? s_mx : nullptr,
+                                                       mf_in(k + 1));
+                const bool end = k + 1 == nstages;
                 if (tid == 0) {
-                    if (cfl && s == 1) {
-#pragma unroll
-                        for (int f = 0; f < W::NMF; ++f) L.forcing[f] = m[f] = s_mx[f];
-                    }
-                    if (cfl && s == 2) {
+                    if (cfl && s == 1) L.forcing[e] = s_mx[e];
+                    if (cfl && s == 2 && e == 0) {
                         L.forcing[4] = dt_sum = __dadd_rn(dt_sum, sA[0].sc.dt);
-                        L.forcing[5] = cfl_step<MODEL>(L, m, s_mx[0]);
+                        L.forcing[5] = cfl_step<MODEL>(L, s_mx[0]);
                     }
-                    // after the last stage nobody waits any more: ready for the next launch
-                    const bool end = n == L.nsteps - 1 && s == 2;
-                    if (end) C->arrive = 0;
-                    st_release_u32(&C->epoch, end ? 0u : k + 1 + e0);
+                    st_release_u32(C->epoch + 32 * e, k + 1 + e0);
+                }
+                if (rec || (end && e == 0)) {
+                    // the others' new fields, for the record (they are not overwritten before this reducer
+                    // has finished another stage); at the end the last use of the others' counters
+                    if (tid < 32) {
+                        const int ok = __all_sync(0xffffffffu, wait_others(k + 1 + e0, lane));
+                        if (lane == 0) ss.ok = ok;
+                    }
+                    __syncthreads();
+                    if (!ss.ok) return;
+                    if (rec) {
+                        cplx* mfs = wide::top_mfs<W>(tot);
+                        for (int i = tid; i < (int)nmfe; i += blockDim.x) mfs[i] = ldc_cg(mf_in(k + 1) + i);
+                        __syncthreads();
+                        if (tid < 32) step_record<W>(sA[s], L.P, tot + W::NE * NZ, mfs, lc.t, tid);
+                    }
+                    // nobody waits any more: ready for the next launch
+                    if (end && tid < NR) C->arrive[32 * tid] = C->epoch[32 * tid] = 0;
                 }
             }
         return;
     }
-    const size_t nlin = (size_t)L.P.nxy * 4 * L.P.nz, nmfe = (size_t)L.P.nmf * L.P.nz;
-    if (FORCED) {
-        __syncthreads();
-        if (tid == 0 && L.noise_on) {
-            lc.nstep = L.step0;
-            sA[2].noise = &s_noise;
-        }
+    if (FORCED && tid == 0 && L.noise_on) {
+        lc.nstep = L.step0;
+        sA[2].noise = &s_noise;
     }
     for (int n = 0; n < L.nsteps; ++n)
         for (int s = 0; s < 3; ++s, ++k) {
             __syncthreads();
             if (cfl && s == 0) {
                 if (tid == 0) {
-                    ss.ok = run_wait(&C->epoch, k + 1, C, L.wait_ns) ? 1 : 0;
+                    ss.ok = run_wait(C->epoch, k + 1, C, L.wait_ns) ? 1 : 0;
                     const double dt = __ldcg(L.forcing + 5);
                     for (int i = 0; i < 3; ++i) sA[i].sc = stage_const(dt, INTEG == INTEG_CN, i);
                     s_noise.multfac = noise_factor(dt, s_noise.tot2);
@@ -1337,6 +1386,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
                 A.lin_in = L.lin[in];
                 A.lin_out = L.lin[in ^ 1];
                 if (L.rec_lin) {
+                    A.mf = mf_in(k);
                     A.rec_lin = L.rec_lin + (size_t)k * nlin;
                     A.rec_mf = L.rec_mf + (size_t)k * nmfe;
                     A.rec_kx = s == 0 ? L.rec_kx + (size_t)n * L.P.nxy : nullptr;
@@ -1346,8 +1396,9 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
             }
             __syncthreads();
             const StageResult r = stage_body<NZ, MODEL, INTEG, true, false, FORCED>(
-                sA[s], L.P, (int)blockIdx.x, ncta, smem_raw, ss, lc, k == 0, &C->arrive,
-                [&]() -> bool { return run_wait(&C->epoch, k + e0, C, L.wait_ns); });
+                sA[s], L.P, (int)blockIdx.x, ncta, smem_raw, ss, lc, k == 0, C->arrive, [&](int r_) -> bool {
+                    return r_ >= NR || run_wait(C->epoch + 32 * r_, k + e0, C, L.wait_ns);
+                });
             if (r == STAGE_ABORT) return;
         }
 }
