@@ -498,60 +498,34 @@ constexpr int QTRACE_MAX_CTAS_PER_SM = 4;  // bound of the queue grid: at most t
 int ens_class(int NZ) { return NZ == 16 ? 0 : NZ == 32 ? 1 : NZ == 64 ? 2 : 3; }
 size_t tw8_offset(int NZ) { return NZ == 16 ? 0 : NZ == 32 ? 16 : NZ == 64 ? 48 : 112; }  // cplx
 
-// Default CTA passes per chunk of each NZ class, before any tuning.  Four passes
-// keep the fixed cost of a chunk small (about 12 us against about 25 us per pass,
-// the same at every NZ by the choice of modes per pass; measured on B200).  When
-// four passes leave CTAs without a chunk (a small batch), the combination of
-// {1, 2, 3, 4} that minimises whole waves of chunks times the mean chunk time is
-// taken instead.
+// Default CTA passes per chunk, before any tuning.  A chunk costs about 12 us besides its
+// passes of about 13.3 us (the same at every NZ by the choice of modes per pass), so long
+// chunks cost less work W per CTA and stage; but a stage of a case takes at least its longest
+// chunk and the mean-field stage, about 8 us, and where that chain is no longer short against
+// W, CTAs wait.  The stage time (W^5 + chain^5)^(1/5) follows the measurements (24 cases: 0.322,
+// 0.305, 0.351 ms a step at 3, 4, 6 passes; 12 cases: 0.297, 0.275, 0.301 at 2, 3, 4; 6 cases: 0.145,
+// 0.142, 0.180 at 1, 2, 3; 16 cases of 32x32 x NZ=64: 0.155, 0.134, 0.166 at 1, 2, 3), so the
+// passes that minimise it are taken, at most four.  Batches of 30 cases and more gain
+// another 7 % from eight (48 cases: 0.626 -> 0.582), which qlgpu_batch_tune finds.
 void default_passes(qlgpu_batch_t* b) {
-    constexpr double PASS_US = 25.0, CHUNK_US = 12.0;
-    const int grid = b->sms;
-    std::vector<int> need(b->ncases), cls(b->ncases);
-    bool present[4] = {false, false, false, false};
-    for (int c = 0; c < b->ncases; ++c) {
-        const CaseHost& h = b->cs[c];
-        const int mpp = ens::modes_per_pass(h.NZ);
-        need[c] = (h.nxy + mpp - 1) / mpp;
-        cls[c] = ens_class(h.NZ);
-        present[cls[c]] = true;
-    }
-    auto chunks_and_work = [&](const int (&p)[4], double* work) {
-        long C = 0;
-        double W = 0.0;
-        for (int c = 0; c < b->ncases; ++c) {
-            const int pc = p[cls[c]];
-            const long n = (need[c] + pc - 1) / pc;
-            C += n;
-            W += (double)n * (pc * PASS_US + CHUNK_US);
+    constexpr double PASS_US = 13.3, CHUNK_US = 12.0, TOP_US = 8.0;
+    double best = 1e300;
+    for (int p = 1; p <= 4; ++p) {
+        double work = 0.0;
+        int longest = 0;
+        for (const CaseHost& h : b->cs) {
+            const int mpp = ens::modes_per_pass(h.NZ), need = (h.nxy + mpp - 1) / mpp;
+            work += need * PASS_US + (need + p - 1) / p * CHUNK_US;
+            longest = std::max(longest, std::min(p, need));
         }
-        *work = W;
-        return C;
-    };
-    int best[4] = {4, 4, 4, 4};
-    double W4 = 0.0;
-    if (chunks_and_work(best, &W4) >= grid) {
-        std::copy(best, best + 4, b->qpasses);
-        return;
-    }
-    double best_est = 1e300;
-    for (int code = 0; code < 256; ++code) {
-        int p[4];
-        bool skip = false;
-        for (int k = 0; k < 4; ++k) {
-            p[k] = 1 + ((code >> (2 * k)) & 3);
-            if (!present[k] && p[k] != 4) skip = true;
-        }
-        if (skip) continue;
-        double W = 0.0;
-        const long C = chunks_and_work(p, &W);
-        const double est = (double)((C + grid - 1) / grid) * (W / (double)C);
-        if (est < best_est - 1e-9) {
-            best_est = est;
-            std::copy(p, p + 4, best);
+        work /= b->sms;
+        const double chain = longest * PASS_US + CHUNK_US + TOP_US;
+        const double est = std::pow(std::pow(work, 5) + std::pow(chain, 5), 0.2);
+        if (est < best - 1e-9) {
+            best = est;
+            std::fill(b->qpasses, b->qpasses + 4, p);
         }
     }
-    std::copy(best, best + 4, b->qpasses);
 }
 
 bool queue_usable(const qlgpu_batch_t* b) { return b->queue_ok && b->engine == QLGPU_BATCH_ENGINE_QUEUE; }
