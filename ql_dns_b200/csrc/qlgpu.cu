@@ -71,6 +71,14 @@ StageArgs base_args(qlgpu_t* h) {
     return A;
 }
 
+// The stage kernel's shared-memory attributes, set where it is launched.
+cudaError_t load_stage_kernel(const qlgpu_t* h) {
+    const cudaError_t e = ensure_smem_attr(h->var.kernel(), h->smem);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(h->var.kernel(), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                cudaSharedmemCarveoutMaxShared);
+}
+
 // One RK3 step = three stage launches (RK3CN_Elin::Step / RK3CN::Step), timed by 4 events recorded
 // before stage 1 and after each stage.
 void enqueue_step(qlgpu_t* h, cudaEvent_t* ev) {
@@ -269,13 +277,12 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     h->smem = var.smem(h->warps);
     h->grid = sg.grid;
     h->per_sm = 1;
-    if (h->smem > (size_t)prop.sharedMemPerBlockOptin || ensure_smem_attr(var.kernel(), h->smem) != cudaSuccess ||
-        ensure_smem_attr(var.run_kernel[0](), h->smem) != cudaSuccess ||
-        ensure_smem_attr(var.run_kernel[1](), h->smem) != cudaSuccess) {
+    // the stage kernel and the forced steps' are loaded by the calls that launch them (2 to 3 ms)
+    if (h->smem > (size_t)prop.sharedMemPerBlockOptin ||
+        ensure_smem_attr(var.run_kernel[0](), h->smem) != cudaSuccess) {
         h->err = "shared memory request too large";
         return bail(QLGPU_ERR_CUDA);
     }
-    cudaFuncSetAttribute(var.kernel(), cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     const int ngroups = (h->grid + RED_GROUP - 1) / RED_GROUP;
 
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
@@ -302,7 +309,7 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     QLGPU_ALLOC(h->d_ky, h->nxy * sizeof(double));
     QLGPU_ALLOC(h->d_kxi, h->nxy * sizeof(int));
     QLGPU_ALLOC(h->d_kyi, h->nxy * sizeof(int));
-    QLGPU_ALLOC(h->d_tw, 2 * h->NZ * sizeof(cplx));
+    QLGPU_ALLOC(h->d_tw, h->NZ * sizeof(cplx));
     QLGPU_ALLOC(h->d_partials, (size_t)h->grid * var.PL * sizeof(double));
     QLGPU_ALLOC(h->d_gpartials, (size_t)ngroups * var.PL * sizeof(double));
     QLGPU_ALLOC(h->d_clk, sizeof(DevClock));
@@ -311,7 +318,7 @@ int qlgpu_create(const qlgpu_params* pp, int device, qlgpu_t** out) {
     QLGPU_ALLOC(h->d_mfr, (size_t)8 * h->NZ * sizeof(double));
     QLGPU_ALLOC(h->d_ekz, (size_t)6 * h->nz * sizeof(double));
     QLGPU_ALLOC(h->d_dbg, sizeof(int));
-    const std::vector<double> tw = stage_twiddles(h->NZ);
+    const std::vector<double> tw = twiddles(h->NZ);
     cudaMemcpyAsync(h->d_tw, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream);
     h->il2_tab = ilap2_table(p, h->nz);
     h->ekz_tab = ekz_table(p, d);
@@ -490,6 +497,7 @@ static int step_forced(qlgpu_t* h, int nsteps, int diag_every, double* diag_out,
     f.diag_max = max_diag;
     h->dp.tv_interval = 0.0;
     double* const d_dt_sum = h->d_forcing + 4;
+    QLGPU_CK(ensure_smem_attr(h->var.run_kernel[1](), h->smem));
     if (f.cfl > 0) QLGPU_CK(cudaMemcpyAsync(d_dt_sum, &h->dt_sum, sizeof(double), cudaMemcpyHostToDevice, h->stream));
     for (int n = 0; n < nsteps; n += RUN_STEPS) {
         f.diag_step0 = n;
@@ -619,6 +627,7 @@ int qlgpu_step_timed(qlgpu_t* h, float* stage_ms) {
     for (int i = 0; i < 4; ++i)
         if (!h->ev[i]) QLGPU_CK(cudaEventCreate(&h->ev[i]));
     h->dp.tv_interval = 0.0;
+    QLGPU_CK(load_stage_kernel(h));
     enqueue_step(h, h->ev);
     int rc = check_launch(h);
     if (rc) return rc;
@@ -664,6 +673,7 @@ int qlgpu_rhs(qlgpu_t* h, double t, double dt_lin, const double* lin_in, const d
     A.sc.t_off = t;
     A.sc.abs_time = 1;
     A.sc.dt_lin = dt_lin;
+    QLGPU_CK(load_stage_kernel(h));
     h->var.launch(A, h->dp, h->grid, h->block, h->smem, h->stream);
     int rc = check_launch(h);
     if (rc) return rc;
@@ -716,6 +726,7 @@ int qlgpu_launch_info(const qlgpu_t* h, int* info8) {
 int qlgpu_kernel_attrs(const qlgpu_t* h, int* attrs8) {
     if (!h || !attrs8) return QLGPU_ERR_ARG;
     cudaFuncAttributes fa;
+    if (load_stage_kernel(h) != cudaSuccess) return QLGPU_ERR_CUDA;
     if (cudaFuncGetAttributes(&fa, h->var.kernel()) != cudaSuccess) return QLGPU_ERR_CUDA;
     int occ0 = 0, occs = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ0, h->var.kernel(), h->block, 0);
@@ -787,7 +798,7 @@ struct NoallocLayout {
 NoallocLayout noalloc_layout(int NZ, int nxy, int nyh, int nz, int grid, int PL) {
     NoallocLayout L;
     size_t o = 0;
-    L.tw = o; o = align256(o + sizeof(cplx) * 2 * NZ);
+    L.tw = o; o = align256(o + sizeof(cplx) * NZ);
     L.ky = o; o = align256(o + sizeof(double) * nxy);
     L.kxi = o; o = align256(o + sizeof(int) * nxy);
     L.kyi = o; o = align256(o + sizeof(int) * nxy);
@@ -802,7 +813,7 @@ NoallocLayout noalloc_layout(int NZ, int nxy, int nyh, int nz, int grid, int PL)
 
 // Fills the wavenumber tables (Kdata.cpp:24-46,100-119), the twiddles of the
 // transform layout and the default kx0, and zeroes the reduction counters.
-__global__ void noalloc_tables_kernel(unsigned char* base, NoallocLayout L, int NZ, int T, int nx, int ny, int nz,
+__global__ void noalloc_tables_kernel(unsigned char* base, NoallocLayout L, int NZ, int nx, int ny, int nz,
                                       double kxL, double kyL, double kzL, int fill_kx0) {
     const int nxy = (nx - 1) * (ny / 2);
     const int nyh = ny / 2, nxh = nx / 2;
@@ -814,10 +825,8 @@ __global__ void noalloc_tables_kernel(unsigned char* base, NoallocLayout L, int 
     double* il2 = reinterpret_cast<double*>(base + L.il2);
     DevClock* clk = reinterpret_cast<DevClock*>(base + L.clk);
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
-    for (int i = tid; i < 2 * NZ; i += nth) {
-        // [P][T] of the adjoint's layout, then [8][NZ/8]
-        const int Tl = i < NZ ? T : NZ / 8, j = i < NZ ? i : i - NZ;
-        const int m = ((j / Tl) * (j % Tl)) % NZ;
+    for (int i = tid; i < NZ; i += nth) {
+        const int T = NZ / 8, m = (i / T) * (i % T) % NZ;
         double sn, cs;
         sincospi(2.0 * (double)m / (double)NZ, &sn, &cs);
         tw[i] = mk(cs, sn);
@@ -930,7 +939,7 @@ extern "C" int qlgpu_rhs_noalloc(const qlgpu_params* pp, double t, double dt_lin
     d.dt = p.dt;
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     unsigned char* b = static_cast<unsigned char*>(base);
-    noalloc_tables_kernel<<<32, 256, 0, st>>>(b, L, p.NZ, var.T, p.nx, p.ny, nz, 2 * kPI / p.L[0], 2 * kPI / p.L[1],
+    noalloc_tables_kernel<<<32, 256, 0, st>>>(b, L, p.NZ, p.nx, p.ny, nz, 2 * kPI / p.L[0], 2 * kPI / p.L[1],
                                              d.kzL, kx0 ? 0 : 1);
     StageArgs A;
     std::memset(&A, 0, sizeof(A));

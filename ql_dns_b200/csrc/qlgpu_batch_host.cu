@@ -937,7 +937,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         h.ky = reinterpret_cast<double*>(take(h.nxy * sizeof(double)));
         h.kxi = reinterpret_cast<int*>(take(h.nxy * sizeof(int)));
         h.kyi = reinterpret_cast<int*>(take(h.nxy * sizeof(int)));
-        h.tw = reinterpret_cast<cplx*>(take(2 * h.NZ * sizeof(cplx)));
+        h.tw = reinterpret_cast<cplx*>(take(h.NZ * sizeof(cplx)));
         h.il2 = reinterpret_cast<double*>(take((size_t)(h.p.ny / 2) * h.nz * sizeof(double)));
         h.partials = reinterpret_cast<double*>(take((size_t)h.max_cta * h.PL * sizeof(double)));
         h.gpartials = reinterpret_cast<double*>(
@@ -949,7 +949,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         std::vector<double> ky;
         std::vector<int> kxi, kyi;
         ktables(h.p, h.kx_tab, ky, kxi, kyi);
-        const std::vector<double> tw = stage_twiddles(h.NZ);
+        const std::vector<double> tw = twiddles(h.NZ);
         const std::vector<double> il2 = ilap2_table(h.p, h.nz);
         const std::vector<double> ekz = ekz_table(h.p, h.dp);
         cudaMemcpyAsync(h.kx0, h.kx_tab.data(), h.nxy * sizeof(double), cudaMemcpyHostToDevice, b->stream);
@@ -1007,7 +1007,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         // 8-point twiddles of the queue engine, tw[q T + t] = exp(2 pi i q t / NZ), T = NZ / 8
         std::vector<double> tw8(480, 0.0);
         for (int NZ : {16, 32, 64, 128}) {
-            const std::vector<double> t = twiddles(NZ, NZ / 8);
+            const std::vector<double> t = twiddles(NZ);
             std::copy(t.begin(), t.end(), tw8.begin() + 2 * tw8_offset(NZ));
         }
         if (cudaMemcpyAsync(b->d_tw8, tw8.data(), sizeof(double) * 480, cudaMemcpyHostToDevice, b->stream) !=

@@ -278,9 +278,9 @@ int qlgpu_dns_create(const qlgpu_dns_params* p, int device, qlgpu_dns_t** out) {
     DNS_AL(h->d_rec, 15 * sizeof(double));
 #undef DNS_AL
     if (rc == QLGPU_OK) {
-        std::vector<double> twz = twiddles(p->NZ, p->NZ / 8);
-        std::vector<double> twx = twiddles(p->Mx, p->Mx / 8);
-        std::vector<double> twy = twiddles(p->My, p->My / 8);
+        std::vector<double> twz = twiddles(p->NZ);
+        std::vector<double> twx = twiddles(p->Mx);
+        std::vector<double> twy = twiddles(p->My);
         cudaError_t e3 = cudaSuccess;
         if (e3 == cudaSuccess) e3 = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
         if (e3 == cudaSuccess) e3 = cudaMemcpy((void*)a.ky, ky.data(), h->nxy * sizeof(double), cudaMemcpyHostToDevice);

@@ -51,6 +51,7 @@
 
 #include "qlgpu_batch.cuh"
 #include "qlgpu_debug.cuh"
+#include "qlgpu_priv.cuh"
 #include "qlgpu_xform.cuh"
 
 namespace qlgpu {
@@ -556,7 +557,7 @@ __device__ __noinline__ void run_chunk(const EnsLaunch& L, ChunkHdr& hd, const R
                 const double L = linop_f<MODEL_BQLIN>(P, lap_end<MODEL_BQLIN>(P, kxe, ky, kz2), f);
                 const double lo = hd.cn_old_init ? lap_init<MODEL_BQLIN>(P, kxo, lap2val(ky, kz2, z0))
                                                  : lap_end<MODEL_BQLIN>(P, kxo, ky, kz2);
-                nv = rk_update<INTEG_CN>(S, L, linop_f<MODEL_BQLIN>(P, lo, f), F[rr], fp, uin, fpm != nullptr);
+                nv = rk_update(S, L, linop_f<MODEL_BQLIN>(P, lo, f), F[rr], fp, uin, fpm != nullptr);
             }
             if (fo) st_stream(fo + f * nzd + sx, F[rr]);
             st_stream(uo + f * nzd + sx, zero ? mk(0.0, 0.0) : nv);

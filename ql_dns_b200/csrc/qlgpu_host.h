@@ -34,7 +34,6 @@ struct Variant {
     run_launch_fn run[2];  // many steps in one cooperative launch: plain, with noise and / or the CFL time step
     kptr_fn run_kernel[2];
     smem_fn smem;
-    int T;          // threads per transform group of the adjoint's layout (Geom)
     int PL;         // partial vector length (doubles)
     int max_warps;  // widest CTA the kernel is compiled for
 };
@@ -93,17 +92,7 @@ inline cudaError_t ensure_smem_attr(const void* kernel, size_t bytes) {
     return e;
 }
 
-// Threads per transform group for a supported NZ (qlgpu_fft.cuh Geom), 0 if unsupported.
-inline int group_threads(int NZ) {
-    switch (NZ) {
-        case 16: return 4;
-        case 32: return 4;
-        case 64: return 8;
-        case 128: return 8;
-        case 256: return 16;
-        default: return 0;
-    }
-}
+inline bool supported_nz(int NZ) { return NZ == 16 || NZ == 32 || NZ == 64 || NZ == 128 || NZ == 256; }
 
 // Modes a team of the stage kernel steps at once and the teams of a CTA (qlgpu_wide.cuh WG).
 inline int block_modes(int NZ) { return 256 / NZ; }
@@ -164,7 +153,7 @@ inline int check_params(const qlgpu_params& p, std::string* msg) {
         *msg = "MHD_BQlin divides by nu (MHD_BQlin.cpp:251); nu must be nonzero";
         return QLGPU_ERR_ARG;
     }
-    if (group_threads(p.NZ) == 0) {
+    if (!supported_nz(p.NZ)) {
         *msg = "unsupported NZ: must be a power of two in [16, 256]";
         return QLGPU_ERR_UNSUPPORTED;
     }
@@ -235,24 +224,17 @@ inline void ktables(const qlgpu_params& p, std::vector<double>& kx, std::vector<
         }
 }
 
-// Twiddles of the transform layout: tw[n2*T + t] = exp(+2 pi i n2 t / NZ), as (re, im) pairs.
-inline std::vector<double> twiddles(int NZ, int T) {
+// Twiddles of the 8-points-per-thread transforms: tw[q T + t] = exp(+2 pi i q t / NZ), q < 8,
+// T = NZ / 8, as (re, im) pairs.
+inline std::vector<double> twiddles(int NZ) {
     std::vector<double> tw(2 * (size_t)NZ);
-    const int P = NZ / T;
-    for (int n2 = 0; n2 < P; ++n2)
+    const int T = NZ / 8;
+    for (int q = 0; q < 8; ++q)
         for (int t = 0; t < T; ++t) {
-            const int m = (n2 * t) % NZ;
-            const double ang = 2.0 * kPI * (double)m / (double)NZ;
-            tw[2 * (n2 * T + t)] = std::cos(ang);
-            tw[2 * (n2 * T + t) + 1] = std::sin(ang);
+            const double ang = 2.0 * kPI * (double)(q * t % NZ) / (double)NZ;
+            tw[2 * (q * T + t)] = std::cos(ang);
+            tw[2 * (q * T + t) + 1] = std::sin(ang);
         }
-    return tw;
-}
-// The table of a case: the adjoint's layout [P][T], then the 8-point layout [8][NZ/8].
-inline std::vector<double> stage_twiddles(int NZ) {
-    std::vector<double> tw = twiddles(NZ, group_threads(NZ));
-    const std::vector<double> t8 = twiddles(NZ, NZ / 8);
-    tw.insert(tw.end(), t8.begin(), t8.end());
     return tw;
 }
 // Diagnostics of a state in one launch (qlgpu_diag.cu): the 15-column record at time t into out.

@@ -49,7 +49,6 @@ Variant make_variant() {
     v.run_kernel[0] = &run_ptr<NZ, MODEL, INTEG, false>;
     v.run_kernel[1] = &run_ptr<NZ, MODEL, INTEG, true>;
     v.smem = &stage_smem<NZ, MODEL>;
-    v.T = Geom<NZ>::T;
     v.PL = wide::WG<NZ, MODEL>::PL;
     v.max_warps = wide::MAX_WARPS<MODEL>;
     return v;

@@ -130,7 +130,7 @@ __device__ __forceinline__ void mean_field_update(const StageArgs& A, const DevP
                                             : cadd(cscale(F[mm], S.n1), m[mm]);
                 nv = cscale(acc, e);
             } else {
-                nv = rk_update<INTEG_CN>(S, Lm, Lm, F[mm], fp, m[mm], S.has_prev);
+                nv = rk_update(S, Lm, Lm, F[mm], fp, m[mm], S.has_prev);
             }
             if (A.Fmf_out) stc(A.Fmf_out + mm * nzd + s, F[mm]);
             stc(mfo + mm * nzd + s, nv);

@@ -1,7 +1,8 @@
-// qlgpu_stage.cuh -- one fused RK3 stage of the quasi-linear shearing-box step
-// on sm_100a.
+// qlgpu_stage.cuh -- what the kernels of the quasi-linear shearing-box step share
+// (sm_100a): loads, wavenumbers, linear operators and the RK update.
 //
-// One launch = one stage of RK3CN_Elin::Step (QL_DNS/Integrators/
+// The fused RK3 stage (stage_body of qlgpu_wide.cuh, the chunks of qlgpu_ens.cuh)
+// is one stage of RK3CN_Elin::Step (QL_DNS/Integrators/
 // RK3CN_Elin.cpp:86-177) or RK3CN::Step (QL_DNS/Integrators/RK3CN.cpp:86-180)
 // for every (kx,ky) mode, fused with the model right-hand side
 // (MHD_BQlin::rhs, QL_DNS/Models/MHD_BQlin.cpp:117-284; MHD_FullQlin::rhs,
@@ -11,14 +12,10 @@
 // last stage the shearing-wave remap (MHD_BQlin.cpp:314-331) and the
 // energy / stress / dissipation diagnostics (MHD_BQlin.cpp:337-488).
 //
-// Work split: a group of T threads owns one mode at a time (qlgpu_fft.cuh).
-// Per-CTA partial sums go through a fixed-order two-level reduction; the CTA
-// that arrives last at the top performs the mean-field stage.  Everything is
-// FP64.
+// Everything is FP64.
 #pragma once
 #include "qlgpu_debug.cuh"
 #include "qlgpu_xform.cuh"
-#include "qlgpu_priv.cuh"
 #include "qlgpu_types.h"
 
 namespace qlgpu {
@@ -103,24 +100,16 @@ __device__ __forceinline__ double linop_f(const DevParams& P, double lap, int f)
     return MODEL == MODEL_BQLIN ? __dmul_rn(P.etanu, Lu) : __dmul_rn(P.eta, lap);
 }
 
-// RK update of one coefficient.  Elin: exp(linC L)(n1 F + n2 Fp + u)
-// (RK3CN_Elin.cpp:102-104).  CN: n1 d F + n2 d Fp + (1 + linC Lold) d u,
+// RK3CN update of one coefficient: n1 d F + n2 d Fp + (1 + linC Lold) d u,
 // d = 1/(1 - linC L) (RK3CN.cpp:105-107).
-template <int INTEG>
 __device__ __forceinline__ cplx rk_update(const StageConst& S, double L, double Lold, cplx F, cplx Fp, cplx u,
                                           bool has_prev) {
-    if (INTEG == INTEG_EXP) {
-        double e = exp(__dmul_rn(S.linC, L));
-        cplx acc = has_prev ? cadd(cadd(cscale(F, S.n1), cscale(Fp, S.n2)), u) : cadd(cscale(F, S.n1), u);
-        return cscale(acc, e);
-    } else {
-        double d = __drcp_rn(__dsub_rn(1.0, __dmul_rn(S.linC, L)));
-        double c1 = __dmul_rn(S.n1, d);
-        double c3 = __dmul_rn(__dadd_rn(1.0, __dmul_rn(S.linC, Lold)), d);
-        cplx r = cscale(F, c1);
-        if (has_prev) r = cadd(r, cscale(Fp, __dmul_rn(S.n2, d)));
-        return cadd(r, cscale(u, c3));
-    }
+    double d = __drcp_rn(__dsub_rn(1.0, __dmul_rn(S.linC, L)));
+    double c1 = __dmul_rn(S.n1, d);
+    double c3 = __dmul_rn(__dadd_rn(1.0, __dmul_rn(S.linC, Lold)), d);
+    cplx r = cscale(F, c1);
+    if (has_prev) r = cadd(r, cscale(Fp, __dmul_rn(S.n2, d)));
+    return cadd(r, cscale(u, c3));
 }
 
 // CN: where the previous stage's operator was evaluated (RK3CN.cpp:119-122)

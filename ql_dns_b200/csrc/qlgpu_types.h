@@ -130,7 +130,7 @@ struct StageArgs {
     const double* ky;
     const int* kxi;
     const int* kyi;
-    const cplx* tw;         // twiddles exp(2 pi i n2 t/NZ): [P][T] (Geom), then [8][NZ/8]
+    const cplx* tw;         // twiddles exp(2 pi i q t / NZ), [8][NZ/8]
     const double* ilap2;    // [Ny/2][nz] 1/lap2 table (Kdata.cpp:100-119)
     double* partials;       // [grid][PL]
     double* gpartials;      // [ngroups][PL]

@@ -288,7 +288,7 @@ struct Put {
         const double L = linop_f<MODEL>(P, lap_end<MODEL>(P, M.kxe, M.b, kz2), f);
         const double lo = cn.old_init ? lap_init<MODEL>(P, M.kxo, lap2val(M.b, kz2, z0))
                                       : lap_end<MODEL>(P, M.kxo, M.b, kz2);
-        return rk_update<INTEG_CN>(S, L, linop_f<MODEL>(P, lo, f), F, fpv, uin, fp != nullptr);
+        return rk_update(S, L, linop_f<MODEL>(P, lo, f), F, fpv, uin, fp != nullptr);
     }
     // store(s): F and the new value
     __device__ __forceinline__ void store(const StageArgs& A, const DevParams& P, const LaneMode& M, int s, double c,
@@ -754,7 +754,7 @@ __device__ __forceinline__ StageResult stage_body(const StageArgs& A, const DevP
     const bool cached = A.mfr_cache && !A.rhs_only && lc.mfr_valid;
     if (fresh)
         for (int i = tid; i < NZ; i += blockDim.x) {
-            tw[i] = ldc_cg(A.tw + NZ + i);
+            tw[i] = ldc_cg(A.tw + i);
             kzc[i] = kzval(i <= W::H ? i : i - NZ, P.kzL);
         }
     if (INTEG == INTEG_EXP) {
@@ -1279,7 +1279,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
         cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
         double* emf = reinterpret_cast<double*>(smem_raw + W::o_ekz);
         double* tot = reinterpret_cast<double*>(smem_raw + W::o_team);
-        for (int i = tid; i < NZ; i += blockDim.x) tw[i] = ldc_cg(L.A[0].tw + NZ + i);
+        for (int i = tid; i < NZ; i += blockDim.x) tw[i] = ldc_cg(L.A[0].tw + i);
         // wait by the first warp's lanes for the other reducers' `target` (lane: its reducer)
         auto wait_others = [&](unsigned target, int r) -> bool {
             return r >= NR || r == e || run_wait(C->epoch + 32 * r, target, C, L.wait_ns);
