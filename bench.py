@@ -444,7 +444,7 @@ def run_dns(args, local):
                         "flops_per_step": flops,
                         "kernels": "dns_inv_zx<64,64>, dns_phys<128>, dns_fwd_xz<64,64>, dns_update (x3 per step)"},
            "energy_at_end": {"t": rec[0], "E_u": rec[3], "E_b": rec[4], "E_By_mean": rec[2]},
-           "gpu_launches_per_step": 14}
+           "gpu_launches_per_step": 13}
     if not args.no_cpu_baseline:
         from oracle.dns_oracle import DNSOracle
         D = DNSOracle(p)
