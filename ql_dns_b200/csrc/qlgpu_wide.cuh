@@ -35,9 +35,13 @@
 // A CTA holds teams = max(1, warps / TS) teams (TS = 5 / 8: the forward tasks of
 // a model), each with its own named barrier and its own blocks.  Partial sums of
 // the stresses are lane-private in shared memory; per-CTA sums go through the
-// fixed-order two-level reduction and the CTA that arrives last runs the
-// mean-field stage, its loads issued before the sums are waited for and its
-// transforms on the same 8-point layout.
+// fixed-order two-level reduction to the mean-field stage (reducer CTAs in
+// run_kernel, else the CTA that arrives last), its loads issued before the sums
+// are waited for and its transforms on the same 8-point layout.
+//
+// Against the pairs of groups, per step inside qlgpu_step: 16x16 x NZ=32 140 us -> 29,
+// 64x64 x NZ=128 171 -> 85, 48x48 x NZ=64 of MHD_FullQlin 171 -> 43, 22x18 x NZ=256
+// 176 -> 41 (issue 29 % and 15 warps per SM at 64x64, where it was 20 % and 8).
 #pragma once
 #include "qlgpu_debug.cuh"
 #include "qlgpu_kernel.cuh"
@@ -1147,8 +1151,11 @@ __device__ __forceinline__ bool run_wait(const unsigned* p, unsigned target, Dev
 // The mean-field side of one stage in the reducer CTA of mean field `e`: the partial sums of
 // stress profile e over all `ncta` CTAs, in the order of the two-level reduction (CTAs within
 // a group of RED_GROUP, then the groups), then the field's part of the mean-field stage, the
-// result in mfo.  What bounds it is one SM's reading of the sums (8-byte loads, 32 a thread in
-// flight): 147 CTAs x NZ = 128 take 5.8 us for both profiles of MHD_BQlin, 3.8 us for one.
+// result in mfo.  What bounds it is one SM's reading of the sums, so 16-byte loads, 16 a thread
+// in flight (the guard is in the value: a guarded load makes the compiler wait for each before the
+// next, 30 % slower overall).  147 CTAs x NZ = 128 took 5.8 us for both profiles of MHD_BQlin and
+// 3.8 for one with 8-byte loads; 40 steps of 64x64 x NZ=128 3.47 -> 3.39 ms with these, 22x18 x
+// NZ=256 1.69 -> 1.63.
 template <int NZ, int MODEL, int INTEG, bool FORCED>
 __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams& P, int e, int ncta,
                                              unsigned char* smem_raw, const cplx* tw, const double* emf, LocalClock& lc,
@@ -1165,30 +1172,23 @@ __device__ __forceinline__ void reduce_stage(const StageArgs& A, const DevParams
     const int ngroups = (ncta + RED_GROUP - 1) / RED_GROUP;
     // columns [col, col + NC) of all rows
     auto sum = [&](auto nc_, int col) {
-        constexpr int NC = decltype(nc_)::value;
-        const double* p0 = A.partials + col;
-        for (int i0 = tid; i0 < ngroups * NC; i0 += 2 * nth) {
-            // two (group, value) pairs at a time, all their loads in flight
-            double v[2][RED_GROUP];
+        constexpr int NC = decltype(nc_)::value, C2 = NC / 2;
+        for (int i = tid; i < ngroups * C2; i += nth) {
+            // a (group, two values) item at a time, all its loads in flight
+            const int q = i / C2, n = min(RED_GROUP, ncta - q * RED_GROUP);
+            const double2* src = reinterpret_cast<const double2*>(A.partials + (size_t)q * RED_GROUP * W::PL + col) +
+                                 (i - q * C2);
+            double2 v[RED_GROUP], t = make_double2(0.0, 0.0);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int i = i0 + h * nth, q = i / NC, idx = i - q * NC;
-                const int n = i < ngroups * NC ? min(RED_GROUP, ncta - q * RED_GROUP) : 0;
-                const double* src = p0 + (size_t)q * RED_GROUP * W::PL + idx;
+            for (int u = 0; u < RED_GROUP; ++u)
+                v[u] = u < n ? __ldcg(src + (size_t)u * (W::PL / 2)) : make_double2(0.0, 0.0);
 #pragma unroll
-                for (int u = 0; u < RED_GROUP; ++u) v[h][u] = u < n ? __ldcg(src + (size_t)u * W::PL) : 0.0;
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int i = i0 + h * nth;
-                if (i >= ngroups * NC) break;
-                const int n = min(RED_GROUP, ncta - i / NC * RED_GROUP);
-                double s = 0.0;
-#pragma unroll
-                for (int u = 0; u < RED_GROUP; ++u)
-                    if (u < n) s += v[h][u];
-                gs[i] = s;
-            }
+            for (int u = 0; u < RED_GROUP; ++u)
+                if (u < n) {
+                    t.x += v[u].x;
+                    t.y += v[u].y;
+                }
+            reinterpret_cast<double2*>(gs)[i] = t;
         }
         __syncthreads();
         for (int idx = tid; idx < NC; idx += nth) {
