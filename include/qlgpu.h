@@ -137,8 +137,9 @@ int qlgpu_status(qlgpu_t* h, int* status);
 
 /* Profiling aid: with QLGPU_TRACE=1 in the environment at qlgpu_create, each
  * stage kernel records %globaltimer stamps (ns) of its phases; out96 receives
- * 3 stages x 32 slots of the most recent step (slot meanings are listed in
- * ql_dns_b200/csrc/qlgpu_kernel.cuh).  Returns QLGPU_ERR_UNSUPPORTED when off. */
+ * 3 stages x 32 slots of the most recent step (CTA 0: 0 start, 1 tables, 6 gate
+ * passed, 7 profiles, 2 blocks done, 3 sums published; mean-field side: 4 sums
+ * read, 5 done).  Returns QLGPU_ERR_UNSUPPORTED when off. */
 int qlgpu_trace(qlgpu_t* h, unsigned long long* out96);
 
 /* Launch geometry of the stage kernel: info8 = {grid, block, dynamic shared
