@@ -422,6 +422,9 @@ int adj_finish(AdjJob& j, double* grad_lin, double* grad_mf) {
     QA_CK(cudaMemcpyAsync(h->d_mf, j.fin_mf, j.nmfe * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
     QA_CK(cudaMemcpyAsync(h->d_kx0, j.fin_kx0, j.nxy * sizeof(double), cudaMemcpyDeviceToDevice, st));
     QA_CK(cudaMemcpyAsync(h->d_clk, j.fin_clk, sizeof(DevClock), cudaMemcpyDeviceToDevice, st));
+    // the handle's mean-field profile cache is of the last recompute (or, where the forward sweep ran in
+    // the batch, of an earlier run): the next step forms the profiles from the restored mean field
+    QA_CK(cudaMemsetAsync(&h->d_clk->mfr_valid, 0, sizeof(int), st));
     return QLGPU_OK;
 }
 

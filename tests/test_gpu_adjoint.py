@@ -271,3 +271,33 @@ def test_crank_nicolson_batch_of_seeds_against_tangent_linear():
         for d in directions(sts[k][0].shape, 2, 70 + k, np.linalg.norm(sts[k][0])):
             _, dJ = O.tlm_maxwell(p, 0.0, *sts[k], d, None, n)
             assert abs(float(np.real(np.vdot(gl[k], d))) - dJ) <= 1e-8 * abs(dJ)
+
+
+@pytest.mark.parametrize("integ", [0, 1])
+@pytest.mark.parametrize("mode", ["single", "persistent", "streams"])
+def test_steps_after_the_adjoint_continue_the_forward_run(mode, integ, monkeypatch):
+    """The handle is left at the end of the forward run: stepping on from there is the run itself,
+    to the 1e-10 bar of a step, whatever the recomputed windows left in the handle's caches."""
+    require_gpu()
+    if mode == "streams":
+        monkeypatch.setenv("QLGPU_ADJ_BATCH", "streams")
+    p = mri_16x16_nz32(nx=8, ny=8, NZ=32, integrator=integ)
+    sts = [initial_state(p, 30 + k, sigma=0.2) for k in range(1 if mode == "single" else 2)]
+    n, ck, more = 18, 5, 2
+    ss = [QLSolver(p) for _ in sts]
+    try:
+        if mode == "single":
+            ss[0].adjoint_maxwell(0.0, *sts[0], n, ck)
+        else:
+            QLSolver.adjoint_maxwell_batch(ss, 0.0, *zip(*sts), n, ck)
+        for s, (lin, mf, kx0) in zip(ss, sts):
+            rec = s.step(more, diag_every=1)
+            t, lo, mo, ko = s.get_state()
+            t2, lo2, mo2, ko2, d2 = O.run(p, 0.0, lin, mf, kx0, n + more, diag_every=1)
+            assert abs(t - t2) < 1e-12 and np.array_equal(ko, ko2)
+            assert rel(lo, lo2) < 1e-10 and rel(mo, mo2) < 1e-10
+            scale = np.abs(d2[1:, 1:13]).max(0)
+            assert np.all(np.abs(rec[:, 1:13] - d2[-more:, 1:13]) <= 1e-10 * scale)
+    finally:
+        for s in ss:
+            s.close()
