@@ -59,7 +59,7 @@ __device__ __forceinline__ void step_record(const StageArgs& A, const DevParams&
     if (r < A.diag_cap)
         put_record(P, ds, v, t_new, A.diag_ring + (size_t)QLGPU_CHECK_INDEX(r, A.diag_cap, &C->status) * 15);
     else
-        C->status |= QLGPU_STATUS_DIAG_FULL;
+        atomicOr(&C->status, QLGPU_STATUS_DIAG_FULL);  // other CTAs of the launch set bits of the same word
     C->ndiag = r + 1;
     C->timevar = __dsub_rn(C->timevar, P.tv_interval);
     C->since = 0;

@@ -6,11 +6,14 @@ two teams per CTA and several blocks per team.  Tolerance against the oracle: th
 the step (relative L2 of the state).  One launch of n steps and n launches of one step run the
 same kernel on the same sums, so their states agree bit for bit.
 """
+import ctypes
+
 import numpy as np
 import pytest
 
 from gpu_util import rel, require_gpu
 from oracle import oracle as O
+from ql_dns_b200 import _capi
 from ql_dns_b200.batch import QLBatch
 from ql_dns_b200.initial import initial_state
 from ql_dns_b200.params import QLParams
@@ -113,3 +116,17 @@ def test_forced_across_launches():
             out.append(s.get_state() + (s.mean_time_step(), rec[-1]))
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("model", [0, 1])
+def test_status_keeps_the_bits_of_every_cta(model):
+    """The first reducer drops records (4) while the others see a non-finite field (1), in the same launch."""
+    require_gpu()
+    p = QLParams(model=model, nx=8, ny=8, NZ=16, dt=0.02)
+    lin, mf, kx0 = initial_state(p, 3, sigma=0.02, B0=0.2)
+    mf[1, 1] = np.nan
+    out, n = np.zeros((2, 15)), ctypes.c_int()
+    with QLSolver(p) as s:
+        s.set_state(0.0, lin, mf, kx0)
+        assert s.L.qlgpu_step(s.h, 6, 1, _capi.dptr(out), 2, ctypes.byref(n)) == 4
+        assert n.value == 2 and s.status() == 5
