@@ -132,8 +132,23 @@ int qlgpu_rhs_noalloc(const qlgpu_params* p, double t, double dt_lin, const void
 
 /* Device status word (solution::Check_Solution, QL_DNS/solution.cpp:169-203):
  * bit 1 non-finite mean field, bit 2 |mean field| > 1e20, bit 4 diagnostic
- * records dropped.  Reading does not clear it; set_state clears it. */
+ * records dropped, bit 8 a wait inside a launch gave up (qlgpu_set_wait).
+ * Reading does not clear it; set_state clears it. */
 int qlgpu_status(qlgpu_t* h, int* status);
+
+/* qlgpu_step and the adjoint's forward run step a case in one cooperative
+ * launch per 256 steps, whose CTAs wait for each other's part of the mean
+ * field.  This bounds one such wait (default 2 s; 0 < seconds <= 60).  It does
+ * not run while the launch itself is held up by other work on the GPU: its
+ * CTAs start together.  After a wait that gave up the call returns
+ * QLGPU_ERR_STATUS, the status word has bit 8, and the state is lost: the
+ * handle is usable again after set_state. */
+int qlgpu_set_wait(qlgpu_t* h, double seconds);
+
+/* Failure-detection test aid: in the launch-th such launch from now (1: the
+ * next) one CTA's first count is missing, so that the others wait for a mean
+ * field that never completes.  0 takes it back. */
+int qlgpu_debug_drop_arrival(qlgpu_t* h, int launch);
 
 /* Profiling aid: with QLGPU_TRACE=1 in the environment at qlgpu_create, each
  * stage kernel records %globaltimer stamps (ns) of its phases; out96 receives

@@ -131,7 +131,7 @@ cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec, const Run
     R.mf_alt = h->d_mf_alt;
     R.cur = h->cur;
     R.nsteps = n;
-    R.wait_ns = 2000000000LL;
+    R.wait_ns = h->wait_ns;
     if (rec) {
         R.rec_lin = rec->lin;
         R.rec_mf = rec->mf;
@@ -150,6 +150,11 @@ cudaError_t qlgpu_enqueue_run(qlgpu_t* h, int n, const RunRecord* rec, const Run
         R.diag_every = force->diag_every;
         R.diag_step0 = force->diag_step0;
         R.diag_max = force->diag_max;
+    }
+    if (h->drop_arrival > 0 && --h->drop_arrival == 0) {
+        // counters of -1: the first stage's last count is missing
+        const cudaError_t d = cudaMemsetAsync(h->d_clk->arrive, 0xff, sizeof(h->d_clk->arrive), h->stream);
+        if (d != cudaSuccess) return d;
     }
     const cudaError_t e = h->var.run[force != nullptr](R, h->grid + h->nmf, h->block, h->smem, h->stream);
     if (e == cudaSuccess) h->cur ^= n & 1;  // three stages per step
@@ -569,6 +574,20 @@ int qlgpu_set_cfl(qlgpu_t* h, double cfl, double dt_max) {
 int qlgpu_mean_time_step(qlgpu_t* h, double* dt_mean) {
     if (!h || !dt_mean) return QLGPU_ERR_ARG;
     *dt_mean = h->steps_taken ? h->dt_sum / (double)h->steps_taken : h->p.dt;
+    return QLGPU_OK;
+}
+
+int qlgpu_set_wait(qlgpu_t* h, double seconds) {
+    if (!h) return QLGPU_ERR_ARG;
+    if (!(seconds > 0) || seconds > 60) return fail(h, QLGPU_ERR_ARG, "wait bound: 0 < seconds <= 60");
+    h->wait_ns = (long long)(seconds * 1e9);
+    return QLGPU_OK;
+}
+
+int qlgpu_debug_drop_arrival(qlgpu_t* h, int launch) {
+    if (!h) return QLGPU_ERR_ARG;
+    if (launch < 0) return fail(h, QLGPU_ERR_ARG, "drop arrival: launch >= 1, or 0 for none");
+    h->drop_arrival = launch;
     return QLGPU_OK;
 }
 

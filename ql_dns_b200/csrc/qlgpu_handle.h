@@ -70,6 +70,8 @@ struct qlgpu_handle {
     int adj_tab_cap = 0;
     qlgpu_batch_t* adj_batch = nullptr;  // of the last qlgpu_adjoint_maxwell_batch whose first handle this is
     std::vector<qlgpu_params> adj_batch_ps;
+    long long wait_ns = 2000000000LL;  // RunArgs::wait_ns
+    int drop_arrival = 0;              // failure-detection aid: launches until one starts a count short
     // pinned block through which small states cross to and from host arrays, and the clock
     unsigned char* h_pin = nullptr;
     size_t pin_bytes = 0;

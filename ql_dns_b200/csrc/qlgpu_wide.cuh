@@ -639,10 +639,11 @@ __device__ __forceinline__ void side_diag(const DevParams& P, const LaneMode& M,
 
 }  // namespace wide
 
-// Static shared words of a stage: the last-arriver flag and the gate's answer.
+// Static shared words of a stage: the last-arriver flag, the gate's answer and, in a reducer of
+// run_kernel, that of its wait for the workers (a word of its own: slower warps may still read the other).
 struct StageShared {
     int last, ok;
-    int pad[2];
+    int arrived, pad;
 };
 
 // A case's clock as this CTA follows it through a launch: every CTA advances its own
@@ -1130,14 +1131,14 @@ __device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
 }
 __device__ __forceinline__ int ld_volatile_i32(const int* p) { return *reinterpret_cast<const volatile int*>(p); }
 
-// Wait (one thread) until *p >= target.  False when the launch was aborted or the wait
+// Wait (one thread) until *p has reached target.  False when the launch was aborted or the wait
 // exceeded wait_ns; the caller's CTA then leaves, and the abort word makes the others leave.
 __device__ __forceinline__ bool run_wait(const unsigned* p, unsigned target, DevClock* C, long long wait_ns) {
     const unsigned long long t0 = gtimer();
     // at least ~16 ns per iteration: the cap ends the wait even if the timer misbehaves
     const long long max_iter = wait_ns / 16 + 1024;
     for (long long it = 0; it < max_iter; ++it) {
-        if (ld_acquire_u32(p) >= target) return true;
+        if ((int)(ld_acquire_u32(p) - target) >= 0) return true;
         if ((it & 63) == 63) {
             if (ld_volatile_i32(&C->abort)) return false;
             if ((long long)(gtimer() - t0) > wait_ns) break;
@@ -1260,6 +1261,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
         reinterpret_cast<unsigned long long*>(sA)[i] = reinterpret_cast<const unsigned long long*>(L.A)[i];
     if (tid == 0) {
         load_clock(lc, C);
+        ss.ok = __ldcg(&C->abort) == 0;
         if (FORCED) {
             lc.every = L.diag_every;
             lc.step = L.diag_step0;
@@ -1268,6 +1270,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
         }
     }
     __syncthreads();
+    if (!ss.ok) return;  // the launch before gave up: its state and counters are no start
     const size_t nlin = (size_t)L.P.nxy * 4 * L.P.nz, nmfe = (size_t)L.P.nmf * L.P.nz;
     const unsigned nstages = 3u * (unsigned)L.nsteps;
     // the mean fields at the start of stage k of the launch
@@ -1319,7 +1322,7 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
                 if (!ss.ok) return;
                 wide::top_prefetch<W>(sA[s], tot);
                 if (tid == 0)
-                    ss.ok = run_wait(C->arrive + 32 * e, (k + 1) * (unsigned)ncta, C, L.wait_ns) ? 1 : 0;
+                    ss.arrived = run_wait(C->arrive + 32 * e, (k + 1) * (unsigned)ncta, C, L.wait_ns) ? 1 : 0;
                 if (INTEG == INTEG_EXP)  // under the wait (the last threads: the first one polls)
                     for (int i = blockDim.x - 1 - tid; i < W::nz; i += blockDim.x) {
                         const double kz2 = kz2val(kzval(i <= W::H ? i : i - W::nz, L.P.kzL));
@@ -1328,7 +1331,10 @@ __global__ void __launch_bounds__(32 * wide::MAX_WARPS<MODEL>, 1) run_kernel(con
                         emf[W::NZE + i] = L.P.ql ? exp(__dmul_rn(lc_, __dmul_rn(L.P.nu, kz2))) : 1.0;
                     }
                 __syncthreads();
-                if (!ss.ok) return;
+                if (!ss.arrived) {
+                    cp_async_wait_all();
+                    return;
+                }
                 const bool rec = e == 0 && record_due<FORCED>(lc, L.P, FORCED ? sA[s].sc.dt : L.P.dt, s == 2);
                 reduce_stage<NZ, MODEL, INTEG, FORCED>(sA[s], L.P, e, ncta, smem_raw, tw,
                                                        INTEG == INTEG_EXP ? emf : nullptr, lc, cfl ? s_mx : nullptr,

@@ -117,6 +117,14 @@ class QLSolver:
         _capi.check(self.L.qlgpu_mean_time_step(self.h, ctypes.byref(v)), self.h)
         return v.value
 
+    def set_wait(self, seconds: float):
+        """Bound on one wait inside a launch of many steps (qlgpu_set_wait)."""
+        _capi.check(self.L.qlgpu_set_wait(self.h, float(seconds)), self.h)
+
+    def debug_drop_arrival(self, launch: int = 1):
+        """Failure-detection test aid (qlgpu_debug_drop_arrival)."""
+        _capi.check(self.L.qlgpu_debug_drop_arrival(self.h, int(launch)), self.h)
+
     def step_timed(self) -> np.ndarray:
         """One step; returns the device time (ms) of each of its three stage kernels."""
         ms = (ctypes.c_float * 3)()

@@ -7,6 +7,8 @@ the step (relative L2 of the state).  One launch of n steps and n launches of on
 same kernel on the same sums, so their states agree bit for bit.
 """
 import ctypes
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -130,3 +132,77 @@ def test_status_keeps_the_bits_of_every_cta(model):
         s.set_state(0.0, lin, mf, kx0)
         assert s.L.qlgpu_step(s.h, 6, 1, _capi.dptr(out), 2, ctypes.byref(n)) == 4
         assert n.value == 2 and s.status() == 5
+
+
+def run_state(s, st, n, forced):
+    s.set_noise(0.02 if forced else 0.0, 0.5, 50.0, 7)
+    s.set_cfl(0.3 if forced else 0.0, 0.05 if forced else 0.0)
+    s.set_state(0.0, *st)
+    rec = s.step(n, diag_every=2)
+    return s.get_state() + (rec,)
+
+
+@pytest.mark.parametrize("forced", [False, True])
+@pytest.mark.parametrize("model,nx,ny,NZ,launch", [(0, 8, 8, 16, 1), (0, 8, 8, 16, 2), (0, 32, 40, 128, 1), (1, 36, 34, 64, 1)])
+def test_wait_bound_reports_timeout(model, nx, ny, NZ, launch, forced):
+    """A count that never comes: the bounded waits end the launch (and those after it) with a status, and
+    the handle is as good as new once a state is set."""
+    require_gpu()
+    p = QLParams(model=model, nx=nx, ny=ny, NZ=NZ, dt=0.02, B0z=0.02 if model else 0.0)
+    st = initial_state(p, 3, sigma=0.02, B0=0.2, mean_u=0.05 if model else 0.0)
+    n = 6 if launch == 1 else 260  # 256 steps a launch
+    with QLSolver(p) as s:
+        good = run_state(s, st, n, forced)
+    with QLSolver(p) as s:
+        s.set_wait(0.2)
+        s.debug_drop_arrival(launch)
+        with pytest.raises(_capi.QLGPUError) as ei:
+            run_state(s, st, n, forced)
+        assert ei.value.code == 4 and "gave up" in str(ei.value)
+        assert s.status() & 8
+        for a, b in zip(run_state(s, st, n, forced), good):
+            assert np.array_equal(a, b)
+        assert s.status() == 0
+
+
+# eighteen steps, a checkpoint every five: four forward launches, then three recomputes
+@pytest.mark.parametrize("launch", [1, 4, 5, 7])
+def test_adjoint_wait_bound_reports_timeout(launch):
+    require_gpu()
+    p = QLParams(nx=8, ny=8, NZ=32, dt=0.02)
+    st = initial_state(p, 3, sigma=0.2)
+    with QLSolver(p) as s:
+        good = s.adjoint_maxwell(0.0, *st, 18, 5)
+    with QLSolver(p) as s:
+        s.set_wait(0.2)
+        s.debug_drop_arrival(launch)
+        with pytest.raises(_capi.QLGPUError) as ei:
+            s.adjoint_maxwell(0.0, *st, 18, 5)
+        assert ei.value.code == 4 and "gave up" in str(ei.value)
+        for a, b in zip(s.adjoint_maxwell(0.0, *st, 18, 5), good):
+            assert np.array_equal(a, b)
+
+
+def test_wait_bound_does_not_run_before_the_launch_does():
+    """Another stream's launch holds most SMs for far longer than the bound: the step waits its turn."""
+    require_gpu()
+    p = QLParams(nx=64, ny=64, NZ=128, dt=0.005)
+    st = initial_state(p, 1)
+    q = QLParams(nx=8, ny=8, NZ=128, dt=1e-4)
+    with QLSolver(p) as s, QLBatch([q] * 100) as b:
+        good = run_state(s, st, 4, False)
+        b.set_mapping(15, [1] * 100)  # a CTA, and so an SM, for each case
+        for c in range(100):
+            b.set_state(c, 0.0, *initial_state(q, 1))
+        steps = int(1500.0 / (b.step_timed(100) / 100))  # 1.5 s
+        s.set_wait(0.1)
+        s.set_state(0.0, *st)
+        th = threading.Thread(target=b.step, args=(steps,))
+        th.start()
+        time.sleep(0.3)
+        t0 = time.time()
+        rec = s.step(4, diag_every=2)
+        assert time.time() - t0 > 0.2, "the step was not held up"
+        th.join()
+        for a, c in zip(s.get_state() + (rec,), good):
+            assert np.array_equal(a, c)
