@@ -382,8 +382,8 @@ int qlgpu_batch_engine(const qlgpu_batch_t* b, int* engine);
  * active. */
 int qlgpu_batch_set_chunks(qlgpu_batch_t* b, const int* passes4);
 /* The current passes per chunk of the four NZ classes: after qlgpu_batch_tune the
- * tuned ones; before, 4 per class, or fewer where 4 would leave SMs without a chunk
- * (a small batch). */
+ * tuned ones; before, at most 4, the same for every class: as many as a model of the
+ * stage time (work per SM against the longest chain of a case) puts first. */
 int qlgpu_batch_chunks(const qlgpu_batch_t* b, int* passes4);
 
 /* Profiling aid of the queue engine (QLGPU_TRACE=1 in the environment at

@@ -498,28 +498,41 @@ constexpr int QTRACE_MAX_CTAS_PER_SM = 4;  // bound of the queue grid: at most t
 int ens_class(int NZ) { return NZ == 16 ? 0 : NZ == 32 ? 1 : NZ == 64 ? 2 : 3; }
 size_t tw8_offset(int NZ) { return NZ == 16 ? 0 : NZ == 32 ? 16 : NZ == 64 ? 48 : 112; }  // cplx
 
+// Passes per chunk of a case that asks for `passes`, raised until its partial-sum slots hold every
+// chunk; *nch receives its chunks per stage.
+int case_passes(const CaseHost& h, int passes, int* nch) {
+    for (;; ++passes) {
+        const int mpc = passes * ens::modes_per_pass(h.NZ);
+        *nch = (h.nxy + mpc - 1) / mpc;
+        if (*nch <= h.max_cta) return passes;
+    }
+}
+
 // Default CTA passes per chunk, before any tuning.  A chunk costs about 12 us besides its
-// passes of about 13.3 us (the same at every NZ by the choice of modes per pass), so long
-// chunks cost less work W per CTA and stage; but a stage of a case takes at least its longest
-// chunk and the mean-field stage, about 8 us, and where that chain is no longer short against
-// W, CTAs wait.  The stage time (W^5 + chain^5)^(1/5) follows the measurements (24 cases: 0.322,
-// 0.305, 0.351 ms a step at 3, 4, 6 passes; 12 cases: 0.297, 0.275, 0.301 at 2, 3, 4; 6 cases: 0.145,
-// 0.142, 0.180 at 1, 2, 3; 16 cases of 32x32 x NZ=64: 0.155, 0.134, 0.166 at 1, 2, 3), so the
-// passes that minimise it are taken, at most four.  Batches of 30 cases and more gain
+// passes of about 13.3 us (the same at every NZ by the choice of modes per pass; 10.2 us since the
+// next chunk is read ahead, which moves none of the choices below), so long chunks cost less work W
+// per CTA and stage; but a stage of a case takes at least the waves of its chunks over the SMs and the
+// mean-field stage, about 8 us, and where that chain is no longer short against W, CTAs wait.  The
+// stage time (W^5 + chain^5)^(1/5) follows the measurements (24 cases: 0.322, 0.305, 0.351 ms a step at
+// 3, 4, 6 passes; 12 cases: 0.297, 0.275, 0.301 at 2, 3, 4; 6 cases: 0.145, 0.142, 0.180 at 1, 2, 3; 16 cases of
+// 32x32 x NZ=64: 0.155, 0.134, 0.166 at 1, 2, 3; one case of 64x64 x NZ=128, 168 passes for 148 SMs:
+// 0.155, 0.132, 0.169 at 1, 2, 3, of 128x128 x NZ=64, 339 passes: 0.241, 0.241, 0.176, 0.215 at 1 to 4), so
+// the passes that minimise it are taken, at most four.  Batches of 30 cases and more gain
 // another 7 % from eight (48 cases: 0.626 -> 0.582), which qlgpu_batch_tune finds.
 void default_passes(qlgpu_batch_t* b) {
     constexpr double PASS_US = 13.3, CHUNK_US = 12.0, TOP_US = 8.0;
     double best = 1e300;
     for (int p = 1; p <= 4; ++p) {
-        double work = 0.0;
-        int longest = 0;
+        double work = 0.0, chain = 0.0;
         for (const CaseHost& h : b->cs) {
             const int mpp = ens::modes_per_pass(h.NZ), need = (h.nxy + mpp - 1) / mpp;
-            work += need * PASS_US + (need + p - 1) / p * CHUNK_US;
-            longest = std::max(longest, std::min(p, need));
+            int nch = 0;
+            const int pc = case_passes(h, p, &nch);
+            work += need * PASS_US + nch * CHUNK_US;
+            const int waves = (nch + b->sms - 1) / b->sms;
+            chain = std::max(chain, waves * (std::min(pc, need) * PASS_US + CHUNK_US) + TOP_US);
         }
         work /= b->sms;
-        const double chain = longest * PASS_US + CHUNK_US + TOP_US;
         const double est = std::pow(std::pow(work, 5) + std::pow(chain, 5), 0.2);
         if (est < best - 1e-9) {
             best = est;
@@ -547,15 +560,9 @@ int queue_plan(qlgpu_batch_t* b) {
     size_t smem = 0;
     for (int c = 0; c < nc; ++c) {
         const CaseHost& h = b->cs[c];
-        const int mpp = ens::modes_per_pass(h.NZ);
-        int passes = std::max(1, b->qpasses[ens_class(h.NZ)]);
-        int nch = 0, mpc = 0;
-        for (;;) {
-            mpc = passes * mpp;
-            nch = (h.nxy + mpc - 1) / mpc;
-            if (nch <= h.max_cta) break;
-            ++passes;
-        }
+        int nch = 0;
+        const int passes = case_passes(h, std::max(1, b->qpasses[ens_class(h.NZ)]), &nch);
+        const int mpc = passes * ens::modes_per_pass(h.NZ);
         ens::EnsCase& e = b->ec[c];
         std::memset(&e, 0, sizeof(e));
         e.NZ = h.NZ;

@@ -434,3 +434,14 @@ def test_default_chunk_passes_give_every_sm_a_chunk():
     with QLBatch(cases) as b:
         b.set_engine("queue")
         assert all(v == 4 for v in b.mapping()["chunk_passes"].values())
+
+
+@pytest.mark.parametrize("n,NZ", [(64, 128), (80, 128), (96, 128), (128, 64)])
+def test_default_chunk_passes_of_one_large_case_are_one_wave(n, NZ):
+    # a single case's chunks beyond the SM count make every stage wait for a second, nearly empty wave
+    require_gpu()
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    with QLBatch([QLParams(nx=n, ny=n, NZ=NZ, dt=0.002)]) as b:
+        m = b.mapping()
+        assert m["ncta"][0] <= sms, m
