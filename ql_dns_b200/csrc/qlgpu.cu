@@ -385,9 +385,10 @@ int qlgpu_dims(const qlgpu_t* h, int* nxy, int* nlin, int* nz, int* nmf) {
     return QLGPU_OK;
 }
 
-// Host arrays of a small state cross through one pinned block: four copies from or to pageable
-// memory each wait for the device (get_state of 16x16 x NZ=32 100 us, through the block 40 us).
-// Larger ones go directly, in the driver's own pieces.
+// A small state comes back to host arrays through one pinned block: each of four copies to pageable
+// memory waits for the device (get_state of 16x16 x NZ=32 100 us, through the block 40 us).
+// Larger ones come directly, in the driver's own pieces, and so does every state on its way in: copies
+// from pageable memory do not wait, and a detour through the block costs 3 us of 32.
 constexpr size_t PIN_MAX = (size_t)1 << 20;
 
 static size_t state_bytes(const qlgpu_t* h) {
@@ -412,22 +413,10 @@ static int set_state_impl(qlgpu_t* h, double t, const void* lin, const void* mf,
     const size_t nl = (size_t)h->nxy * 4 * h->nz * sizeof(cplx), nm = (size_t)h->nmf * h->nz * sizeof(cplx),
                  nk = h->nxy * sizeof(double);
     h->cur = 0;
-    if (!kx0) kx0 = h->kx_tab.data();
-    else if (k == cudaMemcpyDeviceToDevice) {
-        QLGPU_CK(cudaMemcpyAsync(h->d_kx0, kx0, nk, k, h->stream));
-        kx0 = nullptr;  // done
-    }
-    if (k == cudaMemcpyHostToDevice && pinned(h)) {
-        std::memcpy(h->h_pin, lin, nl);
-        std::memcpy(h->h_pin + nl, mf, nm);
-        std::memcpy(h->h_pin + nl + nm, kx0, nk);
-        lin = h->h_pin;
-        mf = h->h_pin + nl;
-        kx0 = h->h_pin + nl + nm;
-    }
     QLGPU_CK(cudaMemcpyAsync(h->d_lin[0], lin, nl, k, h->stream));
     QLGPU_CK(cudaMemcpyAsync(h->d_mf, mf, nm, k, h->stream));
-    if (kx0) QLGPU_CK(cudaMemcpyAsync(h->d_kx0, kx0, nk, cudaMemcpyHostToDevice, h->stream));
+    if (kx0) QLGPU_CK(cudaMemcpyAsync(h->d_kx0, kx0, nk, k, h->stream));
+    else QLGPU_CK(cudaMemcpyAsync(h->d_kx0, h->kx_tab.data(), nk, cudaMemcpyHostToDevice, h->stream));
     int rc = reset_clock(h, t);
     if (rc) return rc;
     // the integrator and model start afresh: no steps, zero mean-field profiles of a previous rhs

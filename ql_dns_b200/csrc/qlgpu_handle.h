@@ -72,7 +72,7 @@ struct qlgpu_handle {
     std::vector<qlgpu_params> adj_batch_ps;
     long long wait_ns = 2000000000LL;  // RunArgs::wait_ns
     int drop_arrival = 0;              // failure-detection aid: launches until one starts a count short
-    // pinned block through which small states cross to and from host arrays, and the clock
+    // pinned block through which a small state comes back to host arrays, and the clock of a step
     unsigned char* h_pin = nullptr;
     size_t pin_bytes = 0;
 };
