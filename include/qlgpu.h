@@ -232,7 +232,10 @@ int qlgpu_fp64_peak(int device, double* tflops);
  * one checkpoint window at a time.  Returns J, grad_lin = dJ/d lin0 (complex
  * [nxy][4][nz]: dJ = Re sum conj(grad_lin) d lin0, i.e. the derivatives with
  * respect to the real and imaginary parts) and, when grad_mf is not NULL,
- * dJ/d mf0 likewise.  The handle is left at the end of the forward run. */
+ * dJ/d mf0 likewise.  The handle is left at the end of the forward run.
+ * Device memory: the checkpoints and one window's records.  Up to 512 MiB of
+ * it stays with the handle for its next call; a larger workspace is freed at
+ * the end of the call. */
 int qlgpu_adjoint_maxwell(qlgpu_t* h, double t0, const double* lin0, const double* mf0, const double* kx0,
                           int nsteps, int checkpoint_every, double* J, double* grad_lin, double* grad_mf);
 
@@ -245,10 +248,17 @@ int qlgpu_adjoint_maxwell(qlgpu_t* h, double t0, const double* lin0, const doubl
  * NULL; J [nseeds], grad_lin / grad_mf like lin0 / mf0.  Each seed's results
  * equal those of qlgpu_adjoint_maxwell on its handle to round-off (the batch
  * kernel sums in another order); with the environment variable
- * QLGPU_ADJ_BATCH=streams every seed runs the single-case path, bit for bit. */
+ * QLGPU_ADJ_BATCH=streams every seed runs the single-case path, bit for bit.
+ * Device memory that stays for the next call: up to 512 MiB with EACH seed's
+ * handle, and with the first one the batch, if its fields take at most
+ * 512 MiB. */
 int qlgpu_adjoint_maxwell_batch(qlgpu_t* const* handles, int nseeds, double t0, const double* lin0,
                                 const double* mf0, const double* kx0, int nsteps, int checkpoint_every, double* J,
                                 double* grad_lin, double* grad_mf);
+
+/* Gives back the device memory that the adjoint calls keep with the handle
+ * (qlgpu_destroy does so too).  The next adjoint call allocates it anew. */
+int qlgpu_adjoint_release(qlgpu_t* h);
 
 /* ------------------------------------------------------------------------
  * Batched ensemble.  No counterpart in the reference, which runs one case per

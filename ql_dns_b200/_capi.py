@@ -43,7 +43,8 @@ EXPORTS = ["qlgpu_create", "qlgpu_destroy", "qlgpu_dims", "qlgpu_set_state", "ql
            "qlgpu_dns_step_timed", "qlgpu_dns_stream", "qlgpu_fp64_peak",
            "qlgpu_set_noise", "qlgpu_set_cfl", "qlgpu_mean_time_step", "qlgpu_adjoint_maxwell_batch",
            "qlgpu_batch_cost_model", "qlgpu_set_noise_fields", "qlgpu_batch_set_noise", "qlgpu_debug_build",
-           "qlgpu_debug_guard_poke", "qlgpu_batch_debug_guard_poke", "qlgpu_set_wait", "qlgpu_debug_drop_arrival"]
+           "qlgpu_debug_guard_poke", "qlgpu_batch_debug_guard_poke", "qlgpu_set_wait", "qlgpu_debug_drop_arrival",
+           "qlgpu_adjoint_release"]
 
 
 class qlgpu_params(ctypes.Structure):
@@ -172,6 +173,7 @@ def load(path: str | None = None):
     L.qlgpu_batch_debug_guard_poke.argtypes = [vp, ctypes.c_int]
     L.qlgpu_batch_set_noise.argtypes = [vp, ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                         ctypes.c_ulonglong, ctypes.c_int, ctypes.c_int]
+    L.qlgpu_adjoint_release.argtypes = [vp]
     L.qlgpu_set_wait.argtypes = [vp, ctypes.c_double]
     L.qlgpu_debug_drop_arrival.argtypes = [vp, ctypes.c_int]
     L.qlgpu_set_cfl.argtypes = [vp, ctypes.c_double, ctypes.c_double]

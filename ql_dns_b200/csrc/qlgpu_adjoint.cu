@@ -95,9 +95,10 @@ static_assert(offsetof(DevClock, dtlin_old) == offsetof(DevClock, t_old) + 8 &&
 
 // The workspace of a handle's adjoint calls: one device block as large as the checkpoints and
 // one window's records ask for, cut into the call's buffers in two passes, sizes first.  A
-// block of at most ADJ_KEEP_BYTES stays with the handle for its next call and is freed with
-// it (25 allocations, clears and frees per seed and call took more than half of a 100-step
-// call of 16 seeds); a larger one is given back at the end of the call.
+// block of at most ADJ_KEEP_BYTES stays with its handle (every seed's has one) for the next call,
+// until qlgpu_adjoint_release or the handle's end (25 allocations, clears and frees per seed and
+// call took more than half of a 100-step call of 16 seeds); a larger one is given back at the end
+// of the call.
 constexpr size_t ADJ_KEEP_BYTES = (size_t)512 << 20;
 
 void adj_trim(qlgpu_t* h) {
@@ -779,6 +780,21 @@ extern "C" int qlgpu_adjoint_maxwell(qlgpu_t* h, double t0, const double* lin0, 
     if (!rc) rc = run_jobs(jobs, J, gl, grad_mf ? gm : nullptr);
     adj_trim(h);
     return rc ? rc : qlgpu_debug_verify(h);
+}
+
+extern "C" int qlgpu_adjoint_release(qlgpu_t* h) {
+    if (!h) return QLGPU_ERR_ARG;
+    QA_CK(cudaSetDevice(h->device));
+    QA_CK(cudaStreamSynchronize(h->stream));
+    if (h->adj_ws) cudaFree(h->adj_ws);
+    if (h->adj_tab) cudaFree(h->adj_tab);
+    if (h->adj_batch) qlgpu_batch_destroy(h->adj_batch);
+    h->adj_ws = h->adj_tab = nullptr;
+    h->adj_batch = nullptr;
+    h->adj_bytes = 0;
+    h->adj_tab_cap = 0;
+    h->adj_batch_ps.clear();
+    return QLGPU_OK;
 }
 
 extern "C" int qlgpu_adjoint_maxwell_batch(qlgpu_t* const* handles, int nseeds, double t0, const double* lin0,

@@ -165,6 +165,10 @@ class QLSolver:
                                                  _capi.dptr(gm)), self.h)
         return J.value, gl, gm
 
+    def release_adjoint(self):
+        """Gives back the device memory kept for the next adjoint call (qlgpu_adjoint_release)."""
+        _capi.check(self.L.qlgpu_adjoint_release(self.h), self.h)
+
     @staticmethod
     def adjoint_maxwell_batch(solvers, t0: float, lin0s, mf0s, kx0s, nsteps: int, checkpoint_every: int = 100):
         """qlgpu_adjoint_maxwell for several initial states at once, one solver (handle and

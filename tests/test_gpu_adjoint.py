@@ -301,3 +301,37 @@ def test_steps_after_the_adjoint_continue_the_forward_run(mode, integ, monkeypat
     finally:
         for s in ss:
             s.close()
+
+
+@pytest.mark.parametrize("seeds", [1, 3])
+def test_kept_workspace_is_given_back(seeds):
+    """What a gradient keeps for the next one: given back on request, and the next one is the same."""
+    require_gpu()
+    import torch
+    p = QLParams(nx=32, ny=32, NZ=64, dt=0.01)
+    st = initial_state(p, 5, sigma=0.05)
+    ss = [QLSolver(p) for _ in range(seeds)]
+
+    def call():
+        if seeds == 1:
+            return ss[0].adjoint_maxwell(0.0, *st, 20, 20)
+        return QLSolver.adjoint_maxwell_batch(ss, 0.0, *([x] * seeds for x in st), 20, 20)
+
+    def release():
+        for s in ss:
+            s.release_adjoint()
+        return torch.cuda.mem_get_info()[0]
+
+    try:
+        first = call()
+        free = release()  # with the kernels loaded
+        again = call()
+        kept = free - torch.cuda.mem_get_info()[0]
+        # sixty stage records of (nx - 1) ny / 2 modes x 4 fields x nz of 16 bytes, per seed
+        assert kept >= seeds * 60 * 16 * p.nxy * 4 * p.nz
+        assert release() == free
+        for a, b in zip(first, again):
+            assert np.array_equal(a, b)
+    finally:
+        for s in ss:
+            s.close()
