@@ -102,9 +102,13 @@ inline int stage_teams(int model, int warps) {
 }
 
 // CTA width and grid of a single case's stage kernel: one CTA per SM (sms: those left beside the
-// CTAs of the mean-field side, run_kernel).  When every team can
-// have its own SM a team gets as many warps as it has inverse transforms (one round of tasks);
-// otherwise a CTA holds the teams that the case has blocks for.
+// CTAs of the mean-field side, run_kernel).  When every team can have its own SM, MHD_FullQlin and
+// NZ >= 128 give a team as many warps as it has inverse transforms (one round of tasks).  MHD_BQlin
+// below that has eight for its nine: the second round is short and runs under the wait for the mean
+// field (a step of 32x32 x NZ=64 27.7 us, 28.0 with nine; 24x24 x NZ=128 33.5 and 32.3), and at 128
+// registers two CTAs of eight warps fit an SM, of nine one, so that two handles step side by side (eight
+// handles of 32x32 x NZ=64 on eight threads 124 us a step of all, 226 with nine).  Otherwise a CTA holds
+// the teams that the case has blocks for.
 struct StageGeom {
     int warps, grid;
 };
@@ -113,7 +117,7 @@ inline StageGeom stage_geometry(int model, int NZ, int nxy, int sms, int max_gri
     const bool bq = model == MODEL_BQLIN;
     const int per_sm = (blocks + sms - 1) / sms;
     StageGeom g;
-    g.warps = bq ? (per_sm <= 1 ? 9 : per_sm == 2 ? 14 : per_sm == 3 ? 15 : max_warps) : (per_sm <= 1 ? 10 : 16);
+    g.warps = bq ? (per_sm <= 1 ? (NZ <= 64 ? 8 : 9) : per_sm == 2 ? 14 : max_warps) : (per_sm <= 1 ? 10 : 16);
     if (g.warps > max_warps) g.warps = max_warps;
     const int teams = stage_teams(model, g.warps);
     g.grid = (blocks + teams - 1) / teams;

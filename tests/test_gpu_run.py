@@ -206,3 +206,29 @@ def test_wait_bound_does_not_run_before_the_launch_does():
         th.join()
         for a, c in zip(s.get_state() + (rec,), good):
             assert np.array_equal(a, c)
+
+
+@pytest.mark.parametrize("nx,ny,NZ", [(32, 32, 64), (64, 64, 16), (48, 48, 32)])
+def test_handles_on_threads_share_the_gpu(nx, ny, NZ):
+    """Launches of handles whose teams have an SM each leave room for a second one, and threads that step
+    their own handles at the same time get what one alone gets."""
+    require_gpu()
+    p = QLParams(nx=nx, ny=ny, NZ=NZ, dt=0.005)
+    st = initial_state(p, 3)
+    ss = [QLSolver(p) for _ in range(4)]
+    try:
+        assert ss[0].kernel_attrs()["ctas_per_sm"] >= 2
+        good = run_state(ss[0], st, 40, False)
+        for s in ss:
+            s.set_state(0.0, *st)
+        th = [threading.Thread(target=s.step, args=(40,)) for s in ss]
+        for t in th:
+            t.start()
+        for t in th:
+            t.join()
+        for s in ss:
+            for a, b in zip(s.get_state(), good):
+                assert np.array_equal(a, b)
+    finally:
+        for s in ss:
+            s.close()
