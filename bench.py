@@ -333,8 +333,20 @@ def run_reference(args):
 # ---------------------------------------------------------------------------
 # GPU arm
 # ---------------------------------------------------------------------------
+def call_ms(ext, call) -> float:
+    """Time between two events on the stream `ext` around a call that works on it and waits for it."""
+    import torch
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record(ext)
+    call()
+    e1.record(ext)
+    e1.synchronize()
+    return e0.elapsed_time(e1)
+
+
 def run_single(args, ext_stream_of, local):
-    """The single-case production workload through the plain path (L2 flushed before each step)."""
+    """The single-case production workload through the plain path: step by step with L2 flushed before
+    each, as one call of all steps, and stage by stage."""
     import torch
     from ql_dns_b200.initial import initial_state
     from ql_dns_b200.solver import QLSolver
@@ -342,16 +354,23 @@ def run_single(args, ext_stream_of, local):
     lin, mf, kx0 = initial_state(p, 1, sigma=1e-3)
     steps = max(1, min(args.steps, 500))
     with QLSolver(p, device=local) as solver:
-        solver.set_state(0.0, lin, mf, kx0)
         ext = ext_stream_of(solver.stream())
         flush = torch.empty(512 * 1024 * 1024 // 4, dtype=torch.float32, device="cuda")
-        for _ in range(args.warmup):
-            solver.step_timed()
-        stage_ms = np.zeros(3)
-        for _ in range(steps):
+
+        def flushed(call):
             with torch.cuda.stream(ext):
                 flush.fill_(1.0)
-            stage_ms += solver.step_timed()
+            return call()
+
+        solver.set_state(0.0, lin, mf, kx0)
+        for _ in range(args.warmup):
+            solver.step(1)
+        ms = sum(flushed(lambda: call_ms(ext, lambda: solver.step(1))) for _ in range(steps))
+        solver.step(steps)
+        run_ms = call_ms(ext, lambda: solver.step(steps))
+        for _ in range(args.warmup):
+            solver.step_timed()
+        stage_ms = sum(flushed(solver.step_timed) for _ in range(steps))
         del flush
     # the same case as a batch of one on the chunk-queue engine: all K steps in one persistent
     # launch, its ~45 MB working set staying in L2 between steps as in a run
@@ -372,33 +391,37 @@ def run_single(args, ext_stream_of, local):
                   "l2": "not flushed: the working set stays in L2 across the steps of the launch",
                   "roofline": {"bound": "hbm", "achieved": p_ach, "peak": peak, "unit": "GB/s", "frac": p_ach / peak,
                                "kernel": "ens_kernel<RK3CN_Elin>"}}
-    return {"workload": SINGLE_WORKLOAD, "value": p.nxy * steps / (stage_ms.sum() / 1e3), "unit": UNIT,
-            "persistent": persistent,
-            "steps": steps, "ms_per_step": float(stage_ms.sum() / steps),
+    in_run = {"path": "QLSolver.step(K): K steps in one launch", "value": p.nxy * steps / (run_ms / 1e3), "unit": UNIT,
+              "ms_per_step": run_ms / steps,
+              "l2": "not flushed: the working set stays in L2 across the steps of the launch"}
+    stages = {"path": "QLSolver.step_timed(): the three stages in launches of their own (a profiling aid)",
+              "ms_per_step": float(stage_ms.sum() / steps), "l2": "flushed (512 MiB write) before every timed step",
+              "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                           "frac": achieved / peak, "kernel": "stage_kernel<128,MHD_BQlin,RK3CN_Elin>",
+                           "traffic": read_traffic("stage_kernel_mri_64x64_nz128.md"),
+                           "algorithmic_bytes_per_launch": sum(sb) / 3,
+                           "avg_launch_ms": float(stage_ms.sum() / (3 * steps))}}
+    s_ach = sum(sb) * steps / (ms / 1e3) / 1e9
+    return {"workload": SINGLE_WORKLOAD, "path": "QLSolver.step(1), events around the call", "value":
+            p.nxy * steps / (ms / 1e3), "unit": UNIT, "steps": steps, "ms_per_step": ms / steps,
             "l2": "flushed (512 MiB write) before every timed step",
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "kernel": "stage_kernel<128,MHD_BQlin,RK3CN_Elin>",
-                         "traffic": read_traffic("stage_kernel_mri_64x64_nz128.md"),
-                         "algorithmic_bytes_per_launch": sum(sb) / 3,
-                         "avg_launch_ms": float(stage_ms.sum() / (3 * steps))}}
+            "roofline": {"bound": "hbm", "achieved": s_ach, "peak": peak, "unit": "GB/s", "frac": s_ach / peak,
+                         "kernel": "run_kernel<128,MHD_BQlin,RK3CN_Elin>"},
+            "in_run": in_run, "stages": stages, "persistent": persistent}
 
 
-def run_plain_per_case(cases, sts, local, steps_per_case: int = 10):
-    """The ensemble case after case through the plain single-case path (device time)."""
+def run_plain_per_case(cases, sts, local, ext_stream_of, steps_per_case: int = 50):
+    """The ensemble case after case through the plain single-case path: one call of QLSolver.step each."""
     from ql_dns_b200.solver import QLSolver
     tot = 0.0
     for p, (lin, mf, kx0) in zip(cases, sts):
         with QLSolver(p, device=local) as s:
             s.set_state(0.0, lin, mf, kx0)
-            for _ in range(3):
-                s.step_timed()
-            t = 0.0
-            for _ in range(steps_per_case):
-                t += float(s.step_timed().sum())
-            tot += t / steps_per_case
+            s.step(3)
+            tot += call_ms(ext_stream_of(s.stream()), lambda: s.step(steps_per_case)) / steps_per_case
     modes = sum(p.nxy for p in cases)
     return {"value": modes / (tot / 1e3), "unit": UNIT, "ms_per_step": tot,
-            "sample": f"{steps_per_case} steps of each case, one case after another, 3 stage launches per step"}
+            "sample": f"{steps_per_case} steps of each case in one QLSolver.step call, one case after another"}
 
 
 DNS_WORKLOAD = ("full 3-D DNS MRI, MHD shearing box 64x128x64 grid (2/3 dealiased in x, y, z; 1849 (kx,ky) columns x "
@@ -640,7 +663,7 @@ def run_gpu(args):
     batch.close()
 
     parity = ensemble_parity(cases, sts, recs_all, outs, timed_out, args) if rank == 0 else None
-    plain = run_plain_per_case(cases, sts, local) if rank == 0 else None
+    plain = run_plain_per_case(cases, sts, local, torch.cuda.ExternalStream) if rank == 0 else None
     single = run_single(args, torch.cuda.ExternalStream, local) if rank == 0 else None
     dns = run_dns(args, local) if rank == 0 else None
 
