@@ -158,8 +158,8 @@ int qlgpu_debug_drop_arrival(qlgpu_t* h, int launch);
 int qlgpu_trace(qlgpu_t* h, unsigned long long* out96);
 
 /* Launch geometry of the stage kernel: info8 = {grid, block, dynamic shared
- * bytes, CTAs per SM, TMEM columns per CTA, threads per transform, modes, warps
- * per CTA}. */
+ * bytes, CTAs per SM, 0 (tensor memory columns: the stage kernel has none),
+ * threads per transform, modes, warps per CTA}. */
 int qlgpu_launch_info(const qlgpu_t* h, int* info8);
 
 /* Compiled attributes of the stage kernel: attrs8 = {registers per thread,

@@ -91,8 +91,11 @@ struct Item {
 };
 
 struct CostModel {
-    // defaults as fitted on a B200 (12 MHD_FullQlin or MHD_BQlin cases of the ensemble law: a pass
-    // is 256 points per team at every NZ, so its cost hardly depends on the class)
+    // Defaults that plan well, one table for both models: a pass is 256 points per team at every NZ, so
+    // its cost hardly depends on the class.  They are not the measured costs (with every SM busy 12 to
+    // 14.4 us of MHD_BQlin, 8.9 to 11.9 of MHD_FullQlin): a table of those per model packed 12 cases of
+    // MHD_FullQlin into a step 7 % faster and 8, 16 or 20 into one 9 to 10 % slower, by how the items happen to
+    // fall.  qlgpu_batch_tune measures the batch at hand.
     double alpha = 20.0;                               // us per stage, per launch
     double beta = 8.0;                                 // us per work item per stage
     double r[NCLASS] = {9.5, 9.5, 9.8, 12.5, 16.0};    // us per pipeline pass, per NZ class
@@ -908,7 +911,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         o += 3 * gslot(nmfe * sizeof(cplx));                       // mf, Fmf1, Fmf2
         o += 3 * gslot(h.nxy * sizeof(double));                    // kx0, ky, kx_init
         o += 2 * gslot(h.nxy * sizeof(int));                       // kxi, kyi
-        o += gslot(2 * h.NZ * sizeof(cplx));                       // twiddles
+        o += gslot(h.NZ * sizeof(cplx));                           // twiddles
         o += gslot((size_t)(h.p.ny / 2) * h.nz * sizeof(double));  // 1/lap2
         o += gslot((size_t)h.max_cta * h.PL * sizeof(double));     // partials
         o += gslot((size_t)((h.max_cta + RED_GROUP - 1) / RED_GROUP) * h.PL * sizeof(double));
@@ -1050,7 +1053,7 @@ int qlgpu_batch_create(const qlgpu_params* cases, int ncases, int device, qlgpu_
         if (width_limits(b, w, &ps, &sm)) b->wide_warps = w;
     }
     if (!b->wide_warps) {
-        b->err = "batch: no CTA width fits (shared memory / TMEM)";
+        b->err = "batch: no CTA width fits (shared memory)";
         return bail(QLGPU_ERR_UNSUPPORTED);
     }
     int rc = plan_and_apply(b, whole_teams(b, b->wide_warps), nullptr);

@@ -42,9 +42,9 @@ struct qlgpu_handle {
     double* d_linop = nullptr;
     double* d_ilap2 = nullptr;
     int per_sm = 0;
-    unsigned long long* d_trace = nullptr;
+    unsigned long long* d_trace = nullptr;  // QLGPU_TRACE=1: %globaltimer stamps of each stage
     double* d_mfr = nullptr;  // [8][NZ] mean-field profile cache
-    double* d_ekz = nullptr;  // [3 stages][2][nz]  // QLGPU_TRACE=1: %globaltimer stamps of each stage
+    double* d_ekz = nullptr;  // [3 stages][2][nz]
     int grid = 0, warps = 4, block = 128;
     size_t smem = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
