@@ -335,3 +335,26 @@ def test_kept_workspace_is_given_back(seeds):
     finally:
         for s in ss:
             s.close()
+
+
+@pytest.mark.parametrize("integ", [0, 1])
+def test_adjoint_matches_tangent_linear_at_nz256(integ):
+    """The widest transforms (32 lanes): J, and the gradients along a random field and a real mean-field
+    profile, to the bars of the narrower ones."""
+    require_gpu()
+    p = mri_16x16_nz32(nx=8, ny=8, NZ=256, integrator=integ)
+    lin, mf, kx0 = initial_state(p, 7, sigma=0.2)
+    n = 12
+    with QLSolver(p) as s:
+        J, g, gm = s.adjoint_maxwell(0.0, lin, mf, kx0, n, checkpoint_every=5)
+    d = directions(lin.shape, 1, 256, np.linalg.norm(lin))[0]
+    Jo, dJ = O.tlm_maxwell(p, 0.0, lin, mf, kx0, d, None, n)
+    assert abs(J - Jo) <= 1e-10 * abs(Jo)
+    assert abs(float(np.real(np.vdot(g, d))) - dJ) <= 1e-8 * abs(dJ)
+    dm = directions(mf.shape, 1, 99, np.linalg.norm(mf))[0]
+    nzs = mf.shape[1]
+    dm[:, 0] = dm[:, 0].real
+    for s_ in range(1, (nzs - 1) // 2 + 1):
+        dm[:, nzs - s_] = np.conj(dm[:, s_])
+    _, dJm = O.tlm_maxwell(p, 0.0, lin, mf, kx0, np.zeros_like(lin), dm, n)
+    assert abs(float(np.real(np.vdot(gm, dm))) - dJm) <= 1e-8 * abs(dJm)
