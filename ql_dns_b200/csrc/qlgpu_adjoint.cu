@@ -239,7 +239,6 @@ int adj_begin(AdjJob& j, qlgpu_t* h, double t0, const double* lin0, const double
     H.kxi = h->d_kxi;
     H.kyi = h->d_kyi;
     H.ilap2 = h->d_ilap2;
-    H.ekz = h->d_ekz;
     H.tw8 = h->d_tw;
     H.status = h->d_dbg;
     H.nlin = (long long)j.nlin;

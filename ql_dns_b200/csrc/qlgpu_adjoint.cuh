@@ -66,7 +66,6 @@ struct AdjShared {
     const int* kxi;
     const int* kyi;
     const double* ilap2;   // [Ny/2][nz]
-    const double* ekz;     // [3][2][nz] integrating factors exp(linC c kz2) of the stages
     const cplx* tw8;       // transform twiddles [8][NZ/8]
     int* status;           // the first handle's status word (debug-build index checks)
     long long nlin, nmfe;
@@ -103,8 +102,8 @@ struct AG {
     static constexpr size_t o_tw = 0;                                    // [8][T] cplx
     static constexpr size_t o_prof = o_tw + 16 * (size_t)NZ_;           // [5][NZ]
     static constexpr size_t o_kz = o_prof + 8 * 5 * (size_t)NZ_;        // kz per spectral slot
-    static constexpr size_t o_ekz = o_kz + 8 * (size_t)NZ_;             // [2][NZE]
-    static constexpr size_t o_acc = o_ekz + 16 * (size_t)NZE;           // [3][8][32] profile sums
+    static constexpr size_t o_e = o_kz + 8 * (size_t)NZ_;               // [GPW][2][NZE] E or D of the block's modes
+    static constexpr size_t o_acc = o_e + 16 * (size_t)GPW * NZE;       // [3][8][32] profile sums
     static constexpr size_t o_R = o_acc + 8 * 3 * 256;                  // [NR][XW] cplx, a result at [8][32]
     static constexpr size_t o_stg = o_R + 16 * XW * (size_t)NR;        // [GPW][4][nz] cplx: U
     static constexpr size_t o_lf = o_stg + 16 * (size_t)GPW * 4 * nz;   // [GPW][4][nz] cplx: lamF
@@ -119,18 +118,18 @@ enum { A_RU = 0, A_RZ, A_RB, A_RE, A_RUZ, A_RBZ, A_RIK, A_RUY, A_RBY, A_WB, A_WZ
 struct AdjLane {
     int m, kyi, kxi;
     bool valid;
-    double a, b, kxe, kxo, mult, em_u, em_b;
+    double a, b, kxo, mult;
     int old_init;
 };
 
-// E (RK3CN_Elin: em exp(linC c kz2)) or D = 1/(1 - linC L) (RK3CN.cpp:105) of field f.
-template <class W>
-__device__ __forceinline__ double adj_e(const DevParams& P, const StageConst& S, const AdjLane& M, const double* ekz,
-                                        int f, int s, double kz2, int integ) {
-    if (integ == INTEG_CN)
-        return __drcp_rn(__dsub_rn(
-            1.0, __dmul_rn(S.linC, linop_f<MODEL_BQLIN>(P, lap_end<MODEL_BQLIN>(P, M.kxe, M.b, kz2), f))));
-    return f < 2 ? M.em_u * ekz[s] : M.em_b * ekz[W::NZE + s];
+// E = exp(linC L) (RK3CN_Elin.cpp:102-104) or D = 1/(1 - linC L) (RK3CN.cpp:105) of (u, zeta), side 0,
+// or (b, eta), side 1, at stored index s; kxe: kx at the stage end.  One exp: a
+// product of the mode's and kz's factors, as the forward stage takes it, has three roundings, the same at
+// every stage (gradient of 32x32 x NZ=64 over 100 steps 3.4e-15 from the 64-bit restatement, 1.9e-15 so).
+__device__ __forceinline__ double adj_e(const DevParams& P, const StageConst& S, double kxe, double ky, double kz2,
+                                        int side, int integ) {
+    const double L = linop_f<MODEL_BQLIN>(P, lap_end<MODEL_BQLIN>(P, kxe, ky, kz2), 2 * side);
+    return integ == INTEG_CN ? __drcp_rn(__dsub_rn(1.0, __dmul_rn(S.linC, L))) : exp(__dmul_rn(S.linC, L));
 }
 
 // The stage adjoint of the chunk's modes.  What bounds it: the transforms' chain of a block
@@ -150,7 +149,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == ADJ_MANY ? 2 : 1)
     cplx* tw = reinterpret_cast<cplx*>(smem_raw + W::o_tw);
     double* prof = reinterpret_cast<double*>(smem_raw + W::o_prof);
     double* kzc = reinterpret_cast<double*>(smem_raw + W::o_kz);
-    double* ekz = reinterpret_cast<double*>(smem_raw + W::o_ekz);
+    double* e_all = reinterpret_cast<double*>(smem_raw + W::o_e);
     double* acc = reinterpret_cast<double*>(smem_raw + W::o_acc);
     cplx* R = reinterpret_cast<cplx*>(smem_raw + W::o_R);
     cplx* stg_all = reinterpret_cast<cplx*>(smem_raw + W::o_stg);
@@ -182,10 +181,6 @@ __global__ void __launch_bounds__(THREADS, THREADS == ADJ_MANY ? 2 : 1)
         tw[i] = ldc_cg(H.tw8 + i);
         kzc[i] = kzval(i <= W::H ? i : i - NZ, P.kzL);
     }
-    for (int i = tid; i < nzd; i += nth) {
-        ekz[i] = __ldg(H.ekz + (size_t)(2 * X.s) * nzd + i);
-        ekz[W::NZE + i] = __ldg(H.ekz + (size_t)(2 * X.s + 1) * nzd + i);
-    }
     for (int i = tid; i < 3 * 256; i += nth) acc[i] = 0.0;
     const double tclock = B.t_pre[X.n];
     const double ts = __dadd_rn(tclock, S.t_off);
@@ -204,8 +199,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == ADJ_MANY ? 2 : 1)
         const double k0 = kx0[M.m];
         M.a = kx_at(k0, P.q, ts, M.b);
         M.mult = M.valid ? (M.b == 0.0 ? 1.0 : 2.0) : 0.0;
-        M.kxe = __dadd_rn(M.a, __dmul_rn(__dmul_rn(P.q, S.dt_lin), M.b));
-        M.kxo = M.em_u = M.em_b = 0.0;
+        M.kxo = 0.0;
         M.old_init = 0;
         if (H.integ == INTEG_CN) {
             // kx where the previous stage's operator was evaluated (RK3CN.cpp:119-122; the init form
@@ -214,23 +208,27 @@ __global__ void __launch_bounds__(THREADS, THREADS == ADJ_MANY ? 2 : 1)
             M.old_init = cn->old_init;
             if (M.old_init) M.kxo = kx_at(k0, P.q, tclock, M.b);
             else M.kxo = __dadd_rn(kx_at(k0, P.q, cn->t_old, M.b), __dmul_rn(__dmul_rn(P.q, cn->dtlin_old), M.b));
-        } else {
-            const double hxy = __dsub_rn(-__dmul_rn(M.kxe, M.kxe), __dmul_rn(M.b, M.b));
-            M.em_u = exp(S.linC * P.nu * hxy);
-            M.em_b = exp(S.linC * P.cb * hxy);
         }
         const double a = M.a, b = M.b, ab = __dmul_rn(a, b);
         const double* il2row = il2_all + min(g, nv - 1) * nzd;
+        const double* e = e_all + (size_t)min(g, nv - 1) * 2 * W::NZE;  // this mode's E or D
         cplx* lfm = lf_s + (size_t)min(g, nv - 1) * 4 * nzd;  // this mode's lamF
         const cplx* lo = lo_all + (size_t)M.m * 4 * nzd;
         const cplx* lf = lf_all ? lf_all + (size_t)M.m * 4 * nzd : nullptr;
         // lamF of field f at stored index s: n1 E lamU' + lamF_out
-        auto lam_F = [&](int f, int s, double kz2) -> cplx {
-            cplx r = cscale(ldc(lo + f * nzd + s), __dmul_rn(S.n1, adj_e<W>(P, S, M, ekz, f, s, kz2, H.integ)));
+        auto lam_F = [&](int f, int s) -> cplx {
+            cplx r = cscale(ldc(lo + f * nzd + s), __dmul_rn(S.n1, e[(f >> 1) * W::NZE + s]));
             if (lf) r = cadd(r, ldc(lf + f * nzd + s));
             return r;
         };
         if (base != first) stage_block(base);
+        // E of the block's modes, while the fields are on their way
+        for (int i = tid; i < 2 * nv * nzd; i += nth) {
+            const int q = i / nzd, s = i - q * nzd, m = base + (q >> 1);
+            const double ky = __ldg(H.ky + m);
+            const double kxe = __dadd_rn(kx_at(kx0[m], P.q, ts, ky), __dmul_rn(__dmul_rn(P.q, S.dt_lin), ky));
+            e_all[q * W::NZE + s] = adj_e(P, S, kxe, ky, kz2val(kzval(s <= W::H ? s : s - nzd, P.kzL)), q & 1, H.integ);
+        }
         cp_async_wait_all();
         __syncthreads();
         // ---- fourteen inverse transforms
@@ -256,7 +254,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == ADJ_MANY ? 2 : 1)
                         v = task == A_RIK ? imul(v, sc * c) : cscale(v, sc);
                     } else {
                         const int f = task == A_WB ? 2 : task == A_WZ ? 1 : task == A_WE ? 3 : 0;
-                        v = lam_F(f, s, kz2);
+                        v = lam_F(f, s);
                         if (task != A_WU2) {
                             if (M.valid) lfm[f * nzd + s] = v;  // kept for the spectral chain
                         } else {
@@ -364,7 +362,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == ADJ_MANY ? 2 : 1)
                 const double c = kzc[t + T * r], kz2 = kz2val(c);
                 const bool z0 = (M.kyi == 0 && s == 0);
                 const double il2 = il2row[s];
-                const cplx mu = cscale(lov[i], adj_e<W>(P, S, M, ekz, f, s, kz2, H.integ));
+                const cplx mu = cscale(lov[i], e[(f >> 1) * W::NZE + s]);
                 cplx v = mu;
                 if (H.integ == INTEG_CN) {
                     // the direct term (1 + linC Lold) D lamU' (RK3CN.cpp:107)

@@ -358,3 +358,37 @@ def test_adjoint_matches_tangent_linear_at_nz256(integ):
         dm[:, nzs - s_] = np.conj(dm[:, s_])
     _, dJm = O.tlm_maxwell(p, 0.0, lin, mf, kx0, np.zeros_like(lin), dm, n)
     assert abs(float(np.real(np.vdot(gm, dm))) - dJm) <= 1e-8 * abs(dJm)
+
+
+def test_gradient_takes_the_integrating_factor_in_one_rounding():
+    """Pure decay (no shear, no mean field): b_n = b_0 E^n, and the gradient is w (2 a b_y b_0 + i c eta_0) / lap2
+    sum_n E^2n / N in closed form.  The roundings of E repeat at every step, so errors grow with their
+    number: the forward state's after N steps is N d_f, of the factors' product (two exps and a product: 0.5
+    ulp rms), the gradient's N/2 (d_f + d_a).  With d_a of one exp (0.3 ulp, not the product's) that is
+    0.5 sqrt(1 + 0.36) = 0.58 of the state's; with the product again, d_a = d_f, it is the whole of it."""
+    require_gpu()
+    from ql_dns_b200.ktables import ktables
+    p = QLParams(nx=16, ny=16, NZ=32, q=0.0, nu=1e-4, eta=1e-4, dt=0.01, quasilinear=0, remap=0)
+    lin, mf, kx0 = initial_state(p, 3, sigma=0.1, B0=0.0)
+    N = 200
+    with QLSolver(p) as s:
+        _, g, _ = s.adjoint_maxwell(0.0, lin, mf, kx0, N, 50)
+        _, end, _, _ = s.get_state()
+    kt = ktables(p)
+    a, b, c = (np.asarray(kt[k], dtype=np.longdouble) for k in ("kx", "ky", "kz"))
+    a, b, c = a[:, None], b[:, None], c[None, :]
+    E = np.exp(-np.longdouble(p.eta) * np.longdouble(p.dt) * (a * a + b * b + c * c))
+    use = (b * b + c * c > 0) & (np.abs(lin[:, 2]) > 0) & (np.abs(lin[:, 3]) > 0)
+    b0, e0 = lin[:, 2].astype(np.clongdouble), lin[:, 3].astype(np.clongdouble)
+    n = np.arange(1, N + 1, dtype=np.longdouble)[:, None, None]
+    w = np.where(b == 0, 1, 2) * np.longdouble(p.L[2]) / np.longdouble(p.nx * p.ny * p.NZ) ** 2 / N
+    il2 = -1 / np.where(use, b * b + c * c, 1)
+    exact = w * il2 * (2 * a * b * b0 + 1j * c * e0) * (E[None] ** (2 * n)).sum(0)
+    state = b0 * E ** N
+
+    def rms(x, y, at):
+        return float(np.sqrt(np.mean(np.abs((x - y)[at] / y[at]) ** 2)))
+
+    r_g, r_f = rms(g[:, 2], exact, use & (np.abs(exact) > 0)), rms(end[:, 2], state, use)
+    assert r_f > 20 * 2.0 ** -53  # the repeated roundings, not the single ones
+    assert r_g <= 0.8 * r_f, (r_g, r_f)
