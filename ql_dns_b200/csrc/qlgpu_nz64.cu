@@ -1,4 +1,4 @@
-// Stage kernels for NZ = 64 (all models, integrators and private-store backings).
+// Stage kernels for NZ = 64 (all models and integrators).
 #include "qlgpu_inst.cuh"
 
 QLGPU_DEFINE_NZ(64)
