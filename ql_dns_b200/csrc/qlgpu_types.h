@@ -279,6 +279,6 @@ struct EnsLaunch {
 #define QLGPU_STATUS_NONFINITE 1   // solution::Check_Solution NaN/Inf (solution.cpp:194)
 #define QLGPU_STATUS_UNSTABLE 2    // |mean field| > 1e20 (solution.cpp:184)
 #define QLGPU_STATUS_DIAG_FULL 4   // diagnostic ring overflowed (records dropped)
-#define QLGPU_STATUS_TIMEOUT 8     // batch: a CTA gave up waiting for the other CTAs of its case
+#define QLGPU_STATUS_TIMEOUT 8     // a CTA gave up waiting for the other CTAs of its case
 #define QLGPU_STATUS_BOUNDS 16     // debug build: a device index check failed (the access was redirected)
 #define QLGPU_STATUS_CANARY 32     // debug build: a guard zone after a device buffer was overwritten
